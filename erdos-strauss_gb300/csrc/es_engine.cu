@@ -1232,14 +1232,14 @@ static u64 classes_below(const es_engine *e, u64 x) {
   return i;
 }
 
-// x / M and x mod M for any 64-bit x: a double estimate of the quotient (off by at most
-// one: x / M < 2^44, and the product's relative error is 2^-52) corrected exactly.
+// x / M and x mod M for any 64-bit x: a double estimate of the quotient, corrected exactly (its
+// relative error is below 2^-51: off by at most one while x / M < 2^51, by a few for smaller M).
 static void divmod_M(const es_engine *e, u64 x, u64 &q, u64 &r) {
   const u64 M = e->M;
   q = (u64)((double)x * e->inv_M);
-  const unsigned __int128 qm = (unsigned __int128)q * M;
-  if (qm > x) { --q; r = x - (u64)(qm - M); }
-  else { r = x - (u64)qm; if (r >= M) { ++q; r -= M; } }
+  unsigned __int128 qm = (unsigned __int128)q * M;
+  for (; qm > x; qm -= M) --q;
+  for (r = x - (u64)qm; r >= M; r -= M) ++q;
 }
 
 static void build_lane_index(es_engine *e) {
