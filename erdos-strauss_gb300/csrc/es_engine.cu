@@ -5,22 +5,23 @@
 //   K0[L][ldk]        u16  per (lane, filter): the residue K0 = K mod s at which filter f
 //                          kills lane l (p = rho_l + M*K), or K0_MISS; 2308 x 3752 x 2 B
 //                          = 17.3 MB for the M = 2042040 table, read coalesced row by row
-//   mtab[L][Wpad]     u64  per lane, one kill mask per distinct stride s: bit x set when some
-//                          filter of stride s kills K = x (mod s), for x < s + SEG_SMALL
-//                          (33.4 KB a lane, 77 MB for the M = 2042040 table)
-//   mdesc             per masked stride (densest first): s, its Qm column, its mask offset
+//   tdense            per group of 128 lanes, the rows of the dense strides: 16 bytes a row, the
+//                     lanes that some filter of stride s kills at K == x (mod s) (209 KB a group,
+//                     4 MB for the M = 2042040 table)
+//   tlane[L]          u32  per lane, the other strides' bits 0 .. s - 1 (26 KB a lane, 60 MB)
+//   mdesc             per stride with a table (densest first): s, its reduction constants, its place
 //   fdesc[nf]         u32  per filter: stride s = mod/gcd(M,mod) and its Qm column
 //   tdp/tde                trial-division table: 6541 odd primes < 2^16 with inverses
-// Per run: window and short-window descriptors, Qm[window][stride] = (lo / M) mod s, the
-// survivor list, prime/direct index lists, records, counters and the hard board.
+// Per run: window descriptors, row pieces and rows, candidate chunks, Qm[window][stride] =
+// (lo / M) mod s where windows are marked by segments, the survivor list, prime/direct index lists, records, counters and the hard board.
 //
 // Pipeline per run (one CUDA stream, replayed as a CUDA graph for batches):
-//   k_prep        Qm for every window and stride
-//   k_mark_short  a CTA per pair of lanes with their mask rows in shared memory; each warp
-//                 walks short windows (and 128-position pieces of long ones): rounds of 32
-//                 strides, one funnel-shift extraction of 32 positions per stride and chunk,
-//                 a warp OR, stopping when every position is dead; survivors appended
-//   k_mark        the alternative for long windows: a byte map per segment in shared memory,
+//   k_rows        the windows cut into rows (one K, all lanes) and pieces of 32 rows, with each
+//                 piece's place in every dense stride's table
+//   k_mark_short  a lane group's dense slice in an SM's shared memory; a thread per row ORs one
+//                 16-byte read per dense stride: the 0.2% of positions left become candidates
+//   k_sift        the candidates against the other strides; survivors appended
+//   k_prep, k_mark  the alternative for long windows: a byte map per segment in shared memory,
 //                 each filter clears its progression, warp-aggregated compaction
 //   k_mr          a thread per survivor: the base-2 strong-probable-prime round
 //   k_mr2         a warp per number that passed base 2: the 12-base test, one base per lane
@@ -296,428 +297,529 @@ __global__ void __launch_bounds__(BLOCK) k_mark(const MarkParams P, int persiste
   }
 }
 
-// ---------------------------------------------------------------- short windows
-// A CTA holds the kill-mask tables of SHORT_LANES consecutive lanes in shared memory; each
-// warp takes one short window at a time and marks the segments of those lanes in it. The
-// per-window work that does not depend on the lane -- the stride descriptor and the
-// segment-start residue (lo / M) mod s -- is done once for all SHORT_LANES lanes.
-#ifndef ES_SHORT_LANES
-#define ES_SHORT_LANES 2
-#endif
-constexpr int SHORT_LANES = ES_SHORT_LANES;
-// Windows with at most SPARSE_N positions in either lane of a k_mark_short CTA take the sparse
-// first round (short_sparse_round). Measured on the 4096-window batch: 0.87 ms for the kernel
-// with 32, 0.98 without the sparse round, 0.88 with 16, 0.93 with 48 or 64 (a second chunk
-// per lane: the task path marks those windows for less).
-#ifndef ES_SPARSE_N
-#define ES_SPARSE_N 32
-#endif
-constexpr u32 SPARSE_N = ES_SPARSE_N;
-static_assert(SPARSE_N <= 32, "a sparse window's positions fit one 32-position chunk per lane");
-constexpr u32 HAND_WORDS = SHORT_LANES;          // alive words per window handed on, one per lane
-constexpr u32 SMD_MAX = 512;       // stride descriptors staged in shared memory
+// ---------------------------------------------------------------- marking by rows
+// A row is one K of one window: the positions p = rho_l + M K of all lanes l (contiguous in
+// integer order, so a window is a run of rows whose first and last are cut at a lane). For a
+// stride s the filters kill the lanes of row K by a bit vector that depends on K mod s alone.
+// Dense strides (the first n1, densest first) keep these vectors by group of GROUP_LANES lanes,
+// each stride's rows 0 .. s - 1 followed by PIECE_ROWS - 1 repeats, so that the rows of a piece (at
+// most PIECE_ROWS consecutive K of one window) that starts at K0 are consecutive from K0 mod s; one
+// group's slice fits an SM's shared memory. The other strides keep, per lane, the bits 0 .. s - 1.
 
+// x mod s for x < 2^32, m = floor((2^32 - 1) / s) (the quotient estimate is low by at most one)
+__device__ __forceinline__ u32 mod_s(u32 x, u32 s, u32 m) {
+  const u32 v = x - __umulhi(x, m) * s;
+  return min(v, v - s);
+}
+// K mod s for d = {s, m, 2^32 mod s, ..}; wide: K may reach 2^48
+__device__ __forceinline__ u32 mod_stride(u64 K, const uint4 &d, bool wide) {
+  u32 hi = (u32)(K >> 32);
+  if (wide) hi = mod_s(hi, d.x, d.y);
+  return mod_s(hi * d.z + mod_s((u32)K, d.x, d.y), d.x, d.y);        // below 2^16 (2^16 - 1) + 2^16
+}
 
-__device__ __forceinline__ u32 warp_or32(u32 v) { return __reduce_or_sync(0xFFFFFFFFu, v); }
-
-// Mask strides [m0, m1) over the segments of SHORT_LANES lanes, in rounds of 32 strides (one
-// per lane of the warp). alive[q][c] holds the positions 32c + j of lane q's segment not yet
-// killed; it is the same in every lane of the warp. A segment starts at K == Qrow[d] + b[q]
-// (mod s_d); mask bits come out 32 at a time: word r/32 + c and the next, funnel-shifted right
-// by r mod 32. After each round the warp ORs its kill words into alive, and it stops as soon
-// as nothing is left alive: the strides come densest first, so most segments are dead after
-// one or two rounds. Returns nonzero if a position is still alive.
-
-#ifndef ES_FIRST_SH
-#define ES_FIRST_SH 1
-#endif
-template <int NC>
-__device__ __forceinline__ u32 short_mask_rounds(u32 (&alive)[SHORT_LANES][NC], const u32 (&b)[SHORT_LANES],
-                                                 const u32 *tab, u32 tab_words, const MaskDesc *smd, u32 m0,
-                                                 u32 m1, const u16 *__restrict__ Qrow, u32 q0_first, u32 lane,
-                                                 const MaskDesc &md_first) {
-  u32 kill[SHORT_LANES][NC];
-  // Round one (strides m0 .. m0 + 31, q0_first loaded by the caller ahead of time): every
-  // chunk, one mask word load per chunk, no per-chunk tests.
-  u32 k = m0 + lane;
-  u32 q0 = k + 32 < m1 ? (u32)__ldg(Qrow + smd[k + 32].d) : 0u;    // the next round's residue
-  if (k < m1) {
-    const MaskDesc md = md_first;                    // this lane's stride of the first round
-    // SH: the round's row layout (the same for all its strides), a constant in each copy
-    auto first = [&](auto shc) {
-      constexpr u32 SH = decltype(shc)::value;
-      u32 r = 0;
-      #pragma unroll
-      for (int q = 0; q < SHORT_LANES; ++q) {
-        if (q == 0 || b[q] != b[0]) {                // lanes whose segments start together share r
-          r = q0_first + b[q];
-          r = r >= md.s ? r - md.s : r;
-        }
-        // the mask repeats for SEG_SMALL bits past s, so chunk c is words r/32 + c, + c + 1
-        const u32 *wp = tab + q * tab_words + md.off + ((r >> 5) << (SH == 1 ? md.sh : SH));
-        const u32 sh = r & 31;
-        u32 w0 = wp[0];
-        #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          const u32 w1 = wp[(c + 1) << (SH == 1 ? md.sh : SH)];
-          kill[q][c] = __funnelshift_r(w0, w1, sh);
-          w0 = w1;
-        }
-      }
-    };
-    if (!ES_FIRST_SH) first(std::integral_constant<u32, 1>{});   // 1: the layout read at run time
-    else if (md.sh == 5) first(std::integral_constant<u32, 5>{});
-    else first(std::integral_constant<u32, 0>{});
-  } else {
-    #pragma unroll
-    for (int q = 0; q < SHORT_LANES; ++q)
-      #pragma unroll
-      for (int c = 0; c < NC; ++c) kill[q][c] = 0;
+// The batch's row windows cut into pieces: a warp per piece finds its window (32-way search over
+// the windows' first pieces), writes the piece, its rows, and per dense stride the slice row of the
+// piece's first K. Bound by the latency of its few dependent loads.
+__global__ void k_rows(const RowParams P) {
+  const u32 lane = threadIdx.x & 31;
+  const u32 nw = P.hdr->nshort, npieces = P.hdr->npieces;
+  const u32 warps = gridDim.x * blockDim.x / 32;
+  for (u32 pc = (blockIdx.x * blockDim.x + threadIdx.x) / 32; pc < npieces; pc += warps) {
+    u32 w0 = 0, cnt = nw;                            // the last window whose first piece is <= pc
+    while (cnt > 1) {
+      const u32 step = (cnt + 31) / 32, off = lane * step;
+      const bool le = off < cnt && P.roww[w0 + off].piece0 <= pc;
+      const u32 k = __popc(__ballot_sync(FULL, le)) - 1;          // lane 0 always holds
+      w0 += k * step;
+      cnt = min(step, cnt - k * step);
+    }
+    const RowWin W = P.roww[w0];
+    const u32 t = pc - W.piece0;
+    Piece x;
+    x.K0 = W.K0 + (u64)t * PIECE_ROWS;
+    x.row0 = W.row0 + t * PIECE_ROWS;
+    x.win = W.wi;
+    x.n = min(PIECE_ROWS, W.nrows - t * PIECE_ROWS);
+    const bool last = t * PIECE_ROWS + x.n == W.nrows;
+    x.la = t == 0 ? W.la : 0;
+    x.lb = last ? W.lb : P.L;
+    x.pad = 0;
+    if (lane == 0) P.piece[pc] = x;
+    if (lane < x.n) {
+      const bool cut = (lane == 0 && x.la) || (lane == x.n - 1 && x.lb < P.L);
+      P.rowinfo[x.row0 + lane] = pc * PIECE_ROWS + lane + (cut ? ROW_CUT : 0u);
+    }
+    for (u32 m = lane; m < P.n1p; m += 32) {
+      const uint4 d = __ldg(P.mdesc + m);
+      P.pidx[(size_t)pc * P.n1p + m] = (u16)(d.w + mod_stride(x.K0, d, P.wide));
+    }
   }
-  u32 any = 0;
+}
+
+// Bulk copies into shared memory, and the bounded wait for them.
+__device__ __forceinline__ u32 smem_addr(const void *p) { return (u32)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(u32 bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ void bar_expect(u32 bar, u32 bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_copy(u32 dst, const void *src, u32 bytes, u32 bar) {   // bytes: a multiple of 16
+  for (u32 o = 0; o < bytes; o += BULK_COPY)
+    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst + o),
+                 "l"((const char *)src + o), "r"(min(BULK_COPY, bytes - o)), "r"(bar)
+                 : "memory");
+}
+// Every thread of the block waits for the barrier's phase; false (never: the copies take
+// microseconds) when one gave up, with the status set and the copies waited for once more.
+__device__ __forceinline__ bool bulk_wait(u32 bar, u32 parity, u32 *status) {
+  auto wait = [&]() {
+    u32 ok = 0;
+    for (u32 i = 0; !ok && i < (1u << 20); ++i)
+      asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                   : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok;
+  };
+  if (__syncthreads_and(wait())) return true;
+  if (threadIdx.x == 0) atomicOr(status, ST_QUEUE_TIMEOUT);
+  wait();
+  return false;
+}
+
+// The lanes of word w of group g that have a position in the row `ri`.
+__device__ __forceinline__ void row_lanes(const RowParams &P, u32 ri, u32 g, u32 (&al)[GROUP_WORDS]) {
+  u32 a = 0, b = ri == ROW_NONE ? 0 : P.L;
+  if (ri != ROW_NONE && (ri & ROW_CUT)) {
+    const u32 j = ri % PIECE_ROWS;
+    const Piece x = P.piece[(ri & ~ROW_CUT) / PIECE_ROWS];
+    if (j == 0) a = x.la;
+    if (j == x.n - 1) b = x.lb;
+  }
   #pragma unroll
-  for (int q = 0; q < SHORT_LANES; ++q)
-    #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      alive[q][c] &= ~warp_or32(kill[q][c]);
-      any |= alive[q][c];
+  for (u32 w = 0; w < GROUP_WORDS; ++w) {              // bits [a, b) of lanes l0 .. l0 + 31
+    const u32 l0 = g * GROUP_LANES + w * 32;
+    const u32 lo = a > l0 ? min(a - l0, 32u) : 0u, hi = b > l0 ? min(b - l0, 32u) : 0u;
+    al[w] = lo < hi ? (~0u << lo) & (~0u >> (32 - hi)) : 0u;
+  }
+}
+
+// A warp's n <= 32 candidates of group g as a chunk. Chunks past the capacity are counted only
+// (the host runs again with room for them).
+__device__ __forceinline__ void put_chunk(const RowParams &P, u32 g, const uint2 *buf, u32 n, u32 lane) {
+  u64 id = 0;
+  if (lane == 0) id = atomicAdd(P.chunk_count, 1ull);
+  id = __shfl_sync(FULL, id, 0);
+  if (id >= P.chunk_cap) return;
+  if (lane == 0) P.chunk[id] = g << 8 | n;
+  if (lane < n) P.cand[id * 32 + lane] = buf[lane];
+}
+
+// Marks the tiles (32 consecutive rows of the batch, one per thread of a warp) of every lane
+// group by the dense strides. The (group, tile) items are dealt to the CTAs (one per SM) in equal
+// runs, so a CTA holds one group's slice or two in turn; its warps take tiles from a counter, the
+// next tile's rows loaded while one is marked. Per tile a thread ORs its row's bit vectors over the
+// strides: one 16-byte shared-memory read per stride decides GROUP_LANES positions, and consecutive
+// rows read consecutive words. The positions left (0.2% with the gpu table) go to k_sift in chunks
+// of up to 32 of one group.
+// Bound by shared-memory bandwidth: on a 2^40-integer window (1.24e9 positions) 0.257 ms at 94% of
+// the LSU data pipe's peak; the 4096-window batch takes 0.052 ms. Per-lane masks of one stride per
+// lane of a warp, which this replaced, took 1.9 ms and 0.83 ms with the survivors' other strides
+// included. Rows of 8 bytes hold 64 strides in a slice but were bound by address arithmetic (0.47
+// ms with next to no candidates left); with 16-byte rows and k_sift, 40, 48 and 56 dense strides
+// (the last cut to 50 by the slice) took 0.71, 0.60 and 0.61 ms together on that window.
+__global__ void __launch_bounds__(ROW_THREADS, 1) k_mark_short(const RowParams P) {
+  extern __shared__ __align__(128) unsigned char rowmem[];
+  __shared__ __align__(8) u64 s_bar;
+  __shared__ u32 s_next;
+  const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const u32 nrows = P.hdr->nrows;
+  const u32 ntiles = (nrows + 31) / 32;
+  const u64 items = (u64)ntiles * P.ngroups;
+  u64 item = items * blockIdx.x / gridDim.x;
+  const u64 end = items * (blockIdx.x + 1) / gridDim.x;
+  if (item >= end) return;
+  uint2 *buf = reinterpret_cast<uint2 *>(rowmem + P.slice_bytes) + warp * 64;   // fewer than 32, then at most 32 more
+  const u32 bar = smem_addr(&s_bar), tab = smem_addr(rowmem);
+  if (threadIdx.x == 0) bar_init(bar);
+  u32 parity = 0;
+  auto row_at = [&](u32 t, u32 t1) {
+    const u32 row = t * 32 + lane;
+    return t < t1 && row < nrows ? __ldg(P.rowinfo + row) : ROW_NONE;
+  };
+  while (item < end) {
+    const u32 g = (u32)(item / ntiles), t0 = (u32)(item % ntiles);
+    const u32 t1 = (u32)min((u64)ntiles, t0 + (end - item));
+    item += t1 - t0;
+    u32 al[GROUP_WORDS];
+    // A run no longer than the warps may hold no position of the group at all (windows shorter
+    // than M): then its slice is not needed. The barrier also ends the previous run's reads.
+    bool some = true;
+    u32 t = t0 + warp, ri = row_at(t, t1);
+    if (t1 - t0 <= ROW_THREADS / 32) {
+      row_lanes(P, ri, g, al);
+      some = al[0] | al[1] | al[2] | al[3];
     }
-  // Later rounds, rarely more than one or two: only the chunks still alive.
-  for (u32 kb = m0 + 32; kb < m1 && any; kb += 32) {
-    k = kb + lane;
-    const u32 q0_next = k + 32 < m1 ? (u32)__ldg(Qrow + smd[k + 32].d) : 0u;
-    #pragma unroll
-    for (int q = 0; q < SHORT_LANES; ++q)
-      #pragma unroll
-      for (int c = 0; c < NC; ++c) kill[q][c] = 0;
-    if (k < m1) {
-      const MaskDesc md = smd[k];
-      #pragma unroll
-      for (int q = 0; q < SHORT_LANES; ++q) {
-        u32 r = q0 + b[q];
-        r = r >= md.s ? r - md.s : r;
-        const u32 *wp = tab + q * tab_words + md.off + ((r >> 5) << md.sh);
-        const u32 sh = r & 31;
-        #pragma unroll
-        for (int c = 0; c < NC; ++c)
-          if (alive[q][c]) kill[q][c] = __funnelshift_r(wp[c << md.sh], wp[(c + 1) << md.sh], sh);
+    if (!__syncthreads_or(some)) continue;
+    if (threadIdx.x == 0) {
+      s_next = t0 + ROW_THREADS / 32;
+      bar_expect(bar, P.slice_bytes);
+      bulk_copy(tab, P.tdense + (size_t)g * P.slice_bytes, P.slice_bytes, bar);
+    }
+    if (!bulk_wait(bar, parity, P.status)) return;
+    parity ^= 1;
+    u32 nbuf = 0;                                      // candidates in the warp's buffer
+    while (t < t1) {
+      const u32 now = ri;
+      if (lane == 0) t = atomicAdd(&s_next, 1u);
+      t = __shfl_sync(FULL, t, 0);
+      ri = row_at(t, t1);
+      row_lanes(P, now, g, al);
+      if (!__any_sync(FULL, al[0] | al[1] | al[2] | al[3])) continue;
+      const u32 pj = now == ROW_NONE ? 0 : now & ~ROW_CUT, j = pj % PIECE_ROWS;
+      const uint4 *ip = reinterpret_cast<const uint4 *>(P.pidx + (size_t)(pj / PIECE_ROWS) * P.n1p);
+      const u32 base = tab + j * 16;
+      u32 a0 = 0, a1 = 0, a2 = 0, a3 = 0;
+      auto take = [&](u32 row) {
+        u32 x, y, z, w;
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(base + row * 16));
+        a0 |= x; a1 |= y; a2 |= z; a3 |= w;
+      };
+      uint4 nx = P.n1p ? __ldg(ip) : make_uint4(0, 0, 0, 0);
+      for (u32 m = 0; m < P.n1p; m += 8) {
+        const uint4 c = nx;
+        if (m + 8 < P.n1p) nx = __ldg(ip + m / 8 + 1);
+        take(c.x & 0xFFFFu); take(c.x >> 16);
+        take(c.y & 0xFFFFu); take(c.y >> 16);
+        take(c.z & 0xFFFFu); take(c.z >> 16);
+        take(c.w & 0xFFFFu); take(c.w >> 16);
       }
-    }
-    q0 = q0_next;
-    any = 0;
-    #pragma unroll
-    for (int q = 0; q < SHORT_LANES; ++q)
+      al[0] &= ~a0; al[1] &= ~a1; al[2] &= ~a2; al[3] &= ~a3;
       #pragma unroll
-      for (int c = 0; c < NC; ++c)
-        if (alive[q][c]) {
-          alive[q][c] &= ~warp_or32(kill[q][c]);
-          any |= alive[q][c];
+      for (u32 w = 0; w < GROUP_WORDS; ++w)
+        for (unsigned who; (who = __ballot_sync(FULL, al[w] != 0));) {
+          if (al[w]) {
+            buf[nbuf + __popc(who & ((1u << lane) - 1))] = make_uint2(pj / PIECE_ROWS, j * GROUP_LANES + w * 32 + __ffs(al[w]) - 1);
+            al[w] &= al[w] - 1;
+          }
+          nbuf += __popc(who);
+          __syncwarp();
+          if (nbuf < 32) continue;
+          nbuf -= 32;
+          put_chunk(P, g, buf + nbuf, 32, lane);
+          __syncwarp();
         }
-  }
-  return any;
-}
-
-// kill[q][c] gets bit j set when position 32c + j of lane q's segment is hit by one of the
-// filters lfil[l0, l1) (the strides without a mask), checked one by one from the first-hit
-// table. Lanes of the warp split the filters; the caller reduces.
-template <int NC>
-__device__ __forceinline__ void short_list_kill(u32 (&kill)[SHORT_LANES][NC], const u32 (&n)[SHORT_LANES],
-                                                const u32 (&b)[SHORT_LANES], const u32 *__restrict__ lfil, u32 l0,
-                                                u32 l1, const u16 *const (&K0row)[SHORT_LANES],
-                                                const u32 *__restrict__ fdesc, const u16 *__restrict__ Qrow,
-                                                u32 lane) {
-  for (u32 k = l0 + lane; k < l1; k += 32) {
-    const u32 f = lfil[k];
-    const u32 fd = __ldg(fdesc + f);
-    const u32 s = fd & 0xFFFFu;
-    const u32 q0 = (u32)__ldg(Qrow + (fd >> 16));
-    #pragma unroll
-    for (int q = 0; q < SHORT_LANES; ++q) {
-      const u32 k0 = K0row[q][f];
-      if (k0 == K0_MISS) continue;
-      u32 r = q0 + b[q];
-      r = r >= s ? r - s : r;
-      int off = (int)k0 - (int)r;
-      if (off < 0) off += (int)s;
-      for (u32 j = (u32)off; j < n[q]; j += s) {
-        #pragma unroll
-        for (int c = 0; c < NC; ++c)
-          if ((j >> 5) == (u32)c) kill[q][c] |= 1u << (j & 31);
-      }
     }
+    if (nbuf) put_chunk(P, g, buf, nbuf, lane);
+    __syncwarp();
   }
 }
 
-// One phase (covers, or the stage-B' primes) over alive: the mask strides [m0, m1), then, if
-// anything survived them, the unmasked filters lfil[l0, l1). Returns the positions alive.
-template <int NC>
-__device__ __forceinline__ u32 short_phase(u32 (&alive)[SHORT_LANES][NC], const ShortParams &P, const u32 *tab,
-                                           u32 tab_words, const MaskDesc *smd, u32 m0, u32 m1, u32 l0, u32 l1,
-                                           const u32 (&n)[SHORT_LANES], const u32 (&b)[SHORT_LANES],
-                                           const u16 *const (&K0row)[SHORT_LANES], const u16 *Qrow, u32 q0_first,
-                                           u32 lane, const MaskDesc &md_first) {
-  const u32 any = short_mask_rounds<NC>(alive, b, tab, tab_words, smd, m0, m1, Qrow, q0_first, lane, md_first);
-  if (any && l1 > l0) {
-    u32 kill[SHORT_LANES][NC];
-    #pragma unroll
-    for (int q = 0; q < SHORT_LANES; ++q)
-      #pragma unroll
-      for (int c = 0; c < NC; ++c) kill[q][c] = 0;
-    short_list_kill<NC>(kill, n, b, P.lfil, l0, l1, K0row, P.fdesc, Qrow, lane);
-    #pragma unroll
-    for (int q = 0; q < SHORT_LANES; ++q)
-      #pragma unroll
-      for (int c = 0; c < NC; ++c) alive[q][c] &= ~warp_or32(kill[q][c]);
-  }
-  u32 cnt = 0;
-  #pragma unroll
-  for (int q = 0; q < SHORT_LANES; ++q)
-    #pragma unroll
-    for (int c = 0; c < NC; ++c) cnt += __popc(alive[q][c]);
-  return cnt;
-}
-
-
-// The segments of SHORT_LANES lanes in one short window, NC 32-position chunks each.
-// The window a warp is marking: its index, and the lane of the warp holding its descriptor
-// (whose q_lo/q_hi registers carry Q = lo / M, read only when there are survivors).
-struct WinRef {
-  u32 wi, q_lo, q_hi;
-  int src;
+// A position the strides so far left: lane l at K, of window win.
+struct __align__(16) Cand {
+  u64 K;
+  u32 win, l;
 };
 
-template <int NC>
-__device__ __forceinline__ void short_segments(const ShortParams &P, const u32 *tab, u32 tab_words,
-                                               const MaskDesc *smd, u32 l_first, const WinRef &R,
-                                               const u64 (&rho)[SHORT_LANES], const u32 (&n)[SHORT_LANES],
-                                               const u32 (&b)[SHORT_LANES], const u16 *const (&K0row)[SHORT_LANES],
-                                               u32 q0_first, u32 lane, const MaskDesc &md0, const u32 *hand_j) {
-  const u32 wi = R.wi;
-  const u16 *Qrow = P.Qm + (size_t)wi * P.Dq;
-  u32 alive[SHORT_LANES][NC];
-  u32 cnt;
-  if (NC == 1 && hand_j) {                         // the sparse round did the first round
-    #pragma unroll
-    for (int q = 0; q < SHORT_LANES; ++q) alive[q][0] = hand_j[q];
-    const u32 k = 32 + lane;
-    const MaskDesc md1 = k < P.nm_cov ? smd[k] : MaskDesc{1, 0, 0, 0};
-    const u32 q1 = k < P.nm_cov ? (u32)__ldg(Qrow + md1.d) : 0u;
-    cnt = short_phase<NC>(alive, P, tab, tab_words, smd, min(32u, P.nm_cov), P.nm_cov, 0, P.nl_cov, n, b, K0row,
-                          Qrow, q1, lane, md1);
-  } else {
-    #pragma unroll
-    for (int q = 0; q < SHORT_LANES; ++q)
-      #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const u32 lo = 32 * c;
-        alive[q][c] = n[q] >= lo + 32 ? ~0u : (n[q] > lo ? (1u << (n[q] - lo)) - 1 : 0u);
-      }
-    cnt = short_phase<NC>(alive, P, tab, tab_words, smd, 0, P.nm_cov, 0, P.nl_cov, n, b, K0row, Qrow, q0_first,
-                          lane, md0);
-  }
-  if (cnt && (P.nm_all > P.nm_cov || P.nl_all > P.nl_cov)) {          // stage B'
-    if (lane == 0) atomicAdd(&P.cnt[wi].after_covers, (unsigned long long)cnt);
-    const u32 k = P.nm_cov + lane;
-    const u32 q0b = k < P.nm_all ? (u32)__ldg(Qrow + smd[k].d) : 0u;
-    const MaskDesc mdb = k < P.nm_all ? smd[k] : MaskDesc{1, 0, 0, 0};
-    cnt = short_phase<NC>(alive, P, tab, tab_words, smd, P.nm_cov, P.nm_all, P.nl_cov, P.nl_all, n, b, K0row, Qrow,
-                          q0b, lane, mdb);
-  }
-  if (!cnt) return;
-  // survivors are rare: the window's first position index comes from its lane, and lane 0
-  // writes the survivors in order
-  const u64 Q = (u64)__shfl_sync(FULL, R.q_lo, R.src) | ((u64)__shfl_sync(FULL, R.q_hi, R.src) << 32);
-  if (lane == 0) {
-    u64 slot = atomicAdd(P.surv_count, (unsigned long long)cnt);
-    atomicAdd(&P.cnt[wi].surv, (unsigned long long)cnt);
-    #pragma unroll
-    for (int q = 0; q < SHORT_LANES; ++q)
-      #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        u32 x = alive[q][c];
-        while (x) {
-          const u32 k = __ffs(x) - 1;
-          x &= x - 1;
-          if (slot < P.surv_cap) {
-            const u64 J = 32 * c + k;
-            Surv sv;
-            sv.p = rho[q] + P.M * (Q + b[q] + J);        // the segment starts at K = Q + b
-            sv.J = J;
-            sv.win = wi;
-            sv.lane = l_first + q;
-            P.surv[slot] = sv;
-          }
-          ++slot;
-        }
-      }
-  }
+// Kill bit of stride d = {s, m, c, first word} at K in a lane's table: NEAR, in shared memory from
+// word `at` of the dynamic part on; else in L2, from word `at` of P.tlane on.
+template <bool NEAR>
+__device__ __forceinline__ u32 stride_kills(const RowParams &P, const uint4 &d, u64 K, size_t at) {
+  extern __shared__ __align__(128) unsigned char rowmem[];
+  const u32 r = mod_stride(K, d, P.wide);
+  const u32 x = NEAR ? reinterpret_cast<const u32 *>(rowmem)[(u32)at + d.w + (r >> 5)] : __ldg(P.tlane + at + d.w + (r >> 5));
+  return __funnelshift_r(x, 0, r) & 1u;
 }
 
-// The sparse windows of a 32-window group (at most SPARSE_N positions in either lane of the
-// CTA: windows shorter than a few wheel periods) get the first round of strides alone, window
-// after window with the next window's residue loaded ahead: lane k extracts the kill word of
-// stride k for both lanes' positions, one warp OR each, and nothing else -- no task set-up.
-// The first round kills all but ~1% of positions, so almost every sparse window ends there;
-// the few with a position still alive are returned as a mask of the group's lanes, their alive
-// words left in hand[window][lane], and the task path goes on with them from the second round.
-// Counters and survivors are the task path's alone.
-
-// SH is the first round's row layout, the same for every stride of the round: 5 when its rows
-// are interleaved (word w of the stride in slot j at 32 w + j), 0 when they are packed.
-template <u32 SH>
-__device__ __forceinline__ unsigned short_sparse_round(const ShortParams &P, const u32 *tab, u32 tab_words,
-                                                       const MaskDesc &md0, u32 xwi, u32 pk, unsigned sp,
-                                                       u32 *hand, u32 lane) {
-  static_assert(SHORT_LANES == 2, "two lanes per CTA");
-  const bool has = lane < P.nm_cov;                // lane k holds the first round's stride k
-  auto ldq = [&](u32 wi) { return has ? (u32)__ldg(P.Qm + (size_t)wi * P.Dq + md0.d) : 0u; };
-  unsigned again = 0;
-  // this lane's own window of the group: its positions in the CTA's two lanes as bit masks
-  // (at most SPARSE_N each when the window is sparse)
-  const u32 n0l = pk & 255u, n1l = (pk >> 8) & 255u;
-  const u32 lm0 = n0l >= 32 ? ~0u : (1u << n0l) - 1, lm1 = n1l >= 32 ? ~0u : (1u << n1l) - 1;
-  u32 qn = ldq(__shfl_sync(FULL, xwi, __ffs(sp) - 1));
-  while (sp) {
-    const int j = __ffs(sp) - 1;
-    sp &= sp - 1;
-    const u32 pj = __shfl_sync(FULL, pk, j);
-    const u32 m0 = __shfl_sync(FULL, lm0, j), m1 = __shfl_sync(FULL, lm1, j);
-    const u32 qd = qn;
-    if (sp) qn = ldq(__shfl_sync(FULL, xwi, __ffs(sp) - 1));
-    u32 kill0 = 0, kill1 = 0;
-    if (has) {
-      u32 r = qd + ((pj >> 24) & 1u);
-      r = r >= md0.s ? r - md0.s : r;
-      const u32 *wp = tab + md0.off + ((r >> 5) << SH);
-      kill0 = __funnelshift_r(wp[0], wp[1u << SH], r & 31);
-      if ((pj ^ (pj >> 1)) & (1u << 24)) {       // the two lanes' segments start apart (rare)
-        r = qd + ((pj >> 25) & 1u);
-        r = r >= md0.s ? r - md0.s : r;
-      }
-      wp = tab + tab_words + md0.off + ((r >> 5) << SH);
-      kill1 = __funnelshift_r(wp[0], wp[1u << SH], r & 31);
-    }
-    const u32 a0 = m0 & ~warp_or32(kill0);
-    const u32 a1 = m1 & ~warp_or32(kill1);
-    if (a0 | a1) {                                  // the task path goes on from the second round
-      again |= 1u << j;
-      if (lane == 0) { hand[j * HAND_WORDS] = a0; hand[j * HAND_WORDS + 1] = a1; }
-    }
-  }
-  __syncwarp();
-  return again;
-}
-
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 2) k_mark_short(const ShortParams P) {
-  extern __shared__ __align__(16) u32 tab[];
-  const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (P.hdr->nshort == 0) return;
-  const u32 tab_words = P.Wpad * 2;                    // 32-bit words per lane table
-  // the stride descriptors (at most SMD_MAX, the host keeps any further strides unmasked)
-  MaskDesc *smd = reinterpret_cast<MaskDesc *>(tab + SHORT_LANES * tab_words);
-  for (u32 k = threadIdx.x; k < P.nm_all; k += BLOCK) smd[k] = P.mdesc[k];
-  u32 *hand = reinterpret_cast<u32 *>(smd + P.nm_all) + warp * 32 * HAND_WORDS;   // this warp's hand-on
-  const u32 nshort = P.hdr->nshort;
-  for (u32 l0 = blockIdx.x * SHORT_LANES; l0 < P.L; l0 += gridDim.x * SHORT_LANES) {
-    for (int q = 0; q < SHORT_LANES; ++q) {
-      const u32 l = min(l0 + q, P.L - 1);              // a missing last lane loads a copy; it stays inactive
-      const uint4 *src = reinterpret_cast<const uint4 *>(P.mtab + (size_t)l * P.Wpad);
-      uint4 *dst = reinterpret_cast<uint4 *>(tab + q * tab_words);
-      for (u32 i = threadIdx.x; i < P.Wpad / 2; i += BLOCK) dst[i] = __ldg(src + i);
-    }
-    __syncthreads();
-    u64 rho[SHORT_LANES];
-    const u16 *K0row[SHORT_LANES];
+// The strides sdesc[m0, m1) against candidates c[0, N), whose tables start at word at[i], a stride
+// per lane of the warp: one round of 32, which half of them die in, then four rounds at a time, the
+// loads of all candidates in flight together (past m1 the last stride is read again). Returns the
+// candidates of `mask` left, in every lane.
+template <bool NEAR, int N>
+__device__ __forceinline__ u32 strides_leave(const RowParams &P, const uint4 *sdesc, u32 m0, u32 m1, const Cand (&c)[N],
+                                             const size_t (&at)[N], u32 mask, u32 lane) {
+  for (u32 mb = m0; mb < m1 && mask;) {
+    u32 kill[N];
     #pragma unroll
-    for (int q = 0; q < SHORT_LANES; ++q) {
-      const u32 l = min(l0 + q, P.L - 1);
-      rho[q] = P.rho[l];
-      K0row[q] = P.K0 + (size_t)l * P.ldk;
-    }
-    // This warp's windows are i = warp + WS t. They are read 32 at a time, one descriptor per
-    // lane in one load, and each lane works out the segments of this CTA's lanes in its window
-    // (positions n and start offset b); a ballot keeps the windows where either lane has a
-    // position and the warp walks those, taking n and b packed in one shuffle. The first
-    // round's stride residue of the next window is loaded while a window is marked.
-    constexpr u32 WS = BLOCK / 32;
-    const uint4 *sw4 = reinterpret_cast<const uint4 *>(P.shortw);
-    const MaskDesc md0 = lane < P.nm_cov ? smd[lane] : MaskDesc{1, 0, 0, 0};   // the first round's stride
-    const u32 sh0 = P.nm_cov ? smd[0].sh : 0u;          // its layout (the same for the round's strides)
-    const u32 d_first = md0.d;
-    auto load_q0 = [&](u32 wi) {
-      return lane < P.nm_cov ? (u32)__ldg(P.Qm + (size_t)wi * P.Dq + d_first) : 0u;
+    for (int i = 0; i < N; ++i) kill[i] = 0;
+    auto round = [&]() {
+      const uint4 d = sdesc[min(mb + lane, m1 - 1)];
+      #pragma unroll
+      for (int i = 0; i < N; ++i) kill[i] |= stride_kills<NEAR>(P, d, c[i].K, at[i]);
+      mb += 32;
     };
-    static_assert(SHORT_LANES <= 3 && SEG_SMALL < 256, "n (8 bits) and b of each lane are packed in one word");
-    for (u32 t0 = 0; warp + WS * t0 < nshort; t0 += 32) {
-      const u32 my = warp + WS * (t0 + lane);
-      uint4 x = make_uint4(0, 0, 0, 0), y = make_uint4(0, 0, 0, 0);
-      if (my < nshort) { x = __ldg(sw4 + 2 * (size_t)my); y = __ldg(sw4 + 2 * (size_t)my + 1); }
-      // fields: x = {Q lo, Q hi, lomod, wi}, y = {la, lb, lq, lr}
-      u32 pk = 0;                                  // n_q at bit 8q, b_q at bit 24 + q
-      if (my < nshort) {
-        #pragma unroll
-        for (int q = 0; q < SHORT_LANES; ++q) {
-          const u32 l = l0 + q;
-          const u32 r = (u32)rho[q];
-          const u32 bq = r < x.z ? 1u : 0u;
-          const u32 d = r + (bq ? (u32)P.M : 0u) - x.z;              // (rho - lo) mod M
-          const u32 nq = (l < P.L && l >= y.x && l < y.y) ? y.z + (d < y.w ? 1u : 0u) : 0u;
-          pk |= (nq << (8 * q)) | (bq << (24 + q));
-        }
-      }
-      u32 nmax_w = 0;
+    if (mb == m0) round();
+    else {
       #pragma unroll
-      for (int q = 0; q < SHORT_LANES; ++q) nmax_w = max(nmax_w, (pk >> (8 * q)) & 255u);
-      unsigned todo = __ballot_sync(FULL, nmax_w > SPARSE_N);
-      unsigned hand_mask = 0;                      // windows the sparse round handed on
-      if (SPARSE_N) {
-        const unsigned sp = __ballot_sync(FULL, nmax_w > 0 && nmax_w <= SPARSE_N);
-        if (sp) hand_mask = sh0 ? short_sparse_round<5>(P, tab, tab_words, md0, x.w, pk, sp, hand, lane)
-                                : short_sparse_round<0>(P, tab, tab_words, md0, x.w, pk, sp, hand, lane);
-        todo |= hand_mask;
-      }
-      u32 q0n = todo ? load_q0(__shfl_sync(FULL, x.w, __ffs(todo) - 1)) : 0u;
-      while (todo) {
-        const int j = __ffs(todo) - 1;
-        todo &= todo - 1;
-        const u32 pj = __shfl_sync(FULL, pk, j);
-        const u32 wi = __shfl_sync(FULL, x.w, j);
-        const u32 q0_first = q0n;
-        if (todo) q0n = load_q0(__shfl_sync(FULL, x.w, __ffs(todo) - 1));
-        u32 n[SHORT_LANES], b[SHORT_LANES], nmax = 0;
-        #pragma unroll
-        for (int q = 0; q < SHORT_LANES; ++q) {
-          n[q] = (pj >> (8 * q)) & 255u;
-          b[q] = (pj >> (24 + q)) & 1u;
-          nmax = max(nmax, n[q]);
-        }
-        const WinRef R{wi, x.x, x.y, j};
-        const u32 *hj = (hand_mask >> j) & 1u ? hand + j * HAND_WORDS : nullptr;
-        // chunks per lane; one chunk is by far the commonest case, so it is tested first.
-        const u32 nc = (nmax + 31) >> 5;
-        // instantiations for 1, 2 and 4 chunks (8 too when SEG_SMALL is 256) measured faster
-        // than one per chunk count: the kernel's code stays small enough for the instruction
-        // cache
-        if (nc == 1) short_segments<1>(P, tab, tab_words, smd, l0, R, rho, n, b, K0row, q0_first, lane, md0, hj);
-        else if (nc == 2) short_segments<2>(P, tab, tab_words, smd, l0, R, rho, n, b, K0row, q0_first, lane, md0, hj);
-        else if constexpr (SEG_SMALL > 128) {
-          if (nc <= 4) short_segments<4>(P, tab, tab_words, smd, l0, R, rho, n, b, K0row, q0_first, lane, md0, hj);
-          else short_segments<8>(P, tab, tab_words, smd, l0, R, rho, n, b, K0row, q0_first, lane, md0, hj);
-        } else if constexpr (SEG_SMALL > 64) {
-          short_segments<4>(P, tab, tab_words, smd, l0, R, rho, n, b, K0row, q0_first, lane, md0, hj);
-        }
+      for (u32 r = 0; r < 4; ++r) round();
+    }
+    #pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (__any_sync(FULL, kill[i])) mask &= ~(1u << i);
+  }
+  return mask;
+}
+
+// Whether one of the filters lfil[l0, l1) (strides with no table) kills lane l at K.
+__device__ __forceinline__ bool list_kills(const RowParams &P, u32 l0, u32 l1, u64 K, u32 l, u32 lane) {
+  u32 kill = 0;
+  for (u32 k = l0 + lane; k < l1; k += 32) {
+    const u32 f = P.lfil[k], s = P.fdesc[f] & 0xFFFFu;
+    kill |= (u32)P.K0[(size_t)l * P.ldk + f] == (u32)(K % s);       // K0_MISS is no residue
+  }
+  return __any_sync(FULL, kill);
+}
+
+// The root of a perfect square p, else 0: a float root (off by less than 2^10 for p < 2^64) and one
+// Newton step, whose error is then below 2^-12.
+__device__ __forceinline__ u64 square_root(u64 p) {
+  const float f = sqrtf((float)p);
+  u64 s = (u64)f;
+  const float d = (float)(long long)(p - s * s) / (2.0f * f);       // wraps at s = 2^32: still p - s^2
+  s += (u64)(long long)rintf(d);
+  return s * s == p ? s : 0;
+}
+// Whether p = rho_l + M K is a square that passes every cover (see k_square_mask): n is prime to
+// the listed primes q (n < 2^32 is a multiple of q when n / q, as a product with q's inverse mod
+// 2^32, does not exceed (2^32 - 1) / q).
+__device__ __forceinline__ bool free_square(const RowParams &P, u64 K, u32 l) {
+  if (!P.squares) return false;
+  const u32 n = (u32)square_root(P.rho[l] + P.M * K);
+  bool ok = n != 0;
+  if (ok)
+    for (u32 i = 0; i < P.nsq; ++i) ok = ok && n * P.sq_inv[i] > P.sq_lim[i];
+  return ok;
+}
+
+// A chunk's candidate as a position.
+__device__ __forceinline__ Cand cand_of(const RowParams &P, uint2 e, u32 g) {
+  const Piece &x = P.piece[e.x];
+  return Cand{x.K0 + e.y / GROUP_LANES, x.win, g * GROUP_LANES + e.y % GROUP_LANES};
+}
+
+// Candidates c[0, n) against the covers' strides from m0 on (those below n2 in shared memory, from
+// word near[i] on), the filters without tables and stage B'; what is left is appended to the
+// survivors. The whole warp calls.
+constexpr int CAND_ILP = 2;
+__device__ __forceinline__ void take_candidates(const RowParams &P, const uint4 *sdesc, u32 m0, u32 n2,
+                                                const Cand (&c)[CAND_ILP], const size_t (&near)[CAND_ILP], int n,
+                                                u32 lane) {
+  u32 left = (1u << n) - 1;
+  if (m0 < n2) left = strides_leave<true>(P, sdesc, m0, n2, c, near, left, lane);
+  size_t far[CAND_ILP];
+  #pragma unroll
+  for (int i = 0; i < CAND_ILP; ++i) far[i] = (size_t)c[i].l * P.lane_words;
+  left = strides_leave<false>(P, sdesc, max(m0, n2), P.nm_cov, c, far, left, lane);
+  while (left) {
+    const int k = __ffs(left) - 1;
+    left &= left - 1;
+    Cand x[1] = {c[0]};
+    size_t y[1] = {far[0]};
+    #pragma unroll
+    for (int i = 1; i < CAND_ILP; ++i)
+      if (k == i) { x[0] = c[i]; y[0] = far[i]; }
+    const u64 K = x[0].K;
+    const u32 l = x[0].l, win = x[0].win;
+    if (P.nl_cov && list_kills(P, 0, P.nl_cov, K, l, lane)) continue;
+    if (P.nm_all > P.nm_cov || P.nl_all > P.nl_cov) {                 // stage B'
+      if (lane == 0) atomicAdd(&P.cnt[win].after_covers, 1ull);
+      if (!strides_leave<false>(P, sdesc, P.nm_cov, P.nm_all, x, y, 1, lane)) continue;
+      if (P.nl_all > P.nl_cov && list_kills(P, P.nl_cov, P.nl_all, K, l, lane)) continue;
+    }
+    if (lane == 0) {
+      const u64 slot = atomicAdd(P.surv_count, 1ull);
+      atomicAdd(&P.cnt[win].surv, 1ull);
+      if (slot < P.surv_cap) {
+        const WinDev &W = P.win[win];
+        const u32 rho = P.rho[l];
+        Surv sv;
+        sv.p = rho + P.M * K;
+        sv.J = K - W.Q - (rho < W.lomod ? 1 : 0);                     // lane l starts at K = Q or Q + 1
+        sv.win = win;
+        sv.lane = l;
+        P.surv[slot] = sv;
       }
     }
-    __syncthreads();
   }
 }
 
-// Kill masks from the first-hit table: bit x of lane l's mask for filter f's stride, for
-// every x == K0[l][f] (mod s) below s + SEG_SMALL (the repeat that a segment of up to
-// SEG_SMALL positions starting below s may reach).
-__global__ void k_build_masks(const u16 *__restrict__ K0, u32 L, u32 ldk, u32 nf, const int *__restrict__ fmask,
-                              const MaskDesc *__restrict__ mdesc, u32 Wpad, u64 *__restrict__ mtab) {
+// Whether strides sdesc[m0, m1) leave a thread's candidate (where `on`; x is some position
+// elsewhere), its lane's table at word `at`; the warp stops when none is left.
+template <bool NEAR>
+__device__ __forceinline__ bool thread_leaves(const RowParams &P, const uint4 *sdesc, u32 m0, u32 m1, const Cand &x,
+                                              size_t at, bool on) {
+  for (u32 m = m0; m < m1 && __any_sync(FULL, on); m += 8) {
+    u32 kill = 0;
+    #pragma unroll
+    for (u32 i = 0; i < 8; ++i) kill |= stride_kills<NEAR>(P, sdesc[min(m + i, m1 - 1)], x.K, at);
+    on = on && !kill;
+  }
+  return on;
+}
+
+// The candidates `left` of a warp's threads, strides below m0 done, by the whole warp.
+template <bool NEAR>
+__device__ __forceinline__ void take_left(const RowParams &P, const uint4 *sdesc, u32 m0, u32 n2, const Cand &x, size_t at,
+                                          unsigned left, u32 lane) {
+  while (left) {
+    Cand c[CAND_ILP];
+    size_t near[CAND_ILP];
+    int n = 0;
+    #pragma unroll
+    for (int i = 0; i < CAND_ILP; ++i) {
+      const int src = left ? __ffs(left) - 1 : 0;
+      n += left != 0;
+      left &= left - 1;
+      c[i].K = __shfl_sync(FULL, x.K, src);
+      c[i].win = __shfl_sync(FULL, x.win, src);
+      c[i].l = __shfl_sync(FULL, x.l, src);
+      near[i] = NEAR ? __shfl_sync(FULL, (u32)at, src) : 0;
+    }
+    take_candidates(P, sdesc, m0, NEAR ? n2 : 0, c, near, n, lane);
+  }
+}
+
+// Whether a thread's candidate needs no test because it is a square; if so it is counted.
+__device__ __forceinline__ bool take_square(const RowParams &P, const Cand &x) {
+  const bool sq = free_square(P, x.K, x.l);
+  if (sq) atomicAdd(&P.cnt[x.win].surv, 1ull);
+  return sq;
+}
+
+// The candidates against the other strides. Up to two per warp of the grid: a warp each. Up to
+// SIFT_FAR chunks: a thread each, reading the lanes' tables (60 MB) from L2, for THREAD_STRIDES[0]
+// strides, then the whole warp for the quarter that is left. Beyond: the CTAs take SIFT_LANES lanes
+// at a time, copy their tables to shared memory, and pick those lanes' candidates out of their
+// group's chunks; a warp walks THREAD_STRIDES[0] strides when it has gathered 32, gathers what is
+// left in a second buffer, walks THREAD_STRIDES[1] more when that holds 32, and takes the few that
+// are left together. The lines: reading tables from L2 costs a sector per test, so beyond a few
+// candidates a thread their traffic is the bound (one kernel without the shared-memory pass took 0.65
+// ms on a 2^40-integer window and 0.55 ms on the 4096-window batch, against 0.60 and 0.21 ms for
+// the two), while copying all lane tables costs 15 us whatever the count: a 2^34 window's 5 K part-
+// filled chunks took 15 us more with them. Bound by instruction issue (58% of peak issue on the 2^40
+// window: 0.35 ms for 2.3 M candidates).
+#ifndef ES_SIFT_FAR
+#define ES_SIFT_FAR 8192
+#endif
+constexpr u32 SIFT_FAR = ES_SIFT_FAR;
+constexpr u32 THREAD_STRIDES[2] = {32, 64};
+__global__ void __launch_bounds__(ROW_THREADS, 1) k_sift(const RowParams P) {
+  extern __shared__ __align__(128) unsigned char rowmem[];
+  __shared__ __align__(8) u64 s_bar;
+  const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const u32 nchunks = (u32)min(*P.chunk_count, (unsigned long long)P.chunk_cap);
+  if (!nchunks) return;
+  uint4 *sdesc = reinterpret_cast<uint4 *>(rowmem + 2 * CAND_SMEM) - P.n1;              // indexed from n1
+  constexpr u32 near = (2 * CAND_SMEM + STRIDES_MAX * 16) / 4;                          // the tables' first word
+  for (u32 m = P.n1 + threadIdx.x; m < P.nm_all; m += ROW_THREADS) sdesc[m] = P.mdesc[P.n1p - P.n1 + m];
+  const u32 warps = gridDim.x * (ROW_THREADS / 32), w0 = blockIdx.x + warp * gridDim.x;   // spread over the SMs
+  __syncthreads();
+  if (nchunks * 32 <= 2 * warps) {
+    for (u32 i = w0; i < nchunks * 32; i += warps) {
+      const u32 h = P.chunk[i / 32];
+      if (i % 32 >= (h & 255u)) continue;
+      const Cand x = cand_of(P, P.cand[i], h >> 8), c[CAND_ILP] = {x, x};
+      const size_t none[CAND_ILP] = {};
+      if (free_square(P, c[0].K, c[0].l)) {
+        if (lane == 0) atomicAdd(&P.cnt[c[0].win].surv, 1ull);
+        continue;
+      }
+      take_candidates(P, sdesc, P.n1, 0, c, none, 1, lane);
+    }
+    return;
+  }
+  if (nchunks <= SIFT_FAR) {
+    const u32 m1 = min(P.n1 + THREAD_STRIDES[0], P.nm_cov);
+    for (u32 i = w0; i < nchunks; i += warps) {
+      const u32 h = P.chunk[i];
+      bool on = lane < (h & 255u);
+      Cand x{0, 0, 0};
+      if (on) x = cand_of(P, P.cand[(size_t)i * 32 + lane], h >> 8);
+      const size_t far = (size_t)x.l * P.lane_words;
+      on = on && !take_square(P, x);
+      on = thread_leaves<false>(P, sdesc, P.n1, m1, x, far, on);
+      take_left<false>(P, sdesc, m1, 0, x, far, __ballot_sync(FULL, on), lane);
+    }
+    return;
+  }
+  uint2 *buf = reinterpret_cast<uint2 *>(rowmem) + warp * 128, *buf2 = buf + 64;
+  const u32 bar = smem_addr(&s_bar);
+  if (threadIdx.x == 0) bar_init(bar);
+  u32 parity = 0;
+  // the words of the strides below n2, whole 16-byte units (a lane's table is one too)
+  const u32 n2 = min(P.n2, P.nm_cov);
+  const u32 nwords = P.n2 < P.nm_all ? P.mdesc[P.n1p - P.n1 + P.n2].w & ~3u : P.lane_words;
+  const u32 m1 = min(P.n1 + THREAD_STRIDES[0], n2), m2 = min(m1 + THREAD_STRIDES[1], n2);
+  for (u32 l0 = blockIdx.x * SIFT_LANES; l0 < P.L; l0 += gridDim.x * SIFT_LANES) {
+    __syncthreads();                                   // the barrier's init, the previous lanes' reads
+    if (threadIdx.x == 0) {
+      const u32 nl = min(SIFT_LANES, P.L - l0);
+      bar_expect(bar, nl * nwords * 4);
+      for (u32 q = 0; q < nl; ++q)
+        bulk_copy(smem_addr(rowmem) + (near + q * nwords) * 4, P.tlane + (size_t)(l0 + q) * P.lane_words, nwords * 4, bar);
+    }
+    if (!bulk_wait(bar, parity, P.status)) return;
+    parity ^= 1;
+    const u32 g = l0 / GROUP_LANES, o0 = l0 % GROUP_LANES / SIFT_LANES;
+    u32 nbuf = 0, nbuf2 = 0;                           // fewer than 32, then at most 32 more
+    auto load = [&](const uint2 *from, u32 n, uint2 &e, Cand &x) {
+      e = make_uint2(0, 0);
+      x = Cand{0, 0, l0};
+      if (lane < n) { e = from[lane]; x = cand_of(P, e, g); }
+      __syncwarp();
+      return near + (x.l - l0) * nwords;
+    };
+    auto drain2 = [&](u32 n) {
+      uint2 e;
+      Cand x;
+      nbuf2 -= n;
+      const u32 at = load(buf2 + nbuf2, n, e, x);
+      const bool on = thread_leaves<true>(P, sdesc, m1, m2, x, at, lane < n);
+      take_left<true>(P, sdesc, m2, n2, x, at, __ballot_sync(FULL, on), lane);
+    };
+    auto drain = [&](u32 n) {
+      uint2 e;
+      Cand x;
+      nbuf -= n;
+      const u32 at = load(buf + nbuf, n, e, x);
+      bool on = lane < n && !take_square(P, x);
+      on = thread_leaves<true>(P, sdesc, P.n1, m1, x, at, on);
+      const unsigned left = __ballot_sync(FULL, on);
+      if (on) buf2[nbuf2 + __popc(left & ((1u << lane) - 1))] = e;
+      nbuf2 += __popc(left);
+      __syncwarp();
+      if (nbuf2 >= 32) drain2(32);
+    };
+    for (u32 c0 = warp * 32; c0 < nchunks; c0 += ROW_THREADS) {
+      const u32 h = c0 + lane < nchunks ? __ldg(P.chunk + c0 + lane) : ~0u;
+      unsigned mine = __ballot_sync(FULL, h >> 8 == g);
+      auto entry = [&](int k) {                        // of chunk c0 + k, no lane's past its end
+        const u32 n = __shfl_sync(FULL, h, k) & 255u;
+        return lane < n ? __ldg(P.cand + (size_t)(c0 + k) * 32 + lane) : make_uint2(0, ~0u);
+      };
+      uint2 next = mine ? entry(__ffs(mine) - 1) : make_uint2(0, ~0u);
+      while (mine) {
+        const uint2 e = next;
+        mine &= mine - 1;
+        if (mine) next = entry(__ffs(mine) - 1);       // loaded while this chunk is taken
+        const unsigned hit = __ballot_sync(FULL, e.y != ~0u && e.y % GROUP_LANES / SIFT_LANES == o0);
+        if (hit >> lane & 1) buf[nbuf + __popc(hit & ((1u << lane) - 1))] = e;
+        nbuf += __popc(hit);
+        __syncwarp();
+        if (nbuf >= 32) drain(32);
+      }
+    }
+    if (nbuf) drain(nbuf);
+    if (nbuf2) drain2(nbuf2);
+  }
+}
+
+// The tables' bits from the first-hit table, a thread per (lane, filter) that hits: in the
+// dense slices every row x == K0 (mod s) of the stride's s + PIECE_ROWS - 1, elsewhere one bit.
+__global__ void k_build_rows(const u16 *__restrict__ K0, u32 L, u32 ldk, u32 nf, const int *__restrict__ fmask,
+                             const uint4 *__restrict__ mdesc, u32 n1, u32 n1p, u32 slice_rows, u32 lane_words,
+                             u32 *__restrict__ tdense, u32 *__restrict__ tlane) {
   const u64 idx = (u64)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (u64)L * nf) return;
   const u32 l = (u32)(idx / nf), f = (u32)(idx % nf);
@@ -725,9 +827,31 @@ __global__ void k_build_masks(const u16 *__restrict__ K0, u32 L, u32 ldk, u32 nf
   if (m < 0) return;
   const u32 k0 = K0[(size_t)l * ldk + f];
   if (k0 == K0_MISS) return;
-  const MaskDesc md = mdesc[m];
-  u32 *row = reinterpret_cast<u32 *>(mtab + (size_t)l * Wpad) + md.off;
-  for (u32 x = k0; x < md.s + SEG_SMALL; x += md.s) atomicOr(row + ((x >> 5) << md.sh), 1u << (x & 31));
+  if ((u32)m < n1) {
+    const uint4 d = mdesc[m];
+    u32 *slice = tdense + (size_t)(l / GROUP_LANES) * slice_rows * GROUP_WORDS + l % GROUP_LANES / 32;
+    for (u32 x = k0; x < d.x + PIECE_ROWS - 1; x += d.x) atomicOr(slice + (size_t)(d.w + x) * GROUP_WORDS, 1u << (l & 31));
+  } else {
+    atomicOr(tlane + (size_t)l * lane_words + mdesc[n1p - n1 + m].w + (k0 >> 5), 1u << (k0 & 31));
+  }
+}
+
+// Whether a filter (mod, res) can kill a perfect square: a thread per (filter, x mod mod), hits
+// x^2 == res (mod mod). Such an x shares a factor g with mod, and a square n^2 that the filter kills
+// has n == x, so n shares it too: its least odd prime factor q goes into `primes` as bit q. A hit
+// with no such q below 64 sets bit 0: squares then get no shortcut.
+__global__ void k_square_mask(const u64 *__restrict__ mods, const u64 *__restrict__ ress, u32 nf,
+                              unsigned long long *__restrict__ primes) {
+  for (u32 f = blockIdx.x; f < nf; f += gridDim.x) {
+    const u64 mod = mods[f], res = ress[f] % mod;
+    for (u64 x = threadIdx.x; x < mod; x += blockDim.x) {
+      if (x * x % mod != res) continue;                // mod < 2^32
+      const u64 g = gcd64(x, mod);
+      u64 q = 3;
+      while (q < 64 && g % q) q += 2;
+      atomicOr(primes, q < 64 ? 1ull << q : 1ull);
+    }
+  }
 }
 
 // Miller-Rabin in two passes. Nearly every survivor is composite and fails the base-2
@@ -981,12 +1105,6 @@ __global__ void k_probe_factor(const u64 *n, u64 count, u64 *pr, unsigned char *
 // ============================================================================ host engine
 
 constexpr int MARK_BLOCK = 128;
-#ifndef ES_SHORT_BLOCK
-#define ES_SHORT_BLOCK 512
-#endif
-constexpr int SHORT_BLOCK = ES_SHORT_BLOCK;
-constexpr size_t SHORT_HAND_BYTES = (size_t)(SHORT_BLOCK / 32) * 32 * HAND_WORDS * sizeof(u32);   // 16 warps, 64 registers: two CTAs of two 37 KB lane tables fill an SM
-
 }  // namespace es
 
 namespace es {
@@ -999,7 +1117,7 @@ struct Slot {
   cudaEvent_t ev[12] = {};
   BatchHdr *d_hdr = nullptr, *h_hdr = nullptr;
   WinDev *h_win = nullptr;
-  ShortWin *h_short = nullptr;
+  RowWin *h_roww = nullptr;
   WinCount *h_cnt = nullptr;
   unsigned long long *h_ctr = nullptr;
   u32 *h_status = nullptr;
@@ -1013,26 +1131,28 @@ struct Slot {
   cudaGraphExec_t gexec = nullptr, gexec2 = nullptr;
   WinDev *d_win = nullptr; size_t win_cap = 0;
   WinCount *d_cnt = nullptr;
-  ShortWin *d_shortw = nullptr; size_t shortw_cap = 0;
+  RowWin *d_roww = nullptr;
+  Piece *d_piece = nullptr; u16 *d_pidx = nullptr; u32 *d_rowinfo = nullptr; size_t piece_cap = 0;
+  uint2 *d_cand2 = nullptr; u32 *d_chunk = nullptr; size_t chunk_cap = 0;
   u16 *d_Qm = nullptr; size_t qm_cap = 0;
   Surv *d_surv = nullptr;
   u32 *d_primes = nullptr, *d_direct = nullptr, *d_cand = nullptr;
   RecDev *d_recs = nullptr;
   size_t cap = 0;
   size_t rec_prefix = 0;                // records the captured graph copies back itself
+  u64 graph_launches = 0;               // its kernels
   unsigned long long *d_ctr = nullptr;  // [0] queue [1] surv [2] prime [3] direct [4] rec [5] cand
                                       // [6] rung queue (blocks) [7] rungs done [8] help sessions
-                                      // [9] rung queue (warps), board at [16]
+                                      // [9] rung queue (warps) [10] candidate chunks, board at [16]
   u32 *d_status = nullptr;
   es_timing_t timing{};
   struct HostScratch {                  // per-run host vectors, kept with their capacity
     std::vector<WinDev> wd;
-    std::vector<ShortWin> shortw;
+    std::vector<RowWin> roww;
     std::vector<u64> npos;
     std::vector<RecDev> hr;
     std::vector<u32> start, pos;
-    std::vector<uint8_t> mag;
-    std::vector<es_window> dw;          // the long-window split (run_windows)
+    std::vector<es_window> dw;          // runs in passes (run_windows)
     std::vector<std::pair<u32, u64>> dmap;
     std::vector<es_counters> pc;
     std::vector<es_record> all;
@@ -1042,6 +1162,7 @@ struct Slot {
 
 constexpr int SERVE_SLOTS = 2;
 // run counters (16 words) followed by the hard board, cleared together before every run
+constexpr size_t CTR_OUT = 11;          // counters copied back to the host
 constexpr size_t CTR_BYTES = 16 * sizeof(unsigned long long) + HARD_SLOTS * sizeof(HardSlot);
 
 // A serving request: windows in, counters and records out.
@@ -1081,11 +1202,17 @@ struct es_engine {
   // resident device tables
   es::u32 *d_rho = nullptr, *d_fdesc = nullptr, *d_sdist = nullptr, *d_tdp = nullptr;
   es::u16 *d_K0 = nullptr;
-  // short-window kill masks
-  es::u64 *d_mtab = nullptr;
-  es::MaskDesc *d_mdesc = nullptr;
+  // the row tables: dense slices by lane group, the other strides' rows, the strides' descriptors
+  // ([0, n1) dense, padded to n1p, then the others), the filters of the strides without rows
+  unsigned char *d_tdense = nullptr;
+  es::u32 *d_tlane = nullptr;
+  uint4 *d_mdesc = nullptr;
   es::u32 *d_lfil = nullptr;
-  uint32_t Wpad = 0, nm_cov = 0, nm_all = 0, nl_cov = 0, nl_all = 0, m_inter = 0;
+  bool squares = false;                 // see RowParams
+  std::vector<uint32_t> sq;             // the primes a root has to avoid
+  es::u64 pass_rows = 0;                // rows a run marks at a time (run_windows)
+  double cand_rate = 0;                 // candidates per position after the dense strides, estimated
+  uint32_t lane_words = 0, n2 = 0, ngroups = 0, n1 = 0, n1p = 0, slice_rows = 0, nm_cov = 0, nm_all = 0, nl_cov = 0, nl_all = 0;
   es::TdEntry *d_tde = nullptr;
   es::u64 *d_tdi = nullptr;
   uint2 *d_tdqm = nullptr;              // {d, floor(2^32 / d)} for the same primes
@@ -1134,32 +1261,54 @@ static void drop_graph(Slot *sl) {
   sl->graph = sl->graph2 = nullptr;
 }
 
-// Device buffers for nwin windows and a survivor capacity of cap, with their pinned host
+// Device buffers for nwin windows, npieces row pieces, nchunks candidate chunks and a survivor
+// capacity of cap, with their pinned host
 // staging. Growing any of them invalidates the captured graph (its copies and kernel
 // parameters name the old buffers and sizes).
-static es_status ensure_capacity(es_engine *e, Slot *sl, size_t nwin, size_t cap) {
+static es_status ensure_capacity(es_engine *e, Slot *sl, size_t nwin, size_t npieces, size_t nchunks, size_t cap) {
   if (!sl->d_hdr) {
     CU(cudaMalloc(&sl->d_hdr, sizeof(BatchHdr)));
     CU(cudaMallocHost(&sl->h_hdr, sizeof(BatchHdr)));
-    CU(cudaMallocHost(&sl->h_ctr, 8 * sizeof(unsigned long long)));
+    CU(cudaMallocHost(&sl->h_ctr, CTR_OUT * sizeof(unsigned long long)));
     CU(cudaMallocHost(&sl->h_status, sizeof(u32)));
   }
   if (nwin > sl->win_cap) {
     drop_graph(sl);
-    cudaFree(sl->d_win); cudaFree(sl->d_cnt); cudaFree(sl->d_shortw); cudaFree(sl->d_Qm);
-    cudaFreeHost(sl->h_win); cudaFreeHost(sl->h_short); cudaFreeHost(sl->h_cnt);
-    sl->d_win = nullptr; sl->d_cnt = nullptr; sl->d_shortw = nullptr; sl->d_Qm = nullptr;
-    sl->h_win = nullptr; sl->h_short = nullptr; sl->h_cnt = nullptr;
+    cudaFree(sl->d_win); cudaFree(sl->d_cnt); cudaFree(sl->d_roww); cudaFree(sl->d_Qm);
+    cudaFreeHost(sl->h_win); cudaFreeHost(sl->h_roww); cudaFreeHost(sl->h_cnt);
+    sl->d_win = nullptr; sl->d_cnt = nullptr; sl->d_roww = nullptr; sl->d_Qm = nullptr;
+    sl->h_win = nullptr; sl->h_roww = nullptr; sl->h_cnt = nullptr;
+    sl->win_cap = 0;
     const size_t want = std::max<size_t>(nwin, 64);
     CU(cudaMalloc(&sl->d_win, want * sizeof(WinDev)));
     CU(cudaMalloc(&sl->d_cnt, want * sizeof(WinCount)));
-    CU(cudaMalloc(&sl->d_shortw, want * sizeof(ShortWin)));
+    CU(cudaMalloc(&sl->d_roww, want * sizeof(RowWin)));
     CU(cudaMalloc(&sl->d_Qm, want * std::max<u32>(e->Dq, 8) * sizeof(u16)));
     CU(cudaMallocHost(&sl->h_win, want * sizeof(WinDev)));
-    CU(cudaMallocHost(&sl->h_short, want * sizeof(ShortWin)));
+    CU(cudaMallocHost(&sl->h_roww, want * sizeof(RowWin)));
     CU(cudaMallocHost(&sl->h_cnt, want * sizeof(WinCount)));
-    sl->win_cap = sl->shortw_cap = want;
+    sl->win_cap = want;
     sl->qm_cap = want * std::max<u32>(e->Dq, 8);
+  }
+  if (npieces > sl->piece_cap) {
+    drop_graph(sl);
+    cudaFree(sl->d_piece); cudaFree(sl->d_pidx); cudaFree(sl->d_rowinfo);
+    sl->d_piece = nullptr; sl->d_pidx = nullptr; sl->d_rowinfo = nullptr;
+    sl->piece_cap = 0;
+    const size_t want = std::max<size_t>(npieces + npieces / 4, 256);
+    CU(cudaMalloc(&sl->d_piece, want * sizeof(Piece)));
+    CU(cudaMalloc(&sl->d_pidx, want * std::max<u32>(e->n1p, 8) * sizeof(u16)));
+    CU(cudaMalloc(&sl->d_rowinfo, want * PIECE_ROWS * sizeof(u32)));
+    sl->piece_cap = want;
+  }
+  if (nchunks > sl->chunk_cap) {
+    drop_graph(sl);
+    cudaFree(sl->d_cand2); cudaFree(sl->d_chunk);
+    sl->d_cand2 = nullptr; sl->d_chunk = nullptr;
+    sl->chunk_cap = 0;
+    CU(cudaMalloc(&sl->d_cand2, nchunks * 32 * sizeof(uint2)));
+    CU(cudaMalloc(&sl->d_chunk, nchunks * sizeof(u32)));
+    sl->chunk_cap = nchunks;
   }
   if (cap > sl->cap) {
     drop_graph(sl);
@@ -1215,8 +1364,28 @@ static TailParams tail_params(const es_engine *e, const Slot *sl) {
   return T;
 }
 
-static size_t short_smem(const es_engine *e) {
-  return (size_t)SHORT_LANES * e->Wpad * 8 + (size_t)e->nm_all * sizeof(MaskDesc) + SHORT_HAND_BYTES;
+static RowParams row_params(const es_engine *e, const Slot *sl) {
+  RowParams S;
+  S.rho = e->d_rho; S.K0 = e->d_K0; S.fdesc = e->d_fdesc; S.tdense = e->d_tdense; S.tlane = e->d_tlane;
+  S.mdesc = e->d_mdesc; S.lfil = e->d_lfil; S.win = sl->d_win; S.roww = sl->d_roww; S.piece = sl->d_piece;
+  S.pidx = sl->d_pidx; S.rowinfo = sl->d_rowinfo; S.cand = sl->d_cand2; S.chunk = sl->d_chunk;
+  S.chunk_count = sl->d_ctr + 10; S.chunk_cap = (u32)sl->chunk_cap;
+  S.surv = sl->d_surv; S.surv_count = sl->d_ctr + 1; S.cnt = sl->d_cnt; S.surv_cap = sl->cap; S.M = e->M;
+  S.status = sl->d_status; S.hdr = sl->d_hdr;
+  S.L = (u32)e->classes.size(); S.ldk = e->ldk; S.lane_words = e->lane_words; S.ngroups = e->ngroups;
+  S.slice_bytes = e->slice_rows * 4 * GROUP_WORDS; S.n1 = e->n1; S.n1p = e->n1p; S.n2 = e->n2;
+  S.nm_cov = e->nm_cov; S.nm_all = e->nm_all; S.nl_cov = e->nl_cov; S.nl_all = e->nl_all;
+  S.wide = (DIRECT_PMAX / e->M) >> 48 != 0;
+  S.squares = e->squares;
+  S.nsq = (u32)e->sq.size();
+  for (u32 i = 0; i < S.nsq; ++i) {
+    const u32 q = e->sq[i];
+    u32 v = q;                                       // q^-1 mod 2^32 by Newton, from 3 bits
+    for (int k = 0; k < 4; ++k) v *= 2 - q * v;
+    S.sq_inv[i] = v;
+    S.sq_lim[i] = ~0u / q;
+  }
+  return S;
 }
 
 static size_t mark_smem(const es_engine *e) {
@@ -1253,50 +1422,59 @@ static void build_lane_index(es_engine *e) {
   e->inv_M = 1.0 / (double)e->M;
 }
 
-// Window descriptors and their marking items. Short windows (at most SEG_SMALL positions
-// per lane) go to k_mark_short, which walks them lane by lane; long windows get one lane per
-// item and segments of SEG_BIG positions in k_mark.
-static u64 describe(const es_engine *e, const es_window *w, size_t n, std::vector<WinDev> &out,
-                    std::vector<ShortWin> &shortw) {
+// Window descriptors and their marking work. Windows marked by rows (all of them with
+// sched.long_split, else those with at most sched.short_max positions in any lane) get their run
+// of rows: K = lo / M from the first class at or above lo mod M on, to the last class below hi.
+// The others get one lane per item and segments of SEG_BIG positions in k_mark. npos[i] is the
+// window's wheel positions; the totals go to `run`.
+struct RunShape {
+  u64 items = 0, rows = 0, pieces = 0;
+};
+static RunShape describe(const es_engine *e, const es_window *w, size_t n, std::vector<WinDev> &out,
+                         std::vector<RowWin> &roww, std::vector<u64> &npos) {
   out.resize(n);
-  shortw.clear();
-  shortw.reserve(n);
-  u64 items = 0;
-  const u64 L = e->classes.size(), M = e->M;
+  npos.resize(n);
+  roww.clear();
+  roww.reserve(n);
+  RunShape run;
+  const u64 L = e->classes.size();
   for (size_t i = 0; i < n; ++i) {
     WinDev &d = out[i];
     d.lo = w[i].lo; d.hi = std::max(w[i].lo, w[i].hi);
-    u64 q, r;
+    u64 q, r, qh, rh;
     divmod_M(e, d.lo, q, r);
+    divmod_M(e, d.hi, qh, rh);
     d.Q = q;
     d.lomod = (u32)r;
-    const u64 len = d.hi - d.lo;
-    u64 maxpos = 0, rem_;                                // most positions any lane can hold
-    if (len) { divmod_M(e, len - 1, maxpos, rem_); ++maxpos; }
-    d.item0 = items;
+    d.item0 = run.items;
     d.G = 1; d.lane0 = 0;
-    if (maxpos <= e->sched.short_max) {
-      d.seg = SEG_SMALL; d.nseg = 0; d.groups = 0;
-      if (maxpos) {
-        // Shorter than M: only the classes in [lo mod M, lo mod M + len) have a position,
-        // a contiguous lane range unless it wraps past M.
-        u64 la = 0, lb = L;
-        if (len < M && d.lomod + len <= M) {
-          la = classes_below(e, d.lomod);
-          lb = classes_below(e, d.lomod + len);
-        }
-        if (la < lb) {
-          u64 lq, lr;
-          divmod_M(e, len, lq, lr);
-          shortw.push_back(ShortWin{d.Q, d.lomod, (u32)i, (u32)la, (u32)lb, (u32)lq, (u32)lr});
-        }
-      }
+    d.seg = SEG_SMALL; d.nseg = 0; d.groups = 0;
+    // positions before lo and before hi, both counted from K = q
+    const u64 before = classes_below(e, r), upto = (qh - q) * L + classes_below(e, rh);
+    npos[i] = upto - before;
+    if (!npos[i]) continue;
+    u64 maxpos, rem_;                                    // most positions any lane can hold
+    divmod_M(e, d.hi - d.lo - 1, maxpos, rem_);
+    ++maxpos;
+    if (e->sched.long_split || maxpos <= e->sched.short_max) {
+      const u64 k0 = before / L, k1 = (upto - 1) / L;    // first and last row holding a position, from q
+      RowWin x;
+      x.K0 = q + k0;
+      x.nrows = (u32)(k1 - k0 + 1);
+      x.la = (u32)(before - k0 * L);
+      x.lb = (u32)(upto - k1 * L);
+      x.wi = (u32)i;
+      x.row0 = (u32)run.rows;
+      x.piece0 = (u32)run.pieces;
+      roww.push_back(x);
+      run.rows += x.nrows;
+      run.pieces += (x.nrows + PIECE_ROWS - 1) / PIECE_ROWS;
     } else {
       d.seg = SEG_BIG; d.nseg = (u32)((maxpos + SEG_BIG - 1) / SEG_BIG); d.groups = (u32)L;
+      run.items += (u64)d.groups * d.nseg;
     }
-    items += (u64)d.groups * d.nseg;
   }
-  return items;
+  return run;
 }
 
 // Wheel positions in [lo, hi): L per full period of M, plus the classes among the residues
@@ -1313,14 +1491,13 @@ static u64 positions_in(const es_engine *e, u64 lo, u64 hi) {
 }
 
 // One pass of the funnel on the engine's stream: reset the counters, copy the batch header
-// and descriptors from pinned staging (ncopy windows), the marking kernels, the survivor
-// tail, and the copies of the run counters back to pinned memory. With `capture` the event
-// records are external graph nodes, so that the kernels can still be timed when the
-// sequence runs as a graph. `items_hint` sizes k_mark's grid for the plain schedule.
-// The funnel's front on the slot's stream: run counters cleared, batch header and window
-// descriptors copied in, residues, marking (short and long windows), Miller-Rabin.
-static es_status enqueue_front(es_engine *e, Slot *sl, bool persistent, WinCount *cnt, size_t ncopy, size_t nshort_copy,
-                               u64 items_hint, bool capture) {
+// and descriptors from pinned staging (ncopy windows, nrow_copy of them marked by rows), the
+// marking kernels, the survivor tail, and the copies of the run counters back to pinned memory.
+// With `capture` the event records are external graph nodes, so that the kernels can still be
+// timed when the sequence runs as a graph. `segments`: some windows may go to the segment marking
+// (k_mark, sized by `items_hint` in the plain schedule). Adds its kernel launches to `launches`.
+static es_status enqueue_front(es_engine *e, Slot *sl, bool persistent, WinCount *cnt, size_t ncopy, size_t nrow_copy,
+                               bool segments, u64 items_hint, bool capture, u64 &launches) {
   MarkParams P = mark_params(e, sl);
   TailParams T = tail_params(e, sl);
   P.cnt = cnt;
@@ -1333,31 +1510,42 @@ static es_status enqueue_front(es_engine *e, Slot *sl, bool persistent, WinCount
   CU(cudaMemsetAsync(sl->d_status, 0, sizeof(u32), st));
   CU(cudaMemcpyAsync(sl->d_hdr, sl->h_hdr, sizeof(BatchHdr), cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync(sl->d_win, sl->h_win, ncopy * sizeof(WinDev), cudaMemcpyHostToDevice, st));
-  if (nshort_copy) CU(cudaMemcpyAsync(sl->d_shortw, sl->h_short, nshort_copy * sizeof(ShortWin), cudaMemcpyHostToDevice, st));
+  if (nrow_copy) CU(cudaMemcpyAsync(sl->d_roww, sl->h_roww, nrow_copy * sizeof(RowWin), cudaMemcpyHostToDevice, st));
   CU(rec(0));
-  k_prep<<<e->sm_count * 4, 256, 0, st>>>(sl->d_hdr, sl->d_win, e->d_sdist, e->D, e->Dq, sl->d_Qm);
-  CU(cudaGetLastError());
-  CU(rec(7));
-  {
-    ShortParams S;
-    S.rho = e->d_rho; S.K0 = e->d_K0; S.fdesc = e->d_fdesc; S.Qm = sl->d_Qm; S.mtab = e->d_mtab;
-    S.mdesc = e->d_mdesc; S.lfil = e->d_lfil; S.win = sl->d_win; S.shortw = sl->d_shortw;
-    S.surv = sl->d_surv; S.surv_count = sl->d_ctr + 1; S.cnt = cnt; S.surv_cap = sl->cap; S.M = e->M;
-    S.L = (u32)e->classes.size(); S.ldk = e->ldk; S.D = e->D; S.Dq = e->Dq; S.Wpad = e->Wpad; S.hdr = sl->d_hdr;
-    S.nm_cov = e->nm_cov; S.nm_all = e->nm_all; S.nl_cov = e->nl_cov; S.nl_all = e->nl_all;
-    k_mark_short<SHORT_BLOCK><<<(S.L + SHORT_LANES - 1) / SHORT_LANES, SHORT_BLOCK, short_smem(e), st>>>(S);
+  RowParams S = row_params(e, sl);
+  S.cnt = cnt;
+  if (nrow_copy) {
+    k_rows<<<e->sm_count * 4, 256, 0, st>>>(S);
     CU(cudaGetLastError());
+    ++launches;
+  }
+  if (segments) {
+    k_prep<<<e->sm_count * 4, 256, 0, st>>>(sl->d_hdr, sl->d_win, e->d_sdist, e->D, e->Dq, sl->d_Qm);
+    CU(cudaGetLastError());
+    ++launches;
+  }
+  CU(rec(7));
+  if (nrow_copy) {
+    k_mark_short<<<e->sm_count, ROW_THREADS, e->slice_rows * 4 * GROUP_WORDS + CAND_SMEM, st>>>(S);
+    CU(cudaGetLastError());
+    k_sift<<<e->sm_count, ROW_THREADS, ROW_SMEM, st>>>(S);
+    CU(cudaGetLastError());
+    launches += 2;
   }
   CU(rec(8));
-  const unsigned grid = persistent ? (unsigned)((u64)e->sm_count * e->mark_occupancy)
-                                   : (unsigned)std::max<u64>(1, std::min<u64>(items_hint, 0x7FFFFFFFull));
-  k_mark<MARK_BLOCK><<<grid, MARK_BLOCK, mark_smem(e), st>>>(P, persistent ? 1 : 0);
-  CU(cudaGetLastError());
+  if (segments) {
+    const unsigned grid = persistent ? (unsigned)((u64)e->sm_count * e->mark_occupancy)
+                                     : (unsigned)std::max<u64>(1, std::min<u64>(items_hint, 0x7FFFFFFFull));
+    k_mark<MARK_BLOCK><<<grid, MARK_BLOCK, mark_smem(e), st>>>(P, persistent ? 1 : 0);
+    CU(cudaGetLastError());
+    ++launches;
+  }
   CU(rec(1));
   k_mr<<<e->sm_count * ES_MR_BLOCKS_PER_SM, 256, 0, st>>>(T);
   CU(cudaGetLastError());
   k_mr2<<<e->sm_count * 2, 256, 0, st>>>(T);
   CU(cudaGetLastError());
+  launches += 2;
   CU(rec(2));
   return ES_OK;
 }
@@ -1376,7 +1564,7 @@ static es_status enqueue_tail(es_engine *e, Slot *sl, WinCount *cnt, bool captur
   k_direct<<<e->sm_count, 32, 0, st>>>(T);
   CU(cudaGetLastError());
   CU(rec(4));
-  CU(cudaMemcpyAsync(sl->h_ctr, sl->d_ctr, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+  CU(cudaMemcpyAsync(sl->h_ctr, sl->d_ctr, CTR_OUT * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
   CU(cudaMemcpyAsync(sl->h_status, sl->d_status, sizeof(u32), cudaMemcpyDeviceToHost, st));
   return ES_OK;
 }
@@ -1391,7 +1579,9 @@ static es_status capture_graph(es_engine *e, Slot *sl) {
   CU(cudaStreamBeginCapture(sl->stream, cudaStreamCaptureModeThreadLocal));
   es_status s = ES_OK;
   const cudaError_t m = cudaMemsetAsync(sl->d_cnt, 0, sl->win_cap * sizeof(WinCount), sl->stream);
-  if (m == cudaSuccess) s = enqueue_front(e, sl, true, sl->d_cnt, sl->win_cap, sl->shortw_cap, 0, true);
+  u64 launches = 2;                                // the tail's two kernels
+  if (m == cudaSuccess)
+    s = enqueue_front(e, sl, true, sl->d_cnt, sl->win_cap, sl->win_cap, !e->sched.long_split, 0, true, launches);
   cudaGraph_t g = nullptr;
   cudaError_t end = cudaStreamEndCapture(sl->stream, &g);
   if (m != cudaSuccess) return fail(e, ES_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(m));
@@ -1418,6 +1608,7 @@ static es_status capture_graph(es_engine *e, Slot *sl) {
   if (end != cudaSuccess) return fail(e, ES_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(end));
   sl->graph2 = g;
   CU(cudaGraphInstantiate(&sl->gexec2, g, 0));
+  sl->graph_launches = launches;
   return ES_OK;
 }
 
@@ -1472,23 +1663,24 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
       return fail(e, ES_ERR_RANGE, "LO must exceed max pmin of the filter table (" + std::to_string(floor_) + ")");
   }
   std::vector<WinDev> &wd = sl->hs.wd;
-  std::vector<ShortWin> &shortw = sl->hs.shortw;
-  const u64 total_items = describe(e, w, n, wd, shortw);
+  std::vector<RowWin> &roww = sl->hs.roww;
   std::vector<u64> &npos = sl->hs.npos;
-  npos.resize(n);
+  const RunShape shape = describe(e, w, n, wd, roww, npos);
   u64 positions_bound = 0;
-  for (size_t i = 0; i < n; ++i) positions_bound += (npos[i] = positions_in(e, w[i].lo, w[i].hi));
+  for (size_t i = 0; i < n; ++i) positions_bound += npos[i];
   size_t cap = (size_t)std::min<u64>(std::max<u64>(positions_bound / 64, 1 << 16), 1ull << 26);
   cap = std::max(cap, sl->cap);
+  // candidate chunks: half as many again as the estimate, and a part-filled one per warp and run
+  size_t chunks = (size_t)(1.5 * e->cand_rate * (double)positions_bound / 32) + 4 * (size_t)e->sm_count * (ROW_THREADS / 32);
   const bool persistent = schedule == ES_SCHED_PERSISTENT;
   std::vector<RecDev> &hr = sl->hs.hr;
   hr.clear();
   bool done = false;
   for (int attempt = 0; attempt < 4 && !done; ++attempt) {
-    es_status s = ensure_capacity(e, sl, n, cap);
+    es_status s = ensure_capacity(e, sl, n, shape.pieces, chunks, cap);
     if (s) return s;
     double mark_ms = 0, mr_ms = 0, rung_ms = 0, direct_ms = 0, prep_ms = 0, short_ms = 0, long_ms = 0;
-    u64 launches = 0, surv_max = 0, surv_total = 0, prime_total = 0;
+    u64 launches = 0, surv_max = 0, chunk_max = 0, prime_total = 0;
     u32 status = 0;
     hr.clear();
     size_t have_recs = 0;                 // records already on the host (the graph's prefix copy)
@@ -1499,7 +1691,8 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
       rung_ms += ev_ms(sl->ev[2], sl->ev[3]); direct_ms += ev_ms(sl->ev[3], sl->ev[4]);
       const unsigned long long *ctr = sl->h_ctr;
       surv_max = std::max<u64>(surv_max, ctr[1]);
-      surv_total += ctr[1]; prime_total += ctr[2];
+      chunk_max = std::max<u64>(chunk_max, ctr[10]);
+      prime_total += ctr[2];
       status |= *sl->h_status;
       if (ctr[1] > sl->cap) return ES_OK;
       const size_t nrec = (size_t)std::min<u64>(ctr[4], sl->cap);
@@ -1513,28 +1706,13 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
       return ES_OK;
     };
     if (persistent) {
-      sl->h_hdr->total_items = total_items;
+      sl->h_hdr->total_items = shape.items;
       sl->h_hdr->nwin = (u32)n;
-      sl->h_hdr->nshort = (u32)shortw.size();
+      sl->h_hdr->nshort = (u32)roww.size();
+      sl->h_hdr->nrows = (u32)shape.rows;
+      sl->h_hdr->npieces = (u32)shape.pieces;
       memcpy(sl->h_win, wd.data(), n * sizeof(WinDev));
-      if (!shortw.empty()) {
-        // largest first: the warps of a k_mark_short CTA deal the windows round robin, so the
-        // CTA's last window is a small one
-        // a counting sort on the work's binary order of magnitude (largest first, ties in
-        // input order) is all the balance needs
-        const size_t ns = shortw.size();
-        std::vector<uint8_t> &mag = sl->hs.mag;
-        mag.resize(ns);
-        u32 start[34] = {0};
-        for (size_t k = 0; k < ns; ++k) {
-          const ShortWin &x = shortw[k];
-          const u64 work = (u64)(x.lb - x.la) * (x.lq + 1);          // < 2^21
-          mag[k] = (uint8_t)(32 - __builtin_clz((u32)work | 1u));    // 1 .. 22
-          ++start[33 - mag[k]];
-        }
-        for (int b = 1; b < 34; ++b) start[b] += start[b - 1];
-        for (size_t k = 0; k < ns; ++k) sl->h_short[start[32 - mag[k]]++] = shortw[k];
-      }
+      if (!roww.empty()) memcpy(sl->h_roww, roww.data(), roww.size() * sizeof(RowWin));
       if (!sl->gexec || !sl->gexec2) { s = capture_graph(e, sl); if (s) return s; }
       setup_ms = ms_since(t_start);
       const auto t_launch = std::chrono::steady_clock::now();
@@ -1542,59 +1720,66 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
       if (s) return s;
       CU(cudaStreamSynchronize(sl->stream));
       device_ms = ms_since(t_launch);
-      launches = 7;
+      launches = sl->graph_launches;
       have_recs = sl->rec_prefix;
       s = collect();
       if (s) return s;
     } else {
       // The plain schedule: the same kernels, one launch sequence per window.
       CU(cudaMemsetAsync(sl->d_cnt, 0, n * sizeof(WinCount), sl->stream));
-      size_t k = 0;                      // next short-window entry (describe emits them in order)
+      size_t k = 0;                      // next window marked by rows (describe emits them in order)
       for (size_t i = 0; i < n; ++i) {
         sl->h_win[0] = wd[i];
         sl->h_win[0].item0 = 0;
         const u64 items = (u64)wd[i].nseg * wd[i].groups;
-        u32 nshort = 0;
-        if (k < shortw.size() && shortw[k].wi == i) { sl->h_short[0] = shortw[k++]; sl->h_short[0].wi = 0; nshort = 1; }
-        sl->h_hdr->total_items = items; sl->h_hdr->nwin = 1; sl->h_hdr->nshort = nshort;
-        s = enqueue_front(e, sl, false, sl->d_cnt + i, 1, nshort, items, false);
+        BatchHdr &h = *sl->h_hdr;
+        h.total_items = items; h.nwin = 1; h.nshort = h.nrows = h.npieces = 0;
+        if (k < roww.size() && roww[k].wi == i) {
+          RowWin &x = sl->h_roww[0];
+          x = roww[k++];
+          x.wi = x.row0 = x.piece0 = 0;
+          h.nshort = 1; h.nrows = x.nrows; h.npieces = (x.nrows + PIECE_ROWS - 1) / PIECE_ROWS;
+        }
+        s = enqueue_front(e, sl, false, sl->d_cnt + i, 1, h.nshort, items != 0, items, false, launches);
         if (s) return s;
         s = enqueue_tail(e, sl, sl->d_cnt + i, false);
         if (s) return s;
         CU(cudaStreamSynchronize(sl->stream));
-        launches += 7;
+        launches += 2;
         const size_t base = hr.size();
         s = collect();
         if (s) return s;
-        if (surv_max > sl->cap) break;
+        if (surv_max > sl->cap || chunk_max > sl->chunk_cap) break;
         for (size_t r = base; r < hr.size(); ++r) hr[r].win = (u32)i;
       }
       CU(cudaMemcpyAsync(sl->h_cnt, sl->d_cnt, n * sizeof(WinCount), cudaMemcpyDeviceToHost, sl->stream));
       CU(cudaStreamSynchronize(sl->stream));
     }
-    if (surv_max > sl->cap) {            // overflow: grow to the exact need and re-run
-      cap = (size_t)(surv_max + surv_max / 4 + 1024);
+    if (surv_max > sl->cap || chunk_max > sl->chunk_cap) {   // overflow: grow to the exact need and re-run
+      if (surv_max > sl->cap) cap = (size_t)(surv_max + surv_max / 4 + 1024);
+      if (chunk_max > sl->chunk_cap) chunks = (size_t)(chunk_max + chunk_max / 4);
       continue;
     }
     if (status) return fail(e, ES_ERR_DEVICE_STATUS, "device status:" + status_text(status));
     sl->timing.total_ms = mark_ms + mr_ms + rung_ms + direct_ms;   // kernels only, inputs resident
     sl->timing.mark_ms = mark_ms; sl->timing.mr_ms = mr_ms;
     sl->timing.prep_ms = prep_ms; sl->timing.mark_short_ms = short_ms; sl->timing.mark_long_ms = long_ms;
-    sl->timing.short_pairs = (u64)shortw.size() * e->classes.size();
-    sl->timing.mask_bytes = shortw.empty() ? 0 : (u64)e->classes.size() * e->Wpad * 8;
+    sl->timing.short_pairs = (u64)roww.size() * e->classes.size();
+    sl->timing.mask_bytes = roww.empty() ? 0 : (u64)e->ngroups * e->slice_rows * 4 * GROUP_WORDS;
     sl->timing.rung_ms = rung_ms; sl->timing.direct_ms = direct_ms;
     sl->timing.marks_kernel_launches = persistent ? 1 : n;
     sl->timing.kernel_launches = launches;
-    sl->timing.mark_items = total_items;
-    sl->timing.survivors = surv_total;
+    sl->timing.mark_items = shape.items;
     sl->timing.primes = prime_total;
     done = true;
   }
   if (!done) return fail(e, ES_ERR_NOMEM, "survivor list kept overflowing");
+  sl->timing.survivors = 0;
   for (size_t i = 0; i < n; ++i) {      // the SUMMARY counters (sieve/rung_scan3.cpp:764-772)
     const WinCount &c = sl->h_cnt[i];
     es_counters &o = per_window[i];
     o.positions = npos[i];
+    sl->timing.survivors += c.surv;
     if (e->nf == e->ncov) { o.covered = o.positions - c.surv; o.sieved = 0; }
     else { o.covered = o.positions - c.after_covers; o.sieved = c.after_covers - c.surv; }
     // every prime survivor ends as a rung record, a direct one or an unsolved one, so the
@@ -1632,58 +1817,56 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
   return ES_OK;
 }
 
-// Windows whose lanes hold more than short_max positions are, by default, cut into
-// sub-windows of short_max positions per lane (short_max * M integers; the last one
-// shorter), which the short-window kernel marks with its early exit; with long_split = 0
-// they keep one device window each and go to the segment marking. Sub-window t of a window
-// starts t * short_max positions into every lane, so its records map back to the window by
-// J += t * short_max, and its counters add up to the window's (every counter is a sum over
-// positions). Device windows are run in passes of at most PASS_WINDOWS. Every caller passes
-// per_window zeroed.
-constexpr size_t PASS_WINDOWS = 1u << 18;
-
+// Runs windows in passes of at most e->pass_rows rows. A window
+// that does not fit the pass is cut at whole multiples of M: a part that starts t M
+// integers into the window starts t positions into every lane, so its records map back by J += t,
+// and its counters add up to the window's (every counter is a sum over positions). Every caller
+// passes per_window zeroed.
 static es_status run_windows(es_engine *e, Slot *sl, const es_window *w, size_t n, int schedule,
                              es_counters *per_window, es_records *recs) {
   const u64 M = e->M, S = e->sched.short_max;
   const u64 floor_ = std::max(e->wheel_pmin, e->cover_pmax);
-  bool split = false;
+  u64 rows = 0;
+  // rows of [lo, hi), at most; 0 for a window that goes to the segment marking
+  auto rows_of = [&](u64 lo, u64 hi) -> u64 {
+    const u64 len = hi > lo ? hi - lo : 0;
+    return e->sched.long_split || len <= S * M ? len / M + 2 : 0;
+  };
   for (size_t i = 0; i < n; ++i) {                 // refuse what a run would refuse, first
     if (w[i].hi > DIRECT_PMAX)
       return fail(e, ES_ERR_RANGE, "HI must not exceed the stage-E ceiling " + std::to_string(DIRECT_PMAX));
     if (w[i].lo <= floor_)
       return fail(e, ES_ERR_RANGE, "LO must exceed max pmin of the filter table (" + std::to_string(floor_) + ")");
-    const u64 len = w[i].hi > w[i].lo ? w[i].hi - w[i].lo : 0;
-    // more than S positions per lane; the plain schedule keeps one launch sequence per window
-    if (e->sched.long_split && schedule == ES_SCHED_PERSISTENT && len > S * M) split = true;
+    rows += rows_of(w[i].lo, w[i].hi);
   }
-  if (!split) return run_device_windows(e, sl, w, n, schedule, per_window, recs);
+  if (rows <= e->pass_rows) return run_device_windows(e, sl, w, n, schedule, per_window, recs);
   std::vector<es_record> &all = sl->hs.all;
   all.clear();
   es_timing_t tot{};
   std::vector<es_window> &dw = sl->hs.dw;
   std::vector<std::pair<u32, u64>> &dmap = sl->hs.dmap;   // (window, position offset) per device window
   std::vector<es_counters> &pc = sl->hs.pc;
-  dw.reserve(PASS_WINDOWS);
-  dmap.reserve(PASS_WINDOWS);
-  // device windows are produced a pass at a time: (i, t) is the next sub-window to emit
   size_t i = 0;
-  u64 t = 0;
+  u64 t = 0;                                         // window i is done up to t M integers
   while (i < n) {
     dw.clear();
     dmap.clear();
-    while (i < n && dw.size() < PASS_WINDOWS) {
-      const u64 lo = w[i].lo, hi = std::max(w[i].lo, w[i].hi);
-      const u64 len = hi - lo;
-      if (!e->sched.long_split || len <= S * M) {
+    for (u64 left = e->pass_rows; i < n;) {
+      const u64 lo = w[i].lo + t * M, hi = std::max(w[i].lo, w[i].hi), need = rows_of(lo, hi);
+      if (need <= left) {
         dw.push_back({lo, hi});
-        dmap.push_back({(u32)i, 0});
+        dmap.push_back({(u32)i, t});
+        left -= need;
         ++i;
+        t = 0;
         continue;
       }
-      const u64 step = S * M, a = lo + t * step;  // t * step < len: no overflow
-      dw.push_back({a, a + std::min(step, hi - a)});
-      dmap.push_back({(u32)i, t * S});
-      if (hi - a <= step) { ++i; t = 0; } else ++t;
+      if (e->sched.long_split && left > 2) {         // need > left: (left - 2) M is below hi - lo
+        dw.push_back({lo, lo + (left - 2) * M});
+        dmap.push_back({(u32)i, t});
+        t += left - 2;
+      }
+      break;
     }
     const size_t m = dw.size();
     pc.resize(m);
@@ -1797,7 +1980,7 @@ static es_status build_tables(es_engine *e) {
   }
   // temporaries of the table build, freed on every return path
   struct Temps {
-    void *p[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    void *p[6] = {};
     ~Temps() { for (void *x : p) cudaFree(x); }
   } temps;
   u64 *d_mods = nullptr, *d_ress = nullptr;
@@ -1841,15 +2024,14 @@ static es_status build_tables(es_engine *e) {
   k_build_k0<<<(unsigned)((total + 255) / 256), 256, 0, bs>>>(e->d_rho, L, d_mods, d_ress, d_g, d_inv,
                                                               e->d_fdesc, (u32)nf, e->ldk, e->d_K0);
   CU(cudaGetLastError());
-  // Kill masks for short windows: within each phase (covers, then stage-B' primes), the
-  // smallest strides get a mask while the per-lane table fits MASK_BYTES_MAX; the filters of
-  // the remaining strides are checked one by one from the first-hit table. The masked strides
-  // are then ordered by how many positions they kill -- the sum over lanes and filters of
-  // 1/s where the filter hits the lane (rho == res mod g) -- so that k_mark_short, which stops
-  // once a segment is dead, meets the densest strides first. Kills are ORed, so the order
+  // The strides that get rows: within each phase (covers, then stage-B' primes) the smallest,
+  // while their rows fit the budget; the filters of the remaining strides are checked one by one
+  // from the first-hit table. The strides are then ordered by how many positions they kill -- the
+  // sum over lanes and filters of 1/s where the filter hits the lane (rho == res mod g) -- and the
+  // densest covers whose rows fit a slice become the dense strides. Kills are ORed, so the order
   // cannot change a result.
   {
-    std::vector<MaskDesc> md;
+    std::vector<u32> ms;                               // strides with rows, in marking order
     std::vector<int> fmask(nf, -1);
     std::vector<u32> lfil_cov, lfil_siv;
     std::map<u32, std::unordered_map<u32, u32>> lanes_mod;     // g -> (rho mod g -> lanes)
@@ -1864,79 +2046,108 @@ static es_status build_tables(es_engine *e) {
       const auto it = h.find((u32)(orr[k] % og[k]));
       if (it != h.end()) kills[fdesc[k] & 0xFFFFu] += (double)it->second / (double)(fdesc[k] & 0xFFFFu);
     }
-    u32 words = 0;
+    u64 bits = 0;
+    u32 dense_rows = PIECE_ROWS;                       // the padding's rows
     for (int phase = 0; phase < 2; ++phase) {
       const size_t f0 = phase ? e->ncov : 0, f1 = phase ? nf : e->ncov;
       std::vector<u32> strides;
       for (size_t k = f0; k < f1; ++k) strides.push_back(fdesc[k] & 0xFFFFu);
       std::sort(strides.begin(), strides.end());
       strides.erase(std::unique(strides.begin(), strides.end()), strides.end());
-      std::vector<int> slot_of(65536, -1);
-      const size_t m_first = md.size();
+      const size_t m_first = ms.size();
       for (u32 st : strides) {
-        // bits [0, s + SEG_SMALL) plus one spare word: a segment of up to SEG_SMALL positions
-        // starting at any residue below s reads words r/32 .. r/32 + SEG_SMALL/32 of the slice
-        const u32 wd = (st + SEG_SMALL + 31) / 32 + 1;
-        if ((size_t)(words + wd) * 4 > MASK_BYTES_MAX || md.size() >= SMD_MAX) break;
-        const u32 di = (u32)(std::lower_bound(sd.begin(), sd.end(), st) - sd.begin());
-        md.push_back(MaskDesc{st, di, words, 0});
-        words += wd;
+        if (bits + st > 8ull * MASK_BYTES_MAX || ms.size() >= STRIDES_MAX) break;
+        ms.push_back(st);
+        bits += st;
       }
-      std::stable_sort(md.begin() + m_first, md.end(),
-                       [&](const MaskDesc &x, const MaskDesc &y) { return kills[x.s] > kills[y.s]; });
-      for (size_t m = m_first; m < md.size(); ++m) slot_of[md[m].s] = (int)m;
+      std::stable_sort(ms.begin() + m_first, ms.end(), [&](u32 x, u32 y) { return kills[x] > kills[y]; });
+      if (phase == 0) {
+        std::vector<u32> dense, rest;
+        for (u32 st : ms) {
+          const u32 need = st + PIECE_ROWS - 1;
+          const bool fits = dense.size() < DENSE_MAX && dense_rows + need <= SLICE_ROWS_MAX;
+          (fits ? dense : rest).push_back(st);
+          if (fits) dense_rows += need;
+        }
+        e->n1 = (u32)dense.size();
+        ms = dense;
+        ms.insert(ms.end(), rest.begin(), rest.end());
+        e->nm_cov = (u32)ms.size();
+      }
+      std::vector<int> slot_of(65536, -1);
+      for (size_t m = m_first; m < ms.size(); ++m) slot_of[ms[m]] = (int)m;
       for (size_t k = f0; k < f1; ++k) {
         const int m = slot_of[fdesc[k] & 0xFFFFu];
         fmask[k] = m;
         if (m < 0) (phase ? lfil_siv : lfil_cov).push_back((u32)k);
       }
-      if (phase == 0) e->nm_cov = (u32)md.size();
     }
-    e->nm_all = (u32)md.size();
-    // Final layout: the first INTERLEAVE_ROUNDS rounds of the covers' phase interleaved (each
-    // group of 32 slices padded to its longest), the rest packed; if that no longer fits the
-    // per-lane budget, fewer rounds are interleaved (the layout cannot change a result).
-    for (u32 rounds = std::min<u32>(INTERLEAVE_ROUNDS, e->nm_cov / 32);; --rounds) {
-      const u32 m_inter = 32 * rounds;
-      u32 w2 = 0;
-      for (u32 g = 0; g < rounds; ++g) {
-        u32 maxwd = 0;
-        for (u32 j = 0; j < 32; ++j) maxwd = std::max(maxwd, (md[32 * g + j].s + SEG_SMALL + 31) / 32 + 1);
-        for (u32 j = 0; j < 32; ++j) { md[32 * g + j].off = w2 + j; md[32 * g + j].sh = 5; }
-        w2 += 32 * maxwd;
+    e->nm_all = (u32)ms.size();
+    e->n1p = (e->n1 + 7) & ~7u;
+    e->slice_rows = (dense_rows + 7) & ~7u;            // a slice is whole 128-byte lines
+    e->ngroups = (L + GROUP_LANES - 1) / GROUP_LANES;
+    e->cand_rate = 1.0;
+    for (u32 m = 0; m < e->n1; ++m) e->cand_rate *= std::max(0.0, 1.0 - kills[ms[m]] / L);
+    // a pass of 2^23 full rows holds 60 MB of rows and pieces and, with the tables for wheel 2042040,
+    // up to 450 MB of candidates; tables that leave more candidates take shorter passes
+    e->pass_rows = (u64)std::min(8388608.0, std::max(4096.0, 32.0 * 2097152.0 / (1.5 * e->cand_rate * L + 1e-9)));
+    std::vector<uint4> md(e->n1p + e->nm_all - e->n1);
+    auto desc = [](u32 st, u32 at) { return make_uint4(st, 0xFFFFFFFFu / st, (u32)((1ull << 32) % st), at); };
+    u32 row = PIECE_ROWS, word = 0;
+    for (u32 m = 0; m < e->n1; ++m) { md[m] = desc(ms[m], row); row += ms[m] + PIECE_ROWS - 1; }
+    for (u32 m = e->n1; m < e->n1p; ++m) md[m] = desc(1, 0);
+    e->n2 = e->nm_all;
+    for (u32 m = e->n1; m < e->nm_all; ++m) {
+      const u32 wd = (ms[m] + 31) / 32;
+      if (e->n2 == e->nm_all && ((word + wd + 3) & ~3u) > SIFT_WORDS_MAX) {   // k_sift's copy ends here
+        e->n2 = m;
+        word = (word + 3) & ~3u;
       }
-      for (size_t m = m_inter; m < md.size(); ++m) {
-        md[m].off = w2;
-        md[m].sh = 0;
-        w2 += (md[m].s + SEG_SMALL + 31) / 32 + 1;
-      }
-      if ((size_t)w2 * 4 <= MASK_BYTES_MAX || rounds == 0) { words = w2; e->m_inter = m_inter; break; }
+      md[e->n1p - e->n1 + m] = desc(ms[m], word);
+      word += wd;
     }
+    e->lane_words = std::max(4u, (word + 3) & ~3u);
     e->nl_cov = (u32)lfil_cov.size();
     e->nl_all = (u32)(lfil_cov.size() + lfil_siv.size());
-    e->Wpad = std::max<u32>(2, ((words + 1) / 2 + 1) & ~1u);   // in 64-bit words, even
     std::vector<u32> lfil(lfil_cov);
     lfil.insert(lfil.end(), lfil_siv.begin(), lfil_siv.end());
     int *d_fmask = nullptr;
-    CU(cudaMalloc(&e->d_mtab, (size_t)L * e->Wpad * sizeof(u64)));
-    CU(cudaMalloc(&e->d_mdesc, std::max<size_t>(md.size(), 1) * sizeof(MaskDesc)));
+    const size_t dense_bytes = (size_t)e->ngroups * e->slice_rows * 4 * GROUP_WORDS;
+    const size_t lane_bytes = (size_t)L * e->lane_words * sizeof(u32);
+    CU(cudaMalloc(&e->d_tdense, dense_bytes));
+    CU(cudaMalloc(&e->d_tlane, lane_bytes));
+    CU(cudaMalloc(&e->d_mdesc, std::max<size_t>(md.size(), 1) * sizeof(uint4)));
     CU(cudaMalloc(&e->d_lfil, std::max<size_t>(lfil.size(), 1) * sizeof(u32)));
     CU(cudaMalloc(&d_fmask, std::max<size_t>(nf, 1) * sizeof(int)));
     temps.p[4] = d_fmask;
-    CU(cudaMemsetAsync(e->d_mtab, 0, (size_t)L * e->Wpad * sizeof(u64), bs));
-    if (!md.empty()) CU(cudaMemcpyAsync(e->d_mdesc, md.data(), md.size() * sizeof(MaskDesc), cudaMemcpyHostToDevice, bs));
+    CU(cudaMemsetAsync(e->d_tdense, 0, dense_bytes, bs));
+    CU(cudaMemsetAsync(e->d_tlane, 0, lane_bytes, bs));
+    if (!md.empty()) CU(cudaMemcpyAsync(e->d_mdesc, md.data(), md.size() * sizeof(uint4), cudaMemcpyHostToDevice, bs));
     if (!lfil.empty()) CU(cudaMemcpyAsync(e->d_lfil, lfil.data(), lfil.size() * sizeof(u32), cudaMemcpyHostToDevice, bs));
     if (nf) CU(cudaMemcpyAsync(d_fmask, fmask.data(), nf * sizeof(int), cudaMemcpyHostToDevice, bs));
-    if (nf && !md.empty()) {
+    if (nf && e->nm_all) {
       const u64 tt = (u64)L * nf;
-      k_build_masks<<<(unsigned)((tt + 255) / 256), 256, 0, e->slots[0].stream>>>(e->d_K0, L, e->ldk, (u32)nf, d_fmask,
-                                                                         e->d_mdesc, e->Wpad, e->d_mtab);
+      k_build_rows<<<(unsigned)((tt + 255) / 256), 256, 0, bs>>>(e->d_K0, L, e->ldk, (u32)nf, d_fmask, e->d_mdesc, e->n1,
+                                                                 e->n1p, e->slice_rows, e->lane_words,
+                                                                 (u32 *)e->d_tdense, e->d_tlane);
       CU(cudaGetLastError());
     }
+    // Stage B' primes kill squares by their own rule, and moduli past 2^16 are not searched.
+    unsigned long long hit = 1;
+    if (nf && nf == e->ncov && *std::max_element(om.begin(), om.end()) <= 65536) {
+      CU(cudaMalloc(&temps.p[5], sizeof hit));
+      CU(cudaMemsetAsync(temps.p[5], 0, sizeof hit, bs));
+      k_square_mask<<<(unsigned)std::min<size_t>(nf, 65535), 128, 0, bs>>>(d_mods, d_ress, (u32)nf,
+                                                                          (unsigned long long *)temps.p[5]);
+      CU(cudaGetLastError());
+      CU(cudaMemcpyAsync(&hit, temps.p[5], sizeof hit, cudaMemcpyDeviceToHost, bs));
+    }
     CU(cudaStreamSynchronize(bs));
-    CU(cudaFuncSetAttribute(k_mark_short<SHORT_BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)(SHORT_LANES * (MASK_BYTES_MAX + 16) + SMD_MAX * sizeof(MaskDesc) +
-                                  SHORT_HAND_BYTES)));
+    e->squares = !(hit & 1);
+    for (u32 q = 3; q < 64; ++q)
+      if (hit >> q & 1) e->sq.push_back(q);
+    CU(cudaFuncSetAttribute(k_mark_short, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ROW_SMEM));
+    CU(cudaFuncSetAttribute(k_sift, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ROW_SMEM));
   }
   CU(cudaStreamSynchronize(e->slots[0].stream));
   // occupancy of the marking kernel, for the persistent grid
@@ -1975,7 +2186,7 @@ static u64 request_bytes(const es_engine *e, const es_window *w, size_t n) {
   u64 pos = 0;
   for (size_t i = 0; i < n; ++i) pos += positions_in(e, w[i].lo, w[i].hi);
   const u64 surv = std::min<u64>(std::max<u64>(pos / 64, 1024), 1ull << 26);
-  return n * (sizeof(WinDev) + sizeof(ShortWin) + sizeof(WinCount) + 2ull * e->Dq) +
+  return n * (sizeof(WinDev) + sizeof(RowWin) + sizeof(WinCount) + 2ull * e->Dq) +
          surv * (sizeof(Surv) + 3 * sizeof(u32) + sizeof(RecDev));
 }
 
@@ -2227,17 +2438,18 @@ es_status es_close(es_engine *e) {
   for (Slot &sl : e->slots) {
     if (sl.stream) cudaStreamSynchronize(sl.stream);
     drop_graph(&sl);
-    cudaFree(sl.d_win); cudaFree(sl.d_cnt); cudaFree(sl.d_shortw); cudaFree(sl.d_Qm);
+    cudaFree(sl.d_win); cudaFree(sl.d_cnt); cudaFree(sl.d_roww); cudaFree(sl.d_Qm);
+    cudaFree(sl.d_piece); cudaFree(sl.d_pidx); cudaFree(sl.d_rowinfo); cudaFree(sl.d_cand2); cudaFree(sl.d_chunk);
     cudaFree(sl.d_surv); cudaFree(sl.d_primes); cudaFree(sl.d_direct); cudaFree(sl.d_recs); cudaFree(sl.d_cand);
     cudaFree(sl.d_ctr); cudaFree(sl.d_status); cudaFree(sl.d_hdr);
-    cudaFreeHost(sl.h_hdr); cudaFreeHost(sl.h_win); cudaFreeHost(sl.h_short); cudaFreeHost(sl.h_cnt);
+    cudaFreeHost(sl.h_hdr); cudaFreeHost(sl.h_win); cudaFreeHost(sl.h_roww); cudaFreeHost(sl.h_cnt);
     cudaFreeHost(sl.h_ctr); cudaFreeHost(sl.h_status); cudaFreeHost(sl.h_recs);
     for (auto &ev : sl.ev) if (ev) cudaEventDestroy(ev);
     if (sl.stream) cudaStreamDestroy(sl.stream);
   }
   cudaFree(e->d_rho); cudaFree(e->d_fdesc); cudaFree(e->d_sdist); cudaFree(e->d_tdp);
   cudaFree(e->d_K0); cudaFree(e->d_tde); cudaFree(e->d_tdi); cudaFree(e->d_tdqm);
-  cudaFree(e->d_mtab); cudaFree(e->d_mdesc); cudaFree(e->d_lfil);
+  cudaFree(e->d_tdense); cudaFree(e->d_tlane); cudaFree(e->d_mdesc); cudaFree(e->d_lfil);
   delete e;
   return ES_OK;
 }

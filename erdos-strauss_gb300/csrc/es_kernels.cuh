@@ -10,16 +10,11 @@ constexpr int DMAX = 8192;          // distinct strides held in shared memory pe
 
 // One scan window as the device sees it. Lane l's positions are p = rho_l + M*K for
 // K = Kfirst .. Kfirst + npos - 1, with Kfirst = Q + (rho_l < lo mod M). Segment-marking
-// items (k_mark) are (lane, segment) pairs with segments of SEG_BIG positions. Windows with
-// at most SEG_SMALL positions per lane (and sub-windows of that size cut from longer ones)
-// go to the kill-mask kernel instead; SEG_SMALL is the length of the mask repeat. 128
-// measured best over the 4096-window batch and 10^14-integer windows together (64: 2% faster
-// on the batch, 20% slower on long windows; 256: 6% slower on the batch).
+// items (k_mark) are (lane, segment) pairs with segments of SEG_BIG positions; they take the
+// windows that are not marked by rows (k_mark_short): with es_schedule.long_split = 0, those with
+// more than short_max (at most SEG_SMALL) positions in a lane.
 constexpr u32 GROUP = 16;
-#ifndef ES_SEG_SMALL
-#define ES_SEG_SMALL 128
-#endif
-constexpr u32 SEG_SMALL = ES_SEG_SMALL;
+constexpr u32 SEG_SMALL = 128;
 constexpr u32 SEG_BIG = 16384;
 
 struct WinDev {
@@ -38,7 +33,8 @@ struct WinDev {
 // captured launch sequence (a CUDA graph) serves every batch up to the buffers' capacity.
 struct BatchHdr {
   u64 total_items;   // long-window marking items
-  u32 nwin, nshort;  // windows; short windows
+  u32 nwin, nshort;  // windows; windows marked by rows
+  u32 nrows, npieces;
 };
 
 // A position that no filter killed: (window, lane, J) is its key in the output order.
@@ -79,49 +75,71 @@ struct MarkParams {
   u32 r_bytes;             // shared bytes for the stride residues (16-aligned)
 };
 
-// Short windows (at most SEG_SMALL positions in any lane) are marked from per-(lane, stride)
-// kill masks: for lane l and a stride s shared by several filters, bit x of the mask is set
-// when some filter of that stride kills K == x (mod s); bits [s, s + SEG_SMALL) repeat the
-// pattern so that the positions of a whole segment starting below s are consecutive bits,
-// read 32 at a time as funnel shifts of consecutive words.
-constexpr u32 MASK_BYTES_MAX = 48 * 1024;   // per-lane mask table budget (shared memory)
-
-// One masked stride: s, its index in sdist, the 32-bit word offset of its slice in a lane's
-// table, and the log2 of the distance between the slice's consecutive words. The strides of
-// the first INTERLEAVE_ROUNDS rounds of 32 (the densest, which every short window walks) are
-// stored interleaved -- word w of the stride in slot 32g + j at off = base_g + j, w at
-// off + 32 w, sh = 5 -- so that lane j of a warp reading any word of its own stride reads
-// shared-memory bank j; the other strides are packed one after another (sh = 0).
-struct MaskDesc { u32 s, d, off, sh; };
-#ifndef ES_INTERLEAVE_ROUNDS
-#define ES_INTERLEAVE_ROUNDS 2
+// Marking by rows (k_mark_short). A row is one K of one window: the positions rho_l + M K of all
+// lanes l in [la, lb); a piece is at most PIECE_ROWS consecutive rows of one window.
+constexpr u32 MASK_BYTES_MAX = 48 * 1024;   // stride table budget per lane (strides past it are not tabled)
+constexpr u32 STRIDES_MAX = 512;            // strides with tables, at most
+constexpr u32 PIECE_ROWS = 32;
+constexpr u32 GROUP_WORDS = 4;              // 32-bit words of a dense row
+constexpr u32 GROUP_LANES = 32 * GROUP_WORDS;
+constexpr u32 ROW_THREADS = 1024;           // threads of k_mark_short and k_sift, one CTA of each per SM
+#ifndef ES_DENSE_MAX
+#define ES_DENSE_MAX 48
 #endif
-constexpr u32 INTERLEAVE_ROUNDS = ES_INTERLEAVE_ROUNDS;
+constexpr u32 DENSE_MAX = ES_DENSE_MAX;     // dense strides, at most
+constexpr u32 BULK_COPY = 16384;            // bytes per bulk copy into shared memory
+// Shared memory of a CTA (the rest of the 227 KB an SM can give one is static): per warp 64
+// candidates of 8 bytes (k_sift: twice); k_mark_short's group slice, or k_sift's stride descriptors
+// and lane tables.
+constexpr u32 ROW_SMEM = 226 * 1024;
+constexpr u32 CAND_SMEM = ROW_THREADS / 32 * 64 * 8;
+constexpr u32 SLICE_ROWS_MAX = (ROW_SMEM - CAND_SMEM) / (4 * GROUP_WORDS);
+constexpr u32 SIFT_LANES = 8;               // lanes whose tables k_sift holds at a time
+constexpr u32 SIFT_WORDS_MAX = (ROW_SMEM - 2 * CAND_SMEM - STRIDES_MAX * 16) / (4 * SIFT_LANES);
+static_assert(SLICE_ROWS_MAX < 65536, "slice rows are 16-bit indices");
 
-// A short window as k_mark_short walks it: lanes outside [la, lb) have no position in it.
-// Lane rho holds lq + [(rho - lo) mod M < lr] positions, lq = len / M, lr = len mod M (the
-// count of p == rho (mod M) in [lo, lo + len)).
-struct ShortWin {
-  u64 Q;
-  u32 lomod, wi, la, lb, lq, lr;
+// A window marked by rows: K0, K0 + 1, .. K0 + nrows - 1, the first from lane la on, the last up
+// to lane lb; row0 and piece0 count the rows and pieces of the windows before it.
+struct RowWin {
+  u64 K0;
+  u32 wi, row0, piece0, nrows, la, lb;
 };
+struct __align__(16) Piece {
+  u64 K0;
+  u32 row0, win, n, la, lb, pad;
+};
+// rowinfo: the row's piece and its place in it, and whether the row is cut (la, lb)
+constexpr u32 ROW_CUT = 1u << 31, ROW_NONE = ~0u;
 
-struct ShortParams {
+struct RowParams {
   const u32 *rho;
   const u16 *K0;
   const u32 *fdesc;
-  const u16 *Qm;            // [nwin][Dq]
-  const u64 *mtab;          // [L][Wpad] kill masks
-  const MaskDesc *mdesc;    // covers' mask strides [0, nm_cov), then stage B' [nm_cov, nm_all)
-  const u32 *lfil;          // filters not covered by a mask: covers [0, nl_cov), then B' [nl_cov, nl_all)
+  const unsigned char *tdense;   // [ngroups][slice_bytes]: row x of dense stride m at mdesc[m].w + x
+  const u32 *tlane;         // [L][lane_words]: bit x of another stride at mdesc.w + x / 32
+  const uint4 *mdesc;       // {s, floor((2^32 - 1) / s), 2^32 mod s, first row or word}: n1 dense
+                            // strides padded to n1p with rows that hold no bit, then the covers'
+                            // others up to nm_cov and stage B''s up to nm_all
+  const u32 *lfil;          // filters of strides without tables: covers [0, nl_cov), then B' [nl_cov, nl_all)
   const WinDev *win;
-  const ShortWin *shortw;   // the short windows
+  const RowWin *roww;       // [hdr->nshort]
+  Piece *piece;             // [hdr->npieces]
+  u16 *pidx;                // [npieces][n1p] slice row of the piece's first K per dense stride
+  u32 *rowinfo;             // [nrows]
+  uint2 *cand;              // [chunk_cap][32] positions the dense strides left: piece, place * GROUP_LANES + lane
+  u32 *chunk;               // [chunk_cap] group << 8 | candidates
+  unsigned long long *chunk_count;
   Surv *surv;
   unsigned long long *surv_count;
   WinCount *cnt;
   u64 surv_cap, M;
-  const BatchHdr *hdr;      // nshort
-  u32 L, ldk, D, Dq, Wpad, nm_cov, nm_all, nl_cov, nl_all;
+  const BatchHdr *hdr;
+  u32 *status;
+  bool wide;                // K may reach 2^48
+  bool squares;             // n^2 passes every cover when n is prime to the nsq primes with these inverses
+  u32 nsq, sq_inv[18], sq_lim[18];   // mod 2^32 and quotients of 2^32 - 1 (odd primes below 64)
+  u32 L, ldk, ngroups, slice_bytes, lane_words, chunk_cap;
+  u32 n1, n1p, n2, nm_cov, nm_all, nl_cov, nl_all;   // the first words of strides [n1, n2) fit SIFT_WORDS_MAX
 };
 
 struct HardSlot;

@@ -111,7 +111,7 @@ typedef struct {
   uint64_t n_certified;     /* ncov */
   uint64_t n_filters;       /* certified + stage-B' primes */
   uint64_t mmax;
-  uint64_t short_max_limit; /* largest es_schedule.short_max (the kill-mask repeat, positions) */
+  uint64_t short_max_limit; /* largest es_schedule.short_max (positions) */
   int pinned;               /* 1 if M has a pinned class-table digest */
   char classes_sha256[72];  /* the pin, or "unpinned" */
 } es_info_t;
@@ -120,11 +120,13 @@ typedef struct {
  * total_ms is the sum of the stages (kernels only: no host<->device copies). */
 typedef struct {
   double total_ms, mark_ms, mr_ms, rung_ms, direct_ms;
-  double prep_ms, mark_short_ms, mark_long_ms;   /* the three parts of mark_ms */
+  double prep_ms, mark_short_ms, mark_long_ms;   /* the three parts of mark_ms:
+                                                     rows and residues, marking by rows (k_mark_short
+                                                     and k_sift), segment marking */
   uint64_t marks_kernel_launches, kernel_launches;
   uint64_t mark_items, survivors, primes;
-  uint64_t short_pairs;     /* (lane, short window) pairs, active or not, walked by k_mark_short */
-  uint64_t mask_bytes;      /* kill-mask table bytes one k_mark_short launch reads */
+  uint64_t short_pairs;     /* (lane, window) pairs of the windows marked by rows */
+  uint64_t mask_bytes;      /* dense stride table bytes one k_mark_short launch reads */
   /* host wall time of the call: describing and staging the windows, from the launch to the
    * end of the device work (copies included), and collecting counters and records; and the
    * whole es_run_batch / es_run_window call inside the library (with the long-window split,
@@ -199,13 +201,12 @@ size_t es_format_summary(const es_engine *engine, uint64_t lo, uint64_t hi, cons
  * records; only the time differs. No reference counterpart (the reference's CPU loop has
  * nothing to schedule). */
 typedef struct {
-  uint32_t short_max;            /* windows whose lanes hold at most this many positions
-                                    (1..es_info_t.short_max_limit, 128 in this build) go to the
-                                    short-window kernel as they are; default the limit */
+  uint32_t short_max;            /* with long_split = 0, windows whose lanes hold at most this many
+                                    positions (1..es_info_t.short_max_limit, 128 in this build) are
+                                    marked by rows; default the limit */
   uint32_t rung_blocks_per_sm;   /* stage-D grid in blocks per SM (1..16); default 6 */
-  uint32_t long_split;           /* 1 (default): longer windows are cut into sub-windows of
-                                    short_max positions per lane for the short-window kernel;
-                                    0: they go to the segment marking */
+  uint32_t long_split;           /* 1 (default): every window is marked by rows, long ones in
+                                    passes; 0: longer windows go to the segment marking */
   uint32_t reserved[5];          /* zero */
 } es_schedule;
 
