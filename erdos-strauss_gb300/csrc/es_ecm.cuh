@@ -9,16 +9,13 @@
 // curve with B1 = 40 and B2 = 1200 costs about 1.25 K multiplies and splits a 31-bit prime
 // with a probability of about 0.015, a 24-bit one about 0.12: a round of 32 curves in a warp
 // splits a 31-bit pair about a third of the time, a 24-bit one almost always, and block-mates
-// add rounds of their own. On GB300 a single warp's multiply chain is latency-bound (about
-// 0.1 us per 64-bit Montgomery multiply), so short rounds that fail now and then beat long sure
-// ones: measured on the 4096-window batch, stage D took 0.45 ms with B1 = 40, 0.47 with 50,
-// 0.48 with 60, 0.55 with 85 and 0.49 with 30, whose 2^34 window at 1.8e19 then needed 2.1 ms
-// (too many failed rounds); with B1 = 40 and the curves inversion-free, B2 = 1200 against
-// 2000 and 3000: 0.34 against 0.36 and 0.41 ms here, 0.56-0.58 against 0.59-0.60 and
-// 0.62-0.63 ms on the batch at 1e19, 0.32 against 0.35-0.36 and 0.39-0.40 ms on that 2^34
-// window (B2 = 800 measured within noise of 1200); B1 re-checked with B2 = 1200: 30 lost at 1e19
-// (0.69-0.76 against 0.54-0.56 ms), 50 gained there what it lost on the 4096-window batch
-// (0.53-0.54 against 0.54-0.56, and 0.35-0.37 against 0.34-0.35 ms). The reference factors
+// add rounds of their own. On GB300 a single warp's multiplies are latency-bound here, so short
+// rounds that fail now and then beat long sure ones: B1 = 40 and B2 = 1200 were chosen from B1 = 30
+// to 85 and B2 = 800 to 3000 on batches at all heights and at 1e19 (0.34 ms of stage D on the
+// former with B2 = 1200, 0.36 with 2000, 0.41 with 3000). A round of the curve as written below
+// takes 102 K cycles, 119 K with the multiplies and additions of a step one after another and with
+// three multiplies a pair in stage 2; 820 cycles a ladder step with one warp on a scheduler, 1217 with
+// two, 1495 with four. The reference factors
 // with rho alone (sieve/rung_scan3.cpp:333-369); the factorization of a number is unique, so
 // the method that finds a divisor cannot change any certificate.
 //
@@ -58,7 +55,7 @@ constexpr int ECM_M1 = 20;
 __constant__ const unsigned char ECM_PAIRS[ECM_M1] = {
     0xff, 0xfe, 0xff, 0xdf, 0xfe, 0xef, 0xed, 0xff, 0xf3, 0xfb, 0xfb, 0xef, 0xf6, 0xfd, 0xfe, 0x7e,
     0xef, 0xfe, 0x5c, 0xaa};
-// One round (about 1.25 K Montgomery multiplies: 12 per bit of k, 3 per stage-2 pair, 6 per
+// One round (about 1.2 K Montgomery multiplies: 12 per bit of k, 2 per stage-2 pair, 7 per
 // giant step and baby step) in rho steps of two multiplies.
 constexpr u64 ECM_ROUND_STEPS = 625;
 
@@ -94,7 +91,7 @@ __device__ __forceinline__ u64 proper_gcd(u64 g, u64 n) {
 
 // Giant steps between polls in stage 2, ladder bits between polls in stage 1 (a poll that
 // answers "stop" ends the curve at once: another walk or curve has split the cofactor).
-constexpr int ECM_STAGE2_POLL = 24;
+constexpr int ECM_STAGE2_POLL = 5;
 #ifndef ES_ECM_STAGE1_POLL
 #define ES_ECM_STAGE1_POLL 13
 #endif
@@ -104,8 +101,7 @@ constexpr int ECM_STAGE1_POLL = ES_ECM_STAGE1_POLL;
 // arithmetic Ar (LazyArith needs n < 2^62). Returns a proper divisor of n, or 0 when this curve
 // found none. poll() is called at the same points in every lane (every ECM_STAGE1_POLL ladder
 // bits, after stage 1 and every ECM_STAGE2_POLL giant steps); when it returns true the curve
-// stops early and returns 0. dead
-// lanes keep computing (their result is dropped) so that the lanes of a warp stay in step.
+// stops early and returns 0.
 template <class Ar, class Poll>
 __device__ inline u64 ecm_curve(u64 sigma, const Mont &M, Poll poll) {
   const u64 n = M.n;
@@ -124,45 +120,72 @@ __device__ inline u64 ecm_curve(u64 sigma, const Mont &M, Poll poll) {
   for (int i = 0; i < 4; ++i) den = Ar::add(den, den, M);      // 16 u^3 v
   const XZ P0{u3, v3};
   // --- stage 1: Q = [k]P0, ladder from the top bit of k (the difference of the ladder's two
-  // points is always P0)
+  // points is always P0). A step is R0 = [2]R0, R1 = R0 + R1 with the points swapped where the bit
+  // differs from the last one, in three levels of four independent multiplies.
   XZ R0 = P0, R1 = ecm_dbl<Ar>(R0, num, den, M);
+  u64 last = 0;
+  #pragma unroll 1
   for (int i = ECM_K_BITS - 2; i >= 0; --i) {
-    const bool b = (ECM_K[i >> 5] >> (i & 31)) & 1u;
-    if (b) { const XZ t = R0; R0 = R1; R1 = t; }
-    R1 = ecm_add<Ar>(R0, R1, P0, M);
-    R0 = ecm_dbl<Ar>(R0, num, den, M);
-    if (b) { const XZ t = R0; R0 = R1; R1 = t; }
+    const u64 bit = (ECM_K[i >> 5] >> (i & 31)) & 1u, sw = 0 - (bit ^ last);
+    last = bit;
+    const u64 dx = (R0.x ^ R1.x) & sw, dz = (R0.z ^ R1.z) & sw;
+    R0.x ^= dx; R1.x ^= dx; R0.z ^= dz; R1.z ^= dz;
+    const u64 s0 = Ar::add(R0.x, R0.z, M), d0 = Ar::sub(R0.x, R0.z, M);
+    const u64 s1 = Ar::add(R1.x, R1.z, M), d1 = Ar::sub(R1.x, R1.z, M);
+    const u64 t1 = Ar::mul(s0, s0, M), t2 = Ar::mul(d0, d0, M), f = Ar::mul(d0, s1, M), g = Ar::mul(s0, d1, M);
+    const u64 t3 = Ar::sub(t1, t2, M), p = Ar::add(f, g, M), m = Ar::sub(f, g, M);
+    const u64 c = Ar::mul(den, t2, M), w = Ar::mul(num, t3, M), p2 = Ar::mul(p, p, M), m2 = Ar::mul(m, m, M);
+    R0.x = Ar::mul(t1, c, M); R0.z = Ar::mul(t3, Ar::add(c, w, M), M);
+    R1.x = Ar::mul(P0.z, p2, M); R1.z = Ar::mul(P0.x, m2, M);
     if (i && i % ECM_STAGE1_POLL == 0 && poll()) return 0;
   }
-  const XZ Q = R0;
+  const XZ Q = last ? R1 : R0;
   if (poll()) return 0;
-  // --- stage 2: baby steps [j]Q for odd j <= 31 (kept for j in ECM_J), giant step [60]Q
-  const XZ Q2 = ecm_dbl<Ar>(Q, num, den, M);
-  u64 bx[ECM_NJ], bz[ECM_NJ];
-  bx[0] = Q.x; bz[0] = Q.z;
-  XZ prev = Q, cur = ecm_add<Ar>(Q2, Q, Q, M);                 // [1], [3]
-  int nb = 1;
-  XZ P29{0, 0};
-  #pragma unroll
-  for (int j = 3; j <= 29; j += 2) {                           // cur = [j]
-    if (j % 3 != 0 && j % 5 != 0) { bx[nb] = cur.x; bz[nb] = cur.z; ++nb; }
-    if (j == 29) P29 = cur;
-    const XZ nxt = ecm_add<Ar>(cur, Q2, prev, M);              // [j + 2]
-    prev = cur; cur = nxt;
+  // --- stage 2: baby steps [j]Q for j in ECM_J, with the products X Z: [1] and [5] are stepped by
+  // [6] through 7, 13, 19 and 11, 17, 23, 29 together; then the giant step [60]Q = [2]([17] + [13])
+  u64 bx[ECM_NJ], bz[ECM_NJ], bp[ECM_NJ];
+  auto keep = [&](int i, const XZ &P) { bx[i] = P.x; bz[i] = P.z; bp[i] = Ar::mul(P.x, P.z, M); };
+  XZ G1;
+  {
+    const XZ Q2 = ecm_dbl<Ar>(Q, num, den, M), Q3 = ecm_add<Ar>(Q2, Q, Q, M);
+    const XZ Q4 = ecm_dbl<Ar>(Q2, num, den, M), Q6 = ecm_dbl<Ar>(Q3, num, den, M), Q5 = ecm_add<Ar>(Q3, Q2, Q, M);
+    XZ a = Q, a_last = Q5, b = Q5, b_last = Q, Q13 = Q, Q17 = Q;
+    keep(0, Q);
+    #pragma unroll 1
+    for (int k = 0; k < 4; ++k) {                              // a = [6 k + 1], b = [6 k + 5]
+      const XZ na = ecm_add<Ar>(a, Q6, a_last, M), nb = ecm_add<Ar>(b, Q6, b_last, M);
+      a_last = a; b_last = b; a = na; b = nb;
+      if (k < 3) keep(2 * k + 1, a);
+      keep(2 * k + (k < 3 ? 2 : 1), b);
+      if (k == 1) { Q13 = a; Q17 = b; }
+    }
+    G1 = ecm_dbl<Ar>(ecm_add<Ar>(Q17, Q13, Q4, M), num, den, M);
   }
-  const XZ G1 = ecm_add<Ar>(cur, P29, Q2, M);                  // [31] + [29] = [60]
   // giant steps G_m = [60 m]Q, m = 1 .. ECM_M1; for each prime mD +- j of (B1, B2] the
-  // product gathers X(G_m) Z(j) - X(j) Z(G_m), zero modulo p when [mD]Q = +-[j]Q there. It
-  // starts from Z(Q): a factor stage 1 already found (Q at infinity modulo p) stays in it.
+  // product gathers X(G_m) Z(j) - X(j) Z(G_m) = (X(G_m) - X(j)) (Z(G_m) + Z(j)) - X(G_m) Z(G_m) +
+  // X(j) Z(j), zero modulo p when [mD]Q = +-[j]Q there. It starts from Z(Q): a factor stage 1
+  // already found (Q at infinity modulo p) stays in it. The pairs of a giant step are multiplied
+  // as a tree, a pair with no prime standing for one.
   u64 acc = Q.z;
   XZ Gp = G1, G = G1;
+  #pragma unroll 1
   for (int m = 1; m <= ECM_M1; ++m) {
-    if (m == 2) G = ecm_dbl<Ar>(G1, num, den, M);
-    else if (m > 2) { const XZ t = ecm_add<Ar>(G, G1, Gp, M); Gp = G; G = t; }
+    const u64 gp = Ar::mul(G.x, G.z, M);
     const u32 mask = ECM_PAIRS[m - 1];
+    u64 f[ECM_NJ];
     #pragma unroll
-    for (int i = 0; i < ECM_NJ; ++i)
-      if (mask & (1u << i)) acc = Ar::mul(acc, Ar::sub(Ar::mul(G.x, bz[i], M), Ar::mul(bx[i], G.z, M), M), M);
+    for (int i = 0; i < ECM_NJ; ++i) {
+      const u64 t = Ar::mul(Ar::sub(G.x, bx[i], M), Ar::add(G.z, bz[i], M), M);
+      f[i] = (mask >> i & 1u) ? Ar::add(Ar::sub(t, gp, M), bp[i], M) : M.one;
+    }
+    #pragma unroll
+    for (int o = ECM_NJ / 2; o; o >>= 1)
+      #pragma unroll
+      for (int i = 0; i < o; ++i) f[i] = Ar::mul(f[i], f[i + o], M);
+    acc = Ar::mul(acc, f[0], M);
+    const XZ t = m == 1 ? ecm_dbl<Ar>(G1, num, den, M) : ecm_add<Ar>(G, G1, Gp, M);
+    Gp = G;
+    G = t;
     if (m % ECM_STAGE2_POLL == 0 && poll()) return 0;
   }
   return proper_gcd(Ar::norm(acc, M), n);

@@ -13,7 +13,7 @@
 //   fdesc[nf]         u32  per filter: stride s = mod/gcd(M,mod) and its Qm column
 //   tdp/tde                trial-division table: 6541 odd primes < 2^16 with inverses
 // Per run: window descriptors, row pieces and rows, candidate chunks, Qm[window][stride] =
-// (lo / M) mod s where windows are marked by segments, the survivor list, prime/direct index lists, records, counters and the hard board.
+// (lo / M) mod s where windows are marked by segments, the survivor list, prime/direct index lists, records and counters.
 //
 // Pipeline per run (one CUDA stream, replayed as a CUDA graph for batches):
 //   k_rows        the windows cut into rows (one K, all lanes) and pieces of 32 rows, with each
@@ -26,7 +26,7 @@
 //   k_mr          a thread per survivor: the base-2 strong-probable-prime round
 //   k_mr2         a warp per number that passed base 2: the 12-base test, one base per lane
 //   k_rung        stage D: a warp per prime while primes outnumber the grid's warps, then a
-//                 block of four warps per prime over successive rungs; warp trial division,
+//                 team of four warps per prime over successive rungs; warp trial division,
 //                 Miller-Rabin, Brent's rho, ECM rounds (es_tail.cuh, es_ecm.cuh), the rung
 //                 DP, and the exact certificate check (es_check.cuh) before a record is
 //                 written
@@ -891,39 +891,40 @@ __device__ __forceinline__ void put_record(const TailParams &T, const RecDev &r)
   if (k < T.cap) T.recs[k] = r;
 }
 
-#ifndef ES_RUNG_WARPS
-#define ES_RUNG_WARPS 4
-#endif
-constexpr int RUNG_WARPS = ES_RUNG_WARPS;
-#ifndef ES_RUNG_TAIL_PER_BLOCK
-#define ES_RUNG_TAIL_PER_BLOCK RUNG_WARPS     // primes per block left for the block phase
-#endif
-#ifndef ES_RUNG_MIN_BLOCKS
-#define ES_RUNG_MIN_BLOCKS (16 / RUNG_WARPS)   // resident blocks per SM the register budget allows
-#endif
-#ifndef ES_HELP_BLOCKS_PER_SM
-#define ES_HELP_BLOCKS_PER_SM 1
-#endif
-#ifndef ES_FEW_ECM_DIV
-#define ES_FEW_ECM_DIV 4
-#endif
-#ifndef ES_FEW_ECM_AFTER
-#define ES_FEW_ECM_AFTER 384
-#endif
-#ifndef ES_HELP_FEW_DIV
-#define ES_HELP_FEW_DIV 16
-#endif
-#ifndef ES_HELP_BLOCKS_DIV
-#define ES_HELP_BLOCKS_DIV 1
-#endif
+// Shared memory of a stage-D block of TEAMS teams.
+template <int TEAMS>
+struct RungShared {
+  WarpFac F[TEAMS * TEAM_WARPS];
+  DPWarp D[TEAMS * TEAM_WARPS];
+  u64 rho_slot[TEAMS * TEAM_WARPS];
+  RungResult slot[TEAMS * TEAM_WARPS], out[TEAMS];
+  TdSieve tds[TEAMS];
+  BlockHelp help;
+  unsigned long long next[TEAMS];
+  int best_k[TEAMS];
+  unsigned int busy[TEAMS];
+  __device__ Team team(int t) {
+    return Team{F + TEAM_WARPS * t, D + TEAM_WARPS * t, rho_slot + TEAM_WARPS * t, slot + TEAM_WARPS * t, out + t,
+                tds + t, best_k + t, busy + t, &help, (u32)(TEAM_WARPS * t), (u32)t + 1};
+  }
+  __device__ void init() {                         // every thread calls; the caller synchronizes
+    for (u32 i = threadIdx.x; i < sizeof(BlockHelp) / 4; i += blockDim.x) reinterpret_cast<u32 *>(&help)[i] = 0;
+  }
+};
+constexpr int RUNG_TEAMS = BLOCK_WARPS / TEAM_WARPS, RUNG_THREADS = 32 * BLOCK_WARPS;
+// Every fourth block stays to help the board when it is done: all of them keep their SMs from the next
+// batch's marking (three pipelined batches at 1e19 1.26-1.36 ms against 1.48-1.60 with every block and
+// 1.33-1.51 with none; a 2^34 window at 1.8e19 with the tuned table 0.29-0.35, 0.28-0.35, 0.34-0.40).
+constexpr u32 BOARD_BLOCKS_DIV = 4;
+constexpr u32 FEW_PRIMES_PER_BLOCK = 2;        // up to two a block: the board is on (4 measured the same)
 
-// Stage D. While more primes remain than the grid has warps, every warp takes a prime of its
-// own from a queue and walks its rungs in order (warp_solve_rung: no barrier, no speculative
-// rungs); the last gridDim.x * RUNG_WARPS primes go to whole blocks of RUNG_WARPS warps that
-// try four rungs of one prime at a time (block_solve_rung), so that the run ends on short
-// latencies. A block that finds both queues empty turns its warps into helpers on the hard
-// board (warp_help) until every prime of the run is finished, so that the last, hardest
-// factorizations get more walks than one warp's.
+// Stage D, in blocks of four teams of four warps (one block per SM resident). While more primes
+// remain than the grid has warps, every warp takes a prime of its own from a queue and walks its
+// rungs in order (warp_solve_rung: no barrier, no speculative rungs); the last gridDim.x *
+// BLOCK_WARPS primes go to teams that try four rungs of one prime at a time (team_solve_rung), so
+// that the run ends on short latencies. The later teams of a block come to the queue a little
+// later, so that few primes have an SM each. A team that finds the queue empty turns its warps into
+// helpers on the block's hard cofactors until the block's other teams are done.
 __device__ __forceinline__ void rung_result(const TailParams &T, const Surv &s, u32 si, bool ok,
                                             const RungResult &res) {
   if (ok && !check_rung_cert(s.p, res.A, res.r, res.u)) {
@@ -940,67 +941,54 @@ __device__ __forceinline__ void rung_result(const TailParams &T, const Surv &s, 
   atomicAdd(T.rung_done, 1ull);
 }
 
-__global__ void __launch_bounds__(RUNG_WARPS * 32, ES_RUNG_MIN_BLOCKS) k_rung(const TailParams T, int no_rung) {
-  __shared__ WarpFac F[RUNG_WARPS];
-  __shared__ DPWarp D[RUNG_WARPS];
-  __shared__ u64 rho_slot[RUNG_WARPS];
-  __shared__ int best_k;
-  __shared__ RungResult slot[RUNG_WARPS];
-  __shared__ RungResult res;
-  __shared__ unsigned long long next;
+__global__ void __launch_bounds__(RUNG_THREADS, 1) k_rung(const TailParams T, int no_rung) {
+  extern __shared__ __align__(16) unsigned char rungmem[];
+  RungShared<RUNG_TEAMS> &H = *reinterpret_cast<RungShared<RUNG_TEAMS> *>(rungmem);
   const u64 n = min((u64)*T.prime_count, T.cap);
-  const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  __shared__ BlockHelp bhelp;
-  __shared__ TdSieve tds;
-  HardBoard B;
-  B.slot = T.board; B.sessions = T.help_sessions; B.done = T.rung_done; B.total = n;
-  B.local = nullptr;                                 // the warp phase: no block-mates on one prime
-  // A run of few primes is bound by the latency of its hardest factorizations, on SMs that are
-  // otherwise idle: its cofactors turn to curves sooner.
-  B.ecm_after = (ES_FEW_ECM_DIV && n * ES_FEW_ECM_DIV <= (u64)gridDim.x) ? ES_FEW_ECM_AFTER : 0;
-  const u64 tail = min(n, (u64)gridDim.x * ES_RUNG_TAIL_PER_BLOCK);
+  if (!n) return;
+  const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5, t = w / TEAM_WARPS;
+  const u64 tail = min(n, (u64)gridDim.x * BLOCK_WARPS);
   const u64 nw = n - tail;                           // primes [0, nw): a warp each
+  H.init();
+  const bool few = n <= FEW_PRIMES_PER_BLOCK * (u64)gridDim.x;
+  const Board board{few ? T.board : nullptr, T.help_sessions, T.rung_done};
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    H.help.working = RUNG_TEAMS;
+    H.help.board = board;
+  }
+  __syncthreads();
   for (;;) {
-    u64 i = 0;
-    if (lane == 0) i = atomicAdd(T.rung_next_warp, 1ull);
+    u64 i = nw;
+    if (nw && lane == 0) i = atomicAdd(T.rung_next_warp, 1ull);
     i = __shfl_sync(0xFFFFFFFFu, i, 0);
     if (i >= nw) break;
     const u32 si = T.primes[i];
     const Surv s = T.surv[si];
-    const bool ok = !no_rung && warp_solve_rung(s.p, T.tdp, T.tdi, T.status, F[w], D[w], rho_slot + w, &slot[w], &B,
+    const bool ok = !no_rung && warp_solve_rung(s.p, T.tdp, T.tdi, T.status, H.F[w], H.D[w], H.rho_slot + w, &H.slot[w],
                                                 T.rho_budget, /*use_ecm=*/false);
-    if (lane == 0) rung_result(T, s, si, ok, slot[w]);
+    if (lane == 0) rung_result(T, s, si, ok, H.slot[w]);
     __syncwarp();
   }
-  __syncthreads();
-  B.local = &bhelp;
-  for (;;) {                                          // primes [nw, n): a block each
-    if (threadIdx.x == 0) next = nw + atomicAdd(T.rung_next, 1ull);
-    __syncthreads();
-    const u64 i = next;
+  const Team team = H.team(t);
+  const bool first = threadIdx.x % TEAM_THREADS == 0;
+  __nanosleep(1500 * t);
+  for (;;) {                                         // primes [nw, n): a team each
+    if (first) H.next[t] = nw + atomicAdd(T.rung_next, 1ull);
+    team_sync(team.bar);
+    const u64 i = H.next[t];
     if (i >= n) break;
     const u32 si = T.primes[i];
     const Surv s = T.surv[si];
-    const bool ok = !no_rung &&
-                    block_solve_rung<RUNG_WARPS>(s.p, T.tdp, T.tdi, T.tdqm, &tds, T.status, F, D, rho_slot, &best_k, slot,
-                                                 &res, &B,
-                                                 T.rho_budget);
-    if (threadIdx.x == 0) rung_result(T, s, si, ok, res);
-    __syncthreads();
+    const bool ok = !no_rung && team_solve_rung(s.p, T.tdp, T.tdi, T.tdqm, T.status, team, T.rho_budget);
+    if (first) rung_result(T, s, si, ok, *team.out);
+    team_sync(team.bar);
   }
-  // Helpers come from the first help_blocks blocks only (one per SM): the walks of a hard
-  // cofactor progress at the issue rate their sub-partition gives them, so helpers beyond
-  // one warp per scheduler would only split that rate over more walks, and the expected wait
-  // for the first collision grows with the square root of the number of walks sharing it.
-  // They help only a run of few primes (at most one per ES_HELP_FEW_DIV blocks), whose time
-  // is its slowest factorization on SMs that are otherwise idle: the 2^34 window at 1.8e19
-  // with the tuned table (21 primes) 0.33 against 0.46 ms of stage D. With more primes the
-  // helpers' walks take issue slots from the owners (129 primes: 0.375 against 0.36 ms;
-  // batches: 0.48 against 0.435 ms before this rule), and a pipelined tail would keep its
-  // blocks resident.
-  B.local = nullptr;
-  const bool few = ES_HELP_FEW_DIV == 0 || n * ES_HELP_FEW_DIV <= (u64)gridDim.x;
-  if (!no_rung && few && blockIdx.x < T.help_blocks) warp_help(B, lane);
+  if (first) atomicSub(&H.help.working, 1u);
+  __syncwarp();
+  if (no_rung) return;
+  warp_help(&H.help, &H.help.working, nullptr, lane);
+  if (few && t == 0 && blockIdx.x % BOARD_BLOCKS_DIV == 0) warp_help_board(board, n, lane);
 }
 
 __global__ void k_direct(const TailParams T) {
@@ -1042,21 +1030,18 @@ __global__ void k_probe_prime(const u64 *n, u64 count, unsigned char *out) {
     if (lane == 0) out[i] = pr ? 1 : 0;
   }
 }
-__global__ void __launch_bounds__(RUNG_WARPS * 32, ES_RUNG_MIN_BLOCKS) k_probe_rung(const u64 *p, u64 count, RecDev *out,
+__global__ void __launch_bounds__(TEAM_THREADS, 4) k_probe_rung(const u64 *p, u64 count, RecDev *out,
                                                                unsigned char *found, const u32 *tdp,
                                                                const u64 *tdi, const uint2 *tdqm, u32 *status,
                                                                u64 rho_budget) {
-  __shared__ TdSieve tds;
-  __shared__ WarpFac F[RUNG_WARPS];
-  __shared__ DPWarp D[RUNG_WARPS];
-  __shared__ u64 rho_slot[RUNG_WARPS];
-  __shared__ int best_k;
-  __shared__ RungResult slot[RUNG_WARPS];
-  __shared__ RungResult res;
+  __shared__ RungShared<1> H;
+  H.init();
+  __syncthreads();
+  const Team team = H.team(0);
   for (u64 i = blockIdx.x; i < count; i += gridDim.x) {
-    bool ok = block_solve_rung<RUNG_WARPS>(p[i], tdp, tdi, tdqm, &tds, status, F, D, rho_slot, &best_k, slot, &res,
-                                           nullptr, rho_budget);
+    bool ok = team_solve_rung(p[i], tdp, tdi, tdqm, status, team, rho_budget);
     if (threadIdx.x == 0) {
+      const RungResult &res = *team.out;
       if (ok && !check_rung_cert(p[i], res.A, res.r, res.u)) { atomicOr(status, ST_CERT_BAD); ok = false; }
       found[i] = ok;
       out[i] = ok ? RecDev{ES_REC_RUNG, 0, 0, 0, 0, p[i], res.A, res.r, res.u.lo, res.u.hi}
@@ -1084,7 +1069,7 @@ __global__ void k_probe_factor(const u64 *n, u64 count, u64 *pr, unsigned char *
   const u64 warps = (u64)gridDim.x * blockDim.x / 32;
   for (u64 i = ((u64)blockIdx.x * blockDim.x + threadIdx.x) / 32; i < count; i += warps) {
     WarpFac &f = F[w];
-    const bool ok = warp_factor(n[i], f, tdp, tdi, status, lane, rho_slot + w, nullptr, 0, nullptr, rho_budget);
+    const bool ok = warp_factor(n[i], f, tdp, tdi, status, lane, rho_slot + w, nullptr, 0, nullptr, 0, rho_budget);
     if (lane == 0) {
       const int kk = ok ? f.k : 0;
       for (int a = 1; a < kk; ++a)
@@ -1142,7 +1127,7 @@ struct Slot {
   size_t rec_prefix = 0;                // records the captured graph copies back itself
   u64 graph_launches = 0;               // its kernels
   unsigned long long *d_ctr = nullptr;  // [0] queue [1] surv [2] prime [3] direct [4] rec [5] cand
-                                      // [6] rung queue (blocks) [7] rungs done [8] help sessions
+                                      // [6] rung queue (teams) [7] rung primes done [8] board sessions
                                       // [9] rung queue (warps) [10] candidate chunks, board at [16]
   u32 *d_status = nullptr;
   es_timing_t timing{};
@@ -1161,9 +1146,9 @@ struct Slot {
 };
 
 constexpr int SERVE_SLOTS = 2;
-// run counters (16 words) followed by the hard board, cleared together before every run
 constexpr size_t CTR_OUT = 11;          // counters copied back to the host
-constexpr size_t CTR_BYTES = 16 * sizeof(unsigned long long) + HARD_SLOTS * sizeof(HardSlot);
+// run counters followed by stage D's board, cleared before every run
+constexpr size_t CTR_BYTES = 16 * sizeof(unsigned long long) + BOARD_SLOTS * sizeof(BoardSlot);
 
 // A serving request: windows in, counters and records out.
 struct Request {
@@ -1355,9 +1340,8 @@ static TailParams tail_params(const es_engine *e, const Slot *sl) {
   T.direct = sl->d_direct; T.direct_count = sl->d_ctr + 3;
   T.recs = sl->d_recs; T.rec_count = sl->d_ctr + 4;
   T.rung_next = sl->d_ctr + 6; T.rung_done = sl->d_ctr + 7; T.help_sessions = sl->d_ctr + 8;
+  T.board = reinterpret_cast<BoardSlot *>(sl->d_ctr + 16);
   T.rung_next_warp = sl->d_ctr + 9;
-  T.board = reinterpret_cast<HardSlot *>(sl->d_ctr + 16);
-  T.help_blocks = (u32)(e->sm_count * ES_HELP_BLOCKS_PER_SM / ES_HELP_BLOCKS_DIV);
   T.rho_budget = e->rho_budget;
   T.cnt = sl->d_cnt; T.tdp = e->d_tdp; T.tde = e->d_tde; T.tdi = e->d_tdi; T.tdqm = e->d_tdqm; T.status = sl->d_status;
   T.cap = sl->cap;
@@ -1558,7 +1542,8 @@ static es_status enqueue_tail(es_engine *e, Slot *sl, WinCount *cnt, bool captur
   auto rec = [&](int k) {
     return capture ? cudaEventRecordWithFlags(sl->ev[k], st, cudaEventRecordExternal) : cudaEventRecord(sl->ev[k], st);
   };
-  k_rung<<<e->sm_count * e->sched.rung_blocks_per_sm, RUNG_WARPS * 32, 0, st>>>(T, (e->flags & ES_FLAG_NO_RUNG) ? 1 : 0);
+  const u32 teams = e->sm_count * std::min<u32>(e->sched.rung_blocks_per_sm, RUNG_TEAMS);
+  k_rung<<<(teams + RUNG_TEAMS - 1) / RUNG_TEAMS, RUNG_THREADS, sizeof(RungShared<RUNG_TEAMS>), st>>>(T, (e->flags & ES_FLAG_NO_RUNG) ? 1 : 0);
   CU(cudaGetLastError());
   CU(rec(3));
   k_direct<<<e->sm_count, 32, 0, st>>>(T);
@@ -2160,11 +2145,11 @@ static es_status build_tables(es_engine *e) {
   {
     int max_smem = 0;
     CU(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, e->device));
-    for (const void *f : {(const void *)k_rung, (const void *)k_probe_rung}) {
-      cudaFuncAttributes fa;
-      CU(cudaFuncGetAttributes(&fa, f));
-      const double need = (double)ES_RUNG_MIN_BLOCKS * (fa.sharedSizeBytes + 1024);
-      const int pct = std::min(100, (int)(100.0 * need / std::max(max_smem, 1)) + 1);
+    CU(cudaFuncSetAttribute(k_rung, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RungShared<RUNG_TEAMS>)));
+    const std::pair<const void *, size_t> resident[] = {{(const void *)k_rung, sizeof(RungShared<RUNG_TEAMS>)},
+                                                        {(const void *)k_probe_rung, 4 * sizeof(RungShared<1>)}};
+    for (const auto &[f, bytes] : resident) {
+      const int pct = std::min(100, (int)(100.0 * (bytes + 4096) / std::max(max_smem, 1)) + 1);
       CU(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
     }
   }
@@ -2672,7 +2657,7 @@ es_status es_solve_rung_batch(es_engine *e, const uint64_t *p, size_t count, es_
   if (!count) return ES_OK;
   return probe(e, &e->slots[0], count, count * 8, p, 0, {{out, count * sizeof(es_record)}, {found, count}},
                [&](void *in, std::vector<void *> &o) {
-                 k_probe_rung<<<e->sm_count * 4, RUNG_WARPS * 32, 0, e->slots[0].stream>>>((const u64 *)in, count, (RecDev *)o[0],
+                 k_probe_rung<<<e->sm_count * 4, TEAM_THREADS, 0, e->slots[0].stream>>>((const u64 *)in, count, (RecDev *)o[0],
                                                                      (unsigned char *)o[1], e->d_tdp, e->d_tdi, e->d_tdqm,
                                                                      e->slots[0].d_status, e->rho_budget);
                });

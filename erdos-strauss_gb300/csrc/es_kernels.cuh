@@ -142,7 +142,7 @@ struct RowParams {
   u32 n1, n1p, n2, nm_cov, nm_all, nl_cov, nl_all;   // the first words of strides [n1, n2) fit SIFT_WORDS_MAX
 };
 
-struct HardSlot;
+struct BoardSlot;
 
 struct TailParams {
   Surv *surv;
@@ -162,12 +162,11 @@ struct TailParams {
   const uint2 *tdqm;       // {d, floor(2^32 / d)} (the rung sieve's residues)
   u32 *status;
   u64 cap;                 // capacity of surv/primes/direct/recs
-  unsigned long long *rung_next;      // k_rung's prime queue head, whole blocks (the tail)
-  unsigned long long *rung_next_warp; // k_rung's prime queue head, one warp per prime
+  unsigned long long *rung_next;      // k_rung's prime queue head, a team per prime (the tail)
   unsigned long long *rung_done;      // primes k_rung has finished
-  unsigned long long *help_sessions;  // helping sessions started on the hard board
-  struct HardSlot *board;             // [HARD_SLOTS] cofactors whose rho takes long
-  u32 help_blocks;                    // k_rung blocks [0, help_blocks) help on the board
+  unsigned long long *help_sessions;  // curve rounds started on the board
+  struct BoardSlot *board;            // [BOARD_SLOTS] hard cofactors of a run of few primes
+  unsigned long long *rung_next_warp; // k_rung's prime queue head, one warp per prime
   u64 rho_budget;                     // Brent steps per lane before a factorization gives up
 };
 

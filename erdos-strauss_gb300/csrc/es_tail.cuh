@@ -12,9 +12,11 @@
 //   ECM              in the latency-bound tail, a cofactor rho has not split after ECM_AFTER
 //                    steps gets rounds of one elliptic curve per lane (es_ecm.cuh), the first
 //                    divisor wins
-//   rung DP          lanes own residue classes t mod r and gather
+//   rung DP          the least divisor up to 65536 in the rung's class by 32-bit values; if there is
+//                    none, whether any divisor is in the class; only then the least of all: lanes
+//                    own residue classes t mod r and gather
 //                    nxt[t] = min_j cur[t * pr^-j] * pr^j over j <= e with the bound <= q
-// and a block of four warps walks successive rungs of one prime concurrently, keeping the
+// and a team of four warps walks successive rungs of one prime concurrently, keeping the
 // smallest rung that certifies (the reference's emission rule, sieve/rung_scan3.cpp:574-603).
 #pragma once
 #include "es_arith.cuh"
@@ -56,17 +58,21 @@ __device__ inline bool warp_is_prime(u64 n, u32 lane) {
     for (int i = 0; i < 12; ++i) isb |= (n == MR_BASES[i]);
     return isb;
   }
+  if (!(n & 1)) return false;
   if (lane < 12) {
-    const u64 b = MR_BASES[lane];
-    if (n % b == 0) ok = false;
-    else {
-      const Mont M = mont_init(n);
-      u64 d = n - 1;
-      const int s = __ffsll((long long)d) - 1;
-      d >>= s;
-      const u64 bm = to_mont(b, M);
-      ok = n < LazyArith::NMAX ? sprp_ar<LazyArith>(bm, d, s, M) : sprp_mont(bm, d, s, M);
+    // No division by the base first: a base that divides n > 37 has only multiples of itself as
+    // powers mod n, never +-1, so the round fails. The base's Montgomery form by doublings of 1's.
+    const u32 b = (u32)MR_BASES[lane];
+    const Mont M = mont_one(n);
+    u64 bm = 0;
+    for (int i = 5; i >= 0; --i) {
+      bm = addmod(bm, bm, n);
+      if (b >> i & 1) bm = addmod(bm, M.one, n);
     }
+    u64 d = n - 1;
+    const int s = __ffsll((long long)d) - 1;
+    d >>= s;
+    ok = n < LazyArith::NMAX ? sprp_ar<LazyArith>(bm, d, s, M) : sprp_mont(bm, d, s, M);
   }
   return __all_sync(FULL, ok);
 }
@@ -90,19 +96,20 @@ __device__ __forceinline__ u64 rho_backtrack(u64 x, u64 ys, u64 cm, u64 n, const
 // |x - y| accumulated between gcds, the comparison window doubling -- with two changes that
 // cannot change a result, only when a factor is found: the first window is 16 steps instead
 // of 1 (every cofactor that reaches rho has all its primes above 2^16, so its cycles are far
-// longer) and gcds come every 256 steps instead of 128 (a 64-bit binary gcd costs about as
-// much as twenty steps here). A 64-bit Montgomery multiply is issue-bound on this GPU (the
-// wide integer multiplies issue at a quarter of the low-half rate), so more walks per lane
-// would only add work: the latency-optimal split is one walk per lane.
+// longer) and gcds come every 256 steps, across windows, instead of 128 (a 64-bit binary gcd costs
+// as much as 25 steps here). More walks per lane would only add work: the latency-optimal split
+// is one walk per lane.
 // The lanes run in lockstep (one window schedule for the warp), so that the warp can stop as
-// soon as any lane has a divisor, poll the hard board between batches and be cancelled
-// there. A lane whose batch product shares all of n backtracks one step at a time from the
-// batch start; if that closes without a divisor its walk restarts with its next constant.
+// soon as any lane has a divisor, poll for one from outside every RHO_POLL steps and be cancelled
+// there. A lane whose product shares all of n goes on with its next constant, and the warp then
+// takes gcds within windows, where a lane can backtrack one step at a time from the batch start (as
+// it does from the first for n < 2^40, whose two primes may well be met in one batch).
 // Returns a nontrivial factor of the odd composite n (the same value in every lane), or 0
 // when the budget ran out or the warp was cancelled. The factorization is unique, so which
 // walk wins cannot change any result.
 constexpr u64 RHO_R0 = 16;      // first comparison window
 constexpr u64 RHO_BATCH = 256;  // steps between gcds
+constexpr u64 RHO_POLL = 64;    // steps between polls
 
 // cancel/my_k: the warp is working for rung index my_k of a block whose best certifying rung
 // so far is *cancel; once that drops below my_k nothing this warp finds can matter and it stops
@@ -111,54 +118,44 @@ __device__ __forceinline__ bool cancelled(const volatile int *cancel, int my_k) 
   return cancel && *cancel < my_k;
 }
 
-// The hard board: a cofactor that rho has not split in its first steps is posted here when its
-// owner turns to ECM, and warps with nothing left to do (k_rung blocks that found the prime
-// queue empty) run more rho walks on it with constants of their own. Any nontrivial divisor
-// ends the search; by the birthday bound the wait for the first collision among W walks
-// shrinks like 1/sqrt(W), so with hundreds of idle warps the helpers' walks can beat the
-// owner's fixed-length ECM round, while a cofactor left alone gets the ECM round. The board
-// only speeds things up: the owner checks every divisor it is handed (1 < d < n,
-// n mod d == 0) and its own curves and walks still finish the job alone. No warp ever waits
-// for another.
-constexpr u32 HARD_SLOTS = 32;                 // one per lane of a scanning warp
-#ifndef ES_RHO_POST_STEPS
-#define ES_RHO_POST_STEPS 512
-#endif
-#ifndef ES_HELP_R0
-#define ES_HELP_R0 16
-#endif
-#ifndef ES_HELP_SLEEP_NS
-#define ES_HELP_SLEEP_NS 2000
-#endif
-constexpr u64 RHO_POST_STEPS = ES_RHO_POST_STEPS;  // steps per lane before a cofactor is posted
-constexpr u64 HELP_STEPS = 1ull << 16;         // steps per lane of one helping session
-constexpr u32 HELP_IDLE_POLLS = 4096;          // empty-board polls (2 us apart) before a helper leaves
-constexpr u32 HELP_MAX_ROUNDS = 1024;          // board scans (sessions or polls) per helper, at most
-struct HardSlot {
+// A block's hard cofactors (shared memory): a warp that has to split a cofactor posts it in its own
+// slot, and warps of the block with nothing else to do -- block-mates that have finished their own
+// rungs, and all warps of a team that found the prime queue empty -- run rounds of elliptic curves on
+// it while the owner walks rho and then curves of its own; the first divisor found ends the search
+// (the owner checks it divides n). Only speed depends on the helpers.
+// More curves at once on one SM pay little: two warps on a scheduler take 1.5 times as long as one for
+// a step of a curve (820 and 1217 cycles) and slow the owners' rho and the other rungs as much. So
+// at most CURVE_WARPS helpers, on cofactors that have outlasted rho; in a run of few primes (its
+// cofactors are posted at once, and done SMs help through the board) CURVE_WARPS_FEW. Mean stage-D
+// time of the 4096-window batch at 1e19 (gpu table): 0.80, 0.50, 0.46, 0.46 ms with 0, 3, 5, 8; of the
+// batch over all heights 0.29, 0.32, 0.31, 0.35; of 2^34 windows at 1.8e19 in the few-primes form
+// 0.27, 0.23, 0.25, 0.28 with 0, 1, 3, 8.
+constexpr int BLOCK_WARPS = 16;
+constexpr u32 CURVE_WARPS = 5, CURVE_WARPS_FEW = 1;
+// The grid's hard cofactors (device memory, all free between runs): in a run of few primes, where
+// most blocks are soon done, an owner that turns to curves posts its cofactor here too, and the done
+// blocks run curves on it, one warp per scheduler.
+constexpr u32 BOARD_SLOTS = 64;
+struct BoardSlot {
   unsigned long long n, found;
   unsigned int state, pad;                     // 0 free, 1 being written, 2 posted
   unsigned long long pad2;
 };
-// A block's own hard cofactor (shared memory): when a warp of a block that works on one
-// prime's rungs has walked rho on a cofactor for RHO_POST_STEPS steps, it posts the cofactor
-// here; block-mates that have finished their own rungs run rounds of elliptic curves on it
-// instead of waiting at the block's barrier, and the first divisor found ends the search.
-struct BlockHelp {
-  unsigned long long n, found;                 // the posted cofactor (0: none), a divisor of it
-  unsigned int busy;                           // warps of the block still on their rungs
-  unsigned int sessions;                       // curve rounds started on the block's cofactors
+struct Board {
+  BoardSlot *slot;                             // [BOARD_SLOTS]
+  unsigned long long *sessions, *done;         // curve rounds started on it, primes finished
 };
-struct HardBoard {
-  HardSlot *slot;                              // [HARD_SLOTS], all free between runs
-  unsigned long long *sessions;                // helping sessions started (distinct constants)
-  unsigned long long *done;                    // primes finished by k_rung
-  unsigned long long total;                    // primes k_rung has to finish
-  BlockHelp *local;                            // the block's own slot, or null
-  u64 ecm_after;                               // rho steps per lane before curves (0: ECM_AFTER)
+struct BlockHelp {
+  Board board;                                 // slot null: not in this run
+  unsigned long long n[BLOCK_WARPS], found[BLOCK_WARPS];   // the posted cofactor (0: none), a divisor of it
+  unsigned int curves;                         // helpers at work
+  unsigned int sessions;                       // curve rounds started by helpers (distinct sigmas)
+  unsigned int working;                        // teams that may still post
 };
 
 __device__ __forceinline__ u64 ld_volatile(const unsigned long long *p) { return *(const volatile unsigned long long *)p; }
 __device__ __forceinline__ u32 ld_volatile(const unsigned int *p) { return *(const volatile unsigned int *)p; }
+__device__ __forceinline__ void st_volatile(unsigned long long *p, u64 v) { *(volatile unsigned long long *)p = v; }
 
 // The lockstep walk shared by the owner and its helpers. c0: this lane's first constant,
 // cstep: the distance to its next one. poll() is called by every lane between batches (warp-
@@ -171,112 +168,133 @@ __device__ __forceinline__ u64 rho_walk(u64 n, const Mont &M, u64 c0, u64 cstep,
   u64 c = c0;
   u64 cm = to_mont(c, M);
   u64 y = y0, x = y0, ys = y0, q = M.one;
-  u64 steps = 0;
-  for (u64 r = r0;; r <<= 1) {
-    x = y;
-    if (steps + 2 * r > budget) return 0;
-    for (u64 i = 0; i < r; ++i) y = Ar::add(Ar::mul(y, y, M), cm, M);
-    steps += r;
-    for (u64 k = 0; k < r; k += RHO_BATCH) {
-      ys = y;
-      const u64 lim = RHO_BATCH < r - k ? RHO_BATCH : r - k;
-      for (u64 i = 0; i < lim; ++i) {
-        y = Ar::add(Ar::mul(y, y, M), cm, M);
-        q = Ar::mul(q, x > y ? x - y : y - x, M);     // a closed cycle makes q = 0 mod n
-      }
-      steps += lim;
-      u64 mine = 0;
-      const u64 g = gcd64(q, n);
-      if (g != 1) {
-        if (g != n) mine = g;
-        else {
-          const u64 gb = rho_backtrack<Ar>(x, ys, cm, n, M);
-          if (gb != 1 && gb != n) mine = gb;
-          else {                                        // this walk is spent: next constant
-            c += cstep;
-            cm = to_mont(c, M);
-            y = y0; x = y0; q = M.one;
-          }
+  u64 steps = 0, since = 0;                            // since: steps in q
+  bool fine = n < 1ull << 40;                          // gcds within windows, with backtracking
+  // gcd of the batch in every lane; a divisor found by any lane, or 0
+  auto test = [&]() -> u64 {
+    u64 mine = 0;
+    bool spent = false;
+    const u64 g = gcd64(q, n);
+    if (g != 1) {
+      if (g != n) mine = g;
+      else {
+        const u64 gb = fine ? rho_backtrack<Ar>(x, ys, cm, n, M) : n;
+        if (gb != 1 && gb != n) mine = gb;
+        else {                                          // this walk is spent: next constant
+          spent = true;
+          c += cstep;
+          cm = to_mont(c, M);
+          y = y0; x = y0; q = M.one;
         }
       }
-      const unsigned has = __ballot_sync(FULL, mine != 0);
-      if (has) return __shfl_sync(FULL, mine, __ffs(has) - 1);
-      const u64 ext = poll(steps);
+    }
+    since = 0;
+    const unsigned has = __ballot_sync(FULL, mine != 0);
+    fine = __any_sync(FULL, spent) || fine;
+    return has ? __shfl_sync(FULL, mine, __ffs(has) - 1) : 0;
+  };
+  for (u64 r = r0;; r <<= 1) {
+    x = y;
+    if (steps + 2 * r > budget) return since ? test() : 0;
+    for (u64 i = 0; i < r;) {
+      const u64 lim = RHO_POLL < r - i ? RHO_POLL : r - i;
+      for (u64 k = 0; k < lim; ++k) y = Ar::add(Ar::mul(y, y, M), cm, M);
+      i += lim;
+      const u64 ext = poll();
+      if (ext) return ext == ~0ull ? 0 : ext;
+    }
+    steps += r;
+    for (u64 k = 0; k < r;) {
+      const u64 lim = RHO_POLL < r - k ? RHO_POLL : r - k;
+      if (!since) ys = y;
+      // q takes y while the next y is computed: two independent multiplies in flight
+      y = Ar::add(Ar::mul(y, y, M), cm, M);
+      for (u64 i = 1; i < lim; ++i) {
+        const u64 next = Ar::add(Ar::mul(y, y, M), cm, M);
+        q = Ar::mul(q, x > y ? x - y : y - x, M);     // a closed cycle makes q = 0 mod n
+        y = next;
+      }
+      q = Ar::mul(q, x > y ? x - y : y - x, M);
+      k += lim;
+      steps += lim;
+      since += lim;
+      if (since >= RHO_BATCH || (fine && k == r)) {
+        const u64 d = test();
+        if (d) return d;
+      }
+      const u64 ext = poll();
       if (ext) return ext == ~0ull ? 0 : ext;
     }
   }
 }
 
-// One round of elliptic curves on n, one per lane: lane l takes sigma0 + l. poll()
-// returns what rho_walk's does (a divisor handed in, ~0 to stop, 0 to go on); a nonzero answer
-// ends the round and is left in ext. Returns the first divisor a lane found (the same value in
-// every lane), or 0.
-template <class Ar, class Poll>
-__device__ inline u64 warp_ecm(const Mont &M, u64 sigma0, u32 lane, Poll poll, u64 &ext) {
-  ext = 0;
-  auto p = [&]() -> bool { ext = poll(); return ext != 0; };
-  const u64 d = ecm_curve<Ar>(sigma0 + lane, M, p);
+// When a warp's round of curves on n may stop: its slot was withdrawn or split, its rung became
+// moot, or its team is done. Null pointers ask nothing.
+struct CurveStop {
+  const unsigned long long *n_at, *found, *found2;
+  u64 n;
+  const unsigned int *busy;
+  const volatile int *cancel;
+  int my_k;
+};
+
+// One round of elliptic curves on n < 2^62, one per lane: lane l takes sigma0 + l. Returns the first
+// divisor a lane found (the same value in every lane), or 0. Not inlined: one copy of the curve's
+// code serves owners and helpers, so that it stays in the instruction cache.
+static __device__ __noinline__ u64 warp_ecm(const Mont M, u64 sigma0, u32 lane, const CurveStop stop) {
+  auto poll = [&]() -> bool {
+    int end = 0;
+    if (lane == 0)
+      end = (stop.n_at && ld_volatile(stop.n_at) != stop.n) || (stop.found && ld_volatile(stop.found) != 0) || (stop.found2 && ld_volatile(stop.found2) != 0) ||
+            (stop.busy && ld_volatile(stop.busy) == 0) || cancelled(stop.cancel, stop.my_k);
+    return __shfl_sync(FULL, end, 0) != 0;
+  };
+  const u64 d = ecm_curve<LazyArith>(sigma0 + lane, M, poll);
   const unsigned has = __ballot_sync(FULL, d != 0);
   return has ? __shfl_sync(FULL, d, __ffs(has) - 1) : 0;
 }
 
-// Rho steps per lane before a cofactor goes to ECM: rho is the cheaper method for a prime
-// factor below ~2^22 (its expected walk over 32 lanes is a few hundred steps), ECM above.
-#ifndef ES_ECM_AFTER
-#define ES_ECM_AFTER 512
-#endif
-constexpr u64 ECM_AFTER = ES_ECM_AFTER;
+// Rho steps per lane before the owner of a cofactor turns to ECM: rho is the cheaper method for a
+// prime factor below ~2^20 (its expected walk over 32 lanes is a few hundred steps), ECM above.
+// 230 takes the windows of 16, 32 and 64 steps: 28 us, half a round of curves. Against 512 steps the
+// 2^34 windows at 1e15 took 0.164 instead of 0.185 ms of stage D.
+constexpr u64 ECM_AFTER = 230;
 constexpr u32 ECM_OWNER_ROUNDS = 32;     // 1024 curves: a 31-bit factor survives them w.p. ~2e-7
 constexpr u64 ECM_SIGMA_OWNER = 6;       // owner round r: sigma = 6 + 32 r + lane
-constexpr u64 ECM_SIGMA_HELP = 4096;     // helper session t: sigma = 4096 + 32 t + lane
-constexpr u64 ECM_SIGMA_LOCAL = 1ull << 22;   // block-mate session t: sigma = 2^22 + 32 t + lane
-constexpr u32 LOCAL_HELP_POLLS = 1u << 16;   // empty-slot polls (0.5 us apart) before a block-mate stops
-constexpr u32 LOCAL_HELP_ROUNDS = 1u << 12;  // curve rounds per block-mate and prime, at most
-#ifndef ES_LOCAL_HELP
-#define ES_LOCAL_HELP 1
-#endif
-// Helpers on the hard board run rounds of curves (1) or Brent walks (0).
-#ifndef ES_HELP_ECM
-#define ES_HELP_ECM 0
-#endif
+constexpr u64 ECM_SIGMA_HELP = 1ull << 22;    // helper session t: sigma = 2^22 + 32 t + lane
+constexpr u64 ECM_SIGMA_BOARD = 1ull << 32;   // board session t: sigma = 2^32 + 32 t + lane
+constexpr u32 HELP_POLLS = 1u << 16;     // empty polls (0.5 us apart) before a helper stops
+constexpr u32 BOARD_POLLS = 256;         // the same for the board
+constexpr u32 HELP_ROUNDS = 1u << 12;    // curve rounds per helper and wait, at most
 
 __device__ inline u64 warp_rho(u64 n, u32 lane, volatile u64 *found, u32 *status, const volatile int *cancel = nullptr,
-                               int my_k = 0, const HardBoard *board = nullptr, u64 budget = WARP_RHO_STEPS,
+                               int my_k = 0, BlockHelp *bh = nullptr, u32 slot = 0, u64 budget = WARP_RHO_STEPS,
                                bool use_ecm = true) {
   const Mont M = mont_init(n);
-  int slot = -1;                                   // the board slot this warp posted n in
-  bool local_posted = false;                       // n is in the block's own slot
+  const bool posted = bh && n < LazyArith::NMAX;
   bool stop = false;                               // cancelled (warp-uniform)
-  BlockHelp *const bh = board ? board->local : nullptr;
-  auto poll = [&](u64 steps) -> u64 {
+  const bool few = bh && bh->board.slot;
+  auto post = [&]() {
+    if (!posted || lane) return;
+    st_volatile(&bh->found[slot], 0);
+    __threadfence_block();
+    st_volatile(&bh->n[slot], n);
+  };
+  if (few) post();
+  BoardSlot *far = nullptr;                        // this warp's slot on the board
+  auto poll = [&]() -> u64 {
     u64 ext = 0;
-    if (lane == 0 && bh) {
-      if (!local_posted && steps >= RHO_POST_STEPS && n < LazyArith::NMAX) {
-        local_posted = atomicCAS(&bh->n, 0ull, (unsigned long long)n) == 0ull;
-        if (local_posted) *(volatile unsigned long long *)&bh->found = 0;   // no divisor of an earlier one
-      }
-      if (local_posted) {
-        const u64 d = *(volatile unsigned long long *)&bh->found;
+    if (lane == 0) {
+      if (far) {
+        const u64 d = ld_volatile(&far->found);
         if (d > 1 && d < n && n % d == 0) ext = d;
       }
-    }
-    if (lane == 0 && !ext) {
-      if (cancelled(cancel, my_k)) ext = ~0ull;
-      else if (board && slot < 0 && steps >= RHO_POST_STEPS) {
-        for (u32 j = 0; j < HARD_SLOTS; ++j)
-          if (atomicCAS(&board->slot[j].state, 0u, 1u) == 0u) {
-            board->slot[j].n = n;
-            board->slot[j].found = 0;
-            __threadfence();
-            atomicExch(&board->slot[j].state, 2u);
-            slot = (int)j;
-            break;
-          }
-        if (slot < 0) slot = (int)HARD_SLOTS;      // board full: do not try again
-      } else if (board && slot >= 0 && slot < (int)HARD_SLOTS) {
-        const u64 d = ld_volatile(&board->slot[slot].found);
+      if (posted && !ext) {
+        const u64 d = ld_volatile(&bh->found[slot]);
         if (d > 1 && d < n && n % d == 0) ext = d;
+        else if (d) st_volatile(&bh->found[slot], 0);       // of an earlier cofactor
       }
+      if (!ext && cancelled(cancel, my_k)) ext = ~0ull;
     }
     ext = __shfl_sync(FULL, ext, 0);
     if (ext == ~0ull) stop = true;
@@ -290,33 +308,46 @@ __device__ inline u64 warp_rho(u64 n, u32 lane, volatile u64 *found, u32 *status
   if (n >= LazyArith::NMAX) {
     f = rho_walk<ExactArith>(n, M, 1 + lane, 32, budget, lane, poll);
   } else {
-    const u64 after = board && board->ecm_after ? board->ecm_after : ECM_AFTER;
-    const bool ecm = use_ecm && budget >= after + ECM_ROUND_STEPS;
-    f = rho_walk<LazyArith>(n, M, 1 + lane, 32, ecm ? after : budget, lane, poll);
-    if (!f && !stop && ecm) {
-      u64 steps = after;
-      u64 ext = poll(RHO_POST_STEPS > steps ? RHO_POST_STEPS : steps);   // post n to the board now
-      if (ext && ext != ~0ull) f = ext;
-      for (u32 round = 0; !f && !stop && round < ECM_OWNER_ROUNDS && steps + ECM_ROUND_STEPS <= budget; ++round) {
-        f = warp_ecm<LazyArith>(M, ECM_SIGMA_OWNER + 32 * (u64)round, lane, [&]() -> u64 { return poll(steps); }, ext);
-        steps += ECM_ROUND_STEPS;
-        if (!f && ext && ext != ~0ull) f = ext;
+    const bool ecm = use_ecm && budget >= ECM_AFTER + ECM_ROUND_STEPS;
+    u64 steps = 0;
+    for (u32 part = 0; !f && !stop && part < 2; ++part) {            // rho, curves, rho again
+      const u64 lim = part == 0 && ecm ? ECM_AFTER : budget - steps;
+      if (part == 0 || steps < budget) f = rho_walk<LazyArith>(n, M, 1 + lane + 32 * 1024 * part, 32, lim, lane, poll);
+      steps += lim;
+      if (!ecm) break;
+      if (!few && !f && !stop && part == 0) post();
+      if (few && !f && !stop && part == 0 && posted && lane == 0) {
+        for (u32 j = 0; j < BOARD_SLOTS && !far; ++j) {
+          BoardSlot *const b = bh->board.slot + (slot + blockIdx.x + j) % BOARD_SLOTS;
+          if (atomicCAS(&b->state, 0u, 1u) != 0u) continue;
+          far = b;
+          st_volatile(&b->found, 0);
+          st_volatile(&b->n, n);
+          __threadfence();
+          atomicExch(&b->state, 2u);
+        }
       }
-      if (!f && !stop && steps < budget)
-        f = rho_walk<LazyArith>(n, M, 1 + lane + 32 * 1024, 32, budget - steps, lane, poll);
+      const CurveStop cs{nullptr, posted ? &bh->found[slot] : nullptr, far ? &far->found : nullptr, n, nullptr, cancel, my_k};
+      for (u32 round = 0; part == 0 && !f && !stop && round < ECM_OWNER_ROUNDS && steps + ECM_ROUND_STEPS <= budget; ++round) {
+        f = warp_ecm(M, ECM_SIGMA_OWNER + 32 * (u64)round, lane, cs);
+        steps += ECM_ROUND_STEPS;
+        if (f) break;
+        const u64 ext = poll();
+        if (ext && ext != ~0ull) f = ext;
+      }
     }
   }
-  if (lane == 0 && local_posted) {                 // take n out of the block's slot
-    *(volatile unsigned long long *)&bh->found = 0;
-    __threadfence_block();
-    atomicExch(&bh->n, 0ull);
-  }
-  if (lane == 0 && slot >= 0 && slot < (int)HARD_SLOTS) {  // take n off the board
-    atomicExch(&board->slot[slot].state, 1u);
-    board->slot[slot].n = 0;
-    board->slot[slot].found = 0;
+  if (lane == 0 && far) {                          // withdraw n
+    atomicExch(&far->state, 1u);
+    st_volatile(&far->n, 0);
+    st_volatile(&far->found, 0);
     __threadfence();
-    atomicExch(&board->slot[slot].state, 0u);
+    atomicExch(&far->state, 0u);
+  }
+  if (lane == 0 && posted) {
+    st_volatile(&bh->n[slot], 0);
+    __threadfence_block();
+    st_volatile(&bh->found[slot], 0);
   }
   if (lane == 0) *found = f;
   __syncwarp();
@@ -324,114 +355,80 @@ __device__ inline u64 warp_rho(u64 n, u32 lane, volatile u64 *found, u32 *status
   return f;
 }
 
-// One helping pass of a warp with nothing else to do: pick a posted cofactor, walk HELP_STEPS
-// steps per lane with constants no other walk uses (or run a round of curves, with ecm), and
-// post the first divisor found. Returns 2 when every prime of the run is finished, 0 when the
-// board was empty, 1 otherwise. All lanes call.
-__device__ inline int warp_help_once(const HardBoard &B, u32 lane, bool ecm) {
-  if (ld_volatile(B.done) >= B.total) return 2;
-  const u32 st = lane < HARD_SLOTS ? ld_volatile(&B.slot[lane].state) : 0u;
-  const unsigned posted = __ballot_sync(FULL, st == 2u);
-  if (!posted) return 0;
-  u64 ses = 0;
-  if (lane == 0) ses = atomicAdd(B.sessions, 1ull);
-  ses = __shfl_sync(FULL, ses, 0);
-  u32 pick = (u32)(ses % (u64)__popc(posted)), j = 0;
-  for (unsigned m = posted;; m &= m - 1) {
-    if (pick-- == 0) { j = (u32)(__ffs(m) - 1); break; }
-  }
-  HardSlot *hs = &B.slot[j];
-  const u64 n = ld_volatile(&hs->n);
-  __threadfence();
-  if (ld_volatile(&hs->state) != 2u || n <= 0xFFFFFFFFull || !(n & 1)) return 1;
-  const Mont M = mont_init(n);
-  auto poll = [&](u64) -> u64 {
-    u64 ext = 0;
-    if (lane == 0)
-      ext = (ld_volatile(&hs->state) != 2u || ld_volatile(&hs->n) != n || ld_volatile(&hs->found) != 0) ? ~0ull : 0;
-    return __shfl_sync(FULL, ext, 0);
-  };
-  // A round of curves polls its slot every few ladder bits and every few giant steps, so it
-  // stops as soon as the cofactor is split; its sigmas lie above every owner's (an owner's round
-  // r uses 6 + 32 r + lane, r < ECM_OWNER_ROUNDS) and are distinct per session. Rho walks take
-  // constants above every owner's (an owner walks c = 1 + lane + 32 j with j below 2^12),
-  // distinct per session (2^20 sessions apart before a restart adds 2^25); a posted cofactor has
-  // already outlasted its owner's first walks, so helpers start with a longer window.
-  u64 d = 0;
-  if (ecm && n < LazyArith::NMAX) {
-    u64 ext = 0;
-    d = warp_ecm<LazyArith>(M, ECM_SIGMA_HELP + 32 * (ses & 0xFFFFFull), lane, [&]() -> u64 { return poll(0); },
-                            ext);
-  } else {
-    const u64 c0 = (1ull << 24) + 32 * (ses & 0xFFFFFull) + 1 + lane;
-    d = n < LazyArith::NMAX ? rho_walk<LazyArith>(n, M, c0, 1ull << 25, HELP_STEPS, lane, poll, ES_HELP_R0)
-                            : rho_walk<ExactArith>(n, M, c0, 1ull << 25, HELP_STEPS, lane, poll, ES_HELP_R0);
-  }
-  if (lane == 0 && d > 1 && d < n && n % d == 0 && ld_volatile(&hs->n) == n)
-    atomicCAS(&hs->found, 0ull, (unsigned long long)d);
-  __syncwarp();
-  return 1;
-}
-
-// A warp with nothing left to do helps the posted cofactors until every prime of the run is
-// finished (or the board stays empty for HELP_IDLE_POLLS polls, or after HELP_MAX_ROUNDS
-// sessions). All lanes call.
-__device__ inline void warp_help(const HardBoard &B, u32 lane) {
-  for (u32 idle = 0, round = 0; idle < HELP_IDLE_POLLS && round < HELP_MAX_ROUNDS + HELP_IDLE_POLLS; ++round) {
-    const int h = warp_help_once(B, lane, ES_HELP_ECM);
-    if (h == 2) return;
-    if (h == 0) {
-      ++idle;
-      __nanosleep(ES_HELP_SLEEP_NS);
+// A warp with no rung of its own helps the block's posted cofactors until *done is zero: rounds of
+// curves with sigmas of their own, the open slots in turn by session, at most CURVE_WARPS warps at a
+// time, each round polling its slot every few ladder bits. `busy`: the round stops when it is zero
+// too. Bounded: HELP_POLLS empty polls at most, and every round is bounded. All lanes call.
+__device__ inline void warp_help(BlockHelp *bh, const unsigned int *done, const unsigned int *busy, u32 lane) {
+  for (u32 idle = 0, rounds = 0; idle < HELP_POLLS && rounds < HELP_ROUNDS;) {
+    if (!__shfl_sync(FULL, ld_volatile(done), 0)) return;
+    // lane i looks at slot i: a cofactor not split yet, with the fewest helpers
+    const u64 mine = lane < BLOCK_WARPS ? ld_volatile(&bh->n[lane]) : 0;
+    unsigned open = __ballot_sync(FULL, mine && !ld_volatile(&bh->found[lane % BLOCK_WARPS]));
+    u32 go = 0, ses = 0;
+    if (open && lane == 0) {
+      go = atomicAdd(&bh->curves, 1u) < (bh->board.slot ? CURVE_WARPS_FEW : CURVE_WARPS);
+      if (go) ses = atomicAdd(&bh->sessions, 1u);
+      else atomicSub(&bh->curves, 1u);
     }
-  }
-}
-
-// A warp that has finished its rungs helps the block's posted cofactor until every warp of the
-// block has finished: rounds of curves with sigmas of their own (2^22 + 32 t + lane, t the
-// block's session count), each polling the slot every few ladder bits so that it stops as soon
-// as the cofactor is split or withdrawn. Bounded: LOCAL_HELP_POLLS empty polls at most, and
-// every round is bounded. All lanes call.
-__device__ inline void warp_help_block(BlockHelp *bh, u32 lane) {
-  for (u32 idle = 0, rounds = 0; idle < LOCAL_HELP_POLLS && rounds < LOCAL_HELP_ROUNDS;) {
-    u64 n = 0, found = 0;
-    u32 busy = 0;
-    if (lane == 0) {
-      busy = *(volatile unsigned int *)&bh->busy;
-      n = *(volatile unsigned long long *)&bh->n;
-      found = *(volatile unsigned long long *)&bh->found;
-    }
-    busy = __shfl_sync(FULL, busy, 0);
-    if (!busy) return;
-    n = __shfl_sync(FULL, n, 0);
-    found = __shfl_sync(FULL, found, 0);
-    if (!n || found || n >= LazyArith::NMAX || !(n & 1)) { ++idle; __nanosleep(500); continue; }
+    go = __shfl_sync(FULL, go, 0);
+    if (!go) { ++idle; __nanosleep(500); continue; }
     ++rounds;
-    u32 ses = 0;
-    if (lane == 0) ses = atomicAdd(&bh->sessions, 1u);
     ses = __shfl_sync(FULL, ses, 0);
+    for (u32 skip = ses % __popc(open); skip; --skip) open &= open - 1;
+    const u32 j = __ffs(open) - 1;
+    const u64 n = __shfl_sync(FULL, mine, j);
     const Mont M = mont_init(n);
-    auto poll = [&]() -> u64 {
-      u64 stop = 0;
-      if (lane == 0)
-        stop = (*(volatile unsigned long long *)&bh->n != n || *(volatile unsigned long long *)&bh->found != 0 ||
-                *(volatile unsigned int *)&bh->busy == 0) ? ~0ull : 0;
-      return __shfl_sync(FULL, stop, 0);
-    };
-    u64 ext = 0;
-    const u64 d = warp_ecm<LazyArith>(M, ECM_SIGMA_LOCAL + 32 * (u64)ses, lane, poll, ext);
-    if (lane == 0 && d > 1 && d < n && n % d == 0 && *(volatile unsigned long long *)&bh->n == n)
-      atomicCAS(&bh->found, 0ull, (unsigned long long)d);
+    const u64 d = warp_ecm(M, ECM_SIGMA_HELP + 32 * (u64)ses, lane, CurveStop{&bh->n[j], &bh->found[j], nullptr, n, busy, nullptr, 0});
+    if (lane == 0) {
+      if (d > 1 && d < n && n % d == 0 && ld_volatile(&bh->n[j]) == n) atomicCAS(&bh->found[j], 0ull, (unsigned long long)d);
+      atomicSub(&bh->curves, 1u);
+    }
     __syncwarp();
   }
 }
 
-// The prime factors of a cofactor v > 2^32 with no prime factor below 2^16 (so at most three
-// of them), appended to F: primes and squares at once, anything else split by warp_rho. All
-// lanes call. Returns false when a bound was hit (status says which) or on cancellation.
+// A warp of a block that is done helps the board's cofactors until all `total` primes are. Bounded as
+// warp_help. All lanes call.
+__device__ inline void warp_help_board(const Board &B, u64 total, u32 lane) {
+  for (u32 idle = 0, rounds = 0; idle < BOARD_POLLS && rounds < HELP_ROUNDS;) {
+    if (__shfl_sync(FULL, ld_volatile(B.done), 0) >= total) return;
+    unsigned open[BOARD_SLOTS / 32];
+    u32 count = 0;
+    #pragma unroll
+    for (u32 i = 0; i < BOARD_SLOTS / 32; ++i) {
+      const BoardSlot *b = B.slot + 32 * i + lane;
+      open[i] = __ballot_sync(FULL, ld_volatile(&b->state) == 2u && !ld_volatile(&b->found));
+      count += __popc(open[i]);
+    }
+    if (!count) { ++idle; __nanosleep(500); continue; }
+    ++rounds;
+    u64 ses = 0;
+    if (lane == 0) ses = atomicAdd(B.sessions, 1ull);
+    ses = __shfl_sync(FULL, ses, 0);
+    u32 skip = (u32)(ses % count), i = 0;
+    while (skip >= (u32)__popc(open[i])) skip -= __popc(open[i++]);
+    unsigned m = open[i];
+    for (; skip; --skip) m &= m - 1;
+    BoardSlot *const b = B.slot + 32 * i + (__ffs(m) - 1);
+    u64 n = ld_volatile(&b->n);
+    __threadfence();
+    if (ld_volatile(&b->state) != 2u) n = 0;
+    n = __shfl_sync(FULL, n, 0);
+    if (n <= 0xFFFFFFFFull || n >= LazyArith::NMAX || !(n & 1)) continue;
+    const u64 d = warp_ecm(mont_init(n), ECM_SIGMA_BOARD + 32 * ses, lane, CurveStop{&b->n, &b->found, nullptr, n, nullptr, nullptr, 0});
+    if (lane == 0 && d > 1 && d < n && n % d == 0 && ld_volatile(&b->n) == n) atomicCAS(&b->found, 0ull, (unsigned long long)d);
+    __syncwarp();
+  }
+}
+
+// The prime factors of a cofactor v0 > 2^32 with no prime factor below 2^16 (so at most three
+// of them), appended to F: primes and squares at once, anything else split by warp_rho. `composite`:
+// v0 is known to be neither a prime nor a square. All lanes call. Returns false when a bound was hit
+// (status says which) or on cancellation.
 __device__ inline bool warp_factor_cofactor(u64 v0, WarpFac &F, u32 *status, u32 lane, volatile u64 *rho_slot,
-                                            const volatile int *cancel, int my_k, const HardBoard *board,
-                                            u64 rho_budget, bool use_ecm) {
+                                            const volatile int *cancel, int my_k, BlockHelp *bh, u32 slot,
+                                            u64 rho_budget, bool use_ecm, bool composite) {
   u64 stack[4];
   int sp = 0;
   stack[sp++] = v0;
@@ -440,10 +437,12 @@ __device__ inline bool warp_factor_cofactor(u64 v0, WarpFac &F, u32 *status, u32
     const u64 v = stack[--sp];
     if (v == 1) continue;
     if (cancel && __shfl_sync(FULL, cancelled(cancel, my_k) ? 1 : 0, 0)) return false;
-    if (v <= 0xFFFFFFFFull || warp_is_prime(v, lane)) { wf_add(F, v, 1, lane); continue; }
-    const u64 s = isqrt64(v);
-    if (s * s == v) { wf_add(F, s, 2, lane); continue; }
-    const u64 d = warp_rho(v, lane, rho_slot, status, cancel, my_k, board, rho_budget, use_ecm);
+    if (!composite || guard) {
+      if (v <= 0xFFFFFFFFull || warp_is_prime(v, lane)) { wf_add(F, v, 1, lane); continue; }
+      const u64 s = isqrt64(v);
+      if (s * s == v) { wf_add(F, s, 2, lane); continue; }
+    }
+    const u64 d = warp_rho(v, lane, rho_slot, status, cancel, my_k, bh, slot, rho_budget, use_ecm);
     if (d == 0) return false;                  // budget (status set) or cancelled
     if (sp + 2 > 4) { if (lane == 0) atomicOr(status, ST_STACK_OVERFLOW); return false; }
     stack[sp++] = d;
@@ -486,46 +485,57 @@ __device__ __forceinline__ u32 mod_a0(u32 hi, u32 mid, u32 lo, u32 q, u32 m) {  
 
 // S for A_k = A0 + k, k < TD_RUNGS, A0 < 2^64, from tdqm[i] = {d_i, floor(2^32 / d_i)} over
 // the odd primes d_i below 2^16. Each thread takes SIEVE_BATCH primes at a time, their table
-// entries loaded together before any is used. Every thread of the block calls; the block
-// synchronizes on entry and exit.
+// entries loaded together before any is used. Every thread of a team calls (tid of TEAM_THREADS); the
+// team synchronizes on entry and exit.
+constexpr int TEAM_WARPS = 4, TEAM_THREADS = 32 * TEAM_WARPS;
+// Barrier of a team: hardware barrier `bar` over its threads.
+__device__ __forceinline__ void team_sync(u32 bar) { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(TEAM_THREADS) : "memory"); }
 constexpr int SIEVE_BATCH = 8;
-__device__ inline void block_td_sieve(u64 A0, const uint2 *__restrict__ tdqm, TdSieve &S) {
+__device__ inline void team_td_sieve(u64 A0, const uint2 *__restrict__ tdqm, TdSieve &S, u32 tid, u32 bar) {
   const u32 hi = (u32)(A0 >> 32), mid = (u32)(A0 >> 16) & 0xFFFFu, lo = (u32)A0 & 0xFFFFu;
-  for (int k = threadIdx.x; k < TD_RUNGS; k += blockDim.x) S.n[k] = 0;
-  if (threadIdx.x < TD_SMALL) {
-    const uint2 e = __ldg(tdqm + threadIdx.x);
-    S.qm[threadIdx.x] = e;
-    S.rs[threadIdx.x] = mod_a0(hi, mid, lo, e.x, e.y);
+  for (u32 k = tid; k < TD_RUNGS; k += TEAM_THREADS) S.n[k] = 0;
+  if (tid < TD_SMALL) {
+    const uint2 e = __ldg(tdqm + tid);
+    S.qm[tid] = e;
+    S.rs[tid] = mod_a0(hi, mid, lo, e.x, e.y);
   }
-  __syncthreads();
-  for (int k = threadIdx.x; k < TD_RUNGS; k += blockDim.x) {   // the small primes, rung by rung
+  team_sync(bar);
+  for (u32 k = tid; k < TD_RUNGS; k += TEAM_THREADS) {   // the small primes, rung by rung
     u32 mask = 0;
     #pragma unroll
     for (int i = 0; i < TD_SMALL; ++i) {
       const uint2 e = S.qm[i];
-      if (mod_q16(S.rs[i] + (u32)k, e.x, e.y) == 0) mask |= 1u << i;
+      if (mod_q16(S.rs[i] + k, e.x, e.y) == 0) mask |= 1u << i;
     }
     S.small[k] = mask;
   }
-  for (int i0 = TD_SMALL + threadIdx.x; i0 < NTD; i0 += SIEVE_BATCH * blockDim.x) {
-    uint2 e[SIEVE_BATCH];
+  uint2 e[SIEVE_BATCH], nx[SIEVE_BATCH];
+  auto load = [&](int i0, uint2 (&to)[SIEVE_BATCH]) {
     #pragma unroll
     for (int j = 0; j < SIEVE_BATCH; ++j) {
-      const int i = i0 + j * (int)blockDim.x;
-      e[j] = i < NTD ? __ldg(tdqm + i) : make_uint2(0u, 0u);
+      const int i = i0 + j * TEAM_THREADS;
+      to[j] = i < NTD ? __ldg(tdqm + i) : make_uint2(1u, ~0u);       // 1: residue 0, never a listed prime
     }
+  };
+  load(TD_SMALL + tid, nx);
+  for (int i0 = TD_SMALL + tid; i0 < NTD; i0 += SIEVE_BATCH * TEAM_THREADS) {
+    #pragma unroll
+    for (int j = 0; j < SIEVE_BATCH; ++j) e[j] = nx[j];
+    load(i0 + SIEVE_BATCH * TEAM_THREADS, nx);
+    u32 k[SIEVE_BATCH];
     #pragma unroll
     for (int j = 0; j < SIEVE_BATCH; ++j) {
-      if (!e[j].x) continue;
       const u32 r = mod_a0(hi, mid, lo, e[j].x, e[j].y);
-      const u32 k = r ? e[j].x - r : 0u;                 // q > TD_RUNGS: one rung at most
-      if (k < (u32)TD_RUNGS) {
-        const u32 s = atomicAdd(&S.n[k], 1u);
-        if (s < (u32)TD_LIST_CAP) S.idx[k][s] = (u16)(i0 + j * (int)blockDim.x);
-      }
+      k[j] = r ? e[j].x - r : (e[j].x == 1 ? ~0u : 0u);                // q > TD_RUNGS: one rung at most
     }
+    #pragma unroll
+    for (int j = 0; j < SIEVE_BATCH; ++j)
+      if (k[j] < (u32)TD_RUNGS) {
+        const u32 s = atomicAdd(&S.n[k[j]], 1u);
+        if (s < (u32)TD_LIST_CAP) S.idx[k[j]][s] = (u16)(i0 + j * TEAM_THREADS);
+      }
   }
-  __syncthreads();
+  team_sync(bar);
 }
 
 // Complete factorization of n >= 1 into F (prime order as found). All lanes call.
@@ -536,7 +546,7 @@ __device__ inline void block_td_sieve(u64 A0, const uint2 *__restrict__ tdqm, Td
 __device__ inline bool warp_factor(u64 n, WarpFac &F, const u32 *__restrict__ tdp, const u64 *__restrict__ tdi,
                                    u32 *status, u32 lane, volatile u64 *rho_slot,
                                    const volatile int *cancel = nullptr, int my_k = 0,
-                                   const HardBoard *board = nullptr, u64 rho_budget = WARP_RHO_STEPS,
+                                   BlockHelp *bh = nullptr, u32 slot = 0, u64 rho_budget = WARP_RHO_STEPS,
                                    bool use_ecm = true, u64 *hard_left = nullptr,
                                    const u16 *td_list = nullptr, u32 td_n = ~0u, u32 td_small = 0) {
   if (hard_left) *hard_left = 0;
@@ -646,7 +656,7 @@ __device__ inline bool warp_factor(u64 n, WarpFac &F, const u32 *__restrict__ td
       else if (s * s == cur) wf_add(F, s, 2, lane);     // s is prime: no factor of cur is below 2^16
       else *hard_left = cur;                             // needs rho: left to the caller
     } else {
-      return warp_factor_cofactor(cur, F, status, lane, rho_slot, cancel, my_k, board, rho_budget, use_ecm);
+      return warp_factor_cofactor(cur, F, status, lane, rho_slot, cancel, my_k, bh, slot, rho_budget, use_ecm, false);
     }
   }
   __syncwarp();
@@ -686,6 +696,72 @@ struct ModR {
     return mod32(mod32((u32)(x >> 32)) * c + mod32((u32)x));   // below RCAP^2 + RCAP < 2^32
   }
 };
+
+// Residues of the divisors of a rung, in two forms that are cheaper than the table of least divisors
+// below (10 us of a rung's latency, most of it 128-bit products): `small` is the least divisor up
+// to 65536 in each residue class, from the primes below 2^16 alone (p and every other prime are
+// larger); `met` the classes that any divisor of q^2 lies in. Both push a class's value along its
+// multiples by a prime, in shared memory.
+constexpr u32 SMALL_U = 65536;
+
+// The least divisor u <= SMALL_U of q^2 with u == target (mod r), p > SMALL_U; 0 if there is none.
+__device__ inline u32 warp_small_divisor(const WarpFac &F, const ModR &R, u32 target, DPWarp &D, u32 lane) {
+  u32 *v = reinterpret_cast<u32 *>(D.v[0]), *w = reinterpret_cast<u32 *>(D.v[1]);
+  const u32 r = R.r;
+  for (u32 t = lane; t < r; t += 32) v[t] = t == (r == 1 ? 0u : 1u) ? 1u : ~0u;
+  __syncwarp();
+  const u64 mine = lane < (u32)F.k ? F.pr[lane] : ~0ull;
+  const u32 my_res = mine < SMALL_U ? R.mod32((u32)mine) : 0u;
+  for (int idx = 0; idx < F.k; ++idx) {
+    const u32 pr = (u32)min(__shfl_sync(FULL, mine, idx), (u64)SMALL_U), res = __shfl_sync(FULL, my_res, idx);
+    if (pr >= SMALL_U) continue;
+    const int e = 2 * (int)F.ex[idx];
+    for (u32 t = lane; t < r; t += 32) w[t] = v[t];
+    __syncwarp();
+    for (u32 t = lane; t < r; t += 32) {
+      u32 x = v[t], s = t;
+      if (x == ~0u) continue;
+      for (int j = 0; j < e; ++j) {
+        x *= pr;                                       // below 2^16 2^16
+        if (x > SMALL_U) break;
+        s = R.mod32(s * res);
+        atomicMin(w + s, x);
+      }
+    }
+    __syncwarp();
+    u32 *const t = v; v = w; w = t;
+  }
+  const u32 u = v[target];
+  __syncwarp();
+  return u == ~0u ? 0u : u;
+}
+
+// Whether a divisor of q^2 = (p A)^2, A's factorization complete in F, is == target (mod r). With
+// target == -q, u and q^2 / u are in the class together and one of them is at most q: the least
+// divisor u <= q in the class exists exactly when the class is met.
+__device__ inline bool warp_class_met(u64 p, const WarpFac &F, const ModR &R, u32 target, DPWarp &D, u32 lane) {
+  unsigned char *v = reinterpret_cast<unsigned char *>(D.v[0]), *w = reinterpret_cast<unsigned char *>(D.v[1]);
+  const u32 r = R.r;
+  for (u32 t = lane; t < r; t += 32) v[t] = t == (r == 1 ? 0u : 1u);
+  __syncwarp();
+  const u32 my_res = R.mod64(lane < (u32)F.k ? F.pr[lane] : p);    // lane F.k <= MAXF: p
+  for (int idx = 0; idx <= F.k; ++idx) {
+    const u32 res = __shfl_sync(FULL, my_res, idx);
+    const int e = idx < F.k ? 2 * (int)F.ex[idx] : 2;
+    for (u32 t = lane; t < r; t += 32) w[t] = v[t];
+    __syncwarp();
+    for (u32 t = lane; t < r; t += 32) {
+      if (!v[t]) continue;
+      u32 s = t;
+      for (int j = 0; j < e; ++j) { s = R.mod32(s * res); w[s] = 1; }
+    }
+    __syncwarp();
+    unsigned char *const t = v; v = w; w = t;
+  }
+  const bool met = v[target] != 0;
+  __syncwarp();
+  return met;
+}
 
 // min_div_res (sieve/rung_scan3.cpp:544-565), lanes over residue classes. Returns the
 // least divisor u <= q of q^2 with u == target (mod r), or 0.
@@ -757,36 +833,37 @@ __device__ __forceinline__ bool rung_of(u64 p, u32 k, Rung &g) {
   return true;
 }
 
-// Below this bound a divisor of q^2 = (pA)^2 cannot involve p or a prime factor of a cofactor
-// that trial division left (every such prime is at least 65537, the first prime after the
-// trial-division table's last, 65521).
-constexpr u64 SMALL_U_BOUND = 65536;
-#ifndef ES_SMALL_U
-#define ES_SMALL_U 1
-#endif
-
 // min_div_res of one rung (sieve/rung_scan3.cpp:544-565): the least divisor u <= q of q^2,
 // q = pA, with u == target (mod r), or u = 0 when there is none. A is factored by trial
 // division first; when that leaves a composite cofactor C (prime factors all >= 65537), the
-// divisors of q^2 below 65537 are exactly those of S^2, S = A / C, so the least qualifying
+// divisors of q^2 up to 65536 are exactly those of S^2, S = A / C, so the least qualifying
 // one among them -- found from S's primes alone -- is the answer whenever it exists, and C is
-// factored (rho, ECM) only when it does not. The same u comes out either way. Returns false
-// when a bound was hit or the rung was cancelled.
+// factored (rho, ECM) only when it does not. The table of least divisors is made only when the
+// class holds a divisor and none up to 65536. Returns false when a bound was hit or the rung was
+// cancelled.
 __device__ inline bool rung_divisor(u64 p, u64 A, U128 q, u32 r, u32 target, WarpFac &F, DPWarp &D,
                                     const u32 *tdp, const u64 *tdi, u32 *status, u32 lane,
                                     volatile u64 *rho_slot, const volatile int *cancel, int my_k,
-                                    const HardBoard *board, u64 rho_budget, bool use_ecm, U128 &u,
+                                    BlockHelp *bh, u32 slot, u64 rho_budget, bool use_ecm, U128 &u,
                                     const u16 *td_list = nullptr, u32 td_n = ~0u, u32 td_small = 0) {
+  const ModR R(r);
   u64 hard = 0;
-  if (!warp_factor(A, F, tdp, tdi, status, lane, rho_slot, cancel, my_k, board, rho_budget, use_ecm,
-                   ES_SMALL_U ? &hard : nullptr, td_list, td_n, td_small))
-    return false;
-  if (hard) {
-    u = warp_min_div_res(p, F, U128{SMALL_U_BOUND, 0}, r, target, D, lane);
-    if (u.lo || u.hi) return true;
-    if (!warp_factor_cofactor(hard, F, status, lane, rho_slot, cancel, my_k, board, rho_budget, use_ecm)) return false;
+  if (p <= SMALL_U) {                                  // probes only: the scans' floors are far above
+    if (!warp_factor(A, F, tdp, tdi, status, lane, rho_slot, cancel, my_k, bh, slot, rho_budget, use_ecm, nullptr,
+                     td_list, td_n, td_small))
+      return false;
+    u = warp_min_div_res(p, F, q, r, target, D, lane);
+    return true;
   }
-  u = warp_min_div_res(p, F, q, r, target, D, lane);
+  if (!warp_factor(A, F, tdp, tdi, status, lane, rho_slot, cancel, my_k, bh, slot, rho_budget, use_ecm, &hard, td_list,
+                   td_n, td_small))
+    return false;
+  u = U128{warp_small_divisor(F, R, target, D, lane), 0};
+  if (u.lo) return true;
+  if (hard &&
+      !warp_factor_cofactor(hard, F, status, lane, rho_slot, cancel, my_k, bh, slot, rho_budget, use_ecm, true))
+    return false;
+  if (warp_class_met(p, F, R, target, D, lane)) u = warp_min_div_res(p, F, q, r, target, D, lane);
   return true;
 }
 
@@ -799,15 +876,14 @@ __device__ inline bool rung_divisor(u64 p, u64 A, U128 q, u32 r, u32 target, War
 // stage D with rho alone, 179 ms with ECM), while ECM pays in the latency-bound tail.
 __device__ inline bool warp_solve_rung(u64 p, const u32 *tdp, const u64 *tdi, u32 *status, WarpFac &F,
                                        DPWarp &D, volatile u64 *rho_slot, RungResult *out,
-                                       const HardBoard *board = nullptr, u64 rho_budget = WARP_RHO_STEPS,
-                                       bool use_ecm = true) {
+                                       u64 rho_budget = WARP_RHO_STEPS, bool use_ecm = true) {
   const u32 lane = threadIdx.x & 31;
   const u32 r0 = rung_r0(p);
   for (u32 k = 0; r0 + 4 * k <= RCAP; ++k) {
     Rung g;
     if (!rung_of(p, k, g)) continue;
     U128 u;
-    if (!rung_divisor(p, g.A, g.q, g.r, g.target, F, D, tdp, tdi, status, lane, rho_slot, nullptr, 0, board,
+    if (!rung_divisor(p, g.A, g.q, g.r, g.target, F, D, tdp, tdi, status, lane, rho_slot, nullptr, 0, nullptr, 0,
                       rho_budget, use_ecm, u))
       return false;
     if (u.lo == 0 && u.hi == 0) continue;
@@ -818,61 +894,63 @@ __device__ inline bool warp_solve_rung(u64 p, const u32 *tdp, const u64 *tdi, u3
   return false;
 }
 
-#ifndef ES_TD_SIEVE
-#define ES_TD_SIEVE 1
-#endif
-// The rung walk of one prime by a block of W warps (solve_rung3, sieve/rung_scan3.cpp:
-// 578-603). Warp w takes rung indices k = w, w+W, ... (r = r0 + 4k) in increasing order and
-// stops once k passes the best certifying index found by any warp. With S the block first
-// lists the odd primes below 2^16 of all the prime's rungs at once (block_td_sieve), and each
-// rung divides out only its own. Returns true in every thread when some rung certifies p;
-// the block's result is then in *out.
-template <int W>
-__device__ inline bool block_solve_rung(u64 p, const u32 *tdp, const u64 *tdi, const uint2 *tdqm, TdSieve *S,
-                                        u32 *status, WarpFac *F, DPWarp *D, volatile u64 *rho_slot, int *best_k,
-                                        RungResult *slot, RungResult *out, const HardBoard *board = nullptr,
-                                        u64 rho_budget = WARP_RHO_STEPS) {
-  const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  BlockHelp *const bh = board ? board->local : nullptr;
-  if (threadIdx.x == 0) {
-    *best_k = 0x7FFFFFFF;
-    if (bh) { bh->n = 0; bh->found = 0; bh->busy = W; }
+// The rung walk of one prime by a team of four warps (solve_rung3, sieve/rung_scan3.cpp:
+// 578-603). Warp w takes rung indices k = w, w+4, ... (r = r0 + 4k) in increasing order and
+// stops once k passes the best certifying index found by any warp. The team first lists the odd
+// primes below 2^16 of all the prime's rungs at once (team_td_sieve), and each rung divides out
+// only its own. Returns true in every thread when some rung certifies p; the team's result is
+// then in *out. F, D, rho_slot and slot are the team's four, warp0 its first slot in *bh, *busy
+// the count of its warps still on their rungs.
+struct Team {
+  WarpFac *F;
+  DPWarp *D;
+  u64 *rho_slot;
+  RungResult *slot, *out;
+  TdSieve *S;
+  int *best_k;
+  unsigned int *busy;
+  BlockHelp *bh;
+  u32 warp0, bar;
+};
+__device__ inline bool team_solve_rung(u64 p, const u32 *tdp, const u64 *tdi, const uint2 *tdqm, u32 *status,
+                                       const Team &T, u64 rho_budget) {
+  const u32 lane = threadIdx.x & 31, tid = threadIdx.x % TEAM_THREADS, w = tid >> 5;
+  if (tid == 0) {
+    *T.best_k = 0x7FFFFFFF;
+    *T.busy = TEAM_WARPS;
   }
-  if (lane == 0) slot[w].k = 0x7FFFFFFF;
-  __syncthreads();
-  if (!ES_TD_SIEVE) S = nullptr;
-  if (S) block_td_sieve((p >> 2) + 1, tdqm, *S);   // A_0 = floor(p/4) + 1
+  if (lane == 0) T.slot[w].k = 0x7FFFFFFF;
+  team_sync(T.bar);
+  team_td_sieve((p >> 2) + 1, tdqm, *T.S, tid, T.bar);   // A_0 = floor(p/4) + 1
   const u32 r0 = rung_r0(p);
-  for (u32 k = w; r0 + 4 * k <= RCAP; k += W) {
+  for (u32 k = w; r0 + 4 * k <= RCAP; k += TEAM_WARPS) {
     // warp-uniform: every lane must take the same branch before the warp collectives below
-    if ((int)k >= __shfl_sync(FULL, *(volatile int *)best_k, 0)) break;
+    if ((int)k >= __shfl_sync(FULL, *(volatile int *)T.best_k, 0)) break;
     Rung g;
     if (!rung_of(p, k, g)) continue;
     U128 u;
-    if (!rung_divisor(p, g.A, g.q, g.r, g.target, F[w], D[w], tdp, tdi, status, lane, rho_slot + w, best_k, (int)k,
-                      board, rho_budget, true, u, S ? S->idx[k] : nullptr, S ? S->n[k] : ~0u, S ? S->small[k] : 0u))
+    if (!rung_divisor(p, g.A, g.q, g.r, g.target, T.F[w], T.D[w], tdp, tdi, status, lane, T.rho_slot + w, T.best_k,
+                      (int)k, T.bh, T.warp0 + w, rho_budget, true, u, T.S->idx[k], T.S->n[k], T.S->small[k]))
       break;
     if (u.lo == 0 && u.hi == 0) continue;
     if (lane == 0) {
-      slot[w] = RungResult{g.A, g.r, k, u};
-      atomicMin(best_k, (int)k);
+      T.slot[w] = RungResult{g.A, g.r, k, u};
+      atomicMin(T.best_k, (int)k);
     }
     break;
   }
-  if (bh) {                                     // done with this prime's rungs: help the others
-    if (lane == 0) atomicSub(&bh->busy, 1u);
-    __syncwarp();
-    if (ES_LOCAL_HELP) warp_help_block(bh, lane);
-  }
-  __syncthreads();
-  const int bk = *(volatile int *)best_k;
+  if (lane == 0) atomicSub(T.busy, 1u);           // done with this prime's rungs: help the others
+  __syncwarp();
+  warp_help(T.bh, T.busy, T.busy, lane);
+  team_sync(T.bar);
+  const int bk = *(volatile int *)T.best_k;
   bool ok = false;
   if (bk != 0x7FFFFFFF) {
     ok = true;
-    if (threadIdx.x == 0)
-      for (int i = 0; i < W; ++i) if ((int)slot[i].k == bk) *out = slot[i];
+    if (tid == 0)
+      for (int i = 0; i < TEAM_WARPS; ++i) if ((int)T.slot[i].k == bk) *T.out = T.slot[i];
   }
-  __syncthreads();
+  team_sync(T.bar);
   return ok;
 }
 

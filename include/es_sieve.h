@@ -204,7 +204,8 @@ typedef struct {
   uint32_t short_max;            /* with long_split = 0, windows whose lanes hold at most this many
                                     positions (1..es_info_t.short_max_limit, 128 in this build) are
                                     marked by rows; default the limit */
-  uint32_t rung_blocks_per_sm;   /* stage-D grid in blocks per SM (1..16); default 6 */
+  uint32_t rung_blocks_per_sm;   /* stage-D teams of four warps per SM (1..16, the
+                                    SM holds four); default 6 */
   uint32_t long_split;           /* 1 (default): every window is marked by rows, long ones in
                                     passes; 0: longer windows go to the segment marking */
   uint32_t reserved[5];          /* zero */
