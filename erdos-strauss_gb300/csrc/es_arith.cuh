@@ -205,8 +205,9 @@ __device__ __forceinline__ bool sprp_mont(u64 bm, u64 d, int s, const Mont &M) {
   const u64 mone = M.n - M.one;                       // Montgomery form of n-1
   u64 x = M.one, b = bm, e = d;
   while (e) {
-    if (e & 1) x = mmul(x, b, M);
+    const u64 t = mmul(x, b, M);                      // both in flight, whatever the bit
     b = mmul(b, b, M);
+    if (e & 1) x = t;
     e >>= 1;
   }
   if (x == M.one || x == mone) return true;
@@ -224,8 +225,9 @@ __device__ __forceinline__ bool sprp_ar(u64 bm, u64 d, int s, const Mont &M) {
   const u64 mone = M.n - M.one;
   u64 x = M.one, b = bm, e = d;
   while (e) {
-    if (e & 1) x = Ar::mul(x, b, M);
+    const u64 t = Ar::mul(x, b, M);
     b = Ar::mul(b, b, M);
+    if (e & 1) x = t;
     e >>= 1;
   }
   x = Ar::norm(x, M);
@@ -293,16 +295,17 @@ __device__ inline bool is_prime64(u64 n) {
 }
 
 // Base-2 SPRP (sieve/rung_scan3.cpp:680-689) on an odd n > 2. The base is 2 = one + one in
-// Montgomery form, so r2 (64 doublings) is not needed; below 2^62 the round runs in the lazy
-// arithmetic.
+// Montgomery form, so r2 is not needed; below 2^62 the round runs in the lazy arithmetic.
+__device__ __forceinline__ bool sprp2_round(const Mont &M) {
+  u64 d = M.n - 1;
+  const int s = __ffsll((long long)d) - 1;
+  d >>= s;
+  return M.n < LazyArith::NMAX ? sprp2_ar<LazyArith>(d, s, M) : sprp2_mont(d, s, M);
+}
 __device__ inline bool sprp2_64(u64 n) {
   if (n < 2) return false;
   if (!(n & 1)) return n == 2;
-  const Mont M = mont_one(n);
-  u64 d = n - 1;
-  const int s = __ffsll((long long)d) - 1;
-  d >>= s;
-  return n < LazyArith::NMAX ? sprp2_ar<LazyArith>(d, s, M) : sprp2_mont(d, s, M);
+  return sprp2_round(mont_one(n));
 }
 
 // ---------------------------------------------------------------- gcd, isqrt

@@ -23,8 +23,8 @@
 //   k_sift        the candidates against the other strides; survivors appended
 //   k_prep, k_mark  the alternative for long windows: a byte map per segment in shared memory,
 //                 each filter clears its progression, warp-aggregated compaction
-//   k_mr          a thread per survivor: the base-2 strong-probable-prime round
-//   k_mr2         a warp per number that passed base 2: the 12-base test, one base per lane
+//   k_mr          Miller-Rabin: the base-2 round by a thread per survivor, the other bases by the
+//                 warp (few survivors: a warp each, one base per lane)
 //   k_rung        stage D: a warp per prime while primes outnumber the grid's warps, then a
 //                 team of four warps per prime over successive rungs; warp trial division,
 //                 Miller-Rabin, Brent's rho, ECM rounds (es_tail.cuh, es_ecm.cuh), the rung
@@ -854,35 +854,45 @@ __global__ void k_square_mask(const u64 *__restrict__ mods, const u64 *__restric
   }
 }
 
-// Miller-Rabin in two passes. Nearly every survivor is composite and fails the base-2
-// round (sprp2, sieve/rung_scan3.cpp:680-689), so pass one runs that round with a thread per
-// survivor; the few that pass get the 12-base test (census/rung_scan.cpp:76-92) with one base
-// per lane of a warp. A prime passes base 2, so the two passes give exactly is_prime.
-__global__ void k_mr(const TailParams T) {
-  const u64 n = min((u64)*T.surv_count, T.cap);
-  for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
-    const Surv s = T.surv[i];
-    if (sprp2_64(s.p)) {
-      const unsigned long long k = atomicAdd(T.cand_count, 1ull);
-      if (k < T.cap) T.cand[k] = (u32)i;
-    }
-  }
+// Miller-Rabin of the survivors (sprp2, sieve/rung_scan3.cpp:680-689, and the 12-base test,
+// census/rung_scan.cpp:76-92; a prime passes base 2, so the two give exactly is_prime). Up to one warp
+// a scheduler, a survivor per warp: all 12 bases at once, one per lane, for the latency of one round.
+// Beyond, each warp takes several survivors, a thread each for base 2 and the warp's lanes for the
+// rest (warp_primes): up to 12 while the list is short enough that latency counts (a warp's survivors
+// share one round to each base pass, and 12 rarely fill a second pass of pairs), else 32.
+// Integer-multiply bound on long lists. With its launch: 6 us with no survivor, 10 for 33 survivors, 18
+// for the 1 K of a 2^34 window at 1e15 and 40 for the 7 K of the 4096-window batch at 1e19; two kernels
+// with a list between them, which this replaced, took 9, 16, 22 and 38; with 32 a warp from the first
+// the last two are 38 and 55.
+#ifndef ES_MR_BLOCKS_PER_SM
+#define ES_MR_BLOCKS_PER_SM 6
+#endif
+constexpr u32 MR_BLOCKS_PER_SM = ES_MR_BLOCKS_PER_SM;
+// Numbers a warp takes at a time, of n in all.
+__device__ __forceinline__ u32 mr_share(u64 n) {
+  const u64 warps = (u64)gridDim.x / MR_BLOCKS_PER_SM * 4, share = (n + warps - 1) / warps;
+  return share > 48 ? 32u : (u32)min(share, 12ull);
 }
-
-__global__ void k_mr2(const TailParams T) {
+// This warp's place among the grid's: the first of every block, on the schedulers in turn, then the
+// second of every block and so on.
+__device__ __forceinline__ u64 mr_warp() {
+  const u32 turn = blockIdx.x / (gridDim.x / MR_BLOCKS_PER_SM);
+  return ((threadIdx.x / 32 + 8 - turn % 8) % 8) * (u64)gridDim.x + blockIdx.x;
+}
+__global__ void __launch_bounds__(256, MR_BLOCKS_PER_SM) k_mr(const TailParams T) {
   const u32 lane = threadIdx.x & 31;
-  const u64 warps = (u64)gridDim.x * blockDim.x / 32;
-  const u64 n = min((u64)*T.cand_count, T.cap);
-  for (u64 i = ((u64)blockIdx.x * blockDim.x + threadIdx.x) / 32; i < n; i += warps) {
-    const u32 si = T.cand[i];
-    const Surv s = T.surv[si];
-    const bool prime = warp_is_prime(s.p, lane);
-    if (lane == 0) {
-      if (prime) {
-        const unsigned long long k = atomicAdd(T.prime_count, 1ull);
-        if (k < T.cap) T.primes[k] = si;
-      }
-    }
+  const u64 warps = (u64)gridDim.x * blockDim.x / 32, w = mr_warp();
+  const u64 n = min((u64)*T.surv_count, T.cap);
+  const u32 share = mr_share(n);
+  for (u64 i0 = w * share; i0 < n; i0 += warps * share) {
+    const u64 i = i0 + lane;
+    const bool valid = lane < share && i < n;
+    const unsigned m = share == 1 ? (u32)warp_is_prime(T.surv[i0].p, lane) : warp_primes(valid ? T.surv[i].p : 0, valid, lane);
+    if (!m) continue;
+    unsigned long long k = 0;
+    if (lane == 0) k = atomicAdd(T.prime_count, (unsigned long long)__popc(m));
+    k = __shfl_sync(FULL, k, 0) + __popc(m & ((1u << lane) - 1));
+    if ((m >> lane & 1) && k < T.cap) T.primes[k] = (u32)i;
   }
 }
 
@@ -1022,12 +1032,16 @@ __global__ void k_probe_check(const RecDev *r, u64 count, unsigned char *ok) {
   }
 }
 
-__global__ void k_probe_prime(const u64 *n, u64 count, unsigned char *out) {
+// As k_mr: 200 K odd numbers take 0.13 ms, 1.25 ms with a warp each.
+__global__ void __launch_bounds__(256, MR_BLOCKS_PER_SM) k_probe_prime(const u64 *n, u64 count, unsigned char *out) {
   const u32 lane = threadIdx.x & 31;
-  const u64 warps = (u64)gridDim.x * blockDim.x / 32;
-  for (u64 i = ((u64)blockIdx.x * blockDim.x + threadIdx.x) / 32; i < count; i += warps) {
-    const bool pr = warp_is_prime(n[i], lane);
-    if (lane == 0) out[i] = pr ? 1 : 0;
+  const u64 warps = (u64)gridDim.x * blockDim.x / 32, w = mr_warp();
+  const u32 share = mr_share(count);
+  for (u64 i0 = w * share; i0 < count; i0 += warps * share) {
+    const u64 i = i0 + lane;
+    const bool valid = lane < share && i < count;
+    const unsigned m = share == 1 ? (u32)warp_is_prime(n[i0], lane) : warp_primes(valid ? n[i] : 0, valid, lane);
+    if (valid) out[i] = m >> lane & 1;
   }
 }
 __global__ void __launch_bounds__(TEAM_THREADS, 4) k_probe_rung(const u64 *p, u64 count, RecDev *out,
@@ -1118,15 +1132,15 @@ struct Slot {
   WinCount *d_cnt = nullptr;
   RowWin *d_roww = nullptr;
   Piece *d_piece = nullptr; u16 *d_pidx = nullptr; u32 *d_rowinfo = nullptr; size_t piece_cap = 0;
-  uint2 *d_cand2 = nullptr; u32 *d_chunk = nullptr; size_t chunk_cap = 0;
+  uint2 *d_cand = nullptr; u32 *d_chunk = nullptr; size_t chunk_cap = 0;
   u16 *d_Qm = nullptr; size_t qm_cap = 0;
   Surv *d_surv = nullptr;
-  u32 *d_primes = nullptr, *d_direct = nullptr, *d_cand = nullptr;
+  u32 *d_primes = nullptr, *d_direct = nullptr;
   RecDev *d_recs = nullptr;
   size_t cap = 0;
   size_t rec_prefix = 0;                // records the captured graph copies back itself
   u64 graph_launches = 0;               // its kernels
-  unsigned long long *d_ctr = nullptr;  // [0] queue [1] surv [2] prime [3] direct [4] rec [5] cand
+  unsigned long long *d_ctr = nullptr;  // [0] queue [1] surv [2] prime [3] direct [4] rec
                                       // [6] rung queue (teams) [7] rung primes done [8] board sessions
                                       // [9] rung queue (warps) [10] candidate chunks, board at [16]
   u32 *d_status = nullptr;
@@ -1288,22 +1302,21 @@ static es_status ensure_capacity(es_engine *e, Slot *sl, size_t nwin, size_t npi
   }
   if (nchunks > sl->chunk_cap) {
     drop_graph(sl);
-    cudaFree(sl->d_cand2); cudaFree(sl->d_chunk);
-    sl->d_cand2 = nullptr; sl->d_chunk = nullptr;
+    cudaFree(sl->d_cand); cudaFree(sl->d_chunk);
+    sl->d_cand = nullptr; sl->d_chunk = nullptr;
     sl->chunk_cap = 0;
-    CU(cudaMalloc(&sl->d_cand2, nchunks * 32 * sizeof(uint2)));
+    CU(cudaMalloc(&sl->d_cand, nchunks * 32 * sizeof(uint2)));
     CU(cudaMalloc(&sl->d_chunk, nchunks * sizeof(u32)));
     sl->chunk_cap = nchunks;
   }
   if (cap > sl->cap) {
     drop_graph(sl);
-    cudaFree(sl->d_surv); cudaFree(sl->d_primes); cudaFree(sl->d_direct); cudaFree(sl->d_recs); cudaFree(sl->d_cand);
+    cudaFree(sl->d_surv); cudaFree(sl->d_primes); cudaFree(sl->d_direct); cudaFree(sl->d_recs);
     cudaFreeHost(sl->h_recs);
-    sl->d_surv = nullptr; sl->d_primes = sl->d_direct = sl->d_cand = nullptr; sl->d_recs = nullptr; sl->h_recs = nullptr;
+    sl->d_surv = nullptr; sl->d_primes = sl->d_direct = nullptr; sl->d_recs = nullptr; sl->h_recs = nullptr;
     CU(cudaMalloc(&sl->d_surv, cap * sizeof(Surv)));
     CU(cudaMalloc(&sl->d_primes, cap * sizeof(u32)));
     CU(cudaMalloc(&sl->d_direct, cap * sizeof(u32)));
-    CU(cudaMalloc(&sl->d_cand, cap * sizeof(u32)));
     CU(cudaMalloc(&sl->d_recs, cap * sizeof(RecDev)));
     CU(cudaMallocHost(&sl->h_recs, cap * sizeof(RecDev)));
     sl->cap = cap;
@@ -1324,18 +1337,9 @@ static MarkParams mark_params(const es_engine *e, const Slot *sl) {
   return P;
 }
 
-// k_mr's grid: a base-2 round is one thread's dependent chain of Montgomery squarings, so
-// the launch wants every warp slot the registers allow (40 registers: 8 blocks of 256 per SM);
-// measured on the 4096-window batch, 2, 4 and 8 blocks per SM gave 1.346, 1.331 and 1.319 ms
-// per step.
-#ifndef ES_MR_BLOCKS_PER_SM
-#define ES_MR_BLOCKS_PER_SM 8
-#endif
-
 static TailParams tail_params(const es_engine *e, const Slot *sl) {
   TailParams T;
   T.surv = sl->d_surv; T.surv_count = sl->d_ctr + 1;
-  T.cand = sl->d_cand; T.cand_count = sl->d_ctr + 5;
   T.primes = sl->d_primes; T.prime_count = sl->d_ctr + 2;
   T.direct = sl->d_direct; T.direct_count = sl->d_ctr + 3;
   T.recs = sl->d_recs; T.rec_count = sl->d_ctr + 4;
@@ -1352,7 +1356,7 @@ static RowParams row_params(const es_engine *e, const Slot *sl) {
   RowParams S;
   S.rho = e->d_rho; S.K0 = e->d_K0; S.fdesc = e->d_fdesc; S.tdense = e->d_tdense; S.tlane = e->d_tlane;
   S.mdesc = e->d_mdesc; S.lfil = e->d_lfil; S.win = sl->d_win; S.roww = sl->d_roww; S.piece = sl->d_piece;
-  S.pidx = sl->d_pidx; S.rowinfo = sl->d_rowinfo; S.cand = sl->d_cand2; S.chunk = sl->d_chunk;
+  S.pidx = sl->d_pidx; S.rowinfo = sl->d_rowinfo; S.cand = sl->d_cand; S.chunk = sl->d_chunk;
   S.chunk_count = sl->d_ctr + 10; S.chunk_cap = (u32)sl->chunk_cap;
   S.surv = sl->d_surv; S.surv_count = sl->d_ctr + 1; S.cnt = sl->d_cnt; S.surv_cap = sl->cap; S.M = e->M;
   S.status = sl->d_status; S.hdr = sl->d_hdr;
@@ -1525,11 +1529,9 @@ static es_status enqueue_front(es_engine *e, Slot *sl, bool persistent, WinCount
     ++launches;
   }
   CU(rec(1));
-  k_mr<<<e->sm_count * ES_MR_BLOCKS_PER_SM, 256, 0, st>>>(T);
+  k_mr<<<e->sm_count * MR_BLOCKS_PER_SM, 256, 0, st>>>(T);
   CU(cudaGetLastError());
-  k_mr2<<<e->sm_count * 2, 256, 0, st>>>(T);
-  CU(cudaGetLastError());
-  launches += 2;
+  ++launches;
   CU(rec(2));
   return ES_OK;
 }
@@ -2424,8 +2426,8 @@ es_status es_close(es_engine *e) {
     if (sl.stream) cudaStreamSynchronize(sl.stream);
     drop_graph(&sl);
     cudaFree(sl.d_win); cudaFree(sl.d_cnt); cudaFree(sl.d_roww); cudaFree(sl.d_Qm);
-    cudaFree(sl.d_piece); cudaFree(sl.d_pidx); cudaFree(sl.d_rowinfo); cudaFree(sl.d_cand2); cudaFree(sl.d_chunk);
-    cudaFree(sl.d_surv); cudaFree(sl.d_primes); cudaFree(sl.d_direct); cudaFree(sl.d_recs); cudaFree(sl.d_cand);
+    cudaFree(sl.d_piece); cudaFree(sl.d_pidx); cudaFree(sl.d_rowinfo); cudaFree(sl.d_cand); cudaFree(sl.d_chunk);
+    cudaFree(sl.d_surv); cudaFree(sl.d_primes); cudaFree(sl.d_direct); cudaFree(sl.d_recs);
     cudaFree(sl.d_ctr); cudaFree(sl.d_status); cudaFree(sl.d_hdr);
     cudaFreeHost(sl.h_hdr); cudaFreeHost(sl.h_win); cudaFreeHost(sl.h_roww); cudaFreeHost(sl.h_cnt);
     cudaFreeHost(sl.h_ctr); cudaFreeHost(sl.h_status); cudaFreeHost(sl.h_recs);
@@ -2648,7 +2650,7 @@ es_status es_is_prime_batch(es_engine *e, const uint64_t *n, size_t count, uint8
   if (!e || (!n && count) || (!out && count)) return ES_ERR_ARG;
   if (!count) return ES_OK;
   return probe(e, &e->slots[0], count, count * 8, n, count, {{out, count}}, [&](void *in, std::vector<void *> &o) {
-    k_probe_prime<<<e->sm_count * 2, 256, 0, e->slots[0].stream>>>((const u64 *)in, count, (unsigned char *)o[0]);
+    k_probe_prime<<<e->sm_count * MR_BLOCKS_PER_SM, 256, 0, e->slots[0].stream>>>((const u64 *)in, count, (unsigned char *)o[0]);
   });
 }
 

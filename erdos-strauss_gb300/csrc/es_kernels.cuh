@@ -147,8 +147,6 @@ struct BoardSlot;
 struct TailParams {
   Surv *surv;
   unsigned long long *surv_count;
-  u32 *cand;               // indices into surv that passed the base-2 round
-  unsigned long long *cand_count;
   u32 *primes;             // indices into surv
   unsigned long long *prime_count;
   u32 *direct;             // indices into surv, primes that no rung certified

@@ -47,6 +47,21 @@ __device__ __forceinline__ void wf_add(WarpFac &F, u64 p, int e, u32 lane) {
   __syncwarp();
 }
 
+// One strong-probable-prime round on an odd n > 37 to a prime base b <= 37. No division by the base
+// first: one that divides n has only multiples of itself as powers mod n, never +-1, so the round
+// fails. The base's Montgomery form by doublings of 1's.
+__device__ __forceinline__ bool sprp_round(const Mont &M, u32 b) {
+  u64 bm = 0;
+  for (int i = 5; i >= 0; --i) {
+    bm = addmod(bm, bm, M.n);
+    if (b >> i & 1) bm = addmod(bm, M.one, M.n);
+  }
+  u64 d = M.n - 1;
+  const int s = __ffsll((long long)d) - 1;
+  d >>= s;
+  return M.n < LazyArith::NMAX ? sprp_ar<LazyArith>(bm, d, s, M) : sprp_mont(bm, d, s, M);
+}
+
 // The 12-base deterministic test (census/rung_scan.cpp:76-92) with one base per lane.
 // All lanes must call; returns the same verdict in every lane.
 __device__ inline bool warp_is_prime(u64 n, u32 lane) {
@@ -60,21 +75,43 @@ __device__ inline bool warp_is_prime(u64 n, u32 lane) {
   }
   if (!(n & 1)) return false;
   if (lane < 12) {
-    // No division by the base first: a base that divides n > 37 has only multiples of itself as
-    // powers mod n, never +-1, so the round fails. The base's Montgomery form by doublings of 1's.
-    const u32 b = (u32)MR_BASES[lane];
-    const Mont M = mont_one(n);
-    u64 bm = 0;
-    for (int i = 5; i >= 0; --i) {
-      bm = addmod(bm, bm, n);
-      if (b >> i & 1) bm = addmod(bm, M.one, n);
-    }
-    u64 d = n - 1;
-    const int s = __ffsll((long long)d) - 1;
-    d >>= s;
-    ok = n < LazyArith::NMAX ? sprp_ar<LazyArith>(bm, d, s, M) : sprp_mont(bm, d, s, M);
+    ok = sprp_round(mont_one(n), (u32)MR_BASES[lane]);
   }
   return __all_sync(FULL, ok);
+}
+
+// The primes among the 32 numbers of a warp's threads (where `valid`), as a mask in every lane: the
+// base-2 round of each thread's own number, which nearly every composite fails, then the other 11
+// bases of the numbers that passed, a (number, base) pair per lane, so that no lane idles while
+// another's number is tested. All lanes call.
+__device__ inline unsigned warp_primes(u64 n, bool valid, u32 lane) {
+  bool pass = valid && n >= 2 && ((n & 1) || n == 2);
+  Mont M{3, 0, 0, 0};
+  if (pass && n > 37) {
+    M = mont_one(n);
+    pass = sprp2_round(M);
+  } else if (pass) {
+    pass = false;
+    #pragma unroll
+    for (int i = 0; i < 12; ++i) pass |= n == MR_BASES[i];
+  }
+  unsigned primes = __ballot_sync(FULL, pass);
+  const unsigned test = __ballot_sync(FULL, pass && n > 37);
+  const u32 pairs = 11 * __popc(test);
+  for (u32 i0 = 0; i0 < pairs; i0 += 32) {
+    const u32 i = min(i0 + lane, pairs - 1);
+    unsigned m = test;
+    for (u32 skip = i / 11; skip; --skip) m &= m - 1;
+    const int src = __ffs(m) - 1;
+    Mont Q;
+    Q.n = __shfl_sync(FULL, M.n, src);
+    Q.ninv = __shfl_sync(FULL, M.ninv, src);
+    Q.one = __shfl_sync(FULL, M.one, src);
+    Q.r2 = 0;
+    const bool ok = sprp_round(Q, (u32)MR_BASES[1 + i % 11]);
+    primes &= ~__reduce_or_sync(FULL, ok ? 0u : 1u << src);
+  }
+  return primes;
 }
 
 // Brent's backtrack from ys: step one at a time until gcd(|x - ys|, n) > 1 (bounded by the
