@@ -60,6 +60,8 @@
 
 namespace es {
 
+constexpr size_t CTR_BYTES = CTR_OUT * sizeof(unsigned long long) + BOARD_SLOTS * sizeof(BoardSlot);
+
 // ============================================================================ kernels
 
 // K0 table: for lane l and filter f, p = rho + M*K == res (mod mod) iff
@@ -154,6 +156,7 @@ __global__ void __launch_bounds__(BLOCK) k_mark(const MarkParams P, int persiste
   __shared__ u32 red[BLOCK / 32];
   __shared__ u64 s_item;
   const u32 lane_id = threadIdx.x & 31;
+  stamp(P.ctr, 2);
   const u64 total_items = P.hdr->total_items;
   const u32 nwin = P.hdr->nwin;
   u64 next = blockIdx.x;
@@ -318,42 +321,84 @@ __device__ __forceinline__ u32 mod_stride(u64 K, const uint4 &d, bool wide) {
   return mod_s(hi * d.z + mod_s((u32)K, d.x, d.y), d.x, d.y);        // below 2^16 (2^16 - 1) + 2^16
 }
 
-// The batch's row windows cut into pieces: a warp per piece finds its window (32-way search over
-// the windows' first pieces), writes the piece, its rows, and per dense stride the slice row of the
+// The run's first kernel. It reads the header and the window descriptors from pinned host memory
+// itself, copies them for the kernels that follow and clears the run's counters (three memsets and
+// three copies as nodes of the graph cost 12 us), and cuts the windows marked by rows into pieces:
+// a block takes a run of pieces, finds their first window (32-way search over the windows' first
+// pieces, which are in host memory too: as few dependent reads as possible) and goes on 32 windows
+// at a time; a warp per piece writes the piece, its rows, and per dense stride the slice row of the
 // piece's first K. Bound by the latency of its few dependent loads.
-__global__ void k_rows(const RowParams P) {
-  const u32 lane = threadIdx.x & 31;
-  const u32 nw = P.hdr->nshort, npieces = P.hdr->npieces;
-  const u32 warps = gridDim.x * blockDim.x / 32;
-  for (u32 pc = (blockIdx.x * blockDim.x + threadIdx.x) / 32; pc < npieces; pc += warps) {
-    u32 w0 = 0, cnt = nw;                            // the last window whose first piece is <= pc
+__global__ void __launch_bounds__(256) k_rows(const RowParams P) {
+  __shared__ BatchHdr s_hdr;
+  __shared__ RowWin s_win[32];
+  __shared__ u32 s_first;
+  const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x < sizeof(BatchHdr) / 8)
+    reinterpret_cast<u64 *>(&s_hdr)[threadIdx.x] = reinterpret_cast<const volatile u64 *>(P.h_hdr)[threadIdx.x];
+  __syncthreads();
+  const u32 nw = s_hdr.nshort, npieces = s_hdr.npieces, nwin = s_hdr.nwin;
+  const u32 tid = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
+  if (blockIdx.x == 0) {
+    if (threadIdx.x < sizeof(BatchHdr) / 8) reinterpret_cast<u64 *>(P.hdr)[threadIdx.x] = reinterpret_cast<u64 *>(&s_hdr)[threadIdx.x];
+    if (threadIdx.x == 0) *P.status = 0;
+    for (u32 i = threadIdx.x; i < CTR_BYTES / 8; i += blockDim.x)
+      if (i != STAMP0) P.ctr[i] = 0;
+    stamp(P.ctr, 0);
+  }
+  for (u32 i = tid; i < nwin * (sizeof(WinCount) / 16); i += threads)
+    reinterpret_cast<uint4 *>(P.cnt)[i] = make_uint4(0, 0, 0, 0);
+  for (u32 i = tid; i < nwin * (sizeof(WinDev) / 8); i += threads)
+    reinterpret_cast<u64 *>(P.win)[i] = reinterpret_cast<const volatile u64 *>(P.h_win)[i];
+  const u32 share = (npieces + gridDim.x - 1) / gridDim.x;
+  u32 pc0 = min(blockIdx.x * share, npieces);
+  const u32 pc1 = min(pc0 + share, npieces);
+  if (pc0 == pc1) return;
+  const RowWin *hw = P.h_roww;
+  auto piece0 = [&](u32 w) { return *reinterpret_cast<const volatile u32 *>(&hw[w].piece0); };
+  if (warp == 0) {
+    u32 w0 = 0, cnt = nw;                            // the last window whose first piece is <= pc0
     while (cnt > 1) {
       const u32 step = (cnt + 31) / 32, off = lane * step;
-      const bool le = off < cnt && P.roww[w0 + off].piece0 <= pc;
+      const bool le = off < cnt && piece0(w0 + off) <= pc0;
       const u32 k = __popc(__ballot_sync(FULL, le)) - 1;          // lane 0 always holds
       w0 += k * step;
       cnt = min(step, cnt - k * step);
     }
-    const RowWin W = P.roww[w0];
-    const u32 t = pc - W.piece0;
-    Piece x;
-    x.K0 = W.K0 + (u64)t * PIECE_ROWS;
-    x.row0 = W.row0 + t * PIECE_ROWS;
-    x.win = W.wi;
-    x.n = min(PIECE_ROWS, W.nrows - t * PIECE_ROWS);
-    const bool last = t * PIECE_ROWS + x.n == W.nrows;
-    x.la = t == 0 ? W.la : 0;
-    x.lb = last ? W.lb : P.L;
-    x.pad = 0;
-    if (lane == 0) P.piece[pc] = x;
-    if (lane < x.n) {
-      const bool cut = (lane == 0 && x.la) || (lane == x.n - 1 && x.lb < P.L);
-      P.rowinfo[x.row0 + lane] = pc * PIECE_ROWS + lane + (cut ? ROW_CUT : 0u);
+    if (lane == 0) s_first = w0;
+  }
+  __syncthreads();
+  for (u32 w0 = s_first; pc0 < pc1; w0 += 32) {
+    const u32 have = min(nw - w0, 32u);
+    for (u32 i = threadIdx.x; i < have * (sizeof(RowWin) / 8); i += blockDim.x)
+      reinterpret_cast<u64 *>(s_win)[i] = reinterpret_cast<const volatile u64 *>(hw + w0)[i];
+    __syncthreads();
+    const RowWin &Z = s_win[have - 1];
+    const u32 end = min(pc1, Z.piece0 + (Z.nrows + PIECE_ROWS - 1) / PIECE_ROWS);   // these windows' last piece
+    const u32 mine = lane < have ? s_win[lane].piece0 : ~0u;
+    for (u32 pc = pc0 + warp; pc < end; pc += blockDim.x / 32) {
+      const RowWin W = s_win[__popc(__ballot_sync(FULL, mine <= pc)) - 1];
+      const u32 t = pc - W.piece0;
+      Piece x;
+      x.K0 = W.K0 + (u64)t * PIECE_ROWS;
+      x.row0 = W.row0 + t * PIECE_ROWS;
+      x.win = W.wi;
+      x.n = min(PIECE_ROWS, W.nrows - t * PIECE_ROWS);
+      const bool last = t * PIECE_ROWS + x.n == W.nrows;
+      x.la = t == 0 ? W.la : 0;
+      x.lb = last ? W.lb : P.L;
+      x.pad = 0;
+      if (lane == 0) P.piece[pc] = x;
+      if (lane < x.n) {
+        const bool cut = (lane == 0 && x.la) || (lane == x.n - 1 && x.lb < P.L);
+        P.rowinfo[x.row0 + lane] = pc * PIECE_ROWS + lane + (cut ? ROW_CUT : 0u);
+      }
+      for (u32 m = lane; m < P.n1p; m += 32) {
+        const uint4 d = __ldg(P.mdesc + m);
+        P.pidx[(size_t)pc * P.n1p + m] = (u16)(d.w + mod_stride(x.K0, d, P.wide));
+      }
     }
-    for (u32 m = lane; m < P.n1p; m += 32) {
-      const uint4 d = __ldg(P.mdesc + m);
-      P.pidx[(size_t)pc * P.n1p + m] = (u16)(d.w + mod_stride(x.K0, d, P.wide));
-    }
+    pc0 = end;
+    __syncthreads();
   }
 }
 
@@ -434,6 +479,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) k_mark_short(const RowParams P
   __shared__ __align__(8) u64 s_bar;
   __shared__ u32 s_next;
   const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  stamp(P.ctr, 1);
   const u32 nrows = P.hdr->nrows;
   const u32 ntiles = (nrows + 31) / 32;
   const u64 items = (u64)ntiles * P.ngroups;
@@ -882,6 +928,7 @@ __device__ __forceinline__ u64 mr_warp() {
 __global__ void __launch_bounds__(256, MR_BLOCKS_PER_SM) k_mr(const TailParams T) {
   const u32 lane = threadIdx.x & 31;
   const u64 warps = (u64)gridDim.x * blockDim.x / 32, w = mr_warp();
+  stamp(T.ctr, 3);
   const u64 n = min((u64)*T.surv_count, T.cap);
   const u32 share = mr_share(n);
   for (u64 i0 = w * share; i0 < n; i0 += warps * share) {
@@ -954,6 +1001,7 @@ __device__ __forceinline__ void rung_result(const TailParams &T, const Surv &s, 
 __global__ void __launch_bounds__(RUNG_THREADS, 1) k_rung(const TailParams T, int no_rung) {
   extern __shared__ __align__(16) unsigned char rungmem[];
   RungShared<RUNG_TEAMS> &H = *reinterpret_cast<RungShared<RUNG_TEAMS> *>(rungmem);
+  stamp(T.ctr, 4);
   const u64 n = min((u64)*T.prime_count, T.cap);
   if (!n) return;
   const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5, t = w / TEAM_WARPS;
@@ -1001,21 +1049,54 @@ __global__ void __launch_bounds__(RUNG_THREADS, 1) k_rung(const TailParams T, in
   if (few && t == 0 && blockIdx.x % BOARD_BLOCKS_DIV == 0) warp_help_board(board, n, lane);
 }
 
-__global__ void k_direct(const TailParams T) {
+// The run's last kernel: the direct search, a thread per prime that no rung certified (none in
+// scans), then the run's counters, the windows' counters and the records written to pinned host
+// memory (four copies as nodes of the graph cost 8 us, and a fifth with a second wait brought the
+// records past the first 4096). Without direct primes every block writes its share at once; else the
+// last block to finish them writes all.
+__global__ void __launch_bounds__(256) k_direct(const TailParams T) {
+  __shared__ bool s_last;
+  stamp(T.ctr, 5);
   const u64 n = min((u64)*T.direct_count, T.cap);
-  for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
-    const Surv s = T.surv[T.direct[i]];
-    u64 a, c, d, k;
-    if (solve_direct(s.p, a, c, d, k, T.tdp, T.tde, T.status)) {
-      if (!check_solved_cert(s.p, a, c, d, k)) { atomicOr(T.status, ST_CERT_BAD); continue; }
-      RecDev rec{ES_REC_SOLVED, s.win, s.lane, 0, s.J, s.p, a, c, d, k};
-      put_record(T, rec);
-      atomicAdd(&T.cnt[s.win].direct, 1ull);
-    } else {
-      RecDev rec{ES_REC_SURVIVOR, s.win, s.lane, 0, s.J, s.p, 0, 0, 0, 0};
-      put_record(T, rec);
-      atomicAdd(&T.cnt[s.win].unsolved, 1ull);
+  u32 block = blockIdx.x, blocks = gridDim.x;
+  if (n) {
+    for (u64 i = (u64)threadIdx.x * gridDim.x + blockIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
+      const Surv s = T.surv[T.direct[i]];
+      u64 a, c, d, k;
+      if (solve_direct(s.p, a, c, d, k, T.tdp, T.tde, T.status)) {
+        if (!check_solved_cert(s.p, a, c, d, k)) { atomicOr(T.status, ST_CERT_BAD); continue; }
+        RecDev rec{ES_REC_SOLVED, s.win, s.lane, 0, s.J, s.p, a, c, d, k};
+        put_record(T, rec);
+        atomicAdd(&T.cnt[s.win].direct, 1ull);
+      } else {
+        RecDev rec{ES_REC_SURVIVOR, s.win, s.lane, 0, s.J, s.p, 0, 0, 0, 0};
+        put_record(T, rec);
+        atomicAdd(&T.cnt[s.win].unsolved, 1ull);
+      }
     }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(T.ctr + 5, 1ull) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    block = 0; blocks = 1;
+  }
+  const u64 threads = (u64)blocks * blockDim.x, first = (u64)block * blockDim.x + threadIdx.x;
+  const u64 nrec = min((u64)__ldcg(T.rec_count), T.cap), nwin = T.hdr->nwin;
+  const uint4 *cnt = reinterpret_cast<const uint4 *>(T.cnt), *recs = reinterpret_cast<const uint4 *>(T.recs);
+  for (u64 i = first; i < nwin * (sizeof(WinCount) / 16); i += threads) reinterpret_cast<uint4 *>(T.out.cnt)[i] = __ldcg(cnt + i);
+  for (u64 i = first; i < nrec * (sizeof(RecDev) / 16); i += threads) reinterpret_cast<uint4 *>(T.out.recs)[i] = __ldcg(recs + i);
+  if (block == 0) {
+    if (threadIdx.x == 0) { *T.out.status = __ldcg(T.status); }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned long long t;
+      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+      T.ctr[STAMP0 + 6] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < CTR_OUT) T.out.ctr[threadIdx.x] = __ldcg(T.ctr + threadIdx.x);
   }
 }
 
@@ -1121,16 +1202,15 @@ struct Slot {
   unsigned long long *h_ctr = nullptr;
   u32 *h_status = nullptr;
   RecDev *h_recs = nullptr;
-  // The persistent schedule, captured once per capacity as two graphs: the front (counters
-  // cleared, staging copied in, marking, Miller-Rabin) and the tail (stage D, stage E,
-  // counters and the record prefix copied out). ev[11] is recorded between them on the
-  // slot's stream: the next slot's front waits for it (marking runs one batch at a time, in
-  // launch order) while this slot's tail overlaps the next batch's marking.
+  // The persistent schedule, captured once per capacity. A serving slot has two graphs, the front
+  // (marking, Miller-Rabin) and the tail (stage D, stage E, results written out). ev[11] is
+  // recorded between them on the slot's stream: the next slot's front waits for it (marking runs
+  // one batch at a time, in launch order) while this slot's tail overlaps the next batch's
+  // marking. The synchronous slot has one graph of both.
   cudaGraph_t graph = nullptr, graph2 = nullptr;
   cudaGraphExec_t gexec = nullptr, gexec2 = nullptr;
   WinDev *d_win = nullptr; size_t win_cap = 0;
   WinCount *d_cnt = nullptr;
-  RowWin *d_roww = nullptr;
   Piece *d_piece = nullptr; u16 *d_pidx = nullptr; u32 *d_rowinfo = nullptr; size_t piece_cap = 0;
   uint2 *d_cand = nullptr; u32 *d_chunk = nullptr; size_t chunk_cap = 0;
   u16 *d_Qm = nullptr; size_t qm_cap = 0;
@@ -1138,11 +1218,8 @@ struct Slot {
   u32 *d_primes = nullptr, *d_direct = nullptr;
   RecDev *d_recs = nullptr;
   size_t cap = 0;
-  size_t rec_prefix = 0;                // records the captured graph copies back itself
   u64 graph_launches = 0;               // its kernels
-  unsigned long long *d_ctr = nullptr;  // [0] queue [1] surv [2] prime [3] direct [4] rec
-                                      // [6] rung queue (teams) [7] rung primes done [8] board sessions
-                                      // [9] rung queue (warps) [10] candidate chunks, board at [16]
+  unsigned long long *d_ctr = nullptr;  // run counters (es_kernels.cuh) and stage D's board
   u32 *d_status = nullptr;
   es_timing_t timing{};
   struct HostScratch {                  // per-run host vectors, kept with their capacity
@@ -1160,10 +1237,6 @@ struct Slot {
 };
 
 constexpr int SERVE_SLOTS = 2;
-constexpr size_t CTR_OUT = 11;          // counters copied back to the host
-// run counters followed by stage D's board, cleared before every run
-constexpr size_t CTR_BYTES = 16 * sizeof(unsigned long long) + BOARD_SLOTS * sizeof(BoardSlot);
-
 // A serving request: windows in, counters and records out.
 struct Request {
   uint64_t ticket = 0;
@@ -1273,15 +1346,14 @@ static es_status ensure_capacity(es_engine *e, Slot *sl, size_t nwin, size_t npi
   }
   if (nwin > sl->win_cap) {
     drop_graph(sl);
-    cudaFree(sl->d_win); cudaFree(sl->d_cnt); cudaFree(sl->d_roww); cudaFree(sl->d_Qm);
+    cudaFree(sl->d_win); cudaFree(sl->d_cnt); cudaFree(sl->d_Qm);
     cudaFreeHost(sl->h_win); cudaFreeHost(sl->h_roww); cudaFreeHost(sl->h_cnt);
-    sl->d_win = nullptr; sl->d_cnt = nullptr; sl->d_roww = nullptr; sl->d_Qm = nullptr;
+    sl->d_win = nullptr; sl->d_cnt = nullptr; sl->d_Qm = nullptr;
     sl->h_win = nullptr; sl->h_roww = nullptr; sl->h_cnt = nullptr;
     sl->win_cap = 0;
     const size_t want = std::max<size_t>(nwin, 64);
     CU(cudaMalloc(&sl->d_win, want * sizeof(WinDev)));
     CU(cudaMalloc(&sl->d_cnt, want * sizeof(WinCount)));
-    CU(cudaMalloc(&sl->d_roww, want * sizeof(RowWin)));
     CU(cudaMalloc(&sl->d_Qm, want * std::max<u32>(e->Dq, 8) * sizeof(u16)));
     CU(cudaMallocHost(&sl->h_win, want * sizeof(WinDev)));
     CU(cudaMallocHost(&sl->h_roww, want * sizeof(RowWin)));
@@ -1330,7 +1402,7 @@ static MarkParams mark_params(const es_engine *e, const Slot *sl) {
   P.Qm = sl->d_Qm;
   P.win = sl->d_win; P.queue = reinterpret_cast<u64 *>(sl->d_ctr + 0);
   P.surv = sl->d_surv; P.surv_count = sl->d_ctr + 1; P.cnt = sl->d_cnt;
-  P.hdr = sl->d_hdr; P.surv_cap = sl->cap; P.M = e->M;
+  P.hdr = sl->d_hdr; P.ctr = sl->d_ctr; P.surv_cap = sl->cap; P.M = e->M;
   P.L = (u32)e->classes.size(); P.ldk = e->ldk; P.nf = e->nf; P.ncov = (u32)e->ncov;
   P.D = e->D; P.Dq = e->Dq;
   P.r_bytes = (4 * e->D + 15) & ~15u;
@@ -1339,12 +1411,13 @@ static MarkParams mark_params(const es_engine *e, const Slot *sl) {
 
 static TailParams tail_params(const es_engine *e, const Slot *sl) {
   TailParams T;
+  T.ctr = sl->d_ctr; T.hdr = sl->d_hdr; T.out = HostOut{sl->h_ctr, sl->h_status, sl->h_cnt, sl->h_recs};
   T.surv = sl->d_surv; T.surv_count = sl->d_ctr + 1;
   T.primes = sl->d_primes; T.prime_count = sl->d_ctr + 2;
   T.direct = sl->d_direct; T.direct_count = sl->d_ctr + 3;
   T.recs = sl->d_recs; T.rec_count = sl->d_ctr + 4;
   T.rung_next = sl->d_ctr + 6; T.rung_done = sl->d_ctr + 7; T.help_sessions = sl->d_ctr + 8;
-  T.board = reinterpret_cast<BoardSlot *>(sl->d_ctr + 16);
+  T.board = reinterpret_cast<BoardSlot *>(sl->d_ctr + CTR_OUT);
   T.rung_next_warp = sl->d_ctr + 9;
   T.rho_budget = e->rho_budget;
   T.cnt = sl->d_cnt; T.tdp = e->d_tdp; T.tde = e->d_tde; T.tdi = e->d_tdi; T.tdqm = e->d_tdqm; T.status = sl->d_status;
@@ -1355,7 +1428,8 @@ static TailParams tail_params(const es_engine *e, const Slot *sl) {
 static RowParams row_params(const es_engine *e, const Slot *sl) {
   RowParams S;
   S.rho = e->d_rho; S.K0 = e->d_K0; S.fdesc = e->d_fdesc; S.tdense = e->d_tdense; S.tlane = e->d_tlane;
-  S.mdesc = e->d_mdesc; S.lfil = e->d_lfil; S.win = sl->d_win; S.roww = sl->d_roww; S.piece = sl->d_piece;
+  S.mdesc = e->d_mdesc; S.lfil = e->d_lfil; S.win = sl->d_win; S.piece = sl->d_piece;
+  S.h_hdr = sl->h_hdr; S.h_win = sl->h_win; S.h_roww = sl->h_roww; S.ctr = sl->d_ctr;
   S.pidx = sl->d_pidx; S.rowinfo = sl->d_rowinfo; S.cand = sl->d_cand; S.chunk = sl->d_chunk;
   S.chunk_count = sl->d_ctr + 10; S.chunk_cap = (u32)sl->chunk_cap;
   S.surv = sl->d_surv; S.surv_count = sl->d_ctr + 1; S.cnt = sl->d_cnt; S.surv_cap = sl->cap; S.M = e->M;
@@ -1478,49 +1552,36 @@ static u64 positions_in(const es_engine *e, u64 lo, u64 hi) {
   return ql * e->classes.size() + part;
 }
 
-// One pass of the funnel on the engine's stream: reset the counters, copy the batch header
-// and descriptors from pinned staging (ncopy windows, nrow_copy of them marked by rows), the
-// marking kernels, the survivor tail, and the copies of the run counters back to pinned memory.
-// With `capture` the event records are external graph nodes, so that the kernels can still be
-// timed when the sequence runs as a graph. `segments`: some windows may go to the segment marking
-// (k_mark, sized by `items_hint` in the plain schedule). Adds its kernel launches to `launches`.
-static es_status enqueue_front(es_engine *e, Slot *sl, bool persistent, WinCount *cnt, size_t ncopy, size_t nrow_copy,
-                               bool segments, u64 items_hint, bool capture, u64 &launches) {
+// The funnel's front on the engine's stream: k_rows (which takes the header and the window
+// descriptors from pinned staging and clears the counters), the marking kernels and Miller-Rabin.
+// With `capture` the event record is an external graph node, so that the run can be timed when the
+// sequence is a graph. `rows`, `segments`: some windows may be marked by rows, by segments (k_mark,
+// sized by `items_hint` in the plain schedule). Adds its kernel launches to `launches`.
+static es_status enqueue_front(es_engine *e, Slot *sl, bool persistent, WinCount *cnt, bool rows, bool segments,
+                               u64 items_hint, bool capture, u64 &launches) {
   MarkParams P = mark_params(e, sl);
   TailParams T = tail_params(e, sl);
   P.cnt = cnt;
   T.cnt = cnt;
   cudaStream_t st = sl->stream;
-  auto rec = [&](int k) {
-    return capture ? cudaEventRecordWithFlags(sl->ev[k], st, cudaEventRecordExternal) : cudaEventRecord(sl->ev[k], st);
-  };
-  CU(cudaMemsetAsync(sl->d_ctr, 0, CTR_BYTES, st));
-  CU(cudaMemsetAsync(sl->d_status, 0, sizeof(u32), st));
-  CU(cudaMemcpyAsync(sl->d_hdr, sl->h_hdr, sizeof(BatchHdr), cudaMemcpyHostToDevice, st));
-  CU(cudaMemcpyAsync(sl->d_win, sl->h_win, ncopy * sizeof(WinDev), cudaMemcpyHostToDevice, st));
-  if (nrow_copy) CU(cudaMemcpyAsync(sl->d_roww, sl->h_roww, nrow_copy * sizeof(RowWin), cudaMemcpyHostToDevice, st));
-  CU(rec(0));
+  CU(capture ? cudaEventRecordWithFlags(sl->ev[0], st, cudaEventRecordExternal) : cudaEventRecord(sl->ev[0], st));
   RowParams S = row_params(e, sl);
   S.cnt = cnt;
-  if (nrow_copy) {
-    k_rows<<<e->sm_count * 4, 256, 0, st>>>(S);
-    CU(cudaGetLastError());
-    ++launches;
-  }
+  k_rows<<<e->sm_count * 4, 256, 0, st>>>(S);
+  CU(cudaGetLastError());
+  ++launches;
   if (segments) {
     k_prep<<<e->sm_count * 4, 256, 0, st>>>(sl->d_hdr, sl->d_win, e->d_sdist, e->D, e->Dq, sl->d_Qm);
     CU(cudaGetLastError());
     ++launches;
   }
-  CU(rec(7));
-  if (nrow_copy) {
+  if (rows) {
     k_mark_short<<<e->sm_count, ROW_THREADS, e->slice_rows * 4 * GROUP_WORDS + CAND_SMEM, st>>>(S);
     CU(cudaGetLastError());
     k_sift<<<e->sm_count, ROW_THREADS, ROW_SMEM, st>>>(S);
     CU(cudaGetLastError());
     launches += 2;
   }
-  CU(rec(8));
   if (segments) {
     const unsigned grid = persistent ? (unsigned)((u64)e->sm_count * e->mark_occupancy)
                                      : (unsigned)std::max<u64>(1, std::min<u64>(items_hint, 0x7FFFFFFFull));
@@ -1528,73 +1589,47 @@ static es_status enqueue_front(es_engine *e, Slot *sl, bool persistent, WinCount
     CU(cudaGetLastError());
     ++launches;
   }
-  CU(rec(1));
   k_mr<<<e->sm_count * MR_BLOCKS_PER_SM, 256, 0, st>>>(T);
   CU(cudaGetLastError());
   ++launches;
-  CU(rec(2));
   return ES_OK;
 }
 
-// The funnel's tail on the slot's stream: stage D, stage E, run counters and status copied out.
-static es_status enqueue_tail(es_engine *e, Slot *sl, WinCount *cnt, bool capture) {
+// The funnel's tail on the slot's stream: stage D, stage E, the results written to pinned memory
+// (the windows' counters at out_cnt).
+static es_status enqueue_tail(es_engine *e, Slot *sl, WinCount *cnt, WinCount *out_cnt, bool capture) {
   TailParams T = tail_params(e, sl);
   T.cnt = cnt;
+  T.out.cnt = out_cnt;
   cudaStream_t st = sl->stream;
-  auto rec = [&](int k) {
-    return capture ? cudaEventRecordWithFlags(sl->ev[k], st, cudaEventRecordExternal) : cudaEventRecord(sl->ev[k], st);
-  };
   const u32 teams = e->sm_count * std::min<u32>(e->sched.rung_blocks_per_sm, RUNG_TEAMS);
   k_rung<<<(teams + RUNG_TEAMS - 1) / RUNG_TEAMS, RUNG_THREADS, sizeof(RungShared<RUNG_TEAMS>), st>>>(T, (e->flags & ES_FLAG_NO_RUNG) ? 1 : 0);
   CU(cudaGetLastError());
-  CU(rec(3));
-  k_direct<<<e->sm_count, 32, 0, st>>>(T);
+  k_direct<<<e->sm_count, 256, 0, st>>>(T);
   CU(cudaGetLastError());
-  CU(rec(4));
-  CU(cudaMemcpyAsync(sl->h_ctr, sl->d_ctr, CTR_OUT * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-  CU(cudaMemcpyAsync(sl->h_status, sl->d_status, sizeof(u32), cudaMemcpyDeviceToHost, st));
+  CU(capture ? cudaEventRecordWithFlags(sl->ev[4], st, cudaEventRecordExternal) : cudaEventRecord(sl->ev[4], st));
   return ES_OK;
 }
 
-// The persistent schedule as a CUDA graph: counters cleared, the whole staging area copied,
-// every kernel, and the counters copied back, captured once and replayed per batch.
-constexpr size_t REC_PREFIX = 4096;
-
+// The persistent schedule as CUDA graphs, captured once and replayed per batch: for a serving slot
+// two, the funnel up to Miller-Rabin, and stage D and E with the results written out; for the
+// synchronous slot one (the gap between two is 5 us of a small window's 50).
 static es_status capture_graph(es_engine *e, Slot *sl) {
   drop_graph(sl);
-  // the front: per-window counters cleared, then the funnel up to Miller-Rabin
-  CU(cudaStreamBeginCapture(sl->stream, cudaStreamCaptureModeThreadLocal));
-  es_status s = ES_OK;
-  const cudaError_t m = cudaMemsetAsync(sl->d_cnt, 0, sl->win_cap * sizeof(WinCount), sl->stream);
+  const bool one = sl == &e->slots[0];
   u64 launches = 2;                                // the tail's two kernels
-  if (m == cudaSuccess)
-    s = enqueue_front(e, sl, true, sl->d_cnt, sl->win_cap, sl->win_cap, !e->sched.long_split, 0, true, launches);
-  cudaGraph_t g = nullptr;
-  cudaError_t end = cudaStreamEndCapture(sl->stream, &g);
-  if (m != cudaSuccess) return fail(e, ES_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(m));
-  if (s != ES_OK) { if (g) cudaGraphDestroy(g); return s; }
-  if (end != cudaSuccess) return fail(e, ES_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(end));
-  sl->graph = g;
-  CU(cudaGraphInstantiate(&sl->gexec, g, 0));
-  // the tail: stage D and E, then the counters and the first REC_PREFIX record slots copied
-  // back, so that a batch with fewer records (every 4096-window batch at 1e19 has about
-  // 1.6 K) needs no copy after the run
-  CU(cudaStreamBeginCapture(sl->stream, cudaStreamCaptureModeThreadLocal));
-  s = enqueue_tail(e, sl, sl->d_cnt, true);
-  sl->rec_prefix = std::min<size_t>(sl->cap, REC_PREFIX);
-  if (s == ES_OK) {
-    cudaError_t c2 = cudaMemcpyAsync(sl->h_cnt, sl->d_cnt, sl->win_cap * sizeof(WinCount),
-                                     cudaMemcpyDeviceToHost, sl->stream);
-    if (c2 == cudaSuccess)
-      c2 = cudaMemcpyAsync(sl->h_recs, sl->d_recs, sl->rec_prefix * sizeof(RecDev), cudaMemcpyDeviceToHost, sl->stream);
-    if (c2 != cudaSuccess) s = fail(e, ES_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(c2));
+  for (int part = 0; part < (one ? 1 : 2); ++part) {
+    CU(cudaStreamBeginCapture(sl->stream, cudaStreamCaptureModeThreadLocal));
+    es_status s = ES_OK;
+    if (part == 0) s = enqueue_front(e, sl, true, sl->d_cnt, true, !e->sched.long_split, 0, true, launches);
+    if (s == ES_OK && (one || part == 1)) s = enqueue_tail(e, sl, sl->d_cnt, sl->h_cnt, true);
+    cudaGraph_t g = nullptr;
+    const cudaError_t end = cudaStreamEndCapture(sl->stream, &g);
+    if (s != ES_OK) { if (g) cudaGraphDestroy(g); return s; }
+    if (end != cudaSuccess) return fail(e, ES_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(end));
+    (part == 0 ? sl->graph : sl->graph2) = g;
+    CU(cudaGraphInstantiate(part == 0 ? &sl->gexec : &sl->gexec2, g, 0));
   }
-  g = nullptr;
-  end = cudaStreamEndCapture(sl->stream, &g);
-  if (s != ES_OK) { if (g) cudaGraphDestroy(g); return s; }
-  if (end != cudaSuccess) return fail(e, ES_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(end));
-  sl->graph2 = g;
-  CU(cudaGraphInstantiate(&sl->gexec2, g, 0));
   sl->graph_launches = launches;
   return ES_OK;
 }
@@ -1611,7 +1646,7 @@ static es_status launch_persistent(es_engine *e, Slot *sl) {
     CU(cudaEventRecord(sl->ev[11], sl->stream));
     e->last_front = sl;
   }
-  CU(cudaGraphLaunch(sl->gexec2, sl->stream));
+  if (sl->gexec2) CU(cudaGraphLaunch(sl->gexec2, sl->stream));
   return ES_OK;
 }
 
@@ -1666,16 +1701,19 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
   for (int attempt = 0; attempt < 4 && !done; ++attempt) {
     es_status s = ensure_capacity(e, sl, n, shape.pieces, chunks, cap);
     if (s) return s;
-    double mark_ms = 0, mr_ms = 0, rung_ms = 0, direct_ms = 0, prep_ms = 0, short_ms = 0, long_ms = 0;
+    double total_ms = 0, mark_ms = 0, mr_ms = 0, rung_ms = 0, direct_ms = 0, prep_ms = 0, short_ms = 0, long_ms = 0;
     u64 launches = 0, surv_max = 0, chunk_max = 0, prime_total = 0;
     u32 status = 0;
     hr.clear();
-    size_t have_recs = 0;                 // records already on the host (the graph's prefix copy)
     auto collect = [&]() -> es_status {   // after a pass: timings, counts, records
-      prep_ms += ev_ms(sl->ev[0], sl->ev[7]); short_ms += ev_ms(sl->ev[7], sl->ev[8]);
-      long_ms += ev_ms(sl->ev[8], sl->ev[1]);
-      mark_ms += ev_ms(sl->ev[0], sl->ev[1]); mr_ms += ev_ms(sl->ev[1], sl->ev[2]);
-      rung_ms += ev_ms(sl->ev[2], sl->ev[3]); direct_ms += ev_ms(sl->ev[3], sl->ev[4]);
+      total_ms += ev_ms(sl->ev[0], sl->ev[4]);
+      // a stage runs from its first kernel's start to the next stage's; 0 marks one not launched
+      const unsigned long long *t = sl->h_ctr + STAMP0;
+      auto ms = [](u64 a, u64 b) { return b > a ? (double)(b - a) * 1e-6 : 0.0; };
+      const u64 longs = t[2] ? t[2] : t[3], rows = t[1] ? t[1] : longs;
+      prep_ms += ms(t[0], rows); short_ms += ms(rows, longs); long_ms += ms(longs, t[3]);
+      mark_ms += ms(t[0], t[3]); mr_ms += ms(t[3], t[4]);
+      rung_ms += ms(t[4], t[5]); direct_ms += ms(t[5], t[6]);
       const unsigned long long *ctr = sl->h_ctr;
       surv_max = std::max<u64>(surv_max, ctr[1]);
       chunk_max = std::max<u64>(chunk_max, ctr[10]);
@@ -1683,12 +1721,6 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
       status |= *sl->h_status;
       if (ctr[1] > sl->cap) return ES_OK;
       const size_t nrec = (size_t)std::min<u64>(ctr[4], sl->cap);
-      const size_t have = std::min(nrec, have_recs);
-      if (nrec > have) {
-        CU(cudaMemcpyAsync(sl->h_recs + have, sl->d_recs + have, (nrec - have) * sizeof(RecDev),
-                           cudaMemcpyDeviceToHost, sl->stream));
-        CU(cudaStreamSynchronize(sl->stream));
-      }
       if (nrec) hr.insert(hr.end(), sl->h_recs, sl->h_recs + nrec);
       return ES_OK;
     };
@@ -1700,7 +1732,7 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
       sl->h_hdr->npieces = (u32)shape.pieces;
       memcpy(sl->h_win, wd.data(), n * sizeof(WinDev));
       if (!roww.empty()) memcpy(sl->h_roww, roww.data(), roww.size() * sizeof(RowWin));
-      if (!sl->gexec || !sl->gexec2) { s = capture_graph(e, sl); if (s) return s; }
+      if (!sl->gexec) { s = capture_graph(e, sl); if (s) return s; }
       setup_ms = ms_since(t_start);
       const auto t_launch = std::chrono::steady_clock::now();
       s = launch_persistent(e, sl);
@@ -1708,12 +1740,10 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
       CU(cudaStreamSynchronize(sl->stream));
       device_ms = ms_since(t_launch);
       launches = sl->graph_launches;
-      have_recs = sl->rec_prefix;
       s = collect();
       if (s) return s;
     } else {
       // The plain schedule: the same kernels, one launch sequence per window.
-      CU(cudaMemsetAsync(sl->d_cnt, 0, n * sizeof(WinCount), sl->stream));
       size_t k = 0;                      // next window marked by rows (describe emits them in order)
       for (size_t i = 0; i < n; ++i) {
         sl->h_win[0] = wd[i];
@@ -1727,9 +1757,9 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
           x.wi = x.row0 = x.piece0 = 0;
           h.nshort = 1; h.nrows = x.nrows; h.npieces = (x.nrows + PIECE_ROWS - 1) / PIECE_ROWS;
         }
-        s = enqueue_front(e, sl, false, sl->d_cnt + i, 1, h.nshort, items != 0, items, false, launches);
+        s = enqueue_front(e, sl, false, sl->d_cnt + i, h.nshort != 0, items != 0, items, false, launches);
         if (s) return s;
-        s = enqueue_tail(e, sl, sl->d_cnt + i, false);
+        s = enqueue_tail(e, sl, sl->d_cnt + i, sl->h_cnt + i, false);
         if (s) return s;
         CU(cudaStreamSynchronize(sl->stream));
         launches += 2;
@@ -1739,8 +1769,6 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
         if (surv_max > sl->cap || chunk_max > sl->chunk_cap) break;
         for (size_t r = base; r < hr.size(); ++r) hr[r].win = (u32)i;
       }
-      CU(cudaMemcpyAsync(sl->h_cnt, sl->d_cnt, n * sizeof(WinCount), cudaMemcpyDeviceToHost, sl->stream));
-      CU(cudaStreamSynchronize(sl->stream));
     }
     if (surv_max > sl->cap || chunk_max > sl->chunk_cap) {   // overflow: grow to the exact need and re-run
       if (surv_max > sl->cap) cap = (size_t)(surv_max + surv_max / 4 + 1024);
@@ -1748,7 +1776,7 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
       continue;
     }
     if (status) return fail(e, ES_ERR_DEVICE_STATUS, "device status:" + status_text(status));
-    sl->timing.total_ms = mark_ms + mr_ms + rung_ms + direct_ms;   // kernels only, inputs resident
+    sl->timing.total_ms = total_ms;
     sl->timing.mark_ms = mark_ms; sl->timing.mr_ms = mr_ms;
     sl->timing.prep_ms = prep_ms; sl->timing.mark_short_ms = short_ms; sl->timing.mark_long_ms = long_ms;
     sl->timing.short_pairs = (u64)roww.size() * e->classes.size();
@@ -2425,7 +2453,7 @@ es_status es_close(es_engine *e) {
   for (Slot &sl : e->slots) {
     if (sl.stream) cudaStreamSynchronize(sl.stream);
     drop_graph(&sl);
-    cudaFree(sl.d_win); cudaFree(sl.d_cnt); cudaFree(sl.d_roww); cudaFree(sl.d_Qm);
+    cudaFree(sl.d_win); cudaFree(sl.d_cnt); cudaFree(sl.d_Qm);
     cudaFree(sl.d_piece); cudaFree(sl.d_pidx); cudaFree(sl.d_rowinfo); cudaFree(sl.d_cand); cudaFree(sl.d_chunk);
     cudaFree(sl.d_surv); cudaFree(sl.d_primes); cudaFree(sl.d_direct); cudaFree(sl.d_recs);
     cudaFree(sl.d_ctr); cudaFree(sl.d_status); cudaFree(sl.d_hdr);

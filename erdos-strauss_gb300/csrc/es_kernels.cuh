@@ -69,6 +69,7 @@ struct MarkParams {
   unsigned long long *surv_count;
   WinCount *cnt;           // [nwin]
   const BatchHdr *hdr;     // total_items, nwin
+  unsigned long long *ctr;
   u64 surv_cap;
   u64 M;
   u32 L, ldk, nf, ncov, D, Dq;
@@ -111,6 +112,19 @@ struct __align__(16) Piece {
 // rowinfo: the row's piece and its place in it, and whether the row is cut (la, lb)
 constexpr u32 ROW_CUT = 1u << 31, ROW_NONE = ~0u;
 
+// Run counters: [0] k_mark's queue [1] survivors [2] primes [3] direct [4] records [5] k_direct's blocks
+// done [6] rung queue (teams) [7] rung primes done [8] board sessions [9] rung queue (warps)
+// [10] candidate chunks, [STAMP0 + i] the device clock in ns at the start of k_rows, k_mark_short,
+// k_mark, k_mr, k_rung and k_direct and at its end; then stage D's board.
+constexpr u32 STAMP0 = 16, CTR_OUT = 24;
+__device__ __forceinline__ void stamp(unsigned long long *ctr, u32 i) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    ctr[STAMP0 + i] = t;
+  }
+}
+
 struct RowParams {
   const u32 *rho;
   const u16 *K0;
@@ -121,8 +135,12 @@ struct RowParams {
                             // strides padded to n1p with rows that hold no bit, then the covers'
                             // others up to nm_cov and stage B''s up to nm_all
   const u32 *lfil;          // filters of strides without tables: covers [0, nl_cov), then B' [nl_cov, nl_all)
-  const WinDev *win;
-  const RowWin *roww;       // [hdr->nshort]
+  WinDev *win;
+  // the run's pinned host staging: header, window descriptors, windows marked by rows
+  const BatchHdr *h_hdr;
+  const WinDev *h_win;
+  const RowWin *h_roww;     // [hdr->nshort]
+  unsigned long long *ctr;  // the run's counters (CTR_WORDS), cleared by k_rows
   Piece *piece;             // [hdr->npieces]
   u16 *pidx;                // [npieces][n1p] slice row of the piece's first K per dense stride
   u32 *rowinfo;             // [nrows]
@@ -133,7 +151,7 @@ struct RowParams {
   unsigned long long *surv_count;
   WinCount *cnt;
   u64 surv_cap, M;
-  const BatchHdr *hdr;
+  BatchHdr *hdr;
   u32 *status;
   bool wide;                // K may reach 2^48
   bool squares;             // n^2 passes every cover when n is prime to the nsq primes with these inverses
@@ -144,7 +162,18 @@ struct RowParams {
 
 struct BoardSlot;
 
+// Where a run's results go: pinned host memory, written by k_direct.
+struct HostOut {
+  unsigned long long *ctr;
+  u32 *status;
+  WinCount *cnt;
+  RecDev *recs;
+};
+
 struct TailParams {
+  unsigned long long *ctr;
+  const BatchHdr *hdr;
+  HostOut out;
   Surv *surv;
   unsigned long long *surv_count;
   u32 *primes;             // indices into surv

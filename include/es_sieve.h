@@ -116,8 +116,10 @@ typedef struct {
   char classes_sha256[72];  /* the pin, or "unpinned" */
 } es_info_t;
 
-/* Device time of the last run, per stage, from CUDA events on the engine's stream;
- * total_ms is the sum of the stages (kernels only: no host<->device copies). */
+/* Device time of the last run: total_ms from CUDA events on the engine's stream around its
+ * kernels (results written to host memory included); the stages from the device's clock, each from
+ * its first kernel's start to the next stage's, so the launch gaps between them are included and
+ * their sum is total_ms but for the gap before the first. */
 typedef struct {
   double total_ms, mark_ms, mr_ms, rung_ms, direct_ms;
   double prep_ms, mark_short_ms, mark_long_ms;   /* the three parts of mark_ms:
