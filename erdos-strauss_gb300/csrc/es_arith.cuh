@@ -204,6 +204,7 @@ struct LazyArith {
 __device__ __forceinline__ bool sprp_mont(u64 bm, u64 d, int s, const Mont &M) {
   const u64 mone = M.n - M.one;                       // Montgomery form of n-1
   u64 x = M.one, b = bm, e = d;
+  #pragma unroll 1
   while (e) {
     const u64 t = mmul(x, b, M);                      // both in flight, whatever the bit
     b = mmul(b, b, M);
@@ -211,6 +212,7 @@ __device__ __forceinline__ bool sprp_mont(u64 bm, u64 d, int s, const Mont &M) {
     e >>= 1;
   }
   if (x == M.one || x == mone) return true;
+  #pragma unroll 1
   for (int i = 1; i < s; ++i) {
     x = mmul(x, x, M);
     if (x == mone) return true;
@@ -224,6 +226,7 @@ template <class Ar>
 __device__ __forceinline__ bool sprp_ar(u64 bm, u64 d, int s, const Mont &M) {
   const u64 mone = M.n - M.one;
   u64 x = M.one, b = bm, e = d;
+  #pragma unroll 1
   while (e) {
     const u64 t = Ar::mul(x, b, M);
     b = Ar::mul(b, b, M);
@@ -232,6 +235,7 @@ __device__ __forceinline__ bool sprp_ar(u64 bm, u64 d, int s, const Mont &M) {
   }
   x = Ar::norm(x, M);
   if (x == M.one || x == mone) return true;
+  #pragma unroll 1
   for (int i = 1; i < s; ++i) {
     x = Ar::norm(Ar::mul(x, x, M), M);
     if (x == mone) return true;
@@ -247,12 +251,14 @@ template <class Ar>
 __device__ __forceinline__ bool sprp2_ar(u64 d, int s, const Mont &M) {
   const u64 mone = M.n - M.one;
   u64 x = Ar::add(M.one, M.one, M);                  // 2: the top bit of d (d >= 1)
+  #pragma unroll 1
   for (int i = 62 - __clzll((long long)d); i >= 0; --i) {
     x = Ar::mul(x, x, M);
     if ((d >> i) & 1) x = Ar::add(x, x, M);
   }
   x = Ar::norm(x, M);
   if (x == M.one || x == mone) return true;
+  #pragma unroll 1
   for (int i = 1; i < s; ++i) {
     x = Ar::norm(Ar::mul(x, x, M), M);
     if (x == mone) return true;
@@ -262,11 +268,13 @@ __device__ __forceinline__ bool sprp2_ar(u64 d, int s, const Mont &M) {
 __device__ __forceinline__ bool sprp2_mont(u64 d, int s, const Mont &M) {
   const u64 mone = M.n - M.one;
   u64 x = addmod(M.one, M.one, M.n);
+  #pragma unroll 1
   for (int i = 62 - __clzll((long long)d); i >= 0; --i) {
     x = mmul(x, x, M);
     if ((d >> i) & 1) x = addmod(x, x, M.n);
   }
   if (x == M.one || x == mone) return true;
+  #pragma unroll 1
   for (int i = 1; i < s; ++i) {
     x = mmul(x, x, M);
     if (x == mone) return true;
@@ -314,6 +322,7 @@ __device__ __forceinline__ u64 gcd64(u64 a, u64 b) {           // binary gcd
   if (!b) return a;
   const int sh = __ffsll((long long)(a | b)) - 1;
   a >>= __ffsll((long long)a) - 1;
+  #pragma unroll 1
   do {
     b >>= __ffsll((long long)b) - 1;
     if (a > b) { const u64 t = a; a = b; b = t; }

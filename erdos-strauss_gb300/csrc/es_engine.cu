@@ -949,26 +949,27 @@ __device__ __forceinline__ void put_record(const TailParams &T, const RecDev &r)
 }
 
 // Shared memory of a stage-D block of TEAMS teams.
-template <int TEAMS>
+template <int TEAMS, int SIEVES = TEAMS>
 struct RungShared {
   WarpFac F[TEAMS * TEAM_WARPS];
   DPWarp D[TEAMS * TEAM_WARPS];
   u64 rho_slot[TEAMS * TEAM_WARPS];
   RungResult slot[TEAMS * TEAM_WARPS], out[TEAMS];
-  TdSieve tds[TEAMS];
+  TdSieve tds[SIEVES];                             // a team's: its first warp's, which has a prime of its own first
   BlockHelp help;
   unsigned long long next[TEAMS];
   int best_k[TEAMS];
   unsigned int busy[TEAMS];
   __device__ Team team(int t) {
     return Team{F + TEAM_WARPS * t, D + TEAM_WARPS * t, rho_slot + TEAM_WARPS * t, slot + TEAM_WARPS * t, out + t,
-                tds + t, best_k + t, busy + t, &help, (u32)(TEAM_WARPS * t), (u32)t + 1};
+                tds + SIEVES / TEAMS * t, best_k + t, busy + t, &help, (u32)(TEAM_WARPS * t), (u32)t + 1};
   }
   __device__ void init() {                         // every thread calls; the caller synchronizes
     for (u32 i = threadIdx.x; i < sizeof(BlockHelp) / 4; i += blockDim.x) reinterpret_cast<u32 *>(&help)[i] = 0;
   }
 };
 constexpr int RUNG_TEAMS = BLOCK_WARPS / TEAM_WARPS, RUNG_THREADS = 32 * BLOCK_WARPS;
+typedef RungShared<RUNG_TEAMS, BLOCK_WARPS> RungBlock;
 // Every fourth block stays to help the board when it is done: all of them keep their SMs from the next
 // batch's marking (three pipelined batches at 1e19 1.26-1.36 ms against 1.48-1.60 with every block and
 // 1.33-1.51 with none; a 2^34 window at 1.8e19 with the tuned table 0.29-0.35, 0.28-0.35, 0.34-0.40).
@@ -1000,7 +1001,7 @@ __device__ __forceinline__ void rung_result(const TailParams &T, const Surv &s, 
 
 __global__ void __launch_bounds__(RUNG_THREADS, 1) k_rung(const TailParams T, int no_rung) {
   extern __shared__ __align__(16) unsigned char rungmem[];
-  RungShared<RUNG_TEAMS> &H = *reinterpret_cast<RungShared<RUNG_TEAMS> *>(rungmem);
+  RungBlock &H = *reinterpret_cast<RungBlock *>(rungmem);
   stamp(T.ctr, 4);
   const u64 n = min((u64)*T.prime_count, T.cap);
   if (!n) return;
@@ -1023,8 +1024,8 @@ __global__ void __launch_bounds__(RUNG_THREADS, 1) k_rung(const TailParams T, in
     if (i >= nw) break;
     const u32 si = T.primes[i];
     const Surv s = T.surv[si];
-    const bool ok = !no_rung && warp_solve_rung(s.p, T.tdp, T.tdi, T.status, H.F[w], H.D[w], H.rho_slot + w, &H.slot[w],
-                                                T.rho_budget, /*use_ecm=*/false);
+    const bool ok = !no_rung && warp_solve_rung(s.p, T.tdp, T.tdi, T.tdqm, T.status, H.F[w], H.D[w], H.tds[w], H.rho_slot + w,
+                                                &H.slot[w], T.rho_budget, /*use_ecm=*/false);
     if (lane == 0) rung_result(T, s, si, ok, H.slot[w]);
     __syncwarp();
   }
@@ -1156,7 +1157,7 @@ __global__ void k_probe_direct(const u64 *p, u64 count, RecDev *out, unsigned ch
   }
 }
 // The production factorization (warp_factor), one warp per value; primes sorted ascending.
-__global__ void k_probe_factor(const u64 *n, u64 count, u64 *pr, unsigned char *ex, unsigned char *k,
+__global__ void __launch_bounds__(128, 4) k_probe_factor(const u64 *n, u64 count, u64 *pr, unsigned char *ex, unsigned char *k,
                                const u32 *tdp, const u64 *tdi, u32 *status, u64 rho_budget) {
   __shared__ WarpFac F[4];
   __shared__ u64 rho_slot[4];
@@ -1603,7 +1604,7 @@ static es_status enqueue_tail(es_engine *e, Slot *sl, WinCount *cnt, WinCount *o
   T.out.cnt = out_cnt;
   cudaStream_t st = sl->stream;
   const u32 teams = e->sm_count * std::min<u32>(e->sched.rung_blocks_per_sm, RUNG_TEAMS);
-  k_rung<<<(teams + RUNG_TEAMS - 1) / RUNG_TEAMS, RUNG_THREADS, sizeof(RungShared<RUNG_TEAMS>), st>>>(T, (e->flags & ES_FLAG_NO_RUNG) ? 1 : 0);
+  k_rung<<<(teams + RUNG_TEAMS - 1) / RUNG_TEAMS, RUNG_THREADS, sizeof(RungBlock), st>>>(T, (e->flags & ES_FLAG_NO_RUNG) ? 1 : 0);
   CU(cudaGetLastError());
   k_direct<<<e->sm_count, 256, 0, st>>>(T);
   CU(cudaGetLastError());
@@ -2175,8 +2176,8 @@ static es_status build_tables(es_engine *e) {
   {
     int max_smem = 0;
     CU(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, e->device));
-    CU(cudaFuncSetAttribute(k_rung, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RungShared<RUNG_TEAMS>)));
-    const std::pair<const void *, size_t> resident[] = {{(const void *)k_rung, sizeof(RungShared<RUNG_TEAMS>)},
+    CU(cudaFuncSetAttribute(k_rung, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RungBlock)));
+    const std::pair<const void *, size_t> resident[] = {{(const void *)k_rung, sizeof(RungBlock)},
                                                         {(const void *)k_probe_rung, 4 * sizeof(RungShared<1>)}};
     for (const auto &[f, bytes] : resident) {
       const int pct = std::min(100, (int)(100.0 * (bytes + 4096) / std::max(max_smem, 1)) + 1);

@@ -18,6 +18,14 @@
 //                    nxt[t] = min_j cur[t * pr^-j] * pr^j over j <= e with the bound <= q
 // and a team of four warps walks successive rungs of one prime concurrently, keeping the
 // smallest rung that certifies (the reference's emission rule, sieve/rung_scan3.cpp:574-603).
+//
+// Code size bounds the bulk of it: the warps of an SM are at different places of a long walk, so
+// what they run has to fit the instruction cache. With the compiler's own unrolling of these loops
+// 32-41 % of the fetches missed it and waiting for instructions was the first stall (5.8-8.9 warps a
+// cycle); so the loops that are a chain anyway (multiplies of a power or a walk, lanes' tables) stay
+// rolled (unroll 1) and rare paths are out of line. With that and one sieve a prime in the bulk
+// (td_sieve), stage D of a window of 2^41 integers at 1e15 takes 1.78 ms for 2.88. Calls in the place
+// of whole inlined steps cost more than the misses that they save.
 #pragma once
 #include "es_arith.cuh"
 #include "es_ecm.cuh"
@@ -230,12 +238,14 @@ __device__ __forceinline__ u64 rho_walk(u64 n, const Mont &M, u64 c0, u64 cstep,
     fine = __any_sync(FULL, spent) || fine;
     return has ? __shfl_sync(FULL, mine, __ffs(has) - 1) : 0;
   };
+  #pragma unroll 1
   for (u64 r = r0;; r <<= 1) {
     x = y;
     if (steps + 2 * r > budget) return since ? test() : 0;
     for (u64 i = 0; i < r;) {
       const u64 lim = RHO_POLL < r - i ? RHO_POLL : r - i;
-      for (u64 k = 0; k < lim; ++k) y = Ar::add(Ar::mul(y, y, M), cm, M);
+      #pragma unroll 1
+      for (u32 k = 0; k < (u32)lim; ++k) y = Ar::add(Ar::mul(y, y, M), cm, M);
       i += lim;
       const u64 ext = poll();
       if (ext) return ext == ~0ull ? 0 : ext;
@@ -246,7 +256,8 @@ __device__ __forceinline__ u64 rho_walk(u64 n, const Mont &M, u64 c0, u64 cstep,
       if (!since) ys = y;
       // q takes y while the next y is computed: two independent multiplies in flight
       y = Ar::add(Ar::mul(y, y, M), cm, M);
-      for (u64 i = 1; i < lim; ++i) {
+      #pragma unroll 1
+      for (u32 i = 1; i < (u32)lim; ++i) {
         const u64 next = Ar::add(Ar::mul(y, y, M), cm, M);
         q = Ar::mul(q, x > y ? x - y : y - x, M);     // a closed cycle makes q = 0 mod n
         y = next;
@@ -521,23 +532,28 @@ __device__ __forceinline__ u32 mod_a0(u32 hi, u32 mid, u32 lo, u32 q, u32 m) {  
 }
 
 // S for A_k = A0 + k, k < TD_RUNGS, A0 < 2^64, from tdqm[i] = {d_i, floor(2^32 / d_i)} over
-// the odd primes d_i below 2^16. Each thread takes SIEVE_BATCH primes at a time, their table
-// entries loaded together before any is used. Every thread of a team calls (tid of TEAM_THREADS); the
-// team synchronizes on entry and exit.
+// the odd primes d_i below 2^16. Each thread takes SIEVE_BATCH primes at a time, the next batch's
+// table entries in flight while one is used. Every thread of the team (THREADS = TEAM_THREADS, tid
+// its place, `bar` its barrier) or warp (THREADS = 32) calls; they synchronize on entry and exit.
 constexpr int TEAM_WARPS = 4, TEAM_THREADS = 32 * TEAM_WARPS;
 // Barrier of a team: hardware barrier `bar` over its threads.
 __device__ __forceinline__ void team_sync(u32 bar) { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(TEAM_THREADS) : "memory"); }
-constexpr int SIEVE_BATCH = 8;
-__device__ inline void team_td_sieve(u64 A0, const uint2 *__restrict__ tdqm, TdSieve &S, u32 tid, u32 bar) {
+// In the bulk a warp sieves for its own prime too, in the place of a trial division on each of its
+// rungs (2^43 integers at 1e16, 88 K primes: stage D 9.2 -> 5.2 ms with the rolled loops). 4 entries in
+// flight: 8 spill (2^41 integers at 1e15 1.86 ms for 1.78), 2 are no faster than 4.
+constexpr int SIEVE_BATCH = 4;
+template <int THREADS>
+static __device__ inline void td_sieve(u64 A0, const uint2 *__restrict__ tdqm, TdSieve &S, u32 tid, u32 bar) {
+  auto sync = [&]() { if (THREADS == 32) __syncwarp(); else team_sync(bar); };
   const u32 hi = (u32)(A0 >> 32), mid = (u32)(A0 >> 16) & 0xFFFFu, lo = (u32)A0 & 0xFFFFu;
-  for (u32 k = tid; k < TD_RUNGS; k += TEAM_THREADS) S.n[k] = 0;
+  for (u32 k = tid; k < TD_RUNGS; k += THREADS) S.n[k] = 0;
   if (tid < TD_SMALL) {
     const uint2 e = __ldg(tdqm + tid);
     S.qm[tid] = e;
     S.rs[tid] = mod_a0(hi, mid, lo, e.x, e.y);
   }
-  team_sync(bar);
-  for (u32 k = tid; k < TD_RUNGS; k += TEAM_THREADS) {   // the small primes, rung by rung
+  sync();
+  for (u32 k = tid; k < TD_RUNGS; k += THREADS) {   // the small primes, rung by rung
     u32 mask = 0;
     #pragma unroll
     for (int i = 0; i < TD_SMALL; ++i) {
@@ -550,15 +566,16 @@ __device__ inline void team_td_sieve(u64 A0, const uint2 *__restrict__ tdqm, TdS
   auto load = [&](int i0, uint2 (&to)[SIEVE_BATCH]) {
     #pragma unroll
     for (int j = 0; j < SIEVE_BATCH; ++j) {
-      const int i = i0 + j * TEAM_THREADS;
+      const int i = i0 + j * THREADS;
       to[j] = i < NTD ? __ldg(tdqm + i) : make_uint2(1u, ~0u);       // 1: residue 0, never a listed prime
     }
   };
   load(TD_SMALL + tid, nx);
-  for (int i0 = TD_SMALL + tid; i0 < NTD; i0 += SIEVE_BATCH * TEAM_THREADS) {
+  #pragma unroll 1
+  for (int i0 = TD_SMALL + tid; i0 < NTD; i0 += SIEVE_BATCH * THREADS) {
     #pragma unroll
     for (int j = 0; j < SIEVE_BATCH; ++j) e[j] = nx[j];
-    load(i0 + SIEVE_BATCH * TEAM_THREADS, nx);
+    load(i0 + SIEVE_BATCH * THREADS, nx);
     u32 k[SIEVE_BATCH];
     #pragma unroll
     for (int j = 0; j < SIEVE_BATCH; ++j) {
@@ -569,10 +586,45 @@ __device__ inline void team_td_sieve(u64 A0, const uint2 *__restrict__ tdqm, TdS
     for (int j = 0; j < SIEVE_BATCH; ++j)
       if (k[j] < (u32)TD_RUNGS) {
         const u32 s = atomicAdd(&S.n[k[j]], 1u);
-        if (s < (u32)TD_LIST_CAP) S.idx[k[j]][s] = (u16)(i0 + j * TEAM_THREADS);
+        if (s < (u32)TD_LIST_CAP) S.idx[k[j]][s] = (u16)(i0 + j * THREADS);
       }
   }
-  team_sync(bar);
+  sync();
+}
+
+// Records in F the primes d (one per lane, where `hit`: x = n / d exactly, iv = d^-1 mod 2^64) with
+// their full powers in n; returns the product of the inverses of those powers.
+static __device__ __noinline__ u64 take_primes(WarpFac &F, bool hit, u64 x, u64 iv, u32 d, u32 lane) {
+  const unsigned mask = __ballot_sync(FULL, hit);
+  u64 f = 1;
+  int e = 0;
+  if (hit) {
+    u64 m = x;
+    e = 1;
+    f = iv;
+    #pragma unroll 1
+    for (int g = 0; g < 64; ++g) {
+      x = m * iv;
+      if (__umul64hi(x, (u64)d)) break;
+      m = x; ++e; f *= iv;
+    }
+  }
+  const int base = F.k;
+  __syncwarp();
+  if (hit) {
+    const int pos = base + __popc(mask & ((1u << lane) - 1));
+    if (pos < MAXF) { F.pr[pos] = d; F.ex[pos] = e; }
+  }
+  #pragma unroll
+  for (int o = 16; o; o >>= 1) f *= __shfl_xor_sync(FULL, f, o);
+  __syncwarp();
+  if (lane == 0) {
+    const int nk = base + __popc(mask);
+    if (nk > MAXF) F.overflow = 1;
+    F.k = nk > MAXF ? MAXF : nk;
+  }
+  __syncwarp();
+  return f;                                        // exact: n times it has every d^e divided out
 }
 
 // Complete factorization of n >= 1 into F (prime order as found). All lanes call.
@@ -602,40 +654,8 @@ __device__ inline bool warp_factor(u64 n, WarpFac &F, const u32 *__restrict__ td
   // than one per block. Testing primes past the point where d^2 > cur is harmless (each prime
   // is tested once, against n, and a hit is a genuine factor), so the early exit is checked
   // once per block.
-  // Divides out of cur every prime of this chunk that divides n (hit: x = n / d exactly), with
-  // its full power, and records it in F.
   auto take = [&](bool hit, u64 x, u64 iv, u32 d) {
-    const unsigned mask = __ballot_sync(FULL, hit);
-    if (!mask) return;                             // rare: a prime below 2^16 divides n
-    u64 f = 1;
-    int e = 0;
-    if (hit) {
-      u64 m = x;
-      e = 1;
-      f = iv;
-      for (int g = 0; g < 64; ++g) {
-        x = m * iv;
-        if (__umul64hi(x, (u64)d)) break;
-        m = x; ++e; f *= iv;
-      }
-    }
-    const int base = F.k;
-    __syncwarp();
-    if (hit) {
-      const int pos = base + __popc(mask & ((1u << lane) - 1));
-      if (pos < MAXF) { F.pr[pos] = d; F.ex[pos] = e; }
-    }
-    u64 g = f;
-    #pragma unroll
-    for (int o = 16; o; o >>= 1) g *= __shfl_xor_sync(FULL, g, o);
-    cur *= g;                                      // exact: divides out every d^e found
-    __syncwarp();
-    if (lane == 0) {
-      const int nk = base + __popc(mask);
-      if (nk > MAXF) F.overflow = 1;
-      F.k = nk > MAXF ? MAXF : nk;
-    }
-    __syncwarp();
+    if (__any_sync(FULL, hit)) cur *= take_primes(F, hit, x, iv, d, lane);   // rare: a prime below 2^16 divides n
   };
   if (td_list && td_n <= (u32)TD_LIST_CAP) {       // the block's sieve listed n's odd primes < 2^16
     const u32 ns = __popc(td_small);               // lanes [0, ns): the small ones, then the list
@@ -667,6 +687,7 @@ __device__ inline bool warp_factor(u64 n, WarpFac &F, const u32 *__restrict__ td
     }
   };
   load_block(0, inv, pr);
+  #pragma unroll 1
   for (int cb = 0; cb < TD_CHUNKS; cb += TD_UNROLL) {
     if (cb + TD_UNROLL < TD_CHUNKS) load_block(cb + TD_UNROLL, ninv, npr);
     const int nx = (cb + TD_UNROLL) * 32;
@@ -745,6 +766,7 @@ constexpr u32 SMALL_U = 65536;
 __device__ inline u32 warp_small_divisor(const WarpFac &F, const ModR &R, u32 target, DPWarp &D, u32 lane) {
   u32 *v = reinterpret_cast<u32 *>(D.v[0]), *w = reinterpret_cast<u32 *>(D.v[1]);
   const u32 r = R.r;
+  #pragma unroll 1
   for (u32 t = lane; t < r; t += 32) v[t] = t == (r == 1 ? 0u : 1u) ? 1u : ~0u;
   __syncwarp();
   const u64 mine = lane < (u32)F.k ? F.pr[lane] : ~0ull;
@@ -753,11 +775,14 @@ __device__ inline u32 warp_small_divisor(const WarpFac &F, const ModR &R, u32 ta
     const u32 pr = (u32)min(__shfl_sync(FULL, mine, idx), (u64)SMALL_U), res = __shfl_sync(FULL, my_res, idx);
     if (pr >= SMALL_U) continue;
     const int e = 2 * (int)F.ex[idx];
+    #pragma unroll 1
     for (u32 t = lane; t < r; t += 32) w[t] = v[t];
     __syncwarp();
+    #pragma unroll 1
     for (u32 t = lane; t < r; t += 32) {
       u32 x = v[t], s = t;
       if (x == ~0u) continue;
+      #pragma unroll 1
       for (int j = 0; j < e; ++j) {
         x *= pr;                                       // below 2^16 2^16
         if (x > SMALL_U) break;
@@ -779,17 +804,21 @@ __device__ inline u32 warp_small_divisor(const WarpFac &F, const ModR &R, u32 ta
 __device__ inline bool warp_class_met(u64 p, const WarpFac &F, const ModR &R, u32 target, DPWarp &D, u32 lane) {
   unsigned char *v = reinterpret_cast<unsigned char *>(D.v[0]), *w = reinterpret_cast<unsigned char *>(D.v[1]);
   const u32 r = R.r;
+  #pragma unroll 1
   for (u32 t = lane; t < r; t += 32) v[t] = t == (r == 1 ? 0u : 1u);
   __syncwarp();
   const u32 my_res = R.mod64(lane < (u32)F.k ? F.pr[lane] : p);    // lane F.k <= MAXF: p
   for (int idx = 0; idx <= F.k; ++idx) {
     const u32 res = __shfl_sync(FULL, my_res, idx);
     const int e = idx < F.k ? 2 * (int)F.ex[idx] : 2;
+    #pragma unroll 1
     for (u32 t = lane; t < r; t += 32) w[t] = v[t];
     __syncwarp();
+    #pragma unroll 1
     for (u32 t = lane; t < r; t += 32) {
       if (!v[t]) continue;
       u32 s = t;
+      #pragma unroll 1
       for (int j = 0; j < e; ++j) { s = R.mod32(s * res); w[s] = 1; }
     }
     __syncwarp();
@@ -811,23 +840,28 @@ __device__ inline U128 warp_min_div_res(u64 p, const WarpFac &F, U128 q, u32 r, 
   const u32 pm = R.mod64(p);
   const bool p_fits = !lt128(q, U128{p, 0});
   u32 ph = 0;                                     // D.v[ph] is the current table
+  #pragma unroll 1
   for (u32 t = lane; t < r; t += 32)
     D.v[0][t] = (t == one) ? U128{1, 0} : (p_fits && t == pm) ? U128{p, 0} : INF;
   __syncwarp();
+  #pragma unroll 1
   for (int idx = 0; idx < F.k; ++idx) {
     const u64 pr = F.pr[idx];
     const int e = 2 * (int)F.ex[idx];
     const u32 prm = R.mod64(pr);
     u32 inv = 0;                                 // prm^-1 mod r (prm is a unit: gcd(q, r) = 1)
+    #pragma unroll 1
     for (u32 base = 0; base < r; base += 32) {
       const u32 x = base + lane;
       const unsigned m = __ballot_sync(FULL, x < r && R.mod32(prm * x) == one);
       if (m) { inv = base + __ffs(m) - 1; break; }
     }
+    #pragma unroll 1
     for (u32 t = lane; t < r; t += 32) {
       U128 best = INF;
       u32 s = t;
       U128 pw{1, 0};
+      #pragma unroll 1
       for (int j = 0; j <= e; ++j) {
         if (j) {
           bool over;
@@ -911,17 +945,18 @@ __device__ inline bool rung_divisor(u64 p, u64 A, U128 q, u32 r, u32 target, War
 // cofactors on rho: with every warp of the GPU busy, a round of curves costs more issue slots
 // than the rho steps it saves (a 10^14-integer window at 10^16, a million primes: 108 ms of
 // stage D with rho alone, 179 ms with ECM), while ECM pays in the latency-bound tail.
-__device__ inline bool warp_solve_rung(u64 p, const u32 *tdp, const u64 *tdi, u32 *status, WarpFac &F,
-                                       DPWarp &D, volatile u64 *rho_slot, RungResult *out,
+__device__ inline bool warp_solve_rung(u64 p, const u32 *tdp, const u64 *tdi, const uint2 *tdqm, u32 *status, WarpFac &F,
+                                       DPWarp &D, TdSieve &S, volatile u64 *rho_slot, RungResult *out,
                                        u64 rho_budget = WARP_RHO_STEPS, bool use_ecm = true) {
   const u32 lane = threadIdx.x & 31;
   const u32 r0 = rung_r0(p);
+  td_sieve<32>((p >> 2) + 1, tdqm, S, lane, 0);
   for (u32 k = 0; r0 + 4 * k <= RCAP; ++k) {
     Rung g;
     if (!rung_of(p, k, g)) continue;
     U128 u;
     if (!rung_divisor(p, g.A, g.q, g.r, g.target, F, D, tdp, tdi, status, lane, rho_slot, nullptr, 0, nullptr, 0,
-                      rho_budget, use_ecm, u))
+                      rho_budget, use_ecm, u, S.idx[k], S.n[k], S.small[k]))
       return false;
     if (u.lo == 0 && u.hi == 0) continue;
     if (lane == 0) *out = RungResult{g.A, g.r, k, u};
@@ -934,7 +969,7 @@ __device__ inline bool warp_solve_rung(u64 p, const u32 *tdp, const u64 *tdi, u3
 // The rung walk of one prime by a team of four warps (solve_rung3, sieve/rung_scan3.cpp:
 // 578-603). Warp w takes rung indices k = w, w+4, ... (r = r0 + 4k) in increasing order and
 // stops once k passes the best certifying index found by any warp. The team first lists the odd
-// primes below 2^16 of all the prime's rungs at once (team_td_sieve), and each rung divides out
+// primes below 2^16 of all the prime's rungs at once (td_sieve), and each rung divides out
 // only its own. Returns true in every thread when some rung certifies p; the team's result is
 // then in *out. F, D, rho_slot and slot are the team's four, warp0 its first slot in *bh, *busy
 // the count of its warps still on their rungs.
@@ -958,7 +993,7 @@ __device__ inline bool team_solve_rung(u64 p, const u32 *tdp, const u64 *tdi, co
   }
   if (lane == 0) T.slot[w].k = 0x7FFFFFFF;
   team_sync(T.bar);
-  team_td_sieve((p >> 2) + 1, tdqm, *T.S, tid, T.bar);   // A_0 = floor(p/4) + 1
+  td_sieve<TEAM_THREADS>((p >> 2) + 1, tdqm, *T.S, tid, T.bar);   // A_0 = floor(p/4) + 1
   const u32 r0 = rung_r0(p);
   for (u32 k = w; r0 + 4 * k <= RCAP; k += TEAM_WARPS) {
     // warp-uniform: every lane must take the same branch before the warp collectives below
