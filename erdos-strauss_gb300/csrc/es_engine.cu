@@ -1193,6 +1193,11 @@ namespace es {
 // device buffers and their pinned host staging, and the captured graph. An engine has one
 // slot for its synchronous calls and SERVE_SLOTS more for the serving workers, so that
 // several batches can be in flight on their own streams.
+struct RecKey {                         // a record's place in its window
+  u64 J;
+  u32 lane, idx;
+  bool operator<(const RecKey &o) const { return lane != o.lane ? lane < o.lane : J < o.J; }
+};
 struct Slot {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[12] = {};
@@ -1222,17 +1227,19 @@ struct Slot {
   u64 graph_launches = 0;               // its kernels
   unsigned long long *d_ctr = nullptr;  // run counters (es_kernels.cuh) and stage D's board
   u32 *d_status = nullptr;
+  unsigned char *d_probe = nullptr; size_t probe_cap = 0;
   es_timing_t timing{};
   struct HostScratch {                  // per-run host vectors, kept with their capacity
     std::vector<WinDev> wd;
     std::vector<RowWin> roww;
     std::vector<u64> npos;
-    std::vector<RecDev> hr;
-    std::vector<u32> start, pos;
+    std::vector<RecDev> hr;             // the plain schedule's records, unordered
+    std::vector<RecKey> key, bin;       // order_records
+    std::vector<u32> start, pos, bstart;
     std::vector<es_window> dw;          // runs in passes (run_windows)
     std::vector<std::pair<u32, u64>> dmap;
     std::vector<es_counters> pc;
-    std::vector<es_record> all;
+    std::vector<RecDev> all;            // and their records
   } hs;
   std::mutex mu;                        // one run at a time per slot
 };
@@ -1668,14 +1675,74 @@ static std::string status_text(u32 st) {
   return s;
 }
 
-// Runs windows through the funnel and collects counters and sorted records. Re-runs
-// with larger buffers when the survivor list overflowed (the count is exact even then).
 static double ms_since(std::chrono::steady_clock::time_point t) {
   return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t).count();
 }
 
+constexpr size_t ORDER_BINS_MIN = 64;
+// The caller's copy of m records of n windows, in (window, lane, J) order. What is sorted are
+// 16-byte keys, dealt out by window and, in a window of many, by lane into about as many bins as it
+// has records; each record is then copied once, from where the device wrote it. 88 K records
+// (one window of 2^43 integers at 1e16): 2.4 ms, where sorting the records themselves took 6.2.
+// Below ORDER_BINS_MIN the bins' own passes cost as much as the comparisons that they save.
+static es_status order_records(es_engine *e, Slot *sl, const RecDev *src, size_t m, size_t n, es_records *recs) {
+  static_assert(sizeof(RecDev) == sizeof(es_record), "record layout");
+  recs->n = m;
+  recs->recs = (es_record *)malloc(std::max<size_t>(m, 1) * sizeof(es_record));
+  if (!recs->recs) return fail(e, ES_ERR_NOMEM, "host records");
+  std::vector<u32> &start = sl->hs.start, &pos = sl->hs.pos, &bstart = sl->hs.bstart;
+  std::vector<RecKey> &key = sl->hs.key, &bin = sl->hs.bin;
+  start.assign(n + 1, 0);
+  pos.resize(m);
+  bin.resize(m);
+  for (size_t i = 0; i < m; ++i) {                   // one read of what the device wrote, in its order
+    const RecDev &r = src[i];
+    bin[i] = RecKey{r.J, r.lane, (u32)i};
+    pos[i] = (u32)std::min<size_t>(r.win, n - 1);
+    ++start[pos[i] + 1];
+  }
+  for (size_t i = 0; i < n; ++i) start[i + 1] += start[i];
+  if (n == 1) {
+    key.swap(bin);
+  } else {
+    key.resize(m);
+    bstart.assign(start.begin(), start.end() - 1);
+    for (size_t i = 0; i < m; ++i) key[bstart[pos[i]]++] = bin[i];
+  }
+  const size_t lanes = std::max<size_t>(e->classes.size(), 1);
+  for (size_t i = 0; i < n; ++i) {
+    RecKey *k = key.data() + start[i];
+    const size_t c = start[i + 1] - start[i];
+    if (c > ORDER_BINS_MIN) {
+      u32 shift = 0;
+      while ((lanes - 1) >> shift >= c) ++shift;
+      const size_t bins = ((lanes - 1) >> shift) + 1;
+      auto bin_of = [&](const RecKey &x) { return std::min<size_t>(x.lane >> shift, bins - 1); };
+      bstart.assign(bins + 1, 0);
+      for (size_t j = 0; j < c; ++j) ++bstart[bin_of(k[j]) + 1];
+      for (size_t b = 0; b < bins; ++b) bstart[b + 1] += bstart[b];
+      bin.assign(k, k + c);
+      for (const RecKey &x : bin) k[bstart[bin_of(x)]++] = x;      // bstart[b] is now bin b's end
+      size_t from = 0;
+      for (size_t b = 0; b < bins; from = bstart[b++])
+        if (bstart[b] - from > 1) std::sort(k + from, k + bstart[b]);
+    } else if (c > 1) {
+      std::sort(k, k + c);
+    }
+  }
+  RecDev *out = reinterpret_cast<RecDev *>(recs->recs);
+  for (size_t i = 0; i < m; ++i) {
+    if (i + 16 < m) __builtin_prefetch(&src[key[i + 16].idx]);
+    out[i] = src[key[i].idx];
+  }
+  return ES_OK;
+}
+
+// Runs windows through the funnel and collects counters; the records are left unordered at *src
+// (the slot's, until its next run). Re-runs with larger buffers when the survivor list overflowed
+// (the count is exact even then).
 static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, size_t n, int schedule,
-                                    es_counters *per_window, es_records *recs) {
+                                    es_counters *per_window, const RecDev **src, size_t *nsrc) {
   const auto t_start = std::chrono::steady_clock::now();
   double setup_ms = 0, device_ms = 0;
   const u64 floor_ = std::max(e->wheel_pmin, e->cover_pmax);
@@ -1696,8 +1763,8 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
   // candidate chunks: half as many again as the estimate, and a part-filled one per warp and run
   size_t chunks = (size_t)(1.5 * e->cand_rate * (double)positions_bound / 32) + 4 * (size_t)e->sm_count * (ROW_THREADS / 32);
   const bool persistent = schedule == ES_SCHED_PERSISTENT;
-  std::vector<RecDev> &hr = sl->hs.hr;
-  hr.clear();
+  std::vector<RecDev> &hr = sl->hs.hr;   // the plain schedule's
+  size_t nrec = 0;
   bool done = false;
   for (int attempt = 0; attempt < 4 && !done; ++attempt) {
     es_status s = ensure_capacity(e, sl, n, shape.pieces, chunks, cap);
@@ -1721,8 +1788,7 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
       prime_total += ctr[2];
       status |= *sl->h_status;
       if (ctr[1] > sl->cap) return ES_OK;
-      const size_t nrec = (size_t)std::min<u64>(ctr[4], sl->cap);
-      if (nrec) hr.insert(hr.end(), sl->h_recs, sl->h_recs + nrec);
+      nrec = (size_t)std::min<u64>(ctr[4], sl->cap);
       return ES_OK;
     };
     if (persistent) {
@@ -1764,11 +1830,14 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
         if (s) return s;
         CU(cudaStreamSynchronize(sl->stream));
         launches += 2;
-        const size_t base = hr.size();
+        nrec = 0;
         s = collect();
         if (s) return s;
         if (surv_max > sl->cap || chunk_max > sl->chunk_cap) break;
-        for (size_t r = base; r < hr.size(); ++r) hr[r].win = (u32)i;
+        for (size_t r = 0; r < nrec; ++r) {
+          hr.push_back(sl->h_recs[r]);
+          hr.back().win = (u32)i;
+        }
       }
     }
     if (surv_max > sl->cap || chunk_max > sl->chunk_cap) {   // overflow: grow to the exact need and re-run
@@ -1804,29 +1873,8 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
     o.mr = c.surv; o.composite = c.surv >= primes_w ? c.surv - primes_w : 0; o.rung = c.rung; o.direct = c.direct;
     o.survivors = c.unsolved;
   }
-  if (recs) {
-    // Lane-major order within each window: a counting sort on the window index straight into
-    // the caller's buffer, then (lane, J) order inside each window's few records.
-    static_assert(sizeof(RecDev) == sizeof(es_record), "record layout");
-    recs->n = hr.size();
-    recs->recs = (es_record *)malloc(std::max<size_t>(hr.size(), 1) * sizeof(es_record));
-    if (!recs->recs) return fail(e, ES_ERR_NOMEM, "host records");
-    RecDev *out = reinterpret_cast<RecDev *>(recs->recs);
-    std::vector<u32> &start = sl->hs.start, &pos = sl->hs.pos;
-    start.assign(n + 1, 0);
-    for (const RecDev &r : hr) ++start[std::min<size_t>(r.win, n - 1) + 1];
-    for (size_t i = 0; i < n; ++i) start[i + 1] += start[i];
-    pos.assign(start.begin(), start.end() - 1);
-    for (const RecDev &r : hr) out[pos[std::min<size_t>(r.win, n - 1)]++] = r;
-    for (size_t i = 0; i < n; ++i) {
-      if (start[i + 1] - start[i] > 1)
-        std::sort(out + start[i], out + start[i + 1], [](const RecDev &a, const RecDev &b) {
-          if (a.win != b.win) return a.win < b.win;
-          if (a.lane != b.lane) return a.lane < b.lane;
-          return a.J < b.J;
-        });
-    }
-  }
+  *src = persistent ? sl->h_recs : hr.data();
+  *nsrc = persistent ? nrec : hr.size();
   sl->timing.host_setup_ms = setup_ms;
   sl->timing.host_device_ms = device_ms;
   sl->timing.host_collect_ms = ms_since(t_start) - setup_ms - device_ms;
@@ -1855,8 +1903,22 @@ static es_status run_windows(es_engine *e, Slot *sl, const es_window *w, size_t 
       return fail(e, ES_ERR_RANGE, "LO must exceed max pmin of the filter table (" + std::to_string(floor_) + ")");
     rows += rows_of(w[i].lo, w[i].hi);
   }
-  if (rows <= e->pass_rows) return run_device_windows(e, sl, w, n, schedule, per_window, recs);
-  std::vector<es_record> &all = sl->hs.all;
+  const RecDev *src = nullptr;
+  size_t nsrc = 0;
+  const auto t_start = std::chrono::steady_clock::now();
+  auto finish = [&](const RecDev *from, size_t m) -> es_status {     // the records, ordered
+    if (recs) {
+      const es_status st = order_records(e, sl, from, m, n, recs);
+      if (st != ES_OK) return st;
+    }
+    sl->timing.host_collect_ms = ms_since(t_start) - sl->timing.host_setup_ms - sl->timing.host_device_ms;
+    return ES_OK;
+  };
+  if (rows <= e->pass_rows) {
+    const es_status st = run_device_windows(e, sl, w, n, schedule, per_window, &src, &nsrc);
+    return st != ES_OK ? st : finish(src, nsrc);
+  }
+  std::vector<RecDev> &all = sl->hs.all;
   all.clear();
   es_timing_t tot{};
   std::vector<es_window> &dw = sl->hs.dw;
@@ -1886,24 +1948,21 @@ static es_status run_windows(es_engine *e, Slot *sl, const es_window *w, size_t 
     }
     const size_t m = dw.size();
     pc.resize(m);
-    es_records pr{nullptr, 0};
-    const es_status st = run_device_windows(e, sl, dw.data(), m, schedule, pc.data(), recs ? &pr : nullptr);
-    if (st != ES_OK) { es_free_records(&pr); return st; }
+    const es_status st = run_device_windows(e, sl, dw.data(), m, schedule, pc.data(), &src, &nsrc);
+    if (st != ES_OK) return st;
     for (size_t k = 0; k < m; ++k) {
       es_counters &o = per_window[dmap[k].first];
       const es_counters &c = pc[k];
       o.positions += c.positions; o.covered += c.covered; o.sieved += c.sieved; o.mr += c.mr;
       o.composite += c.composite; o.rung += c.rung; o.direct += c.direct; o.survivors += c.survivors;
     }
-    all.reserve(all.size() + pr.n);
-    for (size_t r = 0; r < pr.n; ++r) {
-      es_record x = pr.recs[r];
-      const auto &mp = dmap[x.window];
-      x.window = mp.first;
+    for (size_t r = 0; recs && r < nsrc; ++r) {
+      all.push_back(src[r]);
+      RecDev &x = all.back();
+      const auto &mp = dmap[std::min<size_t>(x.win, m - 1)];
+      x.win = mp.first;
       x.J += mp.second;
-      all.push_back(x);
     }
-    es_free_records(&pr);
     const es_timing_t &tt = sl->timing;
     tot.total_ms += tt.total_ms; tot.mark_ms += tt.mark_ms; tot.mr_ms += tt.mr_ms; tot.rung_ms += tt.rung_ms;
     tot.direct_ms += tt.direct_ms; tot.prep_ms += tt.prep_ms; tot.mark_short_ms += tt.mark_short_ms;
@@ -1911,29 +1970,9 @@ static es_status run_windows(es_engine *e, Slot *sl, const es_window *w, size_t 
     tot.kernel_launches += tt.kernel_launches; tot.mark_items += tt.mark_items; tot.survivors += tt.survivors;
     tot.primes += tt.primes; tot.short_pairs += tt.short_pairs; tot.mask_bytes += tt.mask_bytes;
     tot.host_setup_ms += tt.host_setup_ms; tot.host_device_ms += tt.host_device_ms;
-    tot.host_collect_ms += tt.host_collect_ms;
   }
   sl->timing = tot;
-  if (recs) {
-    // Each pass's records come in (device window, lane, J) order and the device windows of a
-    // window are consecutive (across passes too), so the records are already grouped by window
-    // in ascending order; only a split window's group needs putting back in (lane, J) order.
-    for (size_t a = 0; a < all.size();) {
-      size_t b = a + 1;
-      while (b < all.size() && all[b].window == all[a].window) ++b;
-      if (b - a > 1)
-        std::sort(all.begin() + a, all.begin() + b, [](const es_record &x, const es_record &y) {
-          if (x.lane != y.lane) return x.lane < y.lane;
-          return x.J < y.J;
-        });
-      a = b;
-    }
-    recs->n = all.size();
-    recs->recs = (es_record *)malloc(std::max<size_t>(all.size(), 1) * sizeof(es_record));
-    if (!recs->recs) return fail(e, ES_ERR_NOMEM, "host records");
-    memcpy(recs->recs, all.data(), all.size() * sizeof(es_record));
-  }
-  return ES_OK;
+  return finish(all.data(), all.size());
 }
 
 static es_status build_tables(es_engine *e) {
@@ -2272,25 +2311,38 @@ static void serve_worker(es_engine *e, int k) {
 using namespace es;
 
 namespace es {
-// Probes: copy in, one kernel, copy out. Small and synchronous.
+// Probes: copy in, one kernel, copy out. Small and synchronous. The buffer stays with the engine up to
+// PROBE_KEEP bytes: an allocation and its release a call took 150 us (the primality of 200 K values
+// 366 -> 217 us, 8 K factorizations 828 -> 677).
+constexpr size_t PROBE_KEEP = 64u << 20;
 template <typename Launch>
 static es_status probe(es_engine *e, Slot *sl, size_t count, size_t in_bytes, const void *in, size_t out_bytes,
                        std::vector<std::pair<void *, size_t>> outs, Launch launch) {
   std::lock_guard<std::mutex> lk(sl->mu);
   cudaSetDevice(e->device);
-  void *d_in = nullptr;
-  std::vector<void *> d_outs(outs.size(), nullptr);
-  struct Release {                                   // the probe's buffers, on every return path
-    void *&in;
-    std::vector<void *> &outs;
+  auto unit = [](size_t b) { return (std::max<size_t>(b, 8) + 255) & ~(size_t)255; };
+  size_t total = unit(in_bytes);
+  for (const auto &o : outs) total += unit(o.second);
+  struct Release {                                   // what is too large to stay, on every return path
+    Slot *sl;
     ~Release() {
-      cudaFree(in);
-      for (void *p : outs) cudaFree(p);
+      if (sl->probe_cap <= PROBE_KEEP) return;
+      cudaFree(sl->d_probe);
+      sl->d_probe = nullptr;
+      sl->probe_cap = 0;
     }
-  } release{d_in, d_outs};
-  (void)out_bytes;
-  CU(cudaMalloc(&d_in, std::max<size_t>(in_bytes, 8)));
-  for (size_t i = 0; i < outs.size(); ++i) CU(cudaMalloc(&d_outs[i], std::max<size_t>(outs[i].second, 8)));
+  } release{sl};
+  if (total > sl->probe_cap) {
+    cudaFree(sl->d_probe);
+    sl->d_probe = nullptr;
+    sl->probe_cap = 0;
+    CU(cudaMalloc(&sl->d_probe, total));
+    sl->probe_cap = total;
+  }
+  void *d_in = sl->d_probe;
+  std::vector<void *> d_outs(outs.size(), nullptr);
+  size_t at = unit(in_bytes);
+  for (size_t i = 0; i < outs.size(); ++i) { d_outs[i] = sl->d_probe + at; at += unit(outs[i].second); }
   // Every copy is queued on the probe's own stream (a non-blocking stream is not ordered after
   // the legacy stream that a plain cudaMemcpy uses), and the host waits for that stream before
   // it reads anything back.
@@ -2457,7 +2509,7 @@ es_status es_close(es_engine *e) {
     cudaFree(sl.d_win); cudaFree(sl.d_cnt); cudaFree(sl.d_Qm);
     cudaFree(sl.d_piece); cudaFree(sl.d_pidx); cudaFree(sl.d_rowinfo); cudaFree(sl.d_cand); cudaFree(sl.d_chunk);
     cudaFree(sl.d_surv); cudaFree(sl.d_primes); cudaFree(sl.d_direct); cudaFree(sl.d_recs);
-    cudaFree(sl.d_ctr); cudaFree(sl.d_status); cudaFree(sl.d_hdr);
+    cudaFree(sl.d_ctr); cudaFree(sl.d_status); cudaFree(sl.d_hdr); cudaFree(sl.d_probe);
     cudaFreeHost(sl.h_hdr); cudaFreeHost(sl.h_win); cudaFreeHost(sl.h_roww); cudaFreeHost(sl.h_cnt);
     cudaFreeHost(sl.h_ctr); cudaFreeHost(sl.h_status); cudaFreeHost(sl.h_recs);
     for (auto &ev : sl.ev) if (ev) cudaEventDestroy(ev);

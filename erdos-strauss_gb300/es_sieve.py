@@ -230,7 +230,7 @@ class Engine:
         n = recs.n
         if n:
             buf = (C.c_char * (n * RECORD_DTYPE.itemsize)).from_address(C.addressof(recs.recs.contents))
-            arr = np.frombuffer(bytes(buf), dtype=RECORD_DTYPE).copy()
+            arr = np.frombuffer(buf, dtype=RECORD_DTYPE).copy()
         else:
             arr = np.zeros(0, dtype=RECORD_DTYPE)
         lib.es_free_records(C.byref(recs))
