@@ -46,6 +46,7 @@
 #include <type_traits>
 #include <chrono>
 #include <cinttypes>
+#include <cmath>
 #include <condition_variable>
 #include <cstdio>
 #include <cstdlib>
@@ -745,10 +746,7 @@ __device__ __forceinline__ bool take_square(const RowParams &P, const Cand &x) {
 // the two), while copying all lane tables costs 15 us whatever the count: a 2^34 window's 5 K part-
 // filled chunks took 15 us more with them. Bound by instruction issue (58% of peak issue on the 2^40
 // window: 0.35 ms for 2.3 M candidates).
-#ifndef ES_SIFT_FAR
-#define ES_SIFT_FAR 8192
-#endif
-constexpr u32 SIFT_FAR = ES_SIFT_FAR;
+constexpr u32 SIFT_FAR = 8192;
 constexpr u32 THREAD_STRIDES[2] = {32, 64};
 __global__ void __launch_bounds__(ROW_THREADS, 1) k_sift(const RowParams P) {
   extern __shared__ __align__(128) unsigned char rowmem[];
@@ -880,6 +878,36 @@ __global__ void k_build_rows(const u16 *__restrict__ K0, u32 L, u32 ldk, u32 nf,
   } else {
     atomicOr(tlane + (size_t)l * lane_words + mdesc[n1p - n1 + m].w + (k0 >> 5), 1u << (k0 & 31));
   }
+}
+
+// Adds to *sum, a lane a thread, the share of its positions that no stride of the tables kills, were
+// the strides independent: what the survivor buffers are sized by. A lane's own product and not the
+// product of the strides' means, since lanes differ: few of them hold most of what is left.
+__global__ void k_lane_rate(const u32 *__restrict__ tdense, const u32 *__restrict__ tlane, const uint4 *__restrict__ mdesc,
+                            u32 n1, u32 n1p, u32 nm, u32 slice_rows, u32 lane_words, u32 L, double *__restrict__ sum) {
+  const u32 l = blockIdx.x * blockDim.x + threadIdx.x;
+  double r = 0;
+  if (l < L) {
+    r = 1;
+    const u32 *slice = tdense + (size_t)(l / GROUP_LANES) * slice_rows * GROUP_WORDS + l % GROUP_LANES / 32;
+    for (u32 m = 0; m < n1; ++m) {
+      const uint4 d = mdesc[m];
+      u32 c = 0;
+      #pragma unroll 8
+      for (u32 x = 0; x < d.x; ++x) c += slice[(size_t)(d.w + x) * GROUP_WORDS] >> (l & 31) & 1u;
+      r *= 1.0 - (double)c / d.x;
+    }
+    for (u32 m = n1; m < nm; ++m) {
+      const uint4 d = mdesc[n1p - n1 + m];
+      u32 c = 0;
+      #pragma unroll 4
+      for (u32 x = 0; x < (d.x + 31) / 32; ++x) c += __popc(tlane[(size_t)l * lane_words + d.w + x]);
+      r *= 1.0 - (double)c / d.x;
+    }
+  }
+  #pragma unroll
+  for (int o = 16; o; o >>= 1) r += __shfl_xor_sync(FULL, r, o);
+  if (!(threadIdx.x & 31)) atomicAdd(sum, r);
 }
 
 // Whether a filter (mod, res) can kill a perfect square: a thread per (filter, x mod mod), hits
@@ -1291,6 +1319,7 @@ struct es_engine {
   bool squares = false;                 // see RowParams
   std::vector<uint32_t> sq;             // the primes a root has to avoid
   es::u64 pass_rows = 0;                // rows a run marks at a time (run_windows)
+  double surv_rate = 0;                 // survivors per position, estimated (k_lane_rate)
   double cand_rate = 0;                 // candidates per position after the dense strides, estimated
   uint32_t lane_words = 0, n2 = 0, ngroups = 0, n1 = 0, n1p = 0, slice_rows = 0, nm_cov = 0, nm_all = 0, nl_cov = 0, nl_all = 0;
   es::TdEntry *d_tde = nullptr;
@@ -1738,6 +1767,24 @@ static es_status order_records(es_engine *e, Slot *sl, const RecDev *src, size_t
   return ES_OK;
 }
 
+// Survivors that a run's buffers are made for: SURV_ROOM times the tables' estimate and, where squares
+// get no shortcut, the squares (they survive what the estimate takes for random), at most all the
+// positions; in powers of two, so that batches a little larger than the last do not each make their
+// own. Over 2^34 to 2^43 integers at 1e12 to 1e19 and three tables 0.6 to 2.2 times the estimate
+// came (up to 15 times at 1e12 with 91 expected, where the squares are most of it). A window of 2^43
+// integers at 1e16 takes 8 M records of room where 1/64 of its positions took 67 M, 4.3 GB of it
+// pinned: the first call of an engine 161 -> 25 ms, the 4096-window batch's 6.9 -> 1.7 ms.
+constexpr double SURV_ROOM = 8;
+static size_t surv_room(const es_engine *e, const es_window *w, size_t n, u64 positions) {
+  double want = SURV_ROOM * e->surv_rate * (double)positions;
+  for (size_t i = 0; i < n && !e->squares; ++i)
+    if (w[i].hi > w[i].lo) want += std::sqrt((double)w[i].hi) - std::sqrt((double)w[i].lo) + 1;
+  want = std::min(want, (double)positions) + 1024;
+  size_t room = 1 << 16;
+  while ((double)room < want && room < (1u << 26)) room <<= 1;
+  return room;
+}
+
 // Runs windows through the funnel and collects counters; the records are left unordered at *src
 // (the slot's, until its next run). Re-runs with larger buffers when the survivor list overflowed
 // (the count is exact even then).
@@ -1758,8 +1805,7 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
   const RunShape shape = describe(e, w, n, wd, roww, npos);
   u64 positions_bound = 0;
   for (size_t i = 0; i < n; ++i) positions_bound += npos[i];
-  size_t cap = (size_t)std::min<u64>(std::max<u64>(positions_bound / 64, 1 << 16), 1ull << 26);
-  cap = std::max(cap, sl->cap);
+  size_t cap = std::max(surv_room(e, w, n, positions_bound), sl->cap);
   // candidate chunks: half as many again as the estimate, and a part-filled one per warp and run
   size_t chunks = (size_t)(1.5 * e->cand_rate * (double)positions_bound / 32) + 4 * (size_t)e->sm_count * (ROW_THREADS / 32);
   const bool persistent = schedule == ES_SCHED_PERSISTENT;
@@ -2035,7 +2081,7 @@ static es_status build_tables(es_engine *e) {
   }
   // temporaries of the table build, freed on every return path
   struct Temps {
-    void *p[6] = {};
+    void *p[7] = {};
     ~Temps() { for (void *x : p) cudaFree(x); }
   } temps;
   u64 *d_mods = nullptr, *d_ress = nullptr;
@@ -2187,6 +2233,12 @@ static es_status build_tables(es_engine *e) {
                                                                  (u32 *)e->d_tdense, e->d_tlane);
       CU(cudaGetLastError());
     }
+    CU(cudaMalloc(&temps.p[6], sizeof(double)));
+    CU(cudaMemsetAsync(temps.p[6], 0, sizeof(double), bs));
+    k_lane_rate<<<(L + 127) / 128, 128, 0, bs>>>((const u32 *)e->d_tdense, e->d_tlane, e->d_mdesc, e->n1, e->n1p,
+                                                 e->nm_all, e->slice_rows, e->lane_words, L, (double *)temps.p[6]);
+    CU(cudaGetLastError());
+    CU(cudaMemcpyAsync(&e->surv_rate, temps.p[6], sizeof(double), cudaMemcpyDeviceToHost, bs));
     // Stage B' primes kill squares by their own rule, and moduli past 2^16 are not searched.
     unsigned long long hit = 1;
     if (nf && nf == e->ncov && *std::max_element(om.begin(), om.end()) <= 65536) {
@@ -2198,6 +2250,7 @@ static es_status build_tables(es_engine *e) {
       CU(cudaMemcpyAsync(&hit, temps.p[5], sizeof hit, cudaMemcpyDeviceToHost, bs));
     }
     CU(cudaStreamSynchronize(bs));
+    e->surv_rate /= L;
     e->squares = !(hit & 1);
     for (u32 q = 3; q < 64; ++q)
       if (hit >> q & 1) e->sq.push_back(q);
@@ -2236,7 +2289,7 @@ constexpr size_t SERVE_QUEUE_WINDOWS = 1 << 20;   // windows waiting, across req
 constexpr size_t SERVE_BATCH_WINDOWS = 8192;      // windows per batch a worker takes
 
 // Device bytes a request's windows need in a slot: descriptors, per-window residues and
-// counters, and the survivor-side buffers sized like run_windows sizes them.
+// counters, and survivor-side buffers for 1/64 of their positions.
 static u64 request_bytes(const es_engine *e, const es_window *w, size_t n) {
   u64 pos = 0;
   for (size_t i = 0; i < n; ++i) pos += positions_in(e, w[i].lo, w[i].hi);
