@@ -1184,31 +1184,50 @@ __global__ void k_probe_direct(const u64 *p, u64 count, RecDev *out, unsigned ch
     out[i] = ok ? RecDev{ES_REC_SOLVED, 0, 0, 0, 0, p[i], a, c, d, k} : RecDev{0, 0, 0, 0, 0, p[i], 0, 0, 0, 0};
   }
 }
-// The production factorization (warp_factor), one warp per value; primes sorted ascending.
-__global__ void __launch_bounds__(128, 4) k_probe_factor(const u64 *n, u64 count, u64 *pr, unsigned char *ex, unsigned char *k,
-                               const u32 *tdp, const u64 *tdi, u32 *status, u64 rho_budget) {
-  __shared__ WarpFac F[4];
-  __shared__ u64 rho_slot[4];
+// The production factorization (warp_factor), one warp per value; primes sorted ascending. A block's
+// warps take its values (every gridDim-th) as they come free, and one that finds none left runs
+// curves for the others' cofactors, as stage D's do: 8 K integers of up to 62 bits 585 -> 435 us, 16 of
+// them 281 -> 148.
+struct FactorShared {
+  WarpFac F[BLOCK_WARPS];
+  u64 rho_slot[BLOCK_WARPS];
+  BlockHelp help;
+  unsigned int next;
+};
+__global__ void __launch_bounds__(RUNG_THREADS, 1) k_probe_factor(const u64 *n, u64 count, u64 *pr, unsigned char *ex,
+                                                                  unsigned char *k, const u32 *tdp, const u64 *tdi,
+                                                                  u32 *status, u64 rho_budget) {
+  __shared__ __align__(16) FactorShared H;
   const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const u64 warps = (u64)gridDim.x * blockDim.x / 32;
-  for (u64 i = ((u64)blockIdx.x * blockDim.x + threadIdx.x) / 32; i < count; i += warps) {
-    WarpFac &f = F[w];
-    const bool ok = warp_factor(n[i], f, tdp, tdi, status, lane, rho_slot + w, nullptr, 0, nullptr, 0, rho_budget);
-    if (lane == 0) {
-      const int kk = ok ? f.k : 0;
-      for (int a = 1; a < kk; ++a)
-        for (int b = a; b > 0 && f.pr[b - 1] > f.pr[b]; --b) {
-          const u64 t = f.pr[b]; f.pr[b] = f.pr[b - 1]; f.pr[b - 1] = t;
-          const u32 e = f.ex[b]; f.ex[b] = f.ex[b - 1]; f.ex[b - 1] = e;
-        }
-      for (int a = 0; a < MAXF; ++a) {
-        pr[i * MAXF + a] = a < kk ? f.pr[a] : 0;
-        ex[i * MAXF + a] = a < kk ? (unsigned char)f.ex[a] : 0;
-      }
-      k[i] = (unsigned char)kk;
+  for (u32 i = threadIdx.x; i < sizeof(BlockHelp) / 4; i += blockDim.x) reinterpret_cast<u32 *>(&H.help)[i] = 0;
+  __syncthreads();
+  if (threadIdx.x == 0) { H.help.working = BLOCK_WARPS; H.next = 0; }
+  __syncthreads();
+  for (;;) {
+    u32 j = 0;
+    if (lane == 0) j = atomicAdd(&H.next, 1u);
+    const u64 i = blockIdx.x + (u64)gridDim.x * __shfl_sync(FULL, j, 0);
+    if (i >= count) break;
+    WarpFac &f = H.F[w];
+    const bool ok = warp_factor<true>(n[i], f, tdp, tdi, status, lane, H.rho_slot + w, nullptr, 0, &H.help, w, rho_budget);
+    const u32 kk = ok ? (u32)f.k : 0;
+    const bool mine = lane < kk;
+    const u64 p = mine ? f.pr[lane] : 0;
+    u32 at = lane;                                   // an empty place, or the prime's rank
+    if (mine) {
+      at = 0;
+      for (u32 b = 0; b < kk; ++b) at += f.pr[b] < p || (f.pr[b] == p && b < lane);
     }
+    if (lane < (u32)MAXF) {
+      pr[i * MAXF + at] = p;
+      ex[i * MAXF + at] = mine ? (unsigned char)f.ex[lane] : 0;
+    }
+    if (lane == 0) k[i] = (unsigned char)kk;
     __syncwarp();
   }
+  if (lane == 0) atomicSub(&H.help.working, 1u);
+  __syncwarp();
+  warp_help(&H.help, &H.help.working, nullptr, lane);
 }
 
 // ============================================================================ host engine
@@ -2815,7 +2834,7 @@ es_status es_factor_batch(es_engine *e, const uint64_t *n, size_t count, uint64_
   if (!count) return ES_OK;
   return probe(e, &e->slots[0], count, count * 8, n, 0, {{pr, count * MAXF * 8}, {ex, count * MAXF}, {k, count}},
                [&](void *in, std::vector<void *> &o) {
-                 k_probe_factor<<<e->sm_count * 4, 128, 0, e->slots[0].stream>>>((const u64 *)in, count, (u64 *)o[0],
+                 k_probe_factor<<<e->sm_count, RUNG_THREADS, 0, e->slots[0].stream>>>((const u64 *)in, count, (u64 *)o[0],
                                                                        (unsigned char *)o[1], (unsigned char *)o[2],
                                                                        e->d_tdp, e->d_tdi, e->slots[0].d_status,
                                                                        e->rho_budget);

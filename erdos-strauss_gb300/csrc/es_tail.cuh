@@ -315,6 +315,34 @@ constexpr u32 HELP_POLLS = 1u << 16;     // empty polls (0.5 us apart) before a 
 constexpr u32 BOARD_POLLS = 256;         // the same for the board
 constexpr u32 HELP_ROUNDS = 1u << 12;    // curve rounds per helper and wait, at most
 
+// A divisor of n >= 2^62 (factorization probes), without helpers: 230 rho steps in exact arithmetic, the
+// owner's rounds of curves, rho again. Two 32-bit primes took 1.5 to 3 ms by rho alone (8 K
+// integers of up to 64 bits 2.7 -> 1.2 ms). Out of line, and not in stage D, whose cofactors are
+// below 2^62 but for the last primes below 2^64: the call put k_rung's spills from 500 to 900 bytes.
+static __device__ __noinline__ u64 warp_split_exact(const Mont M, u32 lane, u64 budget, bool use_ecm,
+                                                    const volatile int *cancel, int my_k) {
+  bool stop = false;
+  auto poll = [&]() -> u64 {
+    stop = __shfl_sync(FULL, lane == 0 && cancelled(cancel, my_k) ? 1 : 0, 0) != 0;
+    return stop ? ~0ull : 0;
+  };
+  const bool ecm = use_ecm && budget >= ECM_AFTER + ECM_ROUND_STEPS;
+  u64 steps = ecm ? ECM_AFTER : budget;
+  u64 f = rho_walk<ExactArith>(M.n, M, 1 + lane, 32, steps, lane, poll);
+  if (!ecm) return f;
+  for (u32 round = 0; !f && !stop && round < ECM_OWNER_ROUNDS && steps + ECM_ROUND_STEPS <= budget; ++round) {
+    const u64 d = ecm_curve<ExactArith>(ECM_SIGMA_OWNER + 32 * (u64)round + lane, M, [&]() { return poll() != 0; });
+    const unsigned has = __ballot_sync(FULL, d != 0);
+    if (has) f = __shfl_sync(FULL, d, __ffs(has) - 1);
+    steps += ECM_ROUND_STEPS;
+  }
+  if (!f && !stop && steps < budget)
+    f = rho_walk<ExactArith>(M.n, M, 1 + lane + 32 * 1024, 32, budget - steps, lane, poll);
+  return f;
+}
+
+// BIG: n is often 2^62 or more.
+template <bool BIG>
 __device__ inline u64 warp_rho(u64 n, u32 lane, volatile u64 *found, u32 *status, const volatile int *cancel = nullptr,
                                int my_k = 0, BlockHelp *bh = nullptr, u32 slot = 0, u64 budget = WARP_RHO_STEPS,
                                bool use_ecm = true) {
@@ -351,10 +379,11 @@ __device__ inline u64 warp_rho(u64 n, u32 lane, volatile u64 *found, u32 *status
   // Brent's rho first; a cofactor it has not split goes to ECM rounds (charged against the same
   // budget), and rho resumes with fresh constants for whatever budget remains after them. Every
   // stage-D cofactor is below 2^62 (A = (p + r)/4 with p below 2^64) and takes the lazy
-  // arithmetic; larger n (factorization probes only) walk rho in exact arithmetic, without ECM.
+  // arithmetic; larger n go to warp_split_exact where there are many, else they walk rho.
   u64 f = 0;
   if (n >= LazyArith::NMAX) {
-    f = rho_walk<ExactArith>(n, M, 1 + lane, 32, budget, lane, poll);
+    f = BIG ? warp_split_exact(M, lane, budget, use_ecm, cancel, my_k)
+            : rho_walk<ExactArith>(n, M, 1 + lane, 32, budget, lane, poll);
   } else {
     const bool ecm = use_ecm && budget >= ECM_AFTER + ECM_ROUND_STEPS;
     u64 steps = 0;
@@ -474,6 +503,7 @@ __device__ inline void warp_help_board(const Board &B, u64 total, u32 lane) {
 // of them), appended to F: primes and squares at once, anything else split by warp_rho. `composite`:
 // v0 is known to be neither a prime nor a square. All lanes call. Returns false when a bound was hit
 // (status says which) or on cancellation.
+template <bool BIG = false>
 __device__ inline bool warp_factor_cofactor(u64 v0, WarpFac &F, u32 *status, u32 lane, volatile u64 *rho_slot,
                                             const volatile int *cancel, int my_k, BlockHelp *bh, u32 slot,
                                             u64 rho_budget, bool use_ecm, bool composite) {
@@ -490,7 +520,7 @@ __device__ inline bool warp_factor_cofactor(u64 v0, WarpFac &F, u32 *status, u32
       const u64 s = isqrt64(v);
       if (s * s == v) { wf_add(F, s, 2, lane); continue; }
     }
-    const u64 d = warp_rho(v, lane, rho_slot, status, cancel, my_k, bh, slot, rho_budget, use_ecm);
+    const u64 d = warp_rho<BIG>(v, lane, rho_slot, status, cancel, my_k, bh, slot, rho_budget, use_ecm);
     if (d == 0) return false;                  // budget (status set) or cancelled
     if (sp + 2 > 4) { if (lane == 0) atomicOr(status, ST_STACK_OVERFLOW); return false; }
     stack[sp++] = d;
@@ -632,6 +662,7 @@ static __device__ __noinline__ u64 take_primes(WarpFac &F, bool hit, u64 x, u64 
 // cofactor that would need rho (no prime factor below 2^16, not a square) is not factored:
 // it is left in *hard_left (0 otherwise) and F holds the other prime factors; the caller
 // finishes with warp_factor_cofactor if it needs the rest.
+template <bool BIG = false>
 __device__ inline bool warp_factor(u64 n, WarpFac &F, const u32 *__restrict__ tdp, const u64 *__restrict__ tdi,
                                    u32 *status, u32 lane, volatile u64 *rho_slot,
                                    const volatile int *cancel = nullptr, int my_k = 0,
@@ -714,7 +745,7 @@ __device__ inline bool warp_factor(u64 n, WarpFac &F, const u32 *__restrict__ td
       else if (s * s == cur) wf_add(F, s, 2, lane);     // s is prime: no factor of cur is below 2^16
       else *hard_left = cur;                             // needs rho: left to the caller
     } else {
-      return warp_factor_cofactor(cur, F, status, lane, rho_slot, cancel, my_k, bh, slot, rho_budget, use_ecm, false);
+      return warp_factor_cofactor<BIG>(cur, F, status, lane, rho_slot, cancel, my_k, bh, slot, rho_budget, use_ecm, false);
     }
   }
   __syncwarp();
