@@ -42,21 +42,16 @@ GPU_TABLE = os.path.join(GOLDEN, "filters", "f_M2042040_mmax2000_gpu.txt")
 # never the parity default): reported beside the reference's table
 GB300_TABLE = os.path.join(ROOT, "erdos-strauss_gb300", "tables", "f_M2042040_mmax2000_gb300.txt")
 METRIC = "verified integers/s at 1e19 (batched vs plain, 1 GB300)"
-# One ncu capture per kernel schedule of the 4096-window batch with the gpu table (the
-# profiles/ summaries give the commands): per launch, the warp instructions
-# (smsp__inst_executed.sum) and DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum).
-# k_mark_short's depend on (short_max, long_split), k_rung's on rung_blocks_per_sm. A schedule
-# with no capture here gets no issue figure rather than another schedule's.
-MARK_SHORT_NCU = {            # (short_max, long_split) -> per launch
-    (32, 1): {"inst": 728342167, "dram": 95922688 + 3819776},
-    (64, 1): {"inst": 718216590, "dram": 95236608 + 3364864},
-    (128, 1): {"inst": 735127673, "dram": 95047680 + 3439104},
-}
-RUNG_NCU = {                  # rung_blocks_per_sm -> per launch
-    4: {"inst": 70295758, "dram": 845824 + 768},
-    6: {"inst": 70433215, "dram": 845824},
-    8: {"inst": 70539276, "dram": 846592},
-}
+# One ncu capture of the 4096-window batch with the gpu table (the profiles/ summaries give the
+# commands): per launch, the warp instructions (smsp__inst_executed.sum) and DRAM bytes
+# (dram__bytes_read.sum + dram__bytes_write.sum). The marking stage is k_mark_short and k_sift, added
+# up; with windows split it marks by rows whatever short_max is, and k_rung is one block of four
+# teams an SM from rung_blocks_per_sm = 4 on, so one capture stands for the schedules that launch the
+# same kernels. A schedule with no capture here gets no issue figure rather than another schedule's.
+_MARK = {"inst": 33068169 + 84492389, "dram": 4929024 + 66668032 + 320256}
+_RUNG = {"inst": 75059324, "dram": 781824}
+MARK_SHORT_NCU = {(32, 1): _MARK, (64, 1): _MARK, (128, 1): _MARK}      # (short_max, long_split) -> per launch
+RUNG_NCU = {4: _RUNG, 6: _RUNG, 8: _RUNG}                               # rung_blocks_per_sm -> per launch
 # Cover/filter marks per integer of the 2042040 wheel with the gpu filter table: 9.0951 marks per
 # position (positions of all 2308 lanes, all 3745 filters) over 2042040 / 2308 integers per position.
 MARKS_PER_INTEGER_GPU = 9.0951 / (2042040 / 2308)
@@ -455,34 +450,36 @@ def pipelined_leg(eng, wins, steps, warmup, flush_async, depth=3):
 
 
 def roofline(args, wins, n_int, kern, stage, last_t, schedule, clocks):
-    """The dominant kernel against the bound that binds it. k_mark_short is instruction-issue
-    bound integer work: `achieved` is its warp instructions per launch (ncu, same schedule)
-    over its live CUDA-event time, `peak` 152 SMs x 4 schedulers x one instruction per cycle at
-    the sampled SM clock. Sub-objects: `hbm` (the kill-mask rows, stride residues and window
-    list one launch reads, over the same time, against the measured copy bandwidth), `marks`
-    (the per-mark view of a segment sieve) and `stage_d` (k_rung, latency-bound)."""
+    """The dominant stage against the bound that binds it. Marking (k_mark_short and k_sift) is
+    instruction-issue bound integer work: `achieved` is the two kernels' warp instructions per launch
+    (ncu, a schedule that launches the same) over their live time, `peak` 152 SMs x 4 schedulers x one
+    instruction per cycle at the sampled SM clock; the same arithmetic for k_rung where stage D takes
+    longer. Sub-objects: `hbm` (the dense rows and the window list one launch reads, over the same
+    time, against the measured copy bandwidth), `marks` (the per-mark view of a segment sieve) and
+    `stage_d` (k_rung, latency-bound)."""
     hbm_peak, peak_kind = peaks()
     mhz = clocks.get("sm_mhz") or 2070.0
     peak_issue = 152 * 4 * mhz * 1e6
-    per_kernel = {"k_mark_short": kern["mark_short_ms"], "k_mark": kern["mark_long_ms"], "k_prep": kern["prep_ms"],
+    per_kernel = {"k_mark_short": kern["mark_short_ms"], "k_mark": kern["mark_long_ms"], "k_rows": kern["prep_ms"],
                   "k_mr": stage["mr_ms"], "k_rung": stage["rung_ms"], "k_direct": stage["direct_ms"]}
     dom = max(per_kernel, key=per_kernel.get)
     ms = per_kernel[dom] / args.steps
     default = args.windows == 4096 and args.sieve == 0
     cap = MARK_SHORT_NCU.get((schedule["short_max"], schedule["long_split"])) if default else None
+    rcap = RUNG_NCU.get(schedule["rung_blocks_per_sm"]) if default else None
+    own = {"k_mark_short": cap, "k_rung": rcap}.get(dom)
     if dom == "k_mark_short":
-        # one kill-mask row per lane (as laid out: the interleaved rounds padded), the per-window
-        # stride residues (u16 rows of 264) and the window list
-        alg = last_t["mask_bytes"] + len(wins) * 264 * 2 + len(wins) * 32
+        # the dense strides' rows and the window list
+        alg = last_t["mask_bytes"] + len(wins) * 32
     else:
         alg = int(last_t["primes"]) * (24 + 64)             # the survivor tail: 24 B in, 64 B out per prime
     roof = {"kernel": dom, "bound": "issue", "unit": "warp inst/s", "peak": peak_issue, "ms_per_launch": ms,
-            "achieved": None, "frac": None, "traffic": cap["dram"] if cap and dom == "k_mark_short" else None,
+            "achieved": None, "frac": None, "traffic": own["dram"] if own else None,
             "schedule": schedule}
-    if cap and dom == "k_mark_short":
-        roof["achieved"] = cap["inst"] / (ms / 1000.0)
+    if own:
+        roof["achieved"] = own["inst"] / (ms / 1000.0)
         roof["frac"] = roof["achieved"] / peak_issue
-        roof["inst_per_launch"] = cap["inst"]
+        roof["inst_per_launch"] = own["inst"]
     else:
         roof["note"] = "no ncu capture for this kernel and schedule: no issue figure"
     gbs = alg / (ms / 1000.0) / 1e9
@@ -490,7 +487,7 @@ def roofline(args, wins, n_int, kern, stage, last_t, schedule, clocks):
                    "algorithmic_bytes": alg, "traffic": roof["traffic"]}
     if dom == "k_mark_short" and args.sieve == 0:
         # The per-mark view: a segment sieve clears one bit per mark with a 4-byte shared-memory
-        # read-modify-write (8 bytes); the kill-mask kernel does no per-mark work, so this is the
+        # read-modify-write (8 bytes); marking by rows does no per-mark work, so this is the
         # bandwidth such a sieve would need to match it, against the nominal shared-memory rate
         # (152 SMs x 128 B per cycle at the sampled clock).
         marks = n_int * MARKS_PER_INTEGER_GPU
@@ -499,7 +496,6 @@ def roofline(args, wins, n_int, kern, stage, last_t, schedule, clocks):
         roof["marks"] = {"per_launch": marks, "achieved": marks / (ms / 1000.0), "unit": "marks/s",
                          "rmw_equivalent_gbs": rmw_gbs, "smem_peak_gbs": smem_peak, "peak_kind": "nominal",
                          "frac": rmw_gbs / smem_peak}
-    rcap = RUNG_NCU.get(schedule["rung_blocks_per_sm"]) if default else None
     if stage["rung_ms"] > 0:
         # The survivor tail (stage D): integer-pipe work bound by the latency of its hardest
         # factorizations; the same issue arithmetic over k_rung's live time.
