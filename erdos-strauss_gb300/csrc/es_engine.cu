@@ -880,34 +880,39 @@ __global__ void k_build_rows(const u16 *__restrict__ K0, u32 L, u32 ldk, u32 nf,
   }
 }
 
-// Adds to *sum, a lane a thread, the share of its positions that no stride of the tables kills, were
+// Adds to *sum, 32 lanes a block, the share of a lane's positions that no stride of the tables kills, were
 // the strides independent: what the survivor buffers are sized by. A lane's own product and not the
-// product of the strides' means, since lanes differ: few of them hold most of what is left.
+// product of the strides' means, since lanes differ: few of them hold most of what is left. A warp takes
+// every RATE_WARPS'th stride (a thread for all of a lane's: 1.4 ms of es_open, latency of the reads).
+constexpr u32 RATE_WARPS = 16;
 __global__ void k_lane_rate(const u32 *__restrict__ tdense, const u32 *__restrict__ tlane, const uint4 *__restrict__ mdesc,
                             u32 n1, u32 n1p, u32 nm, u32 slice_rows, u32 lane_words, u32 L, double *__restrict__ sum) {
-  const u32 l = blockIdx.x * blockDim.x + threadIdx.x;
-  double r = 0;
+  __shared__ double part[RATE_WARPS][32];
+  const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5, l = blockIdx.x * 32 + lane;
+  double r = 1;
   if (l < L) {
-    r = 1;
     const u32 *slice = tdense + (size_t)(l / GROUP_LANES) * slice_rows * GROUP_WORDS + l % GROUP_LANES / 32;
-    for (u32 m = 0; m < n1; ++m) {
-      const uint4 d = mdesc[m];
+    for (u32 m = w; m < nm; m += RATE_WARPS) {
+      const uint4 d = mdesc[m < n1 ? m : n1p - n1 + m];
       u32 c = 0;
-      #pragma unroll 8
-      for (u32 x = 0; x < d.x; ++x) c += slice[(size_t)(d.w + x) * GROUP_WORDS] >> (l & 31) & 1u;
-      r *= 1.0 - (double)c / d.x;
-    }
-    for (u32 m = n1; m < nm; ++m) {
-      const uint4 d = mdesc[n1p - n1 + m];
-      u32 c = 0;
-      #pragma unroll 4
-      for (u32 x = 0; x < (d.x + 31) / 32; ++x) c += __popc(tlane[(size_t)l * lane_words + d.w + x]);
+      if (m < n1) {
+        #pragma unroll 8
+        for (u32 x = 0; x < d.x; ++x) c += slice[(size_t)(d.w + x) * GROUP_WORDS] >> lane & 1u;
+      } else {
+        #pragma unroll 4
+        for (u32 x = 0; x < (d.x + 31) / 32; ++x) c += __popc(tlane[(size_t)l * lane_words + d.w + x]);
+      }
       r *= 1.0 - (double)c / d.x;
     }
   }
+  part[w][lane] = l < L ? r : 0;
+  __syncthreads();
+  if (w) return;
+  for (u32 i = 1; i < RATE_WARPS; ++i) r *= part[i][lane];
+  if (l >= L) r = 0;
   #pragma unroll
   for (int o = 16; o; o >>= 1) r += __shfl_xor_sync(FULL, r, o);
-  if (!(threadIdx.x & 31)) atomicAdd(sum, r);
+  if (lane == 0) atomicAdd(sum, r);
 }
 
 // Whether a filter (mod, res) can kill a perfect square: a thread per (filter, x mod mod), hits
@@ -2254,7 +2259,7 @@ static es_status build_tables(es_engine *e) {
     }
     CU(cudaMalloc(&temps.p[6], sizeof(double)));
     CU(cudaMemsetAsync(temps.p[6], 0, sizeof(double), bs));
-    k_lane_rate<<<(L + 127) / 128, 128, 0, bs>>>((const u32 *)e->d_tdense, e->d_tlane, e->d_mdesc, e->n1, e->n1p,
+    k_lane_rate<<<(L + 31) / 32, 32 * RATE_WARPS, 0, bs>>>((const u32 *)e->d_tdense, e->d_tlane, e->d_mdesc, e->n1, e->n1p,
                                                  e->nm_all, e->slice_rows, e->lane_words, L, (double *)temps.p[6]);
     CU(cudaGetLastError());
     CU(cudaMemcpyAsync(&e->surv_rate, temps.p[6], sizeof(double), cudaMemcpyDeviceToHost, bs));
