@@ -883,7 +883,7 @@ __global__ void k_build_rows(const u16 *__restrict__ K0, u32 L, u32 ldk, u32 nf,
 // Adds to *sum, 32 lanes a block, the share of a lane's positions that no stride of the tables kills, were
 // the strides independent: what the survivor buffers are sized by. A lane's own product and not the
 // product of the strides' means, since lanes differ: few of them hold most of what is left. A warp takes
-// every RATE_WARPS'th stride (a thread for all of a lane's: 1.4 ms of es_open, latency of the reads).
+// every RATE_WARPS'th stride: 0.24 ms of es_open, latency of the reads (a thread for all of a lane's 1.4).
 constexpr u32 RATE_WARPS = 16;
 __global__ void k_lane_rate(const u32 *__restrict__ tdense, const u32 *__restrict__ tlane, const uint4 *__restrict__ mdesc,
                             u32 n1, u32 n1p, u32 nm, u32 slice_rows, u32 lane_words, u32 L, double *__restrict__ sum) {
