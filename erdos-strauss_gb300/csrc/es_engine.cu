@@ -943,10 +943,7 @@ __global__ void k_square_mask(const u64 *__restrict__ mods, const u64 *__restric
 // for the 1 K of a 2^34 window at 1e15 and 40 for the 7 K of the 4096-window batch at 1e19; two kernels
 // with a list between them, which this replaced, took 9, 16, 22 and 38; with 32 a warp from the first
 // the last two are 38 and 55.
-#ifndef ES_MR_BLOCKS_PER_SM
-#define ES_MR_BLOCKS_PER_SM 6
-#endif
-constexpr u32 MR_BLOCKS_PER_SM = ES_MR_BLOCKS_PER_SM;
+constexpr u32 MR_BLOCKS_PER_SM = 6;
 // Numbers a warp takes at a time, of n in all.
 __device__ __forceinline__ u32 mr_share(u64 n) {
   const u64 warps = (u64)gridDim.x / MR_BLOCKS_PER_SM * 4, share = (n + warps - 1) / warps;

@@ -84,10 +84,7 @@ constexpr u32 PIECE_ROWS = 32;
 constexpr u32 GROUP_WORDS = 4;              // 32-bit words of a dense row
 constexpr u32 GROUP_LANES = 32 * GROUP_WORDS;
 constexpr u32 ROW_THREADS = 1024;           // threads of k_mark_short and k_sift, one CTA of each per SM
-#ifndef ES_DENSE_MAX
-#define ES_DENSE_MAX 48
-#endif
-constexpr u32 DENSE_MAX = ES_DENSE_MAX;     // dense strides, at most
+constexpr u32 DENSE_MAX = 48;     // dense strides, at most
 constexpr u32 BULK_COPY = 16384;            // bytes per bulk copy into shared memory
 // Shared memory of a CTA (the rest of the 227 KB an SM can give one is static): per warp 64
 // candidates of 8 bytes (k_sift: twice); k_mark_short's group slice, or k_sift's stride descriptors
