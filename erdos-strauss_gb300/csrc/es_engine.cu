@@ -1975,7 +1975,13 @@ static es_status run_windows(es_engine *e, Slot *sl, const es_window *w, size_t 
   const auto t_start = std::chrono::steady_clock::now();
   auto finish = [&](const RecDev *from, size_t m) -> es_status {     // the records, ordered
     if (recs) {
-      const es_status st = order_records(e, sl, from, m, n, recs);
+      es_status st;
+      try {
+        st = order_records(e, sl, from, m, n, recs);
+      } catch (const std::bad_alloc &) {
+        es_free_records(recs);
+        st = fail(e, ES_ERR_NOMEM, "host records");
+      }
       if (st != ES_OK) return st;
     }
     sl->timing.host_collect_ms = ms_since(t_start) - sl->timing.host_setup_ms - sl->timing.host_device_ms;
