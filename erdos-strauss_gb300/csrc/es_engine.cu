@@ -1394,14 +1394,13 @@ static void drop_graph(Slot *sl) {
 // Device buffers for nwin windows, npieces row pieces, nchunks candidate chunks and a survivor
 // capacity of cap, with their pinned host
 // staging. Growing any of them invalidates the captured graph (its copies and kernel
-// parameters name the old buffers and sizes).
+// parameters name the old buffers and sizes). A group that grows counts as empty until its last
+// allocation has succeeded: after a failure the next call makes all of it again.
 static es_status ensure_capacity(es_engine *e, Slot *sl, size_t nwin, size_t npieces, size_t nchunks, size_t cap) {
-  if (!sl->d_hdr) {
-    CU(cudaMalloc(&sl->d_hdr, sizeof(BatchHdr)));
-    CU(cudaMallocHost(&sl->h_hdr, sizeof(BatchHdr)));
-    CU(cudaMallocHost(&sl->h_ctr, CTR_OUT * sizeof(unsigned long long)));
-    CU(cudaMallocHost(&sl->h_status, sizeof(u32)));
-  }
+  if (!sl->d_hdr) CU(cudaMalloc(&sl->d_hdr, sizeof(BatchHdr)));
+  if (!sl->h_hdr) CU(cudaMallocHost(&sl->h_hdr, sizeof(BatchHdr)));
+  if (!sl->h_ctr) CU(cudaMallocHost(&sl->h_ctr, CTR_OUT * sizeof(unsigned long long)));
+  if (!sl->h_status) CU(cudaMallocHost(&sl->h_status, sizeof(u32)));
   if (nwin > sl->win_cap) {
     drop_graph(sl);
     cudaFree(sl->d_win); cudaFree(sl->d_cnt); cudaFree(sl->d_Qm);
@@ -1444,6 +1443,7 @@ static es_status ensure_capacity(es_engine *e, Slot *sl, size_t nwin, size_t npi
     cudaFree(sl->d_surv); cudaFree(sl->d_primes); cudaFree(sl->d_direct); cudaFree(sl->d_recs);
     cudaFreeHost(sl->h_recs);
     sl->d_surv = nullptr; sl->d_primes = sl->d_direct = nullptr; sl->d_recs = nullptr; sl->h_recs = nullptr;
+    sl->cap = 0;
     CU(cudaMalloc(&sl->d_surv, cap * sizeof(Surv)));
     CU(cudaMalloc(&sl->d_primes, cap * sizeof(u32)));
     CU(cudaMalloc(&sl->d_direct, cap * sizeof(u32)));

@@ -1,0 +1,43 @@
+"""The engine's buffers on the host side, against a CUDA runtime without a device: growing, failing
+and being asked for again."""
+import pytest
+
+import es_sieve
+from conftest import golden
+from fake_cuda import FakeCuda
+
+SMALL = es_sieve.load_filters(golden("filters", "f_M120120_mmax2000_runtime.txt"))
+TABLE = tuple(a[:60] for a in SMALL)
+LO = 10 ** 12
+
+
+@pytest.fixture(scope="module")
+def cuda(tmp_path_factory):
+    return FakeCuda(tmp_path_factory.mktemp("fake"))
+
+
+@pytest.fixture
+def eng(cuda, monkeypatch):
+    e = cuda.engine(monkeypatch, wheel=120120, filters=TABLE)
+    yield e
+    cuda.fail()
+    e.close()
+
+
+# the n-th allocation of a call fails, from the first one of an engine's first call (its header) to
+# the last one of a call that grows every buffer: that call is an error, the next ones run again
+@pytest.mark.parametrize("n", range(1, 24))
+def test_a_call_after_a_failed_allocation(cuda, eng, n):
+    for big in (False, True):
+        wins = [(LO, LO + (1 << 20))] * (300 if big else 1)
+        cuda.fail(alloc=n)
+        if big:
+            cuda.counts(surv=1 << 20, chunks=1 << 20)          # the run has to be made again with more room
+        try:
+            eng.run_batch(wins)
+        except es_sieve.EsError as ex:
+            assert ex.status == es_sieve.ES_ERR_CUDA
+        cuda.fail()
+        for w in (wins, wins[:1], wins):
+            eng.run_batch(w)
+            assert not cuda.bad(), [ln for ln in cuda.log() if ln.startswith("BAD")]
