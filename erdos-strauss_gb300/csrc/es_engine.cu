@@ -1375,11 +1375,15 @@ static es_status fail(es_engine *e, es_status s, const std::string &msg) {
   return s;
 }
 
+// The failure is this call's alone: the runtime forgets it, or the next call would take it for one
+// of its own launches'.
 #define CU(call)                                                                           \
   do {                                                                                     \
     cudaError_t err_ = (call);                                                             \
-    if (err_ != cudaSuccess)                                                               \
+    if (err_ != cudaSuccess) {                                                             \
+      cudaGetLastError();                                                                  \
       return fail(e, ES_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(err_));   \
+    }                                                                                      \
   } while (0)
 
 static void drop_graph(Slot *sl) {
@@ -1683,6 +1687,7 @@ static es_status capture_graph(es_engine *e, Slot *sl) {
     if (s == ES_OK && (one || part == 1)) s = enqueue_tail(e, sl, sl->d_cnt, sl->h_cnt, true);
     cudaGraph_t g = nullptr;
     const cudaError_t end = cudaStreamEndCapture(sl->stream, &g);
+    if (end != cudaSuccess) cudaGetLastError();
     if (s != ES_OK) { if (g) cudaGraphDestroy(g); return s; }
     if (end != cudaSuccess) return fail(e, ES_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(end));
     (part == 0 ? sl->graph : sl->graph2) = g;
@@ -2546,6 +2551,7 @@ es_status es_open(const es_config *cfg, es_engine **out) {
         cudaMalloc(&sl.d_ctr, CTR_BYTES) != cudaSuccess ||
         cudaMalloc(&sl.d_status, sizeof(u32)) != cudaSuccess) {
       g_open_error = "stream or counter allocation failed";
+      cudaGetLastError();
       es_close(e);
       return ES_ERR_CUDA;
     }

@@ -52,6 +52,7 @@ double rate_all = 0, rate_dense = 0;
 long fail_alloc = 0, fail_instantiate = 0;
 size_t bytes_now = 0;
 int bad = 0;
+cudaError_t last = cudaSuccess;                     // of the calls so far, until it is asked for
 
 void note(const std::string &s) { text += s + "\n"; }
 // The n-th from now fails (a countdown; 0: none).
@@ -60,7 +61,7 @@ bool fails(long &n) { return n > 0 && --n == 0; }
 cudaError_t take(void **p, size_t n, const char *what) {
   std::lock_guard<std::recursive_mutex> lk(mu);
   *p = nullptr;
-  if (fails(fail_alloc)) return cudaErrorMemoryAllocation;
+  if (fails(fail_alloc)) return last = cudaErrorMemoryAllocation;
   note(std::string(what) + " " + std::to_string(n));
   *p = calloc(n ? n : 1, 1);
   live[*p] = n;
@@ -165,7 +166,12 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const
   return cudaSuccess;
 }
 const char *cudaGetErrorString(cudaError_t) { return "a failure the test asked for"; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+  std::lock_guard<std::recursive_mutex> lk(mu);
+  const cudaError_t e = last;
+  last = cudaSuccess;
+  return e;
+}
 cudaError_t cudaGetSymbolAddress(void **, const void *) { return cudaErrorInvalidValue; }
 cudaError_t cudaGetDriverEntryPointByVersion(const char *, void **, unsigned, unsigned long long, cudaDriverEntryPointQueryResult *) {
   return cudaErrorInvalidValue;
@@ -212,7 +218,7 @@ cudaError_t cudaStreamEndCapture(cudaStream_t s, cudaGraph_t *g) {
 }
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t *x, cudaGraph_t g, unsigned long long) {
   std::lock_guard<std::recursive_mutex> lk(mu);
-  if (fails(fail_instantiate)) return cudaErrorMemoryAllocation;
+  if (fails(fail_instantiate)) return last = cudaErrorMemoryAllocation;
   note("instantiate");
   *x = (cudaGraphExec_t) new Graph(*(Graph *)g);
   return cudaSuccess;
