@@ -1678,6 +1678,10 @@ static es_status enqueue_tail(es_engine *e, Slot *sl, WinCount *cnt, WinCount *o
 // synchronous slot one (the gap between two is 5 us of a small window's 50).
 static es_status capture_graph(es_engine *e, Slot *sl) {
   drop_graph(sl);
+  struct Undo {                                    // a front without its tail is none, on every return path
+    Slot *sl;
+    ~Undo() { if (sl) drop_graph(sl); }
+  } undo{sl};
   const bool one = sl == &e->slots[0];
   u64 launches = 2;                                // the tail's two kernels
   for (int part = 0; part < (one ? 1 : 2); ++part) {
@@ -1693,6 +1697,7 @@ static es_status capture_graph(es_engine *e, Slot *sl) {
     (part == 0 ? sl->graph : sl->graph2) = g;
     CU(cudaGraphInstantiate(part == 0 ? &sl->gexec : &sl->gexec2, g, 0));
   }
+  undo.sl = nullptr;
   sl->graph_launches = launches;
   return ES_OK;
 }

@@ -41,3 +41,16 @@ def test_a_call_after_a_failed_allocation(cuda, eng, n):
         for w in (wins, wins[:1], wins):
             eng.run_batch(w)
             assert not cuda.bad(), [ln for ln in cuda.log() if ln.startswith("BAD")]
+
+
+def test_a_request_after_a_failed_capture(cuda, eng):
+    """A serving slot's second graph (stage D and the results) fails to be made: the request is an
+    error, and those that follow run both graphs again."""
+    cuda.fail(instantiate=2)
+    with pytest.raises(es_sieve.EsError):
+        eng.poll(eng.submit([(LO, LO + 10 ** 6)]), 1, timeout_ms=60000)
+    cuda.fail()
+    cuda.log()
+    for _ in range(6):
+        eng.poll(eng.submit([(LO, LO + 10 ** 6)]), 1, timeout_ms=60000)
+        assert sum(ln.startswith("graph on") for ln in cuda.log()) == 2
