@@ -1553,6 +1553,7 @@ static void build_lane_index(es_engine *e) {
 // window's wheel positions; the totals go to `run`.
 struct RunShape {
   u64 items = 0, rows = 0, pieces = 0;
+  u64 positions = 0, row_positions = 0;    // of all windows, of those marked by rows
 };
 static RunShape describe(const es_engine *e, const es_window *w, size_t n, std::vector<WinDev> &out,
                          std::vector<RowWin> &roww, std::vector<u64> &npos) {
@@ -1576,6 +1577,7 @@ static RunShape describe(const es_engine *e, const es_window *w, size_t n, std::
     // positions before lo and before hi, both counted from K = q
     const u64 before = classes_below(e, r), upto = (qh - q) * L + classes_below(e, rh);
     npos[i] = upto - before;
+    run.positions += npos[i];
     if (!npos[i]) continue;
     u64 maxpos, rem_;                                    // most positions any lane can hold
     divmod_M(e, d.hi - d.lo - 1, maxpos, rem_);
@@ -1592,6 +1594,7 @@ static RunShape describe(const es_engine *e, const es_window *w, size_t n, std::
       x.piece0 = (u32)run.pieces;
       roww.push_back(x);
       run.rows += x.nrows;
+      run.row_positions += npos[i];
       run.pieces += (x.nrows + PIECE_ROWS - 1) / PIECE_ROWS;
     } else {
       d.seg = SEG_BIG; d.nseg = (u32)((maxpos + SEG_BIG - 1) / SEG_BIG); d.groups = (u32)L;
@@ -1834,11 +1837,9 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
   std::vector<RowWin> &roww = sl->hs.roww;
   std::vector<u64> &npos = sl->hs.npos;
   const RunShape shape = describe(e, w, n, wd, roww, npos);
-  u64 positions_bound = 0;
-  for (size_t i = 0; i < n; ++i) positions_bound += npos[i];
-  size_t cap = std::max(surv_room(e, w, n, positions_bound), sl->cap);
+  size_t cap = std::max(surv_room(e, w, n, shape.positions), sl->cap);
   // candidate chunks: half as many again as the estimate, and a part-filled one per warp and run
-  size_t chunks = (size_t)(1.5 * e->cand_rate * (double)positions_bound / 32) + 4 * (size_t)e->sm_count * (ROW_THREADS / 32);
+  size_t chunks = (size_t)(1.5 * e->cand_rate * (double)shape.row_positions / 32) + 4 * (size_t)e->sm_count * (ROW_THREADS / 32);
   const bool persistent = schedule == ES_SCHED_PERSISTENT;
   std::vector<RecDev> &hr = sl->hs.hr;   // the plain schedule's
   size_t nrec = 0;

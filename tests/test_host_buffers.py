@@ -54,3 +54,13 @@ def test_a_request_after_a_failed_capture(cuda, eng):
     for _ in range(6):
         eng.poll(eng.submit([(LO, LO + 10 ** 6)]), 1, timeout_ms=60000)
         assert sum(ln.startswith("graph on") for ln in cuda.log()) == 2
+
+
+def test_windows_marked_by_segments_need_no_candidate_chunks(cuda, eng):
+    """With long_split = 0 a long window is marked by segments, whose survivors need no room before they
+    are known: its buffers are those of a short one."""
+    eng.set_schedule(long_split=0)
+    eng.run_window(LO, LO + (1 << 20))
+    short = cuda.bytes()
+    eng.run_window(LO, LO + (1 << 38))
+    assert cuda.bytes() == short
