@@ -119,10 +119,10 @@ __device__ __forceinline__ u64 mmul(u64 a, u64 b, const Mont &M) {
 // 64-bit division takes three times as long.
 __device__ __forceinline__ u64 pow64_mod(u64 n) {
   if (n >> 32 == 0) return (0 - n) % n;
-  const float f = (float)n;
-  long long r = (long long)(0 - (u64)(18446744073709551616.0f / f) * n);
-  r -= (long long)rintf((float)r / f) * (long long)n;                // now within n / 2 + 1 of zero
-  return r < 0 ? (u64)(r + (long long)n) : (u64)r;
+  const float f = (float)n;                            // r is a signed remainder, kept unsigned: n passes 2^63
+  u64 r = 0 - (u64)(18446744073709551616.0f / f) * n;
+  r -= (u64)(long long)rintf((float)(long long)r / f) * n;           // now within n / 2 + 1 of zero
+  return r + ((long long)r < 0 ? n : 0);
 }
 
 __device__ __forceinline__ Mont mont_one(u64 n) {    // without r2
