@@ -106,7 +106,7 @@ __device__ __forceinline__ u64 mmul(u64 a, u64 b, const Mont &M) {
       "mul.lo.u32 m, t1, %9;\n\t"
       "mad.lo.cc.u32 t1, m, %7, t1;\n\tmadc.hi.cc.u32 t2, m, %7, t2;\n\taddc.cc.u32 t3, t3, 0;\n\taddc.u32 t0, t0, 0;\n\t"
       "mad.lo.cc.u32 %0, m, %8, t2;\n\tmadc.hi.cc.u32 %1, m, %8, t3;\n\taddc.u32 %2, t0, 0;\n\t}"
-      : "=r"(r0), "=r"(r1), "=r"(c)
+      : "=&r"(r0), "=&r"(r1), "=&r"(c)
       : "r"(a0), "r"(a1), "r"(b0), "r"(b1), "r"(n0), "r"(n1), "r"(ni));
   const u64 s = (u64)r1 << 32 | r0;
   return (c || s >= M.n) ? s - M.n : s;
@@ -183,7 +183,7 @@ struct LazyArith {
         "mul.lo.u32 m, t1, %8;\n\t"
         "mad.lo.cc.u32 t1, m, %6, t1;\n\tmadc.hi.cc.u32 t2, m, %6, t2;\n\taddc.u32 t3, t3, 0;\n\t"
         "mad.lo.cc.u32 %0, m, %7, t2;\n\tmadc.hi.u32 %1, m, %7, t3;\n\t}"
-        : "=r"(r0), "=r"(r1)
+        : "=&r"(r0), "=&r"(r1)
         : "r"(a0), "r"(a1), "r"(b0), "r"(b1), "r"(n0), "r"(n1), "r"(ni));
     return (u64)r1 << 32 | r0;
 #else
