@@ -1261,7 +1261,7 @@ struct Slot {
   // (marking, Miller-Rabin) and the tail (stage D, stage E, results written out). ev[11] is
   // recorded between them on the slot's stream: the next slot's front waits for it (marking runs
   // one batch at a time, in launch order) while this slot's tail overlaps the next batch's
-  // marking. The synchronous slot has one graph of both.
+  // marking. The synchronous slot has one graph of both, ev[11] recorded inside.
   cudaGraph_t graph = nullptr, graph2 = nullptr;
   cudaGraphExec_t gexec = nullptr, gexec2 = nullptr;
   WinDev *d_win = nullptr; size_t win_cap = 0;
@@ -1676,9 +1676,26 @@ static es_status enqueue_tail(es_engine *e, Slot *sl, WinCount *cnt, WinCount *o
   return ES_OK;
 }
 
+// The end of the front (ev[11], which a serving slot's front waits for) inside the synchronous slot's
+// single graph: a leaf of its own beside stage D. As a node between Miller-Rabin and stage D it took
+// 2.2 us of a small window's 39; recorded after the graph, as it was, it made a served request wait for
+// stage D and the results (a request beside a call of 11.7 ms of direct search: 23.6 ms for both, 14.0 so).
+static es_status capture_front_end(es_engine *e, Slot *sl) {
+  cudaStreamCaptureStatus status;
+  unsigned long long id;
+  cudaGraph_t g;
+  const cudaGraphNode_t *deps;
+  const cudaGraphEdgeData *edges;
+  size_t n;
+  CU(cudaStreamGetCaptureInfo(sl->stream, &status, &id, &g, &deps, &edges, &n));
+  cudaGraphNode_t node;
+  CU(cudaGraphAddEventRecordNode(&node, g, deps, n, sl->ev[11]));
+  return ES_OK;
+}
+
 // The persistent schedule as CUDA graphs, captured once and replayed per batch: for a serving slot
 // two, the funnel up to Miller-Rabin, and stage D and E with the results written out; for the
-// synchronous slot one (the gap between two is 5 us of a small window's 50).
+// synchronous slot one, with the front's end recorded inside (the gap between two is 5 us of a small window's 50).
 static es_status capture_graph(es_engine *e, Slot *sl) {
   drop_graph(sl);
   struct Undo {                                    // a front without its tail is none, on every return path
@@ -1691,6 +1708,7 @@ static es_status capture_graph(es_engine *e, Slot *sl) {
     CU(cudaStreamBeginCapture(sl->stream, cudaStreamCaptureModeThreadLocal));
     es_status s = ES_OK;
     if (part == 0) s = enqueue_front(e, sl, true, sl->d_cnt, true, !e->sched.long_split, 0, true, launches);
+    if (s == ES_OK && one) s = capture_front_end(e, sl);
     if (s == ES_OK && (one || part == 1)) s = enqueue_tail(e, sl, sl->d_cnt, sl->h_cnt, true);
     cudaGraph_t g = nullptr;
     const cudaError_t end = cudaStreamEndCapture(sl->stream, &g);
@@ -1714,7 +1732,7 @@ static es_status launch_persistent(es_engine *e, Slot *sl) {
     std::lock_guard<std::mutex> lk(e->front_mu);
     if (e->last_front && e->last_front != sl) CU(cudaStreamWaitEvent(sl->stream, e->last_front->ev[11], 0));
     CU(cudaGraphLaunch(sl->gexec, sl->stream));
-    CU(cudaEventRecord(sl->ev[11], sl->stream));
+    if (sl->gexec2) CU(cudaEventRecord(sl->ev[11], sl->stream));
     e->last_front = sl;
   }
   if (sl->gexec2) CU(cudaGraphLaunch(sl->gexec2, sl->stream));

@@ -216,6 +216,24 @@ cudaError_t cudaStreamEndCapture(cudaStream_t s, cudaGraph_t *g) {
   capturing.erase(streams[s]);
   return cudaSuccess;
 }
+cudaError_t cudaStreamGetCaptureInfo(cudaStream_t s, cudaStreamCaptureStatus *status, unsigned long long *id, cudaGraph_t *g,
+                                     const cudaGraphNode_t **deps, const cudaGraphEdgeData **edges, size_t *n) {
+  std::lock_guard<std::recursive_mutex> lk(mu);
+  static const cudaGraphNode_t last_node = nullptr;  // what the stream's next node would follow
+  const auto c = capturing.find(streams[s]);
+  *status = c == capturing.end() ? cudaStreamCaptureStatusNone : cudaStreamCaptureStatusActive;
+  *id = 0;
+  *g = c == capturing.end() ? nullptr : (cudaGraph_t)c->second;
+  *deps = &last_node;
+  *edges = nullptr;
+  *n = 1;
+  return cudaSuccess;
+}
+cudaError_t cudaGraphAddEventRecordNode(cudaGraphNode_t *, cudaGraph_t, const cudaGraphNode_t *, size_t n, cudaEvent_t e) {
+  std::lock_guard<std::recursive_mutex> lk(mu);
+  note("record " + std::to_string(events[e]) + (n == 1 ? " node" : ""));
+  return cudaSuccess;
+}
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t *x, cudaGraph_t g, unsigned long long) {
   std::lock_guard<std::recursive_mutex> lk(mu);
   if (fails(fail_instantiate)) return last = cudaErrorMemoryAllocation;

@@ -64,3 +64,20 @@ def test_windows_marked_by_segments_need_no_candidate_chunks(cuda, eng):
     short = cuda.bytes()
     eng.run_window(LO, LO + (1 << 38))
     assert cuda.bytes() == short
+
+
+def test_a_synchronous_call_lets_the_next_front_start_after_its_own(cuda, eng):
+    """The end of marking and Miller-Rabin is recorded between them and stage D, in the synchronous
+    slot's single graph too, and not once more after its results: a serving slot that waits for it
+    does not wait for stage D."""
+    eng.run_window(LO, LO + (1 << 20))
+    ops = [ln.split()[1] if ln.startswith("launch") else ln for ln in cuda.log()
+           if ln.startswith(("launch", "record", "graph"))]
+    assert ops[ops.index("k_mr"):] == ["k_mr", "record 11 node", "k_rung", "k_direct", "record 4 node", "graph on 0"]
+    eng.poll(eng.submit([(LO, LO + 10 ** 6)]), 1, timeout_ms=60000)
+    log = cuda.log()
+    served = [ln for ln in log if " waits " in ln]
+    assert len(served) == 1 and served[0].endswith("waits 11") and not served[0].startswith("stream 0")
+    slot = int(served[0].split()[1])
+    ops = [ln.split()[1] if ln.startswith("launch") else ln for ln in log if ln.startswith(("record", "graph"))]
+    assert ops[-3:] == ["graph on %d" % slot, "record %d" % (12 * slot + 11), "graph on %d" % slot]
