@@ -1862,11 +1862,12 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
   std::vector<RecDev> &hr = sl->hs.hr;   // the plain schedule's
   size_t nrec = 0;
   bool done = false;
+  u64 launches = 0;                      // of all attempts
   for (int attempt = 0; attempt < 4 && !done; ++attempt) {
     es_status s = ensure_capacity(e, sl, n, shape.pieces, chunks, cap);
     if (s) return s;
     double total_ms = 0, mark_ms = 0, mr_ms = 0, rung_ms = 0, direct_ms = 0, prep_ms = 0, short_ms = 0, long_ms = 0;
-    u64 launches = 0, surv_max = 0, chunk_max = 0, prime_total = 0;
+    u64 surv_max = 0, chunk_max = 0, prime_total = 0;
     u32 status = 0;
     hr.clear();
     auto collect = [&]() -> es_status {   // after a pass: timings, counts, records
@@ -1902,7 +1903,7 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
       if (s) return s;
       CU(cudaStreamSynchronize(sl->stream));
       device_ms = ms_since(t_launch);
-      launches = sl->graph_launches;
+      launches += sl->graph_launches;
       s = collect();
       if (s) return s;
     } else {

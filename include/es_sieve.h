@@ -125,7 +125,7 @@ typedef struct {
   double prep_ms, mark_short_ms, mark_long_ms;   /* the three parts of mark_ms:
                                                      rows and residues, marking by rows (k_mark_short
                                                      and k_sift), segment marking */
-  uint64_t marks_kernel_launches, kernel_launches;
+  uint64_t marks_kernel_launches, kernel_launches;   /* kernel_launches: of repeated attempts too */
   uint64_t mark_items, survivors, primes;
   uint64_t short_pairs;     /* (lane, window) pairs of the windows marked by rows */
   uint64_t mask_bytes;      /* dense stride table bytes one k_mark_short launch reads */

@@ -81,3 +81,26 @@ def test_a_synchronous_call_lets_the_next_front_start_after_its_own(cuda, eng):
     slot = int(served[0].split()[1])
     ops = [ln.split()[1] if ln.startswith("launch") else ln for ln in log if ln.startswith(("record", "graph"))]
     assert ops[-3:] == ["graph on %d" % slot, "record %d" % (12 * slot + 11), "graph on %d" % slot]
+
+
+# survivors and chunks that do not fit, in the first run and in the second too
+@pytest.mark.parametrize("schedule", [es_sieve.ES_SCHED_PERSISTENT, es_sieve.ES_SCHED_PLAIN])
+@pytest.mark.parametrize("more", [[(1 << 20, 0)], [(0, 1 << 20)], [(1 << 20, 1 << 20)], [(1 << 20, 0), (0, 1 << 21)]])
+def test_a_run_is_made_again_until_it_fits(cuda, eng, schedule, more):
+    eng.run_batch([(LO, LO + (1 << 20))], schedule=schedule)
+    once = eng.timing()["kernel_launches"]
+    for surv, chunks in more:
+        cuda.counts(surv, chunks)
+    eng.run_batch([(LO, LO + (1 << 20))], schedule=schedule)
+    assert eng.timing()["kernel_launches"] == once * (1 + len(more))
+    eng.run_batch([(LO, LO + (1 << 20))], schedule=schedule)
+    assert eng.timing()["kernel_launches"] == once
+    assert not cuda.bad()
+
+
+def test_a_run_that_never_fits_is_an_error(cuda, eng):
+    for k in range(20, 28):
+        cuda.counts(1 << k, 0)
+    with pytest.raises(es_sieve.EsError) as ex:
+        eng.run_window(LO, LO + (1 << 20))
+    assert ex.value.status == es_sieve.ES_ERR_NOMEM
