@@ -880,16 +880,17 @@ __global__ void k_build_rows(const u16 *__restrict__ K0, u32 L, u32 ldk, u32 nf,
   }
 }
 
-// Adds to *sum, 32 lanes a block, the share of a lane's positions that no stride of the tables kills, were
-// the strides independent: what the survivor buffers are sized by. A lane's own product and not the
-// product of the strides' means, since lanes differ: few of them hold most of what is left. A warp takes
-// every RATE_WARPS'th stride: 0.24 ms of es_open, latency of the reads (a thread for all of a lane's 1.4).
+// Adds to sum[0], 32 lanes a block, the share of a lane's positions that no stride of the tables kills, were
+// the strides independent, and to sum[1] that of the dense strides alone: what the buffers of survivors and
+// of candidates are sized by. A lane's own product and not the product of the strides' means, since lanes
+// differ: few of them hold most of what is left. A warp takes every RATE_WARPS'th stride: 0.24 ms of es_open,
+// latency of the reads (a thread for all of a lane's 1.4).
 constexpr u32 RATE_WARPS = 16;
 __global__ void k_lane_rate(const u32 *__restrict__ tdense, const u32 *__restrict__ tlane, const uint4 *__restrict__ mdesc,
                             u32 n1, u32 n1p, u32 nm, u32 slice_rows, u32 lane_words, u32 L, double *__restrict__ sum) {
-  __shared__ double part[RATE_WARPS][32];
+  __shared__ double part[2][RATE_WARPS][32];
   const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5, l = blockIdx.x * 32 + lane;
-  double r = 1;
+  double r = 1, dense = 1;
   if (l < L) {
     const u32 *slice = tdense + (size_t)(l / GROUP_LANES) * slice_rows * GROUP_WORDS + l % GROUP_LANES / 32;
     for (u32 m = w; m < nm; m += RATE_WARPS) {
@@ -898,6 +899,7 @@ __global__ void k_lane_rate(const u32 *__restrict__ tdense, const u32 *__restric
       if (m < n1) {
         #pragma unroll 8
         for (u32 x = 0; x < d.x; ++x) c += slice[(size_t)(d.w + x) * GROUP_WORDS] >> lane & 1u;
+        dense *= 1.0 - (double)c / d.x;
       } else {
         #pragma unroll 4
         for (u32 x = 0; x < (d.x + 31) / 32; ++x) c += __popc(tlane[(size_t)l * lane_words + d.w + x]);
@@ -905,14 +907,15 @@ __global__ void k_lane_rate(const u32 *__restrict__ tdense, const u32 *__restric
       r *= 1.0 - (double)c / d.x;
     }
   }
-  part[w][lane] = l < L ? r : 0;
+  part[0][w][lane] = l < L ? r : 0;
+  part[1][w][lane] = l < L ? dense : 0;
   __syncthreads();
-  if (w) return;
-  for (u32 i = 1; i < RATE_WARPS; ++i) r *= part[i][lane];
-  if (l >= L) r = 0;
+  if (w >= 2) return;                                  // a warp for each sum
+  r = part[w][0][lane];
+  for (u32 i = 1; i < RATE_WARPS; ++i) r *= part[w][i][lane];
   #pragma unroll
   for (int o = 16; o; o >>= 1) r += __shfl_xor_sync(FULL, r, o);
-  if (lane == 0) atomicAdd(sum, r);
+  if (lane == 0) atomicAdd(sum + w, r);
 }
 
 // Whether a filter (mod, res) can kill a perfect square: a thread per (filter, x mod mod), hits
@@ -2244,11 +2247,6 @@ static es_status build_tables(es_engine *e) {
     e->n1p = (e->n1 + 7) & ~7u;
     e->slice_rows = (dense_rows + 7) & ~7u;            // a slice is whole 128-byte lines
     e->ngroups = (L + GROUP_LANES - 1) / GROUP_LANES;
-    e->cand_rate = 1.0;
-    for (u32 m = 0; m < e->n1; ++m) e->cand_rate *= std::max(0.0, 1.0 - kills[ms[m]] / L);
-    // a pass of 2^23 full rows holds 60 MB of rows and pieces and, with the tables for wheel 2042040,
-    // up to 450 MB of candidates; tables that leave more candidates take shorter passes
-    e->pass_rows = (u64)std::min(8388608.0, std::max(4096.0, 32.0 * 2097152.0 / (1.5 * e->cand_rate * L + 1e-9)));
     std::vector<uint4> md(e->n1p + e->nm_all - e->n1);
     auto desc = [](u32 st, u32 at) { return make_uint4(st, 0xFFFFFFFFu / st, (u32)((1ull << 32) % st), at); };
     u32 row = PIECE_ROWS, word = 0;
@@ -2290,12 +2288,13 @@ static es_status build_tables(es_engine *e) {
                                                                  (u32 *)e->d_tdense, e->d_tlane);
       CU(cudaGetLastError());
     }
-    CU(cudaMalloc(&temps.p[6], sizeof(double)));
-    CU(cudaMemsetAsync(temps.p[6], 0, sizeof(double), bs));
+    double rate[2] = {};
+    CU(cudaMalloc(&temps.p[6], sizeof rate));
+    CU(cudaMemsetAsync(temps.p[6], 0, sizeof rate, bs));
     k_lane_rate<<<(L + 31) / 32, 32 * RATE_WARPS, 0, bs>>>((const u32 *)e->d_tdense, e->d_tlane, e->d_mdesc, e->n1, e->n1p,
                                                  e->nm_all, e->slice_rows, e->lane_words, L, (double *)temps.p[6]);
     CU(cudaGetLastError());
-    CU(cudaMemcpyAsync(&e->surv_rate, temps.p[6], sizeof(double), cudaMemcpyDeviceToHost, bs));
+    CU(cudaMemcpyAsync(rate, temps.p[6], sizeof rate, cudaMemcpyDeviceToHost, bs));
     // Stage B' primes kill squares by their own rule, and moduli past 2^16 are not searched.
     unsigned long long hit = 1;
     if (nf && nf == e->ncov && *std::max_element(om.begin(), om.end()) <= 65536) {
@@ -2307,7 +2306,11 @@ static es_status build_tables(es_engine *e) {
       CU(cudaMemcpyAsync(&hit, temps.p[5], sizeof hit, cudaMemcpyDeviceToHost, bs));
     }
     CU(cudaStreamSynchronize(bs));
-    e->surv_rate /= L;
+    e->surv_rate = rate[0] / L;
+    e->cand_rate = rate[1] / L;
+    // a pass of 2^23 full rows holds 60 MB of rows and pieces and, with the tables for wheel 2042040,
+    // up to 450 MB of candidates; tables that leave more candidates take shorter passes
+    e->pass_rows = (u64)std::min(8388608.0, std::max(4096.0, 32.0 * 2097152.0 / (1.5 * e->cand_rate * L + 1e-9)));
     e->squares = !(hit & 1);
     for (u32 q = 3; q < 64; ++q)
       if (hit >> q & 1) e->sq.push_back(q);

@@ -287,6 +287,7 @@ cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 grid, dim3 block, void **arg
     const double L = (double)*(const u32 *)args[8];
     double *sum = *(double **)args[9];
     sum[0] = rate_all * L;
+    sum[1] = rate_dense * L;
   }
   const auto c = capturing.find(l.stream);
   if (c != capturing.end()) c->second->launches.push_back(l);

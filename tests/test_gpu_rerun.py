@@ -36,3 +36,15 @@ def test_a_run_is_made_again_with_more_room(table, length, schedule):
         first = _same(e, want, win, schedule)
         again = _same(e, want, win, schedule)
         assert first == 2 * again
+
+
+def test_lanes_that_differ_are_seen_by_the_room_for_candidates():
+    """Six strides that kill nearly all positions of one half of the lanes and none of the other: half of
+    the positions are candidates, where the means of the strides would say a 50th."""
+    half = [c for c in range(1, 13) if c % 2]
+    table = [(13 * q, r) for q in (17, 19, 23, 29, 31, 37) for r in range(13 * q) if r % 13 in half and r % q != 1] + REST
+    mods, ress = [m for m, _ in table], [r for _, r in table]
+    win = (10 ** 9, 10 ** 9 + 2_400_000_000)
+    want = oracle.scan(*win, M, mods, ress, len(mods))
+    with es_sieve.Engine(wheel=M, filters=(mods, ress)) as e:
+        assert _same(e, want, win, es_sieve.ES_SCHED_PERSISTENT) == _same(e, want, win, es_sieve.ES_SCHED_PERSISTENT)
