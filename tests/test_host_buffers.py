@@ -104,3 +104,25 @@ def test_a_run_that_never_fits_is_an_error(cuda, eng):
     with pytest.raises(es_sieve.EsError) as ex:
         eng.run_window(LO, LO + (1 << 20))
     assert ex.value.status == es_sieve.ES_ERR_NOMEM
+
+
+def _captures(cuda):
+    return sum(ln.startswith("capture") for ln in cuda.log())
+
+
+def test_calls_that_grow_make_buffers_and_graphs_anew_at_doublings_only(cuda, monkeypatch):
+    """Windows and batches each 5% larger than the last: every buffer at most doubles, so the graph is
+    captured no more often than the sizes double, whichever of them does."""
+    e = cuda.engine(monkeypatch, rates=(2e-4, 0.017), wheel=120120, filters=TABLE)
+    length, windows, calls = 1 << 28, 10, 0
+    while length < 1 << 36:
+        e.run_window(LO, LO + length)
+        length, calls = int(length * 1.05), calls + 1
+    pieces, chunks, surv = 8, 5, 3                     # 70 to 18 K pieces, 420 to 107 K chunks, 1 K to 215 K survivors
+    assert calls > 110 and _captures(cuda) <= 1 + pieces + chunks + surv
+    while windows < 4096:
+        e.run_batch([(LO, LO + 1000)] * windows)
+        windows, calls = windows + windows // 20 + 1, calls + 1
+    assert calls > 200 and _captures(cuda) <= 7        # 64 to 4096 windows
+    assert not cuda.bad()
+    e.close()
