@@ -1839,13 +1839,23 @@ static es_status order_records(es_engine *e, Slot *sl, const RecDev *src, size_t
 // integers at 1e16 takes 8 M records of room where 1/64 of its positions took 67 M, 4.3 GB of it
 // pinned: the first call of an engine 161 -> 25 ms, the 4096-window batch's 6.9 -> 1.7 ms.
 constexpr double SURV_ROOM = 8;
-constexpr size_t CHUNKS_MIN = 8192;
-static size_t surv_room(const es_engine *e, const es_window *w, size_t n, u64 positions) {
+constexpr size_t SURV_MIN = 1 << 16;
+static size_t surv_need(const es_engine *e, const es_window *w, size_t n, u64 positions) {
   double want = SURV_ROOM * e->surv_rate * (double)positions;
   for (size_t i = 0; i < n && !e->squares; ++i)
     if (w[i].hi > w[i].lo) want += std::sqrt((double)w[i].hi) - std::sqrt((double)w[i].lo) + 1;
-  want = std::min(want, (double)positions) + 1024;
-  return grown((size_t)std::min(want, (double)(1u << 26)), 1 << 16);
+  return (size_t)std::min(std::min(want, (double)positions) + 1024, (double)(1u << 26));
+}
+// Candidate chunks: half as many again as the tables' estimate. CHUNKS_MIN holds those of 5 G integers with
+// the 120120 wheel's table, 80 G with the gpu table.
+constexpr size_t CHUNKS_MIN = 8192;
+static size_t chunk_need(const es_engine *e, u64 row_positions) {
+  return (size_t)(1.5 * e->cand_rate * (double)row_positions / 32);
+}
+// Rows of [lo, hi), at most; 0 for a window that goes to the segment marking.
+static u64 window_rows(const es_schedule &sched, u64 M, u64 lo, u64 hi) {
+  const u64 len = hi > lo ? hi - lo : 0;
+  return sched.long_split || len <= sched.short_max * M ? len / M + 2 : 0;
 }
 
 // Runs windows through the funnel and collects counters; the records are left unordered at *src
@@ -1866,11 +1876,9 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
   std::vector<RowWin> &roww = sl->hs.roww;
   std::vector<u64> &npos = sl->hs.npos;
   const RunShape shape = describe(e, w, n, wd, roww, npos);
-  size_t cap = std::max(surv_room(e, w, n, shape.positions), sl->cap);
-  // candidate chunks: half as many again as the estimate (CHUNKS_MIN: 5 G integers with the 120120 wheel's
-  // table, 80 G with the gpu table), and a part-filled one per warp and run
-  size_t chunks = grown((size_t)(1.5 * e->cand_rate * (double)shape.row_positions / 32), CHUNKS_MIN) +
-                  4 * (size_t)e->sm_count * (ROW_THREADS / 32);
+  size_t cap = std::max(grown(surv_need(e, w, n, shape.positions), SURV_MIN), sl->cap);
+  size_t chunks = grown(chunk_need(e, shape.row_positions), CHUNKS_MIN) +
+                  4 * (size_t)e->sm_count * (ROW_THREADS / 32);       // a part-filled one per warp and run
   const bool persistent = schedule == ES_SCHED_PERSISTENT;
   std::vector<RecDev> &hr = sl->hs.hr;   // the plain schedule's
   size_t nrec = 0;
@@ -1998,20 +2006,15 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
 // passes per_window zeroed.
 static es_status run_windows(es_engine *e, Slot *sl, const es_window *w, size_t n, int schedule,
                              es_counters *per_window, es_records *recs) {
-  const u64 M = e->M, S = e->sched.short_max;
+  const u64 M = e->M;
   const u64 floor_ = std::max(e->wheel_pmin, e->cover_pmax);
   u64 rows = 0;
-  // rows of [lo, hi), at most; 0 for a window that goes to the segment marking
-  auto rows_of = [&](u64 lo, u64 hi) -> u64 {
-    const u64 len = hi > lo ? hi - lo : 0;
-    return e->sched.long_split || len <= S * M ? len / M + 2 : 0;
-  };
   for (size_t i = 0; i < n; ++i) {                 // refuse what a run would refuse, first
     if (w[i].hi > DIRECT_PMAX)
       return fail(e, ES_ERR_RANGE, "HI must not exceed the stage-E ceiling " + std::to_string(DIRECT_PMAX));
     if (w[i].lo <= floor_)
       return fail(e, ES_ERR_RANGE, "LO must exceed max pmin of the filter table (" + std::to_string(floor_) + ")");
-    rows += rows_of(w[i].lo, w[i].hi);
+    rows += window_rows(e->sched, M, w[i].lo, w[i].hi);
   }
   const RecDev *src = nullptr;
   size_t nsrc = 0;
@@ -2046,7 +2049,7 @@ static es_status run_windows(es_engine *e, Slot *sl, const es_window *w, size_t 
     dw.clear();
     dmap.clear();
     for (u64 left = e->pass_rows; i < n;) {
-      const u64 lo = w[i].lo + t * M, hi = std::max(w[i].lo, w[i].hi), need = rows_of(lo, hi);
+      const u64 lo = w[i].lo + t * M, hi = std::max(w[i].lo, w[i].hi), need = window_rows(e->sched, M, lo, hi);
       if (need <= left) {
         dw.push_back({lo, hi});
         dmap.push_back({(u32)i, t});
@@ -2358,14 +2361,25 @@ static es_status build_tables(es_engine *e) {
 constexpr size_t SERVE_QUEUE_WINDOWS = 1 << 20;   // windows waiting, across requests
 constexpr size_t SERVE_BATCH_WINDOWS = 8192;      // windows per batch a worker takes
 
-// Device bytes a request's windows need in a slot: descriptors, per-window residues and
-// counters, and survivor-side buffers for 1/64 of their positions.
-static u64 request_bytes(const es_engine *e, const es_window *w, size_t n) {
-  u64 pos = 0;
-  for (size_t i = 0; i < n; ++i) pos += positions_in(e, w[i].lo, w[i].hi);
-  const u64 surv = std::min<u64>(std::max<u64>(pos / 64, 1024), 1ull << 26);
-  return n * (sizeof(WinDev) + sizeof(RowWin) + sizeof(WinCount) + 2ull * e->Dq) +
-         surv * (sizeof(Surv) + 3 * sizeof(u32) + sizeof(RecDev));
+// Device bytes a request's windows need in a slot: twice what run_device_windows asks for (its capacities
+// go in doublings), of at most a pass; the floors that every slot has are not a request's.
+static u64 request_bytes(const es_engine *e, const es_schedule &sched, const es_window *w, size_t n) {
+  const u64 L = e->classes.size();
+  u64 pos = 0, row_pos = 0, rows = 0;
+  for (size_t i = 0; i < n; ++i) {
+    const u64 p = positions_in(e, w[i].lo, w[i].hi), r = window_rows(sched, e->M, w[i].lo, w[i].hi);
+    pos += p;
+    rows += r;
+    if (r) row_pos += p;
+  }
+  pos -= row_pos;                                      // those marked by segments
+  rows = std::min(rows, e->pass_rows);
+  row_pos = std::min(row_pos, rows * L);
+  pos += row_pos;
+  return 2 * (n * (sizeof(WinDev) + sizeof(WinCount) + 2ull * e->Dq) +
+              (rows / PIECE_ROWS + n) * (sizeof(Piece) + 2ull * e->n1p + PIECE_ROWS * sizeof(u32)) +
+              chunk_need(e, row_pos) * (32 * sizeof(uint2) + sizeof(u32)) +
+              surv_need(e, w, n, pos) * (sizeof(Surv) + 2 * sizeof(u32) + sizeof(RecDev)));
 }
 
 // A serving worker owns slot k: whenever its slot is free it takes every queued request
@@ -2769,7 +2783,10 @@ es_status es_set_schedule(es_engine *e, const es_schedule *s) {
   std::vector<std::unique_lock<std::mutex>> locks;
   for (Slot &sl : e->slots) locks.emplace_back(sl.mu);
   cudaSetDevice(e->device);
-  e->sched = *s;
+  {
+    std::lock_guard<std::mutex> lk(e->qmu);
+    e->sched = *s;
+  }
   for (Slot &sl : e->slots) drop_graph(&sl);
   return ES_OK;
 }
@@ -2915,7 +2932,12 @@ static es_status submit(es_engine *e, const es_window *w, size_t n, uint64_t *ti
   if (!r) return ES_ERR_NOMEM;
   r->w.assign(w, w + n);
   r->solo = solo;
-  r->mem = request_bytes(e, w, n);
+  es_schedule sched;
+  {
+    std::lock_guard<std::mutex> lk(e->qmu);            // es_set_schedule writes it under qmu
+    sched = e->sched;
+  }
+  r->mem = request_bytes(e, sched, w, n);
   {
     std::lock_guard<std::mutex> lk(e->qmu);
     if (e->stopping) { delete r; return ES_ERR_ARG; }

@@ -126,3 +126,24 @@ def test_calls_that_grow_make_buffers_and_graphs_anew_at_doublings_only(cuda, mo
     assert calls > 200 and _captures(cuda) <= 7        # 64 to 4096 windows
     assert not cuda.bad()
     e.close()
+
+
+# a table that leaves half of the positions (room for them is 64 times 1/64 of them), and one that
+# leaves few; a request of several passes needs the buffers of one
+@pytest.mark.parametrize("rates, log2, budget, fits", [
+    ((0.5, 0.6), 36, 1 << 30, False),
+    ((0.5, 0.6), 30, 1 << 30, True),
+    ((6e-5, 0.017), 43, 3 << 30, True),
+    ((6e-5, 0.017), 43, 1 << 29, False),
+])
+def test_admission_charges_what_a_request_makes(cuda, monkeypatch, rates, log2, budget, fits):
+    e = cuda.engine(monkeypatch, rates=rates, wheel=120120, filters=TABLE, mem_budget=budget)
+    e.poll(e.submit([(LO, LO + 1000)]), 1, timeout_ms=60000)
+    had = cuda.bytes()
+    try:
+        e.poll(e.submit([(LO, LO + (1 << log2))]), 1, timeout_ms=60000)
+        assert fits and cuda.bytes() - had <= budget
+    except es_sieve.EsError as ex:
+        assert ex.status == es_sieve.ES_ERR_BUSY and not fits
+    assert not cuda.bad()
+    e.close()
