@@ -1083,31 +1083,48 @@ __global__ void __launch_bounds__(RUNG_THREADS, 1) k_rung(const TailParams T, in
   if (few && t == 0 && blockIdx.x % BOARD_BLOCKS_DIV == 0) warp_help_board(board, n, lane);
 }
 
-// The run's last kernel: the direct search, a thread per prime that no rung certified (none in
-// scans), then the run's counters, the windows' counters and the records written to pinned host
-// memory (four copies as nodes of the graph cost 8 us, and a fifth with a second wait brought the
-// records past the first 4096). Without direct primes every block writes its share at once; else the
-// last block to finish them writes all.
-__global__ void __launch_bounds__(256) k_direct(const TailParams T) {
-  __shared__ bool s_last;
+// The direct search of one prime that no rung certified.
+__device__ __forceinline__ void direct_one(const TailParams &T, u64 i) {
+  const Surv s = T.surv[T.direct[i]];
+  u64 a, c, d, k;
+  if (solve_direct(s.p, a, c, d, k, T.tdp, T.tde, T.status)) {
+    if (!check_solved_cert(s.p, a, c, d, k)) { atomicOr(T.status, ST_CERT_BAD); return; }
+    RecDev rec{ES_REC_SOLVED, s.win, s.lane, 0, s.J, s.p, a, c, d, k};
+    put_record(T, rec);
+    atomicAdd(&T.cnt[s.win].direct, 1ull);
+  } else {
+    RecDev rec{ES_REC_SURVIVOR, s.win, s.lane, 0, s.J, s.p, 0, 0, 0, 0};
+    put_record(T, rec);
+    atomicAdd(&T.cnt[s.win].unsolved, 1ull);
+  }
+}
+
+// The direct search of an engine without rungs (ES_FLAG_NO_RUNG), where every prime takes it: a prime a warp
+// while there are warps, then as many lanes of each as it takes. Bound by the latency of one thread's trial
+// divisions and rho, and lanes of a warp that part company wait for each other: with 32 to a warp the 2^34
+// windows of the 120120 table at 1e9, 1e12 and 1e15 take 13.3, 26.6 and 26.6 ms, with 4 12.0, 24.3 and 23.6,
+// with one 10.5, 21.5 and 20.8. A kernel of its own because the search in k_direct's blocks of 256 compiles
+// to a slower chain: 4 primes at 1e12 11.7 ms there, 8.9 here.
+__global__ void k_search(const TailParams T) {
   stamp(T.ctr, 5);
   const u64 n = min((u64)*T.direct_count, T.cap);
+  const u32 share = (u32)min((n + gridDim.x - 1) / gridDim.x, 32ull);
+  if (threadIdx.x >= share) return;
+  for (u64 i = (u64)blockIdx.x * share + threadIdx.x; i < n; i += (u64)gridDim.x * share) direct_one(T, i);
+}
+
+// The run's last kernel: the direct search, a thread per prime that no rung certified (none in
+// scans; `searched`: k_search has done it), then the run's counters, the windows' counters and the records
+// written to pinned host memory (four copies as nodes of the graph cost 8 us, and a fifth with a second
+// wait brought the records past the first 4096). Without direct primes every block writes its share at
+// once; else the last block to finish them writes all.
+__global__ void __launch_bounds__(256) k_direct(const TailParams T, int searched) {
+  __shared__ bool s_last;
+  if (!searched) stamp(T.ctr, 5);
+  const u64 n = searched ? 0 : min((u64)*T.direct_count, T.cap);
   u32 block = blockIdx.x, blocks = gridDim.x;
   if (n) {
-    for (u64 i = (u64)threadIdx.x * gridDim.x + blockIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) {
-      const Surv s = T.surv[T.direct[i]];
-      u64 a, c, d, k;
-      if (solve_direct(s.p, a, c, d, k, T.tdp, T.tde, T.status)) {
-        if (!check_solved_cert(s.p, a, c, d, k)) { atomicOr(T.status, ST_CERT_BAD); continue; }
-        RecDev rec{ES_REC_SOLVED, s.win, s.lane, 0, s.J, s.p, a, c, d, k};
-        put_record(T, rec);
-        atomicAdd(&T.cnt[s.win].direct, 1ull);
-      } else {
-        RecDev rec{ES_REC_SURVIVOR, s.win, s.lane, 0, s.J, s.p, 0, 0, 0, 0};
-        put_record(T, rec);
-        atomicAdd(&T.cnt[s.win].unsolved, 1ull);
-      }
-    }
+    for (u64 i = (u64)threadIdx.x * gridDim.x + blockIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) direct_one(T, i);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) s_last = atomicAdd(T.ctr + 5, 1ull) == gridDim.x - 1;
@@ -1673,17 +1690,23 @@ static es_status enqueue_front(es_engine *e, Slot *sl, bool persistent, WinCount
 }
 
 // The funnel's tail on the slot's stream: stage D, stage E, the results written to pinned memory
-// (the windows' counters at out_cnt).
-static es_status enqueue_tail(es_engine *e, Slot *sl, WinCount *cnt, WinCount *out_cnt, bool capture) {
+// (the windows' counters at out_cnt). Adds its kernel launches to `launches`.
+static es_status enqueue_tail(es_engine *e, Slot *sl, WinCount *cnt, WinCount *out_cnt, bool capture, u64 &launches) {
   TailParams T = tail_params(e, sl);
   T.cnt = cnt;
   T.out.cnt = out_cnt;
   cudaStream_t st = sl->stream;
   const u32 teams = e->sm_count * std::min<u32>(e->sched.rung_blocks_per_sm, RUNG_TEAMS);
-  k_rung<<<(teams + RUNG_TEAMS - 1) / RUNG_TEAMS, RUNG_THREADS, sizeof(RungBlock), st>>>(T, (e->flags & ES_FLAG_NO_RUNG) ? 1 : 0);
+  const int no_rung = (e->flags & ES_FLAG_NO_RUNG) ? 1 : 0;
+  k_rung<<<(teams + RUNG_TEAMS - 1) / RUNG_TEAMS, RUNG_THREADS, sizeof(RungBlock), st>>>(T, no_rung);
   CU(cudaGetLastError());
-  k_direct<<<e->sm_count, 256, 0, st>>>(T);
+  if (no_rung) {
+    k_search<<<e->sm_count * 16, 32, 0, st>>>(T);
+    CU(cudaGetLastError());
+  }
+  k_direct<<<e->sm_count, 256, 0, st>>>(T, no_rung);
   CU(cudaGetLastError());
+  launches += 2 + no_rung;
   CU(capture ? cudaEventRecordWithFlags(sl->ev[4], st, cudaEventRecordExternal) : cudaEventRecord(sl->ev[4], st));
   return ES_OK;
 }
@@ -1715,13 +1738,13 @@ static es_status capture_graph(es_engine *e, Slot *sl) {
     ~Undo() { if (sl) drop_graph(sl); }
   } undo{sl};
   const bool one = sl == &e->slots[0];
-  u64 launches = 2;                                // the tail's two kernels
+  u64 launches = 0;
   for (int part = 0; part < (one ? 1 : 2); ++part) {
     CU(cudaStreamBeginCapture(sl->stream, cudaStreamCaptureModeThreadLocal));
     es_status s = ES_OK;
     if (part == 0) s = enqueue_front(e, sl, true, sl->d_cnt, true, !e->sched.long_split, 0, true, launches);
     if (s == ES_OK && one) s = capture_front_end(e, sl);
-    if (s == ES_OK && (one || part == 1)) s = enqueue_tail(e, sl, sl->d_cnt, sl->h_cnt, true);
+    if (s == ES_OK && (one || part == 1)) s = enqueue_tail(e, sl, sl->d_cnt, sl->h_cnt, true, launches);
     cudaGraph_t g = nullptr;
     const cudaError_t end = cudaStreamEndCapture(sl->stream, &g);
     if (end != cudaSuccess) cudaGetLastError();
@@ -1944,10 +1967,9 @@ static es_status run_device_windows(es_engine *e, Slot *sl, const es_window *w, 
         }
         s = enqueue_front(e, sl, false, sl->d_cnt + i, h.nshort != 0, items != 0, items, false, launches);
         if (s) return s;
-        s = enqueue_tail(e, sl, sl->d_cnt + i, sl->h_cnt + i, false);
+        s = enqueue_tail(e, sl, sl->d_cnt + i, sl->h_cnt + i, false, launches);
         if (s) return s;
         CU(cudaStreamSynchronize(sl->stream));
-        launches += 2;
         nrec = 0;
         s = collect();
         if (s) return s;

@@ -101,7 +101,7 @@ void run(const Launch &L) {
     }
     WANT(P.cand, (size_t)P.chunk_cap * 32 * sizeof(uint2)); WANT(P.chunk, (size_t)P.chunk_cap * sizeof(u32));
     WANT(P.surv, P.surv_cap * sizeof(Surv));
-  } else if (L.name == "k_mr" || L.name == "k_rung" || L.name == "k_direct") {
+  } else if (L.name == "k_mr" || L.name == "k_rung" || L.name == "k_search" || L.name == "k_direct") {
     const TailParams &T = *reinterpret_cast<const TailParams *>(L.arg.data());
     WANT(T.surv, T.cap * sizeof(Surv)); WANT(T.primes, T.cap * sizeof(u32)); WANT(T.direct, T.cap * sizeof(u32));
     WANT(T.recs, T.cap * sizeof(RecDev)); WANT(T.out.recs, T.cap * sizeof(RecDev)); WANT(T.out.ctr, 8 * CTR_OUT);
@@ -278,7 +278,7 @@ cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 grid, dim3 block, void **arg
   Launch l{names[(const void *)k], {}, streams[s]};
   note("launch " + l.name + " " + std::to_string(grid.x) + " " + std::to_string(block.x));
   const bool rows = l.name == "k_rows" || l.name == "k_mark_short" || l.name == "k_sift";
-  const bool tail = l.name == "k_mr" || l.name == "k_rung" || l.name == "k_direct";
+  const bool tail = l.name == "k_mr" || l.name == "k_rung" || l.name == "k_search" || l.name == "k_direct";
   if (rows || tail) {
     const unsigned char *a = (const unsigned char *)args[0];
     l.arg.assign(a, a + (rows ? sizeof(RowParams) : sizeof(TailParams)));
