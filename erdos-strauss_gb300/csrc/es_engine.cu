@@ -736,9 +736,12 @@ __device__ __forceinline__ bool take_square(const RowParams &P, const Cand &x) {
 
 // The candidates against the other strides. Up to two per warp of the grid: a warp each. Up to
 // SIFT_FAR chunks: a thread each, reading the lanes' tables (60 MB) from L2, for THREAD_STRIDES[0]
-// strides, then the whole warp for the quarter that is left. Beyond: the CTAs take SIFT_LANES lanes
-// at a time, copy their tables to shared memory, and pick those lanes' candidates out of their
-// group's chunks; a warp walks THREAD_STRIDES[0] strides when it has gathered 32, gathers what is
+// strides, then the whole warp for the quarter that is left. Beyond: the CTAs take parts of SIFT_LANES
+// lanes, copy their tables to shared memory, and pick those lanes' candidates out of their
+// group's chunks; where there are fewer parts than CTAs (the 120120 wheel's 220 lanes make 28), each is
+// taken by several, every nslices'th 32 chunks each: marking of 2^34 and 2^40 windows with that wheel's
+// table 322 us and 15.8 ms with a CTA a part, 120 us and 4.0 ms so (5.3 ms where a slice was a run of chunks,
+// which lie by group). In a part a warp walks THREAD_STRIDES[0] strides when it has gathered 32, gathers what is
 // left in a second buffer, walks THREAD_STRIDES[1] more when that holds 32, and takes the few that
 // are left together. The lines: reading tables from L2 costs a sector per test, so beyond a few
 // candidates a thread their traffic is the bound (one kernel without the shared-memory pass took 0.65
@@ -795,7 +798,9 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) k_sift(const RowParams P) {
   const u32 n2 = min(P.n2, P.nm_cov);
   const u32 nwords = P.n2 < P.nm_all ? P.mdesc[P.n1p - P.n1 + P.n2].w & ~3u : P.lane_words;
   const u32 m1 = min(P.n1 + THREAD_STRIDES[0], n2), m2 = min(m1 + THREAD_STRIDES[1], n2);
-  for (u32 l0 = blockIdx.x * SIFT_LANES; l0 < P.L; l0 += gridDim.x * SIFT_LANES) {
+  const u32 nparts = (P.L + SIFT_LANES - 1) / SIFT_LANES, nslices = max(1u, gridDim.x / nparts);
+  for (u32 item = blockIdx.x; item < nparts * nslices; item += gridDim.x) {
+    const u32 l0 = item % nparts * SIFT_LANES, slice = item / nparts;
     __syncthreads();                                   // the barrier's init, the previous lanes' reads
     if (threadIdx.x == 0) {
       const u32 nl = min(SIFT_LANES, P.L - l0);
@@ -835,7 +840,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) k_sift(const RowParams P) {
       __syncwarp();
       if (nbuf2 >= 32) drain2(32);
     };
-    for (u32 c0 = warp * 32; c0 < nchunks; c0 += ROW_THREADS) {
+    for (u32 c0 = (warp * nslices + slice) * 32; c0 < nchunks; c0 += ROW_THREADS * nslices) {
       const u32 h = c0 + lane < nchunks ? __ldg(P.chunk + c0 + lane) : ~0u;
       unsigned mine = __ballot_sync(FULL, h >> 8 == g);
       auto entry = [&](int k) {                        // of chunk c0 + k, no lane's past its end
