@@ -2820,9 +2820,9 @@ es_status es_set_schedule(es_engine *e, const es_schedule *s) {
 
 es_status es_autotune(es_engine *e, const es_window *w, size_t n, int repeats, es_schedule *chosen) {
   if (!e || !w || n == 0 || repeats < 1 || repeats > 1000) return ES_ERR_ARG;
-  static const uint32_t SHORT[] = {SEG_SMALL / 4, SEG_SMALL / 2, SEG_SMALL};
-  static const uint32_t RUNG[] = {4, 6, 8};
-  static const uint32_t SPLIT[] = {1, 0};
+  // {long_split, short_max}: the schedules that launch different work. Stage D's grid is full from four teams an
+  // SM on, and with long_split = 1 every window is marked by rows.
+  static const uint32_t CAND[][2] = {{1, SEG_SMALL}, {0, SEG_SMALL / 4}, {0, SEG_SMALL / 2}, {0, SEG_SMALL}};
   const es_schedule before = e->sched;
   std::vector<es_counters> base(n), cur(n);
   es_records rbase{nullptr, 0};
@@ -2830,38 +2830,34 @@ es_status es_autotune(es_engine *e, const es_window *w, size_t n, int repeats, e
   double best_ms = 1e300;
   bool first = true;
   es_status st = ES_OK;
-  for (uint32_t sm : SHORT) {
-    for (size_t cand = 0; cand < 6; ++cand) {
-      const uint32_t rb = RUNG[cand % 3], split = SPLIT[cand / 3];
-      es_schedule c = before;
-      c.short_max = sm;
-      c.rung_blocks_per_sm = rb;
-      c.long_split = split;
-      if ((st = es_set_schedule(e, &c)) != ES_OK) break;
-      double ms = 0;                               // mean device time of the timed runs
-      for (int r = 0; r <= repeats && st == ES_OK; ++r) {
-        es_records rc{nullptr, 0};
-        st = es_run_batch(e, w, n, ES_SCHED_PERSISTENT, cur.data(), &rc);
-        if (st != ES_OK) break;
-        if (first) {                               // the first run defines the results
-          base = cur;
-          rbase = rc;
-          first = false;
-          continue;
-        }
-        const bool same = memcmp(cur.data(), base.data(), n * sizeof(es_counters)) == 0 && rc.n == rbase.n &&
-                          (rc.n == 0 || memcmp(rc.recs, rbase.recs, rc.n * sizeof(es_record)) == 0);
-        es_free_records(&rc);
-        if (!same) st = fail(e, ES_ERR_DEVICE_STATUS, "autotune: a schedule changed a result");
-        // run 0 warms up (graph capture). The mean, not the best, of the timed runs: stage D's
-        // time varies from run to run with which walk splits the hardest cofactor first, and
-        // the fastest of a few runs rewards a lucky tail rather than a better schedule.
-        if (r > 0) ms += e->slots[0].timing.total_ms / repeats;
-      }
+  for (const auto &cand : CAND) {
+    es_schedule c = before;
+    c.long_split = cand[0];
+    c.short_max = cand[1];
+    c.rung_blocks_per_sm = RUNG_TEAMS;
+    if ((st = es_set_schedule(e, &c)) != ES_OK) break;
+    double ms = 0;                               // mean device time of the timed runs
+    for (int r = 0; r <= repeats && st == ES_OK; ++r) {
+      es_records rc{nullptr, 0};
+      st = es_run_batch(e, w, n, ES_SCHED_PERSISTENT, cur.data(), &rc);
       if (st != ES_OK) break;
-      if (ms < best_ms) { best_ms = ms; best = c; }
+      if (first) {                               // the first run defines the results
+        base = cur;
+        rbase = rc;
+        first = false;
+        continue;
+      }
+      const bool same = memcmp(cur.data(), base.data(), n * sizeof(es_counters)) == 0 && rc.n == rbase.n &&
+                        (rc.n == 0 || memcmp(rc.recs, rbase.recs, rc.n * sizeof(es_record)) == 0);
+      es_free_records(&rc);
+      if (!same) st = fail(e, ES_ERR_DEVICE_STATUS, "autotune: a schedule changed a result");
+      // run 0 warms up (graph capture). The mean, not the best, of the timed runs: stage D's
+      // time varies from run to run with which walk splits the hardest cofactor first, and
+      // the fastest of a few runs rewards a lucky tail rather than a better schedule.
+      if (r > 0) ms += e->slots[0].timing.total_ms / repeats;
     }
     if (st != ES_OK) break;
+    if (ms < best_ms) { best_ms = ms; best = c; }
   }
   es_free_records(&rbase);
   if (st != ES_OK) { es_set_schedule(e, &before); return st; }

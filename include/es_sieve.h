@@ -207,7 +207,8 @@ typedef struct {
                                     positions (1..es_info_t.short_max_limit, 128 in this build) are
                                     marked by rows; default the limit */
   uint32_t rung_blocks_per_sm;   /* stage-D teams of four warps per SM (1..16, the
-                                    SM holds four); default 6 */
+                                    SM holds four, and more are
+                                    the same); default 6 */
   uint32_t long_split;           /* 1 (default): every window is marked by rows, long ones in
                                     passes; 0: longer windows go to the segment marking */
   uint32_t reserved[5];          /* zero */
@@ -216,10 +217,9 @@ typedef struct {
 es_status es_get_schedule(const es_engine *engine, es_schedule *out);
 /* ES_ERR_ARG for a value out of range; captured batch graphs are rebuilt on the next run. */
 es_status es_set_schedule(es_engine *engine, const es_schedule *s);
-/* Autotuner: runs the windows (persistent schedule) under each candidate schedule -- short_max
- * in {limit/4, limit/2, limit} x rung_blocks_per_sm in {4, 6, 8} x long_split in {1, 0} -- once to warm up
- * and `repeats` times
- * timed, keeps the mean device time of each, checks that every candidate gave identical
+/* Autotuner: runs the windows (persistent schedule) under each candidate schedule -- long_split = 1, and
+ * long_split = 0 with short_max in {limit/4, limit/2, limit}, at four stage-D teams an SM; others
+ * launch the same work as one of these -- once to warm up and `repeats` times timed, keeps the mean device time of each, checks that every candidate gave identical
  * counters and records (ES_ERR_DEVICE_STATUS if not), and sets the fastest. `chosen` may be
  * null. */
 es_status es_autotune(es_engine *engine, const es_window *w, size_t n, int repeats, es_schedule *chosen);

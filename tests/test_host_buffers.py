@@ -147,3 +147,15 @@ def test_admission_charges_what_a_request_makes(cuda, monkeypatch, rates, log2, 
         assert ex.status == es_sieve.ES_ERR_BUSY and not fits
     assert not cuda.bad()
     e.close()
+
+
+def test_autotune_times_each_launch_once(cuda, eng):
+    """A stage-D grid is at most four teams an SM and short_max matters without long_split only, so four
+    of the schedules differ; equal ones are not told apart by noise."""
+    eng.autotune([(LO, LO + (1 << 20))] * 3, repeats=2)
+    log = cuda.log()
+    assert sum(ln.startswith("graph on 0") for ln in log) == 4 * 3
+    grids = {tuple(ln.split()[2:]) for ln in log if ln.startswith("launch k_rung")}
+    assert grids == {("152", "512")}
+    chosen = eng.schedule()
+    assert chosen["rung_blocks_per_sm"] == 4 and (not chosen["long_split"] or chosen["short_max"] == 128)
