@@ -48,8 +48,8 @@ METRIC = "verified integers/s at 1e19 (batched vs plain, 1 GB300)"
 # up; with windows split it marks by rows whatever short_max is, and k_rung is one block of four
 # teams an SM from rung_blocks_per_sm = 4 on, so one capture stands for the schedules that launch the
 # same kernels. A schedule with no capture here gets no issue figure rather than another schedule's.
-_MARK = {"inst": 33068169 + 84492389, "dram": 4929024 + 66668032 + 320256}
-_RUNG = {"inst": 75059324, "dram": 781824}
+_MARK = {"inst": 33069288 + 85197018, "dram": 4929024 + 66672128 + 315648}
+_RUNG = {"inst": 73976260, "dram": 782592 + 256}
 MARK_SHORT_NCU = {(32, 1): _MARK, (64, 1): _MARK, (128, 1): _MARK}      # (short_max, long_split) -> per launch
 RUNG_NCU = {4: _RUNG, 6: _RUNG, 8: _RUNG}                               # rung_blocks_per_sm -> per launch
 # Cover/filter marks per integer of the 2042040 wheel with the gpu filter table: 9.0951 marks per

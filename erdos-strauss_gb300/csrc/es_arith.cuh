@@ -151,8 +151,8 @@ __device__ __forceinline__ u64 to_mont(u64 a, const Mont &M) { return mmul(a % M
 // Exact keeps every residue in [0, n) for any odd n < 2^64. Lazy is for odd n < 2^62 and keeps
 // residues in [0, 2n), each standing for its class mod n: the product of two such values is
 // below 4n^2 < n 2^64, so (T + m n) / 2^64 is already below 2n and the reduction needs no
-// final comparison and subtraction (measured on GB300: 86 instead of 119 cycles for one
-// dependent Montgomery multiply). gcd(x, n) and x mod p for p | n do not depend on which
+// final comparison and subtraction (82 instead of 93 cycles for one dependent
+// Montgomery multiply on GB300). gcd(x, n) and x mod p for p | n do not depend on which
 // representative x is, so a search that only ever takes gcds with n, as rho and ECM do, finds
 // the same divisors either way; norm() gives the representative in [0, n) where a value must
 // be exact (a modular inverse).

@@ -30,7 +30,8 @@
 //                 Miller-Rabin, Brent's rho, ECM rounds (es_tail.cuh, es_ecm.cuh), the rung
 //                 DP, and the exact certificate check (es_check.cuh) before a record is
 //                 written
-//   k_direct      a thread per prime left over: the direct search, else SURVIVOR
+//   k_search      engines without rungs: the direct search of every prime, else SURVIVOR
+//   k_direct      the direct search of primes left over by rungs; the results to pinned memory
 // Records come back unordered; the host puts them in (window, lane, J) order, the
 // reference's lane-major order per window.
 #include "../../include/es_sieve.h"
@@ -888,7 +889,7 @@ __global__ void k_build_rows(const u16 *__restrict__ K0, u32 L, u32 ldk, u32 nf,
 // Adds to sum[0], 32 lanes a block, the share of a lane's positions that no stride of the tables kills, were
 // the strides independent, and to sum[1] that of the dense strides alone: what the buffers of survivors and
 // of candidates are sized by. A lane's own product and not the product of the strides' means, since lanes
-// differ: few of them hold most of what is left. A warp takes every RATE_WARPS'th stride: 0.24 ms of es_open,
+// differ: few of them hold most of what is left. A warp takes every RATE_WARPS'th stride: 0.20 ms of es_open,
 // latency of the reads (a thread for all of a lane's 1.4).
 constexpr u32 RATE_WARPS = 16;
 __global__ void k_lane_rate(const u32 *__restrict__ tdense, const u32 *__restrict__ tlane, const uint4 *__restrict__ mdesc,
@@ -2358,13 +2359,9 @@ static es_status build_tables(es_engine *e) {
     CU(cudaFuncSetAttribute(k_sift, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ROW_SMEM));
   }
   CU(cudaStreamSynchronize(e->slots[0].stream));
-  // occupancy of the marking kernel, for the persistent grid
-  // The attribute is per function and process-wide: set it to the largest size any engine
-  // can ask for (DMAX strides), never to this engine's own size, or a second engine with
-  // fewer strides would shrink it under the first.
   // Stage D's trial division streams its 78 KB prime table once per factorization: ask for
-  // the smallest shared-memory carveout that still holds the resident blocks' static shared
-  // memory, so that the rest of the SM's 256 KB stays L1 and the table stays in it.
+  // the smallest shared-memory carveout that still holds the resident blocks' shared memory,
+  // so that the rest of the SM's 256 KB stays L1 and the table stays in it.
   {
     int max_smem = 0;
     CU(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, e->device));
@@ -2376,6 +2373,9 @@ static es_status build_tables(es_engine *e) {
       CU(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
     }
   }
+  // k_mark's shared memory: the attribute is per function and process-wide, so it is the largest
+  // size any engine can ask for (DMAX strides), never this engine's own, or a second engine with
+  // fewer strides would shrink it under the first; its occupancy sizes the persistent grid.
   const size_t smem = mark_smem(e);
   const size_t smem_max = ((4 * DMAX + 15) & ~15u) + std::max<u32>(SEG_BIG, GROUP * SEG_SMALL) + 16;
   CU(cudaFuncSetAttribute(k_mark<MARK_BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));

@@ -541,7 +541,7 @@ __device__ inline bool warp_factor_cofactor(u64 v0, WarpFac &F, u32 *status, u32
 constexpr int TD_RUNGS = 64;            // rung indices 0 .. 63 (r = r0 + 4k <= RCAP)
 constexpr int TD_SMALL = 17;            // odd primes below TD_RUNGS: 3 .. 61, tdp[0 .. 16]
 constexpr int TD_LIST_CAP = 15;         // with TD_SMALL, at most 32: one prime per lane
-struct TdSieve {                        // shared memory, one per block
+struct TdSieve {                        // shared memory: a warp's in the bulk, then a team's
   u16 idx[TD_RUNGS][TD_LIST_CAP];       // indices into tdp of the primes above 61 dividing A_k
   u32 n[TD_RUNGS];                      // their count (above TD_LIST_CAP: the list is incomplete)
   u32 small[TD_RUNGS];                  // bit i: tdp[i] divides A_k, i < TD_SMALL
@@ -970,7 +970,7 @@ __device__ inline bool rung_divisor(u64 p, u64 A, U128 q, u32 r, u32 target, War
 }
 
 // The rung walk of one prime by one warp, rung after rung (solve_rung3,
-// sieve/rung_scan3.cpp:578-603, in its own order): the throughput form of block_solve_rung
+// sieve/rung_scan3.cpp:578-603, in its own order): the throughput form of team_solve_rung
 // below, for while there are more primes than warps. Returns true in every lane when a rung
 // certifies p, with the result in *out (written by lane 0). use_ecm = false keeps the hard
 // cofactors on rho: with every warp of the GPU busy, a round of curves costs more issue slots
