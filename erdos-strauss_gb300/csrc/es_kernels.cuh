@@ -112,7 +112,7 @@ constexpr u32 ROW_CUT = 1u << 31, ROW_NONE = ~0u;
 // Run counters: [0] k_mark's queue [1] survivors [2] primes [3] direct [4] records [5] k_direct's blocks
 // done [6] rung queue (teams) [7] rung primes done [8] board sessions [9] rung queue (warps)
 // [10] candidate chunks, [STAMP0 + i] the device clock in ns at the start of k_rows, k_mark_short,
-// k_mark, k_mr, k_rung and k_direct and at its end; then stage D's board.
+// k_mark, k_mr, k_rung and k_search or k_direct and at the latter's end; then stage D's board.
 constexpr u32 STAMP0 = 16, CTR_OUT = 24;
 __device__ __forceinline__ void stamp(unsigned long long *ctr, u32 i) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
